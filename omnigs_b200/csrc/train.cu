@@ -8,9 +8,10 @@
 // vertical 11-tap pass in shared memory.  The gradient follows from
 //   dSSIM/dimg(p) = 1/N [ (w * A)(p) + 2 img(p) (w * B)(p) + gt(p) (w * Cm)(p) ]
 // with per-pixel A = dS/dmu1, B = dS/d(w * img^2), Cm = dS/d(w * img gt) (the window is
-// symmetric, so the adjoint convolution is the same convolution).  Kernel 1 computes the local
-// statistics, S and A, B, Cm (written to a workspace) and per-block FP64 sums; kernel 2
-// convolves A, B, Cm back and writes dL/dimg; kernel 3 writes the three loss values.
+// symmetric, so the adjoint convolution is the same convolution).  One kernel walks the image down
+// column strips and does all of it in registers and two shared rows: it computes the local
+// statistics, S and A, B, Cm of a row, convolves them back ten rows behind its input and writes
+// dL/dimg, with per-block FP64 sums; a second kernel writes the three loss values.
 //
 // Adam (torch::optim::Adam as configured at src/gaussian_model.cpp:485-518: per-group learning
 // rates, betas (0.9, 0.999), eps 1e-15, no weight decay) of the raw parameters xyz, f_dc, f_rest,
@@ -31,25 +32,26 @@ namespace omnigs {
 namespace {
 
 constexpr int kWin = 11, kHalf = 5;
-constexpr int kLossTileW = 32, kLossTileH = 16;
-constexpr int kLossThreads = kLossTileW * kLossTileH / 2;  // each thread owns two output pixels
 constexpr double kC1 = 0.01 * 0.01, kC2 = 0.03 * 0.03;
 
 struct LossParams {
   const float* img;   // [C][H][W]
   const float* gt;
   float* dimg;        // [C][H][W] gradient; rows >= `rows` are set to 0
-  float* ws;          // [3][C][rows][W]: A, B, Cm
   double* sums;       // [2 * blocks]: per-block sum |img - gt|, sum S
-  float* loss;        // [3]: loss, l1, ssim
   int C, H, W, rows;
+  int chunk;          // output rows of a block
   float lambda;
   float w[kWin];
 };
 
-// Register segment of the sliding 11-tap windows: kSeg outputs from kSeg + 10 loads, so shared
-// memory is read ~1.8 times per output instead of 11 times.
-constexpr int kSeg = 8;
+// A block owns kLossCols output columns of `chunk` rows of one channel; a thread owns one column of
+// the kLossThreads statistics columns these need.
+constexpr int kLossThreads = 128;
+constexpr int kLossCols = kLossThreads - 2 * kHalf;
+constexpr int kLossInCols = kLossThreads + 2 * kHalf;
+constexpr int kLossMinChunk = 16;
+constexpr int kLossBlocksPerSm = 3;  // (168 registers; four measured 171 us against 137)
 
 // Block sums of (a, b) into partials[2 * block] (no contended atomics; loss_finalize adds them).
 __device__ __forceinline__ void block_sum2(double a, double b, double* partials) {
@@ -77,177 +79,163 @@ __device__ __forceinline__ void block_sum2(double a, double b, double* partials)
   }
 }
 
-// Separable 11-tap convolution with zero padding of a [rows][W] plane region, by column strips: a
-// block walks down kStripChunks chunks of 16 output rows of a 32-column strip, each pass sliding
-// the window along register segments, and keeps the horizontal pass's last 10 rows for the next
-// chunk, so each input row is loaded and filtered horizontally once per strip (a 16x32 tile with
-// its own 26-row window re-read 10 halo rows: 0.228 -> 0.213 ms per 2048x1024x3 loss, identical
-// results).
-// `src(ok, y, x, v)` gives the NQ inputs at (y, x) (zeros when !ok, i.e. outside [0, rows) x
-// [0, W)), `out(y, x, v)` receives the NQ convolved values of an output pixel; `s_in` holds up to
-// 16 input rows (later the vertical results), `s_tmp` the horizontal results of input rows
-// y0 - 5 .. y0 + 20 of the current chunk.
-constexpr int kStripChunks = 4;
-constexpr int kStripRows = kStripChunks * kLossTileH;
-
-template <int NQ, class Src, class Out>
-__device__ __forceinline__ void conv_strip(int x0, int ystart, int rows, int W, const float* w,
-                                           float (*s_in)[kLossTileH][kLossTileW + 2 * kHalf],
-                                           float (*s_tmp)[kLossTileH + 2 * kHalf][kLossTileW], Src src, Out out) {
-  constexpr int IW = kLossTileW + 2 * kHalf;
-  constexpr int kRowsPerPass = kLossThreads / kLossTileW;
-  constexpr int kHSegs = kLossTileW / kSeg, kVSegs = kLossTileH / kSeg;
-  const int lx = threadIdx.x % kLossTileW, ly = threadIdx.x / kLossTileW;
-  // input rows [ya, ya + n) (with the x halo) into s_in rows [0, n), their horizontal pass into
-  // s_tmp rows [dst, dst + n)
-  auto load_and_filter = [&](int ya, int n, int dst) {
-    for (int ty = ly; ty < n; ty += kRowsPerPass) {
-      for (int tx = lx; tx < IW; tx += kLossTileW) {
-        const int y = ya + ty, x = x0 + tx - kHalf;
-        const bool ok = y >= 0 && y < rows && x >= 0 && x < W;
-        float v[NQ];
-        src(ok, y, x, v);
+// acc[j] holds the window sum of the row that is complete in j + 1 more rows; a row's value v enters
+// all eleven windows that contain it, and the one that it completes comes back.
+__device__ __forceinline__ float window_step(float (&acc)[kWin - 1], const float* w, float v) {
+  const float done = fmaf(w[kWin - 1], v, acc[0]);
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) s_in[q][ty][tx] = v[q];
-      }
-    }
-    __syncthreads();
-    for (int t = threadIdx.x; t < NQ * n * kHSegs; t += kLossThreads) {
-      const int q = t / (n * kHSegs), rem = t - q * (n * kHSegs);
-      const int ty = rem / kHSegs, xs = (rem - ty * kHSegs) * kSeg;
-      float r[kSeg + kWin - 1];
+  for (int j = 0; j < kWin - 2; ++j) acc[j] = fmaf(w[kWin - 2 - j], v, acc[j + 1]);
+  acc[kWin - 2] = w[0] * v;
+  return done;
+}
+// The same for two quantities in packed arithmetic (each lane rounded as the scalar form).
+__device__ __forceinline__ float2 window_step(float2 (&acc)[kWin - 1], const float2* w2, float2 v) {
+  const float2 done = __ffma2_rn(w2[kWin - 1], v, acc[0]);
 #pragma unroll
-      for (int k = 0; k < kSeg + kWin - 1; ++k) r[k] = s_in[q][ty][xs + k];
-#pragma unroll
-      for (int j = 0; j < kSeg; ++j) {
-        float acc = 0.f;
-#pragma unroll
-        for (int k = 0; k < kWin; ++k) acc = fmaf(w[k], r[j + k], acc);
-        s_tmp[q][dst + ty][xs + j] = acc;
-      }
-    }
-    __syncthreads();
-  };
-
-  load_and_filter(ystart - kHalf, 2 * kHalf, 0);  // rows ystart - 5 .. ystart + 4
-  for (int ch = 0; ch < kStripChunks; ++ch) {
-    const int y0 = ystart + ch * kLossTileH;
-    if (y0 >= rows) break;  // block-uniform
-    load_and_filter(y0 + kHalf, kLossTileH, 2 * kHalf);  // rows y0 + 5 .. y0 + 20
-    // vertical pass of the chunk's 16 output rows into s_in
-    for (int t = threadIdx.x; t < NQ * kLossTileW * kVSegs; t += kLossThreads) {
-      const int q = t / (kLossTileW * kVSegs), rem = t - q * (kLossTileW * kVSegs);
-      const int ys = (rem / kLossTileW) * kSeg, tx = rem % kLossTileW;
-      float r[kSeg + kWin - 1];
-#pragma unroll
-      for (int k = 0; k < kSeg + kWin - 1; ++k) r[k] = s_tmp[q][ys + k][tx];
-#pragma unroll
-      for (int j = 0; j < kSeg; ++j) {
-        float acc = 0.f;
-#pragma unroll
-        for (int k = 0; k < kWin; ++k) acc = fmaf(w[k], r[j + k], acc);
-        s_in[q][ys + j][tx] = acc;
-      }
-    }
-    __syncthreads();
-    // outputs of the chunk; meanwhile the horizontal rows the next chunk shares move to the front
-    for (int ty = ly; ty < kLossTileH; ty += kRowsPerPass) {
-      float v[NQ];
-#pragma unroll
-      for (int q = 0; q < NQ; ++q) v[q] = s_in[q][ty][lx];
-      const int y = y0 + ty, x = x0 + lx;
-      if (y < rows && x < W) out(y, x, v);
-    }
-    for (int t = threadIdx.x; t < NQ * 2 * kHalf * kLossTileW; t += kLossThreads) {
-      const int q = t / (2 * kHalf * kLossTileW), rem = t - q * (2 * kHalf * kLossTileW);
-      const int r = rem / kLossTileW, x = rem - r * kLossTileW;
-      s_tmp[q][r][x] = s_tmp[q][kLossTileH + r][x];
-    }
-    __syncthreads();
-  }
+  for (int j = 0; j < kWin - 2; ++j) acc[j] = __ffma2_rn(w2[kWin - 2 - j], v, acc[j + 1]);
+  acc[kWin - 2] = __fmul2_rn(w2[0], v);
+  return done;
 }
 
-// Kernel 1: local statistics of one 32-column strip of kStripRows rows of one channel (blockIdx.z).
-__global__ void __launch_bounds__(kLossThreads) ssim_stats_kernel(const __grid_constant__ LossParams p) {
-  __shared__ float s_in[5][kLossTileH][kLossTileW + 2 * kHalf];
-  __shared__ float s_tmp[5][kLossTileH + 2 * kHalf][kLossTileW];
-  const int c = blockIdx.z;
-  const int x0 = blockIdx.x * kLossTileW, ystart = blockIdx.y * kStripRows;
+// Loss and gradient in one walk down a strip.  Row y of the inputs is in shared memory; a thread
+// filters it horizontally at its column (img, gt and their three products), the vertical windows are
+// running sums in registers, and they complete the statistics of row y - 5.  Their A, B, Cm go through
+// a second shared row and a second set of windows, which a row later complete the gradient of row
+// y - 11.  Both shared rows are double buffered, so a row costs one barrier; the inputs are loaded three
+// rows ahead.  Every sum runs over its taps in the order of a direct 11-tap pass, rounded tap by tap.
+//
+// The pass is bound by instruction issue and the latency of its FMA chains (363 instructions a row and
+// warp, three warps a scheduler, 64 % issue active), not by memory: 75 MB at 2048x1024x3.  Measured
+// there on a B200, against two kernels through a 75 MB workspace, each with its horizontal and
+// vertical pass in shared memory: 213 -> 137 us (157 us with the pairs in scalar arithmetic, 140 us
+// with the two horizontal passes on either side of the barrier).  Strips recompute ten columns a side
+// and chunks ten rows at each end, so a chunk is as high as a grid of one wave allows
+// (omnigs_l1_dssim).
+__global__ void __launch_bounds__(kLossThreads, kLossBlocksPerSm) ssim_loss_kernel(const __grid_constant__ LossParams p) {
+  __shared__ float2 s_in[2][kLossInCols];          // (img, gt) of the current and next input row
+  __shared__ float2 s_ab[2][kLossInCols];          // (A, B) of a statistics row, from column xs - 5 of thread 0
+  __shared__ float s_c[2][kLossInCols];            // Cm
+  const int t = threadIdx.x;
+  const int x0 = blockIdx.x * kLossCols;           // first output column
+  const int xs = x0 - kHalf + t;                   // this thread's column
+  const int ya = blockIdx.y * p.chunk, yb = min(ya + p.chunk, p.rows);
   const size_t plane = (size_t)p.H * p.W;
-  const float* a = p.img + c * plane;
-  const float* b = p.gt + c * plane;
-  const size_t ws_plane = (size_t)p.rows * p.W;
-  float* A = p.ws + c * ws_plane;
-  float* B = p.ws + (p.C + c) * ws_plane;
-  float* Cm = p.ws + (2 * p.C + c) * ws_plane;
-  double l1 = 0.0, ssum = 0.0;
-  auto src = [&](bool ok, int y, int x, float v[5]) {
-    const float u = ok ? a[(size_t)y * p.W + x] : 0.f;
-    const float g = ok ? b[(size_t)y * p.W + x] : 0.f;
-    v[0] = u;
-    v[1] = g;
-    v[2] = u * u;
-    v[3] = g * g;
-    v[4] = u * g;
-  };
-  auto out = [&](int y, int x, const float m[5]) {
-    const float mu1 = m[0], mu2 = m[1];
-    const float mu1_sq = mu1 * mu1, mu2_sq = mu2 * mu2, mu1_mu2 = mu1 * mu2;
-    const float s1 = m[2] - mu1_sq, s2 = m[3] - mu2_sq, s12 = m[4] - mu1_mu2;
-    const float a1 = 2.f * mu1_mu2 + (float)kC1, a2 = 2.f * s12 + (float)kC2;
-    const float b1 = mu1_sq + mu2_sq + (float)kC1, b2 = s1 + s2 + (float)kC2;
-    const float inv = 1.f / (b1 * b2);
-    const float S = a1 * a2 * inv;
-    const size_t o = (size_t)y * p.W + x;
-    // dS/dmu1, dS/d(w * img^2), dS/d(w * img gt) with mu2 and the gt moments fixed
-    A[o] = 2.f * mu2 * (a2 - a1) * inv - 2.f * mu1 * S * (1.f / b1 - 1.f / b2);
-    B[o] = -S / b2;
-    Cm[o] = 2.f * a1 * inv;
-    ssum += (double)S;
-    l1 += (double)fabsf(a[o] - b[o]);
-  };
-  conv_strip<5>(x0, ystart, p.rows, p.W, p.w, s_in, s_tmp, src, out);
-  block_sum2(l1, ssum, p.sums);
-}
-
-// Kernel 2: dL/dimg of one 32-column strip of kStripRows rows of one channel.
-__global__ void __launch_bounds__(kLossThreads) ssim_grad_kernel(const __grid_constant__ LossParams p) {
-  __shared__ float s_in[3][kLossTileH][kLossTileW + 2 * kHalf];
-  __shared__ float s_tmp[3][kLossTileH + 2 * kHalf][kLossTileW];
-  const int c = blockIdx.z;
-  const int x0 = blockIdx.x * kLossTileW, ystart = blockIdx.y * kStripRows;
-  const size_t plane = (size_t)p.H * p.W;
-  const float* a = p.img + c * plane;
-  const float* b = p.gt + c * plane;
-  float* d = p.dimg + c * plane;
-  const size_t ws_plane = (size_t)p.rows * p.W;
-  const float* A = p.ws + c * ws_plane;
-  const float* B = p.ws + (p.C + c) * ws_plane;
-  const float* Cm = p.ws + (2 * p.C + c) * ws_plane;
+  const float* img = p.img + blockIdx.z * plane;
+  const float* gt = p.gt + blockIdx.z * plane;
+  float* d = p.dimg + blockIdx.z * plane;
+  const bool in_x = xs >= 0 && xs < p.W;
+  const bool owner = in_x && t >= kHalf && t < kLossThreads - kHalf;
   const float invN = (float)(1.0 / ((double)p.C * p.rows * p.W));
   const float k_l1 = (1.f - p.lambda) * invN, k_ssim = -p.lambda * invN;
-  auto src = [&](bool ok, int y, int x, float v[3]) {
-    const size_t o = (size_t)y * p.W + x;
-    v[0] = ok ? A[o] : 0.f;
-    v[1] = ok ? B[o] : 0.f;
-    v[2] = ok ? Cm[o] : 0.f;
-  };
-  auto out = [&](int y, int x, const float m[3]) {
-    const size_t o = (size_t)y * p.W + x;
-    const float u = a[o], g = b[o];
-    const float diff = u - g;
-    const float sgn = diff > 0.f ? 1.f : (diff < 0.f ? -1.f : 0.f);
-    const float dssim = m[0] + 2.f * u * m[1] + g * m[2];
-    d[o] = k_l1 * sgn + k_ssim * dssim;
-  };
-  conv_strip<3>(x0, ystart, p.rows, p.W, p.w, s_in, s_tmp, src, out);
-  // rows below `rows` are not part of the loss
-  if (blockIdx.y == gridDim.y - 1) {
-    for (int i = threadIdx.x; i < (p.H - p.rows) * kLossTileW; i += blockDim.x) {
-      const int y = p.rows + i / kLossTileW, x = x0 + i % kLossTileW;
-      if (x < p.W) d[(size_t)y * p.W + x] = 0.f;
+  const float* w = p.w;
+
+  // input columns x0 - 10 + c, c = t and (the first ten threads) c = kLossThreads + t; offsets within a
+  // plane fit 32 bits (at most 2^28 pixels)
+  const int xi = x0 - 2 * kHalf + t, xe = xi + kLossThreads;
+  const bool in_i = xi >= 0 && xi < p.W, in_e = t < 2 * kHalf && xe < p.W;
+  const bool extra = t < 2 * kHalf;
+  auto load = [&](bool ok, int y, int x) {
+    float2 v = make_float2(0.f, 0.f);
+    if (ok && (unsigned)y < (unsigned)p.rows) {
+      const int o = y * p.W + x;
+      v = make_float2(__ldg(img + o), __ldg(gt + o));
     }
+    return v;
+  };
+  float2 n1, n2, n3, e1 = {}, e2 = {}, e3 = {};
+  const int y_first = ya - 2 * kHalf;
+  s_in[y_first & 1][t] = load(in_i, y_first, xi);
+  n1 = load(in_i, y_first + 1, xi);
+  n2 = load(in_i, y_first + 2, xi);
+  if (extra) {
+    s_in[y_first & 1][kLossThreads + t] = load(in_e, y_first, xe);
+    e1 = load(in_e, y_first + 1, xe);
+    e2 = load(in_e, y_first + 2, xe);
   }
+  // (img, gt), (img^2, gt^2) and (A, B) run as packed pairs
+  float2 w2[kWin];
+#pragma unroll
+  for (int k = 0; k < kWin; ++k) w2[k] = make_float2(w[k < kHalf ? k : kWin - 1 - k], w[k < kHalf ? k : kWin - 1 - k]);
+  float2 acc_m[kWin - 1] = {}, acc_s[kWin - 1] = {}, acc_ab[kWin - 1] = {};
+  float acc_x[kWin - 1] = {}, acc_c[kWin - 1] = {};
+  double l1 = 0.0, ssum = 0.0;
+  for (int i = t; i < kLossInCols; i += kLossThreads)  // (the margins are read by threads that own nothing)
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      s_ab[q][i] = make_float2(0.f, 0.f);
+      s_c[q][i] = 0.f;
+    }
+  __syncthreads();
+
+  float2 uo = make_float2(0.f, 0.f), uo_next = uo;  // (img, gt) at the gradient's row and the next one's
+#pragma unroll 1
+  for (int y = y_first; y <= yb + 2 * kHalf; ++y) {
+    const int cur = y & 1;
+    n3 = load(in_i, y + 3, xi);
+    if (extra) e3 = load(in_e, y + 3, xe);
+    const int yo = y - 1 - 2 * kHalf;  // the gradient row that the previous statistics row completes
+    uo = uo_next;
+    if (yo + 1 >= ya) uo_next = load(owner, yo + 1, xs);
+    // the input row and the previous statistics row, filtered horizontally
+    float2 hm = make_float2(0.f, 0.f), hs = hm, hab = hm;
+    float hx = 0.f, hc = 0.f;
+    const float2* in = &s_in[cur][t];
+    const float2* ab = &s_ab[cur ^ 1][t];
+    const float* cm = &s_c[cur ^ 1][t];
+#pragma unroll
+    for (int k = 0; k < kWin; ++k) {
+      const float2 v = in[k];
+      hm = __ffma2_rn(w2[k], v, hm);
+      hs = __ffma2_rn(w2[k], __fmul2_rn(v, v), hs);
+      hx = fmaf(w[k], __fmul_rn(v.x, v.y), hx);
+      hab = __ffma2_rn(w2[k], ab[k], hab);
+      hc = fmaf(w[k], cm[k], hc);
+    }
+    const float2 mu = window_step(acc_m, w2, hm), m2 = window_step(acc_s, w2, hs);
+    const float mu1 = mu.x, mu2 = mu.y, m11 = m2.x, m22 = m2.y;
+    const float m12 = window_step(acc_x, w, hx);
+    const float2 cab = window_step(acc_ab, w2, hab);
+    const float ca = cab.x, cb = cab.y, cc = window_step(acc_c, w, hc);
+    if (owner && yo >= ya) {
+      const float u = uo.x, g = uo.y, diff = u - g;
+      const float sgn = diff > 0.f ? 1.f : (diff < 0.f ? -1.f : 0.f);
+      const float dssim = ca + 2.f * u * cb + g * cc;
+      d[yo * p.W + xs] = k_l1 * sgn + k_ssim * dssim;
+    }
+    // statistics of row y - 5 (0 outside the image, where there is no S, and before the first full window)
+    const int ys = y - kHalf;
+    float A = 0.f, B = 0.f, Cm = 0.f;
+    if (y >= ya && in_x && (unsigned)ys < (unsigned)p.rows) {
+      const float mu1_sq = mu1 * mu1, mu2_sq = mu2 * mu2, mu1_mu2 = mu1 * mu2;
+      const float s1 = m11 - mu1_sq, s2 = m22 - mu2_sq, s12 = m12 - mu1_mu2;
+      const float a1 = 2.f * mu1_mu2 + (float)kC1, a2 = 2.f * s12 + (float)kC2;
+      const float b1 = mu1_sq + mu2_sq + (float)kC1, b2 = s1 + s2 + (float)kC2;
+      const float inv = 1.f / (b1 * b2);
+      const float S = a1 * a2 * inv;
+      // dS/dmu1, dS/d(w * img^2), dS/d(w * img gt) with mu2 and the gt moments fixed
+      A = 2.f * mu2 * (a2 - a1) * inv - 2.f * mu1 * S * (1.f / b1 - 1.f / b2);
+      B = -S / b2;
+      Cm = 2.f * a1 * inv;
+      if (owner && ys >= ya && ys < yb) ssum += (double)S;
+    }
+    if (owner && y >= ya && y < yb) {
+      const float2 v = in[kHalf];
+      l1 += (double)fabsf(v.x - v.y);
+    }
+    s_ab[cur][kHalf + t] = make_float2(A, B);
+    s_c[cur][kHalf + t] = Cm;
+    s_in[cur ^ 1][t] = n1;
+    if (extra) s_in[cur ^ 1][kLossThreads + t] = e1;
+    __syncthreads();
+    n1 = n2;
+    n2 = n3;
+    e1 = e2;
+    e2 = e3;
+  }
+  // rows below `rows` are not part of the loss
+  if (blockIdx.y == gridDim.y - 1 && owner)
+    for (int y = p.rows; y < p.H; ++y) d[y * p.W + xs] = 0.f;
+  block_sum2(l1, ssum, p.sums);
 }
 
 __global__ void __launch_bounds__(1024) loss_finalize_kernel(const double* partials, int blocks, float* loss,
@@ -476,6 +464,14 @@ int validate_params(const OmnigsGaussianParams* prm, const OmnigsActivated* act)
   return OMNIGS_OK;
 }
 
+// Workspace part of the loss kernel's block sums: two doubles per block, whose strips are wider than 32
+// columns and whose chunks are at least kLossMinChunk rows.  (The rest of the workspace holds the
+// gradient when that goes over one of the images.)
+size_t loss_sums_bytes(int C, int H, int W) {
+  const size_t blocks = (size_t)C * ((W + 31) / 32) * ((H + kLossMinChunk - 1) / kLossMinChunk);
+  return align_up(sizeof(double) * 2 * blocks);
+}
+
 }  // namespace
 }  // namespace omnigs
 
@@ -485,8 +481,7 @@ extern "C" {
 
 size_t omnigs_l1_dssim_workspace_bytes(int C, int H, int W) {
   if (C <= 0 || H <= 0 || W <= 0) return 0;
-  const size_t blocks = (size_t)C * ((W + kLossTileW - 1) / kLossTileW) * ((H + kLossTileH - 1) / kLossTileH);
-  return align_up(sizeof(double) * 2 * blocks) + sizeof(float) * 3 * (size_t)C * H * W;
+  return loss_sums_bytes(C, H, W) + sizeof(float) * 3 * (size_t)C * H * W;
 }
 
 int omnigs_l1_dssim(const float* image, const float* gt, int C, int H, int W, int rows, float lambda_dssim,
@@ -504,12 +499,16 @@ int omnigs_l1_dssim(const float* image, const float* gt, int C, int H, int W, in
   LossParams p{};
   p.img = image;
   p.gt = gt;
-  p.dimg = dL_dimage;
-  const dim3 grid((W + kLossTileW - 1) / kLossTileW, (rows + kLossTileH - 1) / kLossTileH, C);
-  const size_t max_blocks = (size_t)C * ((W + kLossTileW - 1) / kLossTileW) * ((H + kLossTileH - 1) / kLossTileH);
   p.sums = static_cast<double*>(workspace);
-  p.ws = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + align_up(sizeof(double) * 2 * max_blocks));
-  p.loss = loss;
+  // The kernel reads pixels around those it has written: a gradient that goes over one of the images
+  // is written to the workspace first.
+  const size_t bytes = sizeof(float) * (size_t)C * H * W;
+  auto overlaps = [&](const float* in) {
+    const uintptr_t x = reinterpret_cast<uintptr_t>(in), y = reinterpret_cast<uintptr_t>(dL_dimage);
+    return x < y + bytes && y < x + bytes;
+  };
+  const bool in_place = overlaps(image) || overlaps(gt);
+  p.dimg = in_place ? reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + loss_sums_bytes(C, H, W)) : dL_dimage;
   p.C = C;
   p.H = H;
   p.W = W;
@@ -523,13 +522,22 @@ int omnigs_l1_dssim(const float* image, const float* gt, int C, int H, int W, in
     sum += p.w[k];
   }
   for (int k = 0; k < kWin; ++k) p.w[k] /= sum;
-  const dim3 strip_grid(grid.x, (rows + kStripRows - 1) / kStripRows, C);
-  const int blocks = (int)(strip_grid.x * strip_grid.y * strip_grid.z);
-  staged(OMNIGS_STAGE_OTHER, 3, s, [&] {
-    ssim_stats_kernel<<<strip_grid, kLossThreads, 0, s>>>(p);
-    ssim_grad_kernel<<<strip_grid, kLossThreads, 0, s>>>(p);
+  // One wave of blocks, each as many rows as that takes (a chunk recomputes 20 rows of statistics and
+  // input filtering), but at least kLossMinChunk.
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int strips = (W + kLossCols - 1) / kLossCols;
+  const int chunks = std::max(1, (int)((int64_t)sms * kLossBlocksPerSm / ((int64_t)strips * C)));
+  p.chunk = std::max(kLossMinChunk, (rows + chunks - 1) / chunks);
+  const dim3 grid(strips, (rows + p.chunk - 1) / p.chunk, C);
+  const int blocks = (int)(grid.x * grid.y * grid.z);
+  staged(OMNIGS_STAGE_OTHER, 2, s, [&] {
+    ssim_loss_kernel<<<grid, kLossThreads, 0, s>>>(p);
     loss_finalize_kernel<<<1, 1024, 0, s>>>(p.sums, blocks, loss, 1.0 / ((double)C * rows * W), lambda_dssim);
   });
+  if (in_place && cudaMemcpyAsync(dL_dimage, p.dimg, bytes, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
+    return check_launch("copy image gradient");
   return check_launch("l1 + d-ssim");
 }
 
