@@ -281,25 +281,47 @@ struct AdamParams {
   const float* dL_dscales;
   const float* dL_drotations;
   const OmnigsAdamHyper* hyper;  // device
+  bool aligned;                  // every array starts on 16 bytes
+  unsigned first_chunk[4];       // first block of the xyz, scaling, rotation and opacity chunks
 };
 
 struct AdamScalars {
   float step_size, bc2_sqrt, beta1, one_minus_beta1, beta2, one_minus_beta2, eps;
 };
 
-// The float coefficients torch::optim::Adam applies (its double options rounded once).
-__device__ __forceinline__ AdamScalars adam_scalars(const OmnigsAdamHyper& h, int group) {
-  const double t = (double)h.step;
+// x^n by repeated squaring: at most two multiplications per bit of n, in every block, where pow()'s
+// latency measured 30 us of a step over 1M Gaussians.  Its error, some 2 log2(n) units in the last place
+// of a double, is far below the rounding to float that follows.
+__device__ __forceinline__ double power_int(double x, long long n) {
+  double r = 1.0;
+  for (long long k = n < 0 ? -n : n; k > 0; k >>= 1, x *= x)
+    if (k & 1) r *= x;
+  return n < 0 ? 1.0 / r : r;
+}
+
+// The float coefficients torch::optim::Adam applies to a group (its double options rounded once);
+// bc: 1 - beta^t.
+__device__ __forceinline__ AdamScalars adam_scalars(const OmnigsAdamHyper& h, int group, const double bc[2]) {
   AdamScalars s;
-  const double bc1 = 1.0 - pow(h.beta1, t), bc2 = 1.0 - pow(h.beta2, t);
-  s.step_size = (float)(h.lr[group] / bc1);
-  s.bc2_sqrt = (float)sqrt(bc2);
+  s.step_size = (float)(h.lr[group] / bc[0]);
+  s.bc2_sqrt = (float)sqrt(bc[1]);
   s.beta1 = (float)h.beta1;
   s.one_minus_beta1 = (float)(1.0 - h.beta1);
   s.beta2 = (float)h.beta2;
   s.one_minus_beta2 = (float)(1.0 - h.beta2);
   s.eps = (float)h.eps;
   return s;
+}
+// Those of groups ga and gb, with the two powers evaluated by two threads of the block (all call it).
+__device__ __forceinline__ void adam_scalars2(const OmnigsAdamHyper& h, int ga, int gb, AdamScalars& a, AdamScalars& b) {
+  __shared__ AdamScalars s_sc[2];
+  __shared__ double s_bc[2];
+  if (threadIdx.x < 2) s_bc[threadIdx.x] = 1.0 - power_int(threadIdx.x ? h.beta2 : h.beta1, h.step);
+  __syncthreads();
+  if (threadIdx.x < 2) s_sc[threadIdx.x] = adam_scalars(h, threadIdx.x ? gb : ga, s_bc);
+  __syncthreads();
+  a = s_sc[0];
+  b = s_sc[1];
 }
 
 // One Adam update of one parameter value (torch::optim::Adam: exp_avg = b1 m + (1 - b1) g,
@@ -312,112 +334,247 @@ __device__ __forceinline__ float adam_update(float& p, float& m, float& v, float
   return p;
 }
 
-__global__ void __launch_bounds__(256) adam_gaussian_kernel(const __grid_constant__ AdamParams p) {
-  __shared__ AdamScalars s_sc[6];
-  const int P = p.prm.P, M = p.prm.M;
-  const int64_t rest_n = (int64_t)P * (M - 1) * 3;
-  if (threadIdx.x < 6) s_sc[threadIdx.x] = adam_scalars(*p.hyper, threadIdx.x);
-  __syncthreads();
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  // per-Gaussian groups: xyz, f_dc, opacity, scaling, rotation
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < P; i += stride) {
-    const int g = (int)i;
-    {  // xyz (group 0): the activated mean is the parameter itself
-      const AdamScalars& s = s_sc[0];
-      for (int k = 0; k < 3; ++k) {
-        const float v = adam_update(p.prm.xyz[3 * g + k], p.st.m_xyz[3 * g + k], p.st.v_xyz[3 * g + k],
-                                    p.dL_dmeans3D[3 * g + k], s);
-        if (p.act.means3D != p.prm.xyz) p.act.means3D[3 * g + k] = v;
-      }
-    }
-    {  // f_dc (group 1) = SH coefficient 0
-      const AdamScalars& s = s_sc[1];
-      for (int k = 0; k < 3; ++k) {
-        const float v = adam_update(p.prm.features_dc[3 * g + k], p.st.m_dc[3 * g + k], p.st.v_dc[3 * g + k],
-                                    p.dL_dsh[(size_t)g * M * 3 + k], s);
-        if (p.act.shs_bf16)
-          reinterpret_cast<__nv_bfloat16*>(p.act.shs)[(size_t)g * M * 3 + k] = __float2bfloat16_rn(v);
+// Every block updates a contiguous piece of one part of the model, so that all loads and stores are
+// coalesced and a block has few arrays open: the first blocks take the SH coefficients (f_dc, f_rest) of
+// kAdamTile Gaussians each, the others kAdamChunk elements of xyz, scaling, opacity or rotation.  A thread
+// loads its elements of p, m, v (16 bytes each when the piece is whole and the arrays are aligned) before
+// it updates any.
+//
+// The pass is bound by HBM: 1.88 GB per step over 1M Gaussians (16 SH coefficients).  Measured there on a
+// B200: a loop over the Gaussians with a thread each (accesses of stride 3 and 4 floats) and one over the
+// f_rest elements 596 us; blocks that take all groups of 64 Gaussians, with 30 arrays open at once,
+// 405-425 us whatever the tile, occupancy or work per thread; this split 318 us, 92 % of the copy rate.
+// A tile's f_rest is 1.9 vectors a thread: 32 Gaussians and 192 threads measured fastest (256 threads
+// 334 us, 128 threads 351 us; tiles of 64 with 256 or 384 threads 349 and 332 us).
+constexpr int kAdamTile = 32;
+constexpr int kAdamThreads = 192;
+constexpr int kAdamChunk = 2 * 4 * kAdamThreads;
+constexpr int kAdamBlocksPerSm = 5;
+
+template <int kW>
+struct AdamVec {
+  float v[kW];
+};
+template <int kW>
+__device__ __forceinline__ AdamVec<kW> adam_load(const float* p, int64_t i) {
+  AdamVec<kW> r;
+  if (kW == 4) {
+    const float4 f = reinterpret_cast<const float4*>(p)[i];
+    r.v[0] = f.x, r.v[1 % kW] = f.y, r.v[2 % kW] = f.z, r.v[3 % kW] = f.w;
+  } else {
+    r.v[0] = p[i];
+  }
+  return r;
+}
+template <int kW>
+__device__ __forceinline__ void adam_store(float* p, int64_t i, const AdamVec<kW>& r) {
+  if (kW == 4)
+    reinterpret_cast<float4*>(p)[i] = make_float4(r.v[0], r.v[1 % kW], r.v[2 % kW], r.v[3 % kW]);
+  else
+    p[i] = r.v[0];
+}
+
+// One vector of one parameter group: p, m, v loaded by the caller, gradients g.
+template <int kW>
+__device__ __forceinline__ void adam_vec(float* prm, float* m, float* v, int64_t i, AdamVec<kW>& pv, AdamVec<kW>& mv,
+                                         AdamVec<kW>& vv, const AdamVec<kW>& g, const AdamScalars& s) {
+#pragma unroll
+  for (int k = 0; k < kW; ++k) adam_update(pv.v[k], mv.v[k], vv.v[k], g.v[k], s);
+  adam_store<kW>(prm, i, pv);
+  adam_store<kW>(m, i, mv);
+  adam_store<kW>(v, i, vv);
+}
+
+// Elements [first, first + kAdamChunk) of a group of n elements, a vector of kW per thread and step:
+// grad(i) and put(i, new values) take the index of a vector.
+template <int kW, class Grad, class Put>
+__device__ __forceinline__ void adam_group(float* prm, float* m, float* v, int64_t first, int64_t n,
+                                           const AdamScalars& s, Grad grad, Put put) {
+  const int64_t end = min(n, first + kAdamChunk) / kW;
+  for (int64_t i = first / kW + threadIdx.x; i < end; i += kAdamThreads) {
+    AdamVec<kW> pv = adam_load<kW>(prm, i), mv = adam_load<kW>(m, i), vv = adam_load<kW>(v, i);
+    const AdamVec<kW> g = grad(i);
+    adam_vec<kW>(prm, m, v, i, pv, mv, vv, g, s);
+    put(i, pv);
+  }
+}
+
+// One chunk of xyz (group 0), scaling (4), opacity (3) or rotation (5).
+template <int kW>
+__device__ __forceinline__ void adam_chunk(const AdamParams& p, int group, int64_t first) {
+  const int64_t P = p.prm.P;
+  AdamScalars s, unused;
+  adam_scalars2(*p.hyper, group, group, s, unused);
+  if (group == 0) {  // the activated mean is the parameter itself
+    adam_group<kW>(p.prm.xyz, p.st.m_xyz, p.st.v_xyz, first, 3 * P, s,
+                   [&](int64_t i) { return adam_load<kW>(p.dL_dmeans3D, i); },
+                   [&](int64_t i, const AdamVec<kW>& x) { if (p.act.means3D != p.prm.xyz) adam_store<kW>(p.act.means3D, i, x); });
+  } else if (group == 4) {  // exp
+    adam_group<kW>(p.prm.scaling, p.st.m_scaling, p.st.v_scaling, first, 3 * P, s,
+                   [&](int64_t i) {
+                     AdamVec<kW> x = adam_load<kW>(p.dL_dscales, i);
+                     const AdamVec<kW> e = adam_load<kW>(p.act.scales, i);  // exp of the current parameter
+#pragma unroll
+                     for (int k = 0; k < kW; ++k) x.v[k] = x.v[k] * e.v[k];
+                     return x;
+                   },
+                   [&](int64_t i, AdamVec<kW> x) {
+#pragma unroll
+                     for (int k = 0; k < kW; ++k) x.v[k] = expf(x.v[k]);
+                     adam_store<kW>(p.act.scales, i, x);
+                   });
+  } else if (group == 3) {  // sigmoid
+    adam_group<kW>(p.prm.opacity, p.st.m_opacity, p.st.v_opacity, first, P, s,
+                   [&](int64_t i) {
+                     AdamVec<kW> x = adam_load<kW>(p.dL_dopacity, i);
+                     const AdamVec<kW> o = adam_load<kW>(p.act.opacities, i);  // sigmoid of the current parameter
+#pragma unroll
+                     for (int k = 0; k < kW; ++k) x.v[k] = x.v[k] * o.v[k] * (1.f - o.v[k]);
+                     return x;
+                   },
+                   [&](int64_t i, AdamVec<kW> x) {
+#pragma unroll
+                     for (int k = 0; k < kW; ++k) x.v[k] = 1.f / (1.f + expf(-x.v[k]));
+                     adam_store<kW>(p.act.opacities, i, x);
+                   });
+  } else {  // rotation: a quaternion per thread, L2 normalisation (F.normalize, eps 1e-12)
+    for (int64_t g = first / 4 + threadIdx.x; g < min(P, (first + kAdamChunk) / 4); g += kAdamThreads) {
+      auto quat = [&](const float* a) {
+        if (kW == 4) return adam_load<4>(a, g);
+        return AdamVec<4>{{a[4 * g], a[4 * g + 1], a[4 * g + 2], a[4 * g + 3]}};
+      };
+      auto put = [&](float* a, const AdamVec<4>& x) {
+        if (kW == 4)
+          adam_store<4>(a, g, x);
         else
-          static_cast<float*>(p.act.shs)[(size_t)g * M * 3 + k] = v;
-      }
-    }
-    {  // opacity (group 3), sigmoid
-      const AdamScalars& s = s_sc[3];
-      const float o = p.act.opacities[g];  // sigmoid of the current parameter (previous forward)
-      const float grad = p.dL_dopacity[g] * o * (1.f - o);
-      const float v = adam_update(p.prm.opacity[g], p.st.m_opacity[g], p.st.v_opacity[g], grad, s);
-      p.act.opacities[g] = 1.f / (1.f + expf(-v));
-    }
-    {  // scaling (group 4), exp
-      const AdamScalars& s = s_sc[4];
-      for (int k = 0; k < 3; ++k) {
-        const float e = p.act.scales[3 * g + k];  // exp of the current parameter
-        const float v = adam_update(p.prm.scaling[3 * g + k], p.st.m_scaling[3 * g + k], p.st.v_scaling[3 * g + k],
-                                    p.dL_dscales[3 * g + k] * e, s);
-        p.act.scales[3 * g + k] = expf(v);
-      }
-    }
-    {  // rotation (group 5), L2 normalisation (F.normalize, eps 1e-12)
-      const AdamScalars& s = s_sc[5];
-      float r[4], gr[4];
-      for (int k = 0; k < 4; ++k) {
-        r[k] = p.prm.rotation[4 * g + k];
-        gr[k] = p.dL_drotations[4 * g + k];
-      }
-      const float n = fmaxf(sqrtf(r[0] * r[0] + r[1] * r[1] + r[2] * r[2] + r[3] * r[3]), 1e-12f);
+          for (int k = 0; k < 4; ++k) a[4 * g + k] = x.v[k];
+      };
+      AdamVec<4> r = quat(p.prm.rotation), gr = quat(p.dL_drotations), m = quat(p.st.m_rotation), v = quat(p.st.v_rotation);
+      const float n = fmaxf(sqrtf(r.v[0] * r.v[0] + r.v[1] * r.v[1] + r.v[2] * r.v[2] + r.v[3] * r.v[3]), 1e-12f);
       const float inv = 1.f / n;
-      const float yg = (r[0] * gr[0] + r[1] * gr[1] + r[2] * gr[2] + r[3] * gr[3]) * inv;  // y . g
-      float nr[4];
-      for (int k = 0; k < 4; ++k) {
-        const float dr = (gr[k] - r[k] * inv * yg) * inv;
-        nr[k] = adam_update(p.prm.rotation[4 * g + k], p.st.m_rotation[4 * g + k], p.st.v_rotation[4 * g + k], dr, s);
-      }
-      const float n2 = fmaxf(sqrtf(nr[0] * nr[0] + nr[1] * nr[1] + nr[2] * nr[2] + nr[3] * nr[3]), 1e-12f);
-      for (int k = 0; k < 4; ++k) p.act.rotations[4 * g + k] = nr[k] / n2;
+      const float yg = (r.v[0] * gr.v[0] + r.v[1] * gr.v[1] + r.v[2] * gr.v[2] + r.v[3] * gr.v[3]) * inv;  // y . g
+#pragma unroll
+      for (int k = 0; k < 4; ++k) adam_update(r.v[k], m.v[k], v.v[k], (gr.v[k] - r.v[k] * inv * yg) * inv, s);
+      const float n2 = fmaxf(sqrtf(r.v[0] * r.v[0] + r.v[1] * r.v[1] + r.v[2] * r.v[2] + r.v[3] * r.v[3]), 1e-12f);
+      AdamVec<4> y;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) y.v[k] = r.v[k] / n2;
+      put(p.prm.rotation, r);
+      put(p.st.m_rotation, m);
+      put(p.st.v_rotation, v);
+      put(p.act.rotations, y);
     }
   }
-  // f_rest (group 2), elementwise (element e of Gaussian g's (M - 1) x 3 rest coefficients; rest_n <
-  // 2^32 is checked on the host, so 32-bit index arithmetic suffices).  Each thread loads
-  // kAdamUnroll elements before updating any, so that many loads are in flight per thread.
-  constexpr int kAdamUnroll = 4;
-  const uint32_t per = (uint32_t)(M - 1) * 3u;
-  // e / per as a multiply-high by ceil(2^32 / per): for every 32-bit e the estimate is the quotient
-  // or one more, and one comparison settles it
-  const uint32_t per_magic = per ? (uint32_t)((0x100000000ull + per - 1) / per) : 0u;
-  const AdamScalars& s = s_sc[2];
-  for (int64_t base = (int64_t)blockIdx.x * blockDim.x * kAdamUnroll + threadIdx.x; base < rest_n;
-       base += stride * kAdamUnroll) {
-    float pv[kAdamUnroll], mv[kAdamUnroll], vv[kAdamUnroll], gv[kAdamUnroll];
-    size_t sh_idx[kAdamUnroll];
-#pragma unroll
-    for (int u = 0; u < kAdamUnroll; ++u) {
-      const int64_t e = base + (int64_t)u * blockDim.x;
-      if (e < rest_n) {
-        uint32_t g = __umulhi((uint32_t)e, per_magic);
-        if ((uint64_t)g * per > (uint64_t)e) --g;
-        const uint32_t r = (uint32_t)e - g * per;
-        sh_idx[u] = (size_t)g * M * 3 + 3 + r;
-        pv[u] = p.prm.features_rest[e];
-        mv[u] = p.st.m_rest[e];
-        vv[u] = p.st.v_rest[e];
-        gv[u] = p.dL_dsh[sh_idx[u]];
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < kAdamUnroll; ++u) {
-      const int64_t e = base + (int64_t)u * blockDim.x;
-      if (e < rest_n) {
-        const float v = adam_update(pv[u], mv[u], vv[u], gv[u], s);
-        p.prm.features_rest[e] = pv[u];
-        p.st.m_rest[e] = mv[u];
-        p.st.v_rest[e] = vv[u];
-        if (p.act.shs_bf16)
-          reinterpret_cast<__nv_bfloat16*>(p.act.shs)[sh_idx[u]] = __float2bfloat16_rn(v);
-        else
-          static_cast<float*>(p.act.shs)[sh_idx[u]] = v;
-      }
+}
+
+// The SH coefficients of Gaussians [g0, g0 + ng): the gradients and the new values, whose rows interleave
+// f_dc (group 1) and f_rest (group 2), pass through shared memory.
+template <int kW>
+__device__ __forceinline__ void adam_sh_tile(const AdamParams& p, float* s_sh, int g0, int ng) {
+  const int M = p.prm.M, per = (M - 1) * 3, row = M * 3, t = threadIdx.x;
+  const float* dsh = p.dL_dsh + (size_t)g0 * row;
+  for (int i = t; i < ng * row / kW; i += kAdamThreads) {
+    if (kW == 4) {
+      const unsigned dst = (unsigned)__cvta_generic_to_shared(s_sh + 4 * i);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(dsh + 4 * i) : "memory");
+    } else {
+      s_sh[i] = dsh[i];
     }
   }
+  // element e of the tile's f_dc and f_rest in shared memory; e / per as a multiply-high by
+  // ceil(2^32 / per), exact for e < 2^16
+  const uint32_t magic = per > 0 ? (uint32_t)((0x100000000ull + per - 1) / per) : 0u;
+  auto rest_at = [&](int e) -> float& { return s_sh[e + 3 * (int)__umulhi((uint32_t)e, magic) + 3]; };
+  auto dc_at = [&](int e) -> float& { const int g = e / 3; return s_sh[g * row + (e - 3 * g)]; };
+  auto update = [&](float* prm, float* m, float* v, int i, AdamVec<kW>& pv, AdamVec<kW>& mv, AdamVec<kW>& vv,
+                    const AdamScalars& s, auto at) {
+    AdamVec<kW> g;
+#pragma unroll
+    for (int k = 0; k < kW; ++k) g.v[k] = at(i * kW + k);
+    adam_vec<kW>(prm, m, v, i, pv, mv, vv, g, s);
+#pragma unroll
+    for (int k = 0; k < kW; ++k) at(i * kW + k) = pv.v[k];
+  };
+  float* dc_p = p.prm.features_dc + (size_t)3 * g0;
+  float* dc_m = p.st.m_dc + (size_t)3 * g0;
+  float* dc_v = p.st.v_dc + (size_t)3 * g0;
+  float* rest_p = per > 0 ? p.prm.features_rest + (size_t)g0 * per : nullptr;
+  float* rest_m = per > 0 ? p.st.m_rest + (size_t)g0 * per : nullptr;
+  float* rest_v = per > 0 ? p.st.v_rest + (size_t)g0 * per : nullptr;
+  const int dc_n = 3 * ng / kW, rest_n = ng * per / kW;
+  AdamScalars s_dc, s_rest;
+  if (kW == 4) {  // a whole tile: everything is loaded before the gradients have arrived
+    constexpr int kRest = (kAdamTile * 45 / 4 + kAdamThreads - 1) / kAdamThreads;
+    static_assert(kAdamTile * 3 / 4 <= kAdamThreads, "one f_dc vector per thread");
+    AdamVec<kW> rp[kRest], rm[kRest], rv[kRest], dp, dm, dv;
+    const int td = kAdamThreads - 1 - t;  // f_dc on the last threads, which have the fewest f_rest vectors
+#pragma unroll
+    for (int u = 0; u < kRest; ++u) {
+      const int i = t + u * kAdamThreads;
+      if (i < rest_n) rp[u] = adam_load<kW>(rest_p, i), rm[u] = adam_load<kW>(rest_m, i), rv[u] = adam_load<kW>(rest_v, i);
+    }
+    if (td < dc_n) dp = adam_load<kW>(dc_p, td), dm = adam_load<kW>(dc_m, td), dv = adam_load<kW>(dc_v, td);
+    adam_scalars2(*p.hyper, 1, 2, s_dc, s_rest);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kRest; ++u)
+      if (t + u * kAdamThreads < rest_n)
+        update(rest_p, rest_m, rest_v, t + u * kAdamThreads, rp[u], rm[u], rv[u], s_rest, rest_at);
+    if (td < dc_n) update(dc_p, dc_m, dc_v, td, dp, dm, dv, s_dc, dc_at);
+  } else {
+    adam_scalars2(*p.hyper, 1, 2, s_dc, s_rest);
+    __syncthreads();
+    for (int i = t; i < rest_n; i += kAdamThreads) {
+      AdamVec<kW> pv = adam_load<kW>(rest_p, i), mv = adam_load<kW>(rest_m, i), vv = adam_load<kW>(rest_v, i);
+      update(rest_p, rest_m, rest_v, i, pv, mv, vv, s_rest, rest_at);
+    }
+    for (int i = t; i < dc_n; i += kAdamThreads) {
+      AdamVec<kW> pv = adam_load<kW>(dc_p, i), mv = adam_load<kW>(dc_m, i), vv = adam_load<kW>(dc_v, i);
+      update(dc_p, dc_m, dc_v, i, pv, mv, vv, s_dc, dc_at);
+    }
+  }
+  __syncthreads();
+  if (p.act.shs_bf16) {
+    __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.act.shs) + (size_t)g0 * row;
+    if (kW == 4) {
+      for (int i = t; i < ng * row / 4; i += kAdamThreads) {
+        const AdamVec<4> f = adam_load<4>(s_sh, i);
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(f.v[0], f.v[1]), hi = __floats2bfloat162_rn(f.v[2], f.v[3]);
+        uint2 u;
+        u.x = *reinterpret_cast<const uint32_t*>(&lo);
+        u.y = *reinterpret_cast<const uint32_t*>(&hi);
+        reinterpret_cast<uint2*>(out)[i] = u;
+      }
+    } else {
+      for (int i = t; i < ng * row; i += kAdamThreads) out[i] = __float2bfloat16_rn(s_sh[i]);
+    }
+  } else {
+    float* out = static_cast<float*>(p.act.shs) + (size_t)g0 * row;
+    for (int i = t; i < ng * row / kW; i += kAdamThreads) adam_store<kW>(out, i, adam_load<kW>(s_sh, i));
+  }
+}
+
+__global__ void __launch_bounds__(kAdamThreads, kAdamBlocksPerSm) adam_gaussian_kernel(const __grid_constant__ AdamParams p) {
+  extern __shared__ float4 s_sh4[];  // [kAdamTile][M][3]
+  // SH tiles first; 16-byte accesses need whole pieces (which then start on 16 bytes if the arrays do)
+  if (blockIdx.x < p.first_chunk[0]) {
+    const int g0 = blockIdx.x * kAdamTile, ng = min(kAdamTile, p.prm.P - g0);
+    if (p.aligned && ng == kAdamTile)
+      adam_sh_tile<4>(p, reinterpret_cast<float*>(s_sh4), g0, ng);
+    else
+      adam_sh_tile<1>(p, reinterpret_cast<float*>(s_sh4), g0, ng);
+    return;
+  }
+  // then the chunks of xyz, scaling, rotation and opacity
+  const int part = (blockIdx.x >= p.first_chunk[1]) + (blockIdx.x >= p.first_chunk[2]) + (blockIdx.x >= p.first_chunk[3]);
+  const int group = part == 0 ? 0 : part == 1 ? 4 : part == 2 ? 5 : 3;
+  const int per = part < 2 ? 3 : part == 2 ? 4 : 1;
+  const int64_t first = (int64_t)(blockIdx.x - p.first_chunk[part]) * kAdamChunk;
+  if (p.aligned && first + kAdamChunk <= (int64_t)p.prm.P * per)
+    adam_chunk<4>(p, group, first);
+  else
+    adam_chunk<1>(p, group, first);
 }
 
 // Activated values from the raw parameters (the first forward of a training run).
@@ -574,12 +731,23 @@ int omnigs_adam_step(const OmnigsGaussianParams* prm, const OmnigsAdamState* st,
   p.dL_dscales = dL_dscales;
   p.dL_drotations = dL_drotations;
   p.hyper = hyper;
-  const int64_t n = (int64_t)prm->P + (int64_t)prm->P * (prm->M - 1) * 3;
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const unsigned blocks = (unsigned)std::min<int64_t>((n + 255) / 256, (int64_t)sms * 8);
-  staged(OMNIGS_STAGE_OTHER, 1, s, [&] { adam_gaussian_kernel<<<blocks, 256, 0, s>>>(p); });
+  const void* arrays[] = {prm->xyz, prm->features_dc, prm->features_rest, prm->opacity, prm->scaling, prm->rotation,
+                          st->m_opacity, st->v_opacity, act->opacities, dL_dopacity, st->m_xyz,
+                          st->v_xyz, st->m_dc, st->v_dc, st->m_rest, st->v_rest, st->m_scaling, st->v_scaling,
+                          st->m_rotation, st->v_rotation, act->means3D, act->shs, act->scales, act->rotations,
+                          dL_dmeans3D, dL_dsh, dL_dscales, dL_drotations};
+  p.aligned = true;
+  for (const void* q : arrays) p.aligned = p.aligned && (reinterpret_cast<uintptr_t>(q) & 15) == 0;
+  // blocks: SH tiles, then chunks of xyz, scaling, rotation and opacity
+  const int64_t P = prm->P;
+  auto chunks = [&](int64_t per) { return (unsigned)((P * per + kAdamChunk - 1) / kAdamChunk); };
+  p.first_chunk[0] = (unsigned)((P + kAdamTile - 1) / kAdamTile);
+  p.first_chunk[1] = p.first_chunk[0] + chunks(3);
+  p.first_chunk[2] = p.first_chunk[1] + chunks(3);
+  p.first_chunk[3] = p.first_chunk[2] + chunks(4);
+  const unsigned blocks = p.first_chunk[3] + chunks(1);
+  const size_t smem = sizeof(float) * kAdamTile * 3 * (size_t)prm->M;
+  staged(OMNIGS_STAGE_OTHER, 1, s, [&] { adam_gaussian_kernel<<<blocks, kAdamThreads, smem, s>>>(p); });
   return check_launch("adam step");
 }
 
