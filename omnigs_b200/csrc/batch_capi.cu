@@ -1,7 +1,6 @@
 // C-ABI entry points of the batched multi-view path (include/omnigs_b200.h, "batched views"):
 // validation, state carving and the launch sequence.  Every stage is one launch for all views:
-//   forward:  batched preprocess -> segmented depth sort (one segment per view) -> duplicate over
-//             all views (global tile ids) -> tile sort -> ranges -> blend of every view's tiles;
+//   forward:  batched preprocess -> binning of all views (run_binning) -> blend of every view's tiles;
 //   backward: blend backward of every view's tiles -> batched backward preprocess.
 // The views' tiles are numbered smallest image first: a small equirect image packs more
 // Gaussians into each tile, so its blocks are the longest and start first.
@@ -28,23 +27,13 @@ struct BatchPlan {
   int P = 0;
 };
 
-// The tile sort of a batch.  Each view's instances leave the duplicate pass contiguous (view after
-// view), so the sort can run per view on view-local tile ids, which need fewer digits than the
-// batch's global ids when the views together hold more than 2^k tiles and the largest alone fewer.
-// Per view, each segment has its own digit histograms (counted by the duplicate pass's emission)
-// and its own look-back chain.
-struct BatchTileSort {
-  TileDigits digits;
-  bool per_view;
-};
-
-BatchTileSort batch_tile_sort(const BatchPlan& plan) {
-  const TileDigits global = TileDigits::from_tiles((uint32_t)plan.tiles);
+// Digit passes that a sort of the instances by tile id would take (per view where that needs fewer): the
+// number that omnigs_batch_state_view reports, whose parity says which buffer holds the sorted list.
+int list_passes(const BatchPlan& plan) {
   int64_t max_view_tiles = 1;
   for (int v = 0; v < plan.V; ++v) max_view_tiles = std::max(max_view_tiles, plan.view_tiles[v]);
-  const TileDigits local = TileDigits::from_tiles((uint32_t)max_view_tiles);
-  const bool per_view = plan.V > 1 && local.passes < global.passes;
-  return {per_view ? local : global, per_view};
+  return std::min(TileDigits::from_tiles((uint32_t)plan.tiles).passes,
+                  TileDigits::from_tiles((uint32_t)max_view_tiles).passes);
 }
 
 int make_plan(int P, int V, const int* W, const int* H, BatchPlan& plan) {
@@ -220,139 +209,39 @@ int omnigs_batch_render(const OmnigsBatchArgs* a, void* state, size_t state_byte
   const BinningLayout BL = BinningLayout::make(capacity);
   if (capacity > kMaxInstances) capacity = kMaxInstances;
   const BatchParams bp = batch_params(a, plan, state, L);
-  GeomHeader* hdr = bp.hdr;
-  uint32_t* thist = at<uint32_t>(binning, BL.hist);
-  uint32_t* dhist = at<uint32_t>(state, L.depth_hist);
-  const int64_t records = (int64_t)a->P * a->V;
-  const int64_t inst_tiles = sort_tiles(BL.capacity);
-
-  staged(OMNIGS_STAGE_OTHER, 1, s, [&] { launch_begin_render(hdr, s); });
-  if (cudaMemsetAsync(at<unsigned char>(state, L.dup_scan), 0, L.zero_end - L.dup_scan, s) != cudaSuccess ||
-      cudaMemsetAsync(thist, 0, sizeof(uint32_t) * kMaxSortPasses * kRadix, s) != cudaSuccess ||
-      cudaMemsetAsync(at<uint2>(state, L.ranges), 0, sizeof(uint2) * plan.tiles, s) != cudaSuccess)
-    return check_launch("memset batch binning state");
-
-  // 1. depth sort of every view's Gaussians: one segment per view, (depth bits, index) order
-  const uint32_t* depth_keys = reinterpret_cast<const uint32_t*>(bp.depth);
-  uint32_t* dkeys[2] = {at<uint32_t>(state, L.dkeys0), at<uint32_t>(state, L.dkeys1)};
-  uint32_t* dvals[2] = {at<uint32_t>(state, L.dvals0), at<uint32_t>(state, L.dvals1)};
-  HistParams hd{};
-  hd.keys = depth_keys;
-  hd.n_host = (uint32_t)records;
-  hd.passes = kDepthPasses;
-  for (int q = 0; q < kDepthPasses; ++q) {
-    hd.shift[q] = kRadixBits * q;
-    hd.mask[q] = kRadix - 1;
-  }
-  hd.hist = dhist;
-  hd.seg_len = (uint32_t)a->P;
-  hd.num_segs = (uint32_t)a->V;
-  staged(OMNIGS_STAGE_SORT, 1, s, [&] { launch_histogram(hd, records, s); });
-  const int64_t depth_tiles = sort_tiles(a->P) * a->V;
-  for (int q = 0; q < kDepthPasses; ++q) {
-    OnesweepParams op{};
-    op.keys_in = q == 0 ? depth_keys : dkeys[(q + 1) & 1];
-    op.vals_in = q == 0 ? nullptr : dvals[(q + 1) & 1];
-    op.keys_out = dkeys[q & 1];
-    op.vals_out = dvals[q & 1];
-    op.shift = kRadixBits * q;
-    op.mask = kRadix - 1;
-    op.n_host = (uint32_t)records;
-    op.hist = dhist + q * kRadix;
-    op.lookback = at<uint32_t>(state, L.depth_lookback) + (size_t)q * depth_tiles * kRadix;
-    op.tile_counter = &hdr->sort_tile_counter[q];
-    op.hdr = hdr;
-    op.seg_len = (uint32_t)a->P;
-    op.num_segs = (uint32_t)a->V;
-    op.hist_seg_stride = kDepthPasses * kRadix;
-    staged(OMNIGS_STAGE_SORT, 1, s, [&] { launch_onesweep(op, records, s); });
-  }
-  const uint32_t* order = dvals[(kDepthPasses - 1) & 1];
-
-  // 2. duplicate every view's instances in that order, keyed by global tile id
-  uint32_t* tkeys[2] = {at<uint32_t>(binning, BL.tkeys0), at<uint32_t>(binning, BL.tkeys1)};
-  uint32_t* tvals[2] = {at<uint32_t>(binning, BL.tvals0), at<uint32_t>(binning, BL.tvals1)};
-  DuplicateParams d{};
-  d.P = a->P;
-  d.V = a->V;
-  d.radii = bp.radii;
-  d.splat = bp.splat;
-  d.order = order;
-  d.tkeys = tkeys[0];
-  d.tvals = tvals[0];
-  d.scan_state = at<unsigned long long>(state, L.dup_scan);
-  d.incl = dkeys[0];  // free once the last depth pass has read it (the sorted keys are in dkeys[1])
-  // the depth sort's other free buffers: its sorted keys and its first value buffer
-  static_assert(((kDepthPasses - 1) & 1) == 1, "the depth order is in dvals[1]");
-  d.rect_row = dvals[0];
-  d.rect_cw = dkeys[1];
-  d.emit_first = at<uint32_t>(binning, BL.emit_first);
-  d.emit_last = at<uint32_t>(binning, BL.emit_last);
-  d.capacity = capacity;
-  d.hdr = hdr;
-  d.seam_wrap = a->seam_wrap;
+  const int fin = list_passes(plan) & 1;
+  BinningPass b{};
+  b.grid.P = a->P;
+  b.grid.V = a->V;
+  b.grid.seam_wrap = a->seam_wrap;
+  b.grid.num_tiles = (uint32_t)plan.tiles;
   for (int v = 0; v < a->V; ++v) {
-    d.gx[v] = bp.views[v].gx;
-    d.gy[v] = bp.views[v].gy;
-    d.tile_base[v] = bp.views[v].tile_base;
+    b.grid.gx[v] = bp.views[v].gx;
+    b.grid.gy[v] = bp.views[v].gy;
+    b.grid.tile_base[v] = bp.views[v].tile_base;
   }
-  // tile sort per view or over the global tile ids (batch_tile_sort)
-  const BatchTileSort ts = batch_tile_sort(plan);
-  const bool per_view = ts.per_view;
-  const TileDigits& tds = ts.digits;
-  uint32_t* tile_hist = per_view ? at<uint32_t>(state, L.tile_hist) : thist + kDepthPasses * kRadix;
-  const int64_t lb_tiles = inst_tiles + a->V;  // look-back tiles per pass (per view: partial tiles)
-  if (cudaMemsetAsync(at<uint32_t>(binning, BL.tile_lookback), 0, sizeof(uint32_t) * tds.passes * lb_tiles * kRadix,
-                      s) != cudaSuccess)
-    return check_launch("memset tile look-back");
-  d.hist = tile_hist;
-  d.hist_passes = tds.passes;
-  d.hist_per_view = per_view ? 1 : 0;
-  d.key_base_out = at<uint32_t>(state, L.view_key_base);
-  for (int q = 0; q < tds.passes; ++q) {
-    d.hist_shift[q] = tds.shift[q];
-    d.hist_mask[q] = tds.mask[q];
-  }
-  staged(OMNIGS_STAGE_DUPLICATE, 1, s, [&] { launch_duplicate(d, s); });
+  b.depth = bp.depth;
+  b.radii = bp.radii;
+  b.splat = bp.splat;
+  b.dkeys[0] = at<uint32_t>(state, L.dkeys0);
+  b.dkeys[1] = at<uint32_t>(state, L.dkeys1);
+  b.dvals[0] = at<uint32_t>(state, L.dvals0);
+  b.dvals[1] = at<uint32_t>(state, L.dvals1);
+  b.zero = at<uint4>(state, L.dup_scan);
+  b.zero_bytes = L.zero_end - L.dup_scan;
+  b.scan_state = at<unsigned long long>(state, L.dup_scan);
+  b.depth_lookback = at<uint32_t>(state, L.depth_lookback);
+  b.depth_hist = at<uint32_t>(state, L.depth_hist);
+  b.binning = binning;
+  b.layout = BL;
+  b.capacity = capacity;
+  b.ranges = at<uint2>(state, L.ranges);
+  b.hdr = bp.hdr;
+  b.out = fin;
+  uint32_t* tvals[2] = {at<uint32_t>(binning, BL.tvals0), at<uint32_t>(binning, BL.tvals1)};
+  if (int rc = run_binning(b, s)) return rc;
 
-  // 3. stable tile sort of all instances (per view when per_view; the digit histograms were
-  // counted by the duplicate pass)
-  for (int q = 0; q < tds.passes; ++q) {
-    OnesweepParams op{};
-    op.keys_in = tkeys[q & 1];
-    op.vals_in = tvals[q & 1];
-    op.keys_out = tkeys[(q + 1) & 1];
-    op.vals_out = tvals[(q + 1) & 1];
-    op.shift = tds.shift[q];
-    op.mask = tds.mask[q];
-    op.count_hdr = hdr;
-    op.capacity = capacity;
-    op.hist = tile_hist + q * kRadix;
-    op.lookback = at<uint32_t>(binning, BL.tile_lookback) + (size_t)q * lb_tiles * kRadix;
-    op.tile_counter = &hdr->sort_tile_counter[kDepthPasses + q];
-    op.hdr = hdr;
-    if (per_view) {
-      op.seg_counts = bp.view_rendered;
-      op.num_segs = (uint32_t)a->V;
-      op.hist_seg_stride = kTilePasses * kRadix;
-      op.add_key_base = q == tds.passes - 1;
-    }
-    staged(OMNIGS_STAGE_SORT, 1, s, [&] { launch_onesweep(op, capacity, s); });
-  }
-  const int fin = tds.passes & 1;
-  if (int rc = check_launch("batch binning")) return rc;
-
-  // 4. tile ranges over all views' tiles
-  RangesParams rp{};
-  rp.keys = tkeys[fin];
-  rp.ranges = at<uint2>(state, L.ranges);
-  rp.num_tiles = (uint32_t)plan.tiles;
-  rp.capacity = capacity;
-  rp.hdr = hdr;
-  staged(OMNIGS_STAGE_RANGES, 1, s, [&] { launch_ranges(rp, s); });
-  if (int rc = check_launch("batch ranges")) return rc;
-
-  // 5. blend every tile of every view
+  // blend every tile of every view
   const BatchRenderParams r = render_params(bp, plan, state, L, tvals[fin], capacity);
   staged(OMNIGS_STAGE_RENDER_FORWARD, 1, s, [&] { launch_batch_render_forward(r, s); });
   return check_launch("batch render forward");
@@ -397,7 +286,7 @@ int omnigs_batch_backward(const OmnigsBatchArgs* a, const OmnigsBatchGrads* g, v
   if (int rc = check_aligned(binning)) return rc;
   const BinningLayout BL = BinningLayout::make(capacity);
   if (capacity > kMaxInstances) capacity = kMaxInstances;
-  const int fin = batch_tile_sort(plan).digits.passes & 1;
+  const int fin = list_passes(plan) & 1;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   const BatchParams bp = batch_params(a, plan, state, L);
   const BatchRenderParams r =
@@ -450,7 +339,7 @@ int omnigs_batch_autotune(const OmnigsBatchArgs* a, void* state, size_t state_by
     return check_launch("read batch status");
   if (h.status != 0)
     return fail(OMNIGS_ERR_DEVICE, "the batch state holds no complete forward (status word set); run omnigs_batch_forward first");
-  const int fin = batch_tile_sort(plan).digits.passes & 1;
+  const int fin = list_passes(plan) & 1;
   const BatchParams bp = batch_params(a, plan, state, L);
   const BatchRenderParams r =
       render_params(bp, plan, state, L, at<uint32_t>(binning, fin ? BL.tvals1 : BL.tvals0), capacity);
@@ -538,7 +427,7 @@ int omnigs_batch_state_view(const void* state, int P, int V, const int* W, const
     out->pixel_base[v] = plan.pixel_base[v];
     out->tile_base[v] = plan.tile_base[v];
   }
-  out->tile_passes = batch_tile_sort(plan).digits.passes;
+  out->tile_passes = list_passes(plan);
   out->depth = at<float>(state, L.depth);
   return OMNIGS_OK;
 }
@@ -552,7 +441,7 @@ int omnigs_batch_binning_view(const void* binning, size_t binning_bytes, int P, 
   const int64_t capacity = BinningLayout::capacity_for(binning_bytes);
   if (capacity < 0) return fail(OMNIGS_ERR_BUFFER_TOO_SMALL, "binning buffer too small");
   const BinningLayout BL = BinningLayout::make(capacity);
-  const int fin = batch_tile_sort(plan).digits.passes & 1;
+  const int fin = list_passes(plan) & 1;
   out->tile_ids = at<uint32_t>(binning, fin ? BL.tkeys1 : BL.tkeys0);
   out->point_list = at<uint32_t>(binning, fin ? BL.tvals1 : BL.tvals0);
   return OMNIGS_OK;

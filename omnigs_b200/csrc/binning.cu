@@ -1,24 +1,32 @@
 // Binning: the reference's sorted instance list and tile ranges (rasterizer_impl.cu:94-167,
-// 622-679) from a depth sort of the Gaussians plus a tile sort of the instances.
+// 622-679) from a depth sort of the Gaussians, a coarse list per bin of 8x4 tiles and, out of it, a
+// compaction per tile.
 //
 // The reference emits one (tile << 32 | depth_bits) key per (Gaussian, tile) pair in Gaussian
 // order and sorts them with a stable LSD radix sort over bits [0, 32 + getHigherMsb(tiles)).  The
 // result is fully determined: instances ordered by tile, then by depth bits, then -- a Gaussian
 // appears at most once per tile and the list starts in Gaussian order -- by Gaussian index.  The
-// same order is produced here with far fewer passes over the instances:
+// same order is produced here without sorting the instances at all:
 //  1. depth sort: a stable LSD radix sort (4 onesweep passes of 8 bits) of the P Gaussians by the
 //     bits of their depth, i.e. the order (depth bits, index);
-//  2. duplicate: a scan of the Gaussians' tile counts in that order (decoupled look-back), then
-//     a load-balanced emission of the instances in that order (every block writes the same number
-//     of instances), counting the digits of the keys it writes for the tile sort;
-//  3. tile sort: a stable LSD radix sort (2 onesweep passes) of the instances by tile id only
-//     (for a batch of views, per view on view-local tile ids when those need fewer passes than
-//     the batch's global ids: each view's instances are contiguous after step 2).
-// Stability makes (1)+(3) equal to the reference's single sort: instance passes drop from six
-// over 12-byte items to two over 8-byte items; the four depth passes run over P, not R, items.
-//  4. ranges: per-tile [start, end) over the sorted tile ids.
+//  2. coarse lists: a scan of the Gaussians' bin counts in that order (decoupled look-back), a
+//     load-balanced emission of the (bin, depth-order position) pairs in that order, and a stable
+//     LSD radix sort of the pairs by bin (one onesweep pass up to 256 bins): every bin's Gaussians
+//     in depth order.  A splat covers far fewer bins than tiles;
+//  3. tile lists: every bin counts its tiles' instances (its pairs' tiles as bit masks), a scan of the
+//     counts in tile order gives the ranges, and every row of a bin's tiles compacts the bin's list
+//     into its tiles' lists, in order (ballots of the masks' bits).
+// Few Gaussians (kRankMaxP) are ordered by counting, which costs less than the five launches of the
+// depth sort: a Gaussian's position is the number of smaller depths.  Where Gaussians times bins are
+// few (kWholeMaxPairs) there are no coarse lists: every bin reads its view's whole order.
 // Counts live on the device: every kernel reads num_rendered from the geometry header and does no
 // work if it exceeds the binning capacity.  Waits on other blocks are bounded.
+//
+// Measured on a B200 against emitting every instance and sorting the list by tile id in two or three
+// passes, all stages of the binning: 1M Gaussians at 2048x1024 (8.6M instances) 353 -> 239 us, 3M at
+// 4096x2048 (72M) 1895 -> 905 us, 16 views over 1M Gaussians (112M) 3.49 -> 2.35 ms, 10,000 at 512x256
+// 115 -> 49 us.  The sort passes over the instances were what it cost (80 us each over 8.2M), and the
+// pairs are a fifth of them.
 #include <algorithm>
 
 #include "device_util.cuh"
@@ -46,11 +54,14 @@ __device__ __forceinline__ bool instances_fit(const GeomHeader* hdr, int64_t cap
   return (hdr->status & kStatusOverflow) == 0 && hdr->num_rendered64 <= (unsigned long long)capacity;
 }
 
-// Element count of a sort/histogram: a host value, or the device num_rendered (0 if it does not
-// fit the capacity, in which case the duplicate pass has flagged the overflow).
+// Number of (Gaussian, bin) pairs, at most one per instance (0 if the instances do not fit the
+// capacity, which the scan has flagged).
+__device__ __forceinline__ uint32_t pair_count(const GeomHeader* hdr, int64_t capacity) {
+  return instances_fit(hdr, capacity) ? (uint32_t)min((long long)hdr->num_pairs, (long long)capacity) : 0u;
+}
+// Element count of a sort/histogram: a host value, or the device's pair count.
 __device__ __forceinline__ uint32_t item_count(const GeomHeader* count_hdr, uint32_t n_host, int64_t capacity) {
-  if (count_hdr == nullptr) return n_host;
-  return instances_fit(count_hdr, capacity) ? count_hdr->num_rendered : 0u;
+  return count_hdr == nullptr ? n_host : pair_count(count_hdr, capacity);
 }
 
 // ---------------------------------------------------------------- digit histograms ------------
@@ -118,9 +129,6 @@ struct SortSmem {
   uint32_t pad[3];
   uint32_t keys[kTile];
   uint32_t vals[kTile];
-  // the block's segment as thread 0 resolved it (variable segments): index (num_segs: none), item
-  // count, tile within the segment, first item, key base
-  uint32_t seg, seg_n, seg_tile, seg_first, seg_key_base;
 };
 
 // Exclusive scan of one value per thread across the block (kSortThreads == kRadix == 256).
@@ -156,68 +164,31 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* s
 // decoupled look-back (tiles are taken in launch order from an atomic counter, so a block only
 // waits on blocks that are already running) and writes runs of equal digits coalesced.  In a
 // segmented sort every segment is an independent sort whose look-back chain starts at the
-// segment's first tile (segments of equal length, or of device-side lengths, whose keys are then
-// segment-local and get seg_key_base added back in the last pass); a value-less first pass numbers
-// items by their global index.
+// segment's first tile; a value-less first pass numbers items by their global index.
 // Launches of this pass measured ~2 us slower each on a B200 with a 136-byte parameter block than
 // with a 128-byte one.
 static_assert(sizeof(OnesweepParams) <= 128, "keep the onesweep parameter block at 128 bytes or less");
 
 // Tiles of kSortTile keys, 16 per thread.  Measured on a B200: 1024-key tiles (4 per thread, five
 // blocks per SM) made the depth passes over 1M Gaussians slower, 22 -> 30 us each (4x the blocks,
-// look-back chains and per-tile scans), so every pass uses the 4096-key tiles.
-template <bool kVarSeg>
-__global__ void __launch_bounds__(kSortThreads, 3) onesweep_kernel(OnesweepParams p) {
-  constexpr int kItems = kSortItems;
-  constexpr int kTile = kSortTile;
+// look-back chains and per-tile scans), so passes over many keys use the 4096-key tiles; passes that
+// 1024-key tiles spread over at most kSmallSortTiles blocks are bound by a tile's own latency and use
+// those: 282 -> 276 us for the whole forward of 150,000 Gaussians (147 tiles), nothing at 300,000 (293).
+template <int kItems, int kMinBlocks, int kLookback>
+__global__ void __launch_bounds__(kSortThreads, kMinBlocks) onesweep_kernel(OnesweepParams p) {
+  constexpr int kTile = kSortThreads * kItems;
   __shared__ SortSmem<kTile> sm;
-  uint32_t n = 0, tiles_per_seg = 1, ntiles = 0;
-  if (!kVarSeg) {
-    n = p.seg_len ? p.seg_len : item_count(p.count_hdr, p.n_host, p.capacity);
-    tiles_per_seg = (n + kTile - 1) / kTile;
-    ntiles = tiles_per_seg * (p.seg_len ? p.num_segs : 1u);
-  }
-  if (threadIdx.x == 0) {
-    const uint32_t t = atomicAdd(p.tile_counter, 1u);
-    sm.tile = t;
-    if (kVarSeg) {  // variable segments: tickets run over the segments' tiles in order
-      const bool fit = instances_fit(p.count_hdr, p.capacity);
-      uint32_t first_tile = 0, first_item = 0;
-      sm.seg = p.num_segs;
-      for (uint32_t sg = 0; sg < p.num_segs; ++sg) {
-        const uint32_t ns = fit ? (uint32_t)p.seg_counts[sg] : 0u;
-        const uint32_t ts = (ns + kTile - 1) / kTile;
-        if (t < first_tile + ts) {
-          sm.seg = sg;
-          sm.seg_n = ns;
-          sm.seg_tile = t - first_tile;
-          sm.seg_first = first_item;
-          sm.seg_key_base = reinterpret_cast<const uint32_t*>(p.seg_counts + kMaxBatchViews)[sg];
-          break;
-        }
-        first_tile += ts;
-        first_item += ns;
-      }
-    }
-  }
+  const uint32_t n = p.seg_len ? p.seg_len : item_count(p.count_hdr, p.n_host, p.capacity);
+  const uint32_t tiles_per_seg = (n + kTile - 1) / kTile;
+  const uint32_t ntiles = tiles_per_seg * (p.seg_len ? p.num_segs : 1u);
+  if (threadIdx.x == 0) sm.tile = atomicAdd(p.tile_counter, 1u);
   for (int i = threadIdx.x; i < (kSortThreads / 32) * kRadix; i += kSortThreads) (&sm.warp_hist[0][0])[i] = 0;
   __syncthreads();
   const uint32_t ticket = sm.tile;
-  // this block's segment, its item count and first item, and the tile index within it
-  uint32_t seg, tile;
-  size_t seg_base;
-  if (kVarSeg) {
-    seg = sm.seg;
-    if (seg >= p.num_segs) return;
-    n = sm.seg_n;
-    tile = sm.seg_tile;
-    seg_base = sm.seg_first;
-  } else {
-    if (ticket >= ntiles) return;
-    seg = ticket / tiles_per_seg;
-    tile = ticket - seg * tiles_per_seg;  // tile index within the segment
-    seg_base = (size_t)seg * n;
-  }
+  if (ticket >= ntiles) return;
+  const uint32_t seg = ticket / tiles_per_seg;
+  const uint32_t tile = ticket - seg * tiles_per_seg;  // tile index within the segment
+  const size_t seg_base = (size_t)seg * n;
   const uint32_t* keys_in = p.keys_in + seg_base;
   const uint32_t* vals_in = p.vals_in ? p.vals_in + seg_base : nullptr;
   uint32_t* keys_out = p.keys_out + seg_base;
@@ -294,12 +265,12 @@ __global__ void __launch_bounds__(kSortThreads, 3) onesweep_kernel(OnesweepParam
     int64_t j = (int64_t)tile - 1;
     bool gave_up = false, found = false;
     while (!found) {
-      uint32_t w[kLookbackBatch];
+      uint32_t w[kLookback];
 #pragma unroll
-      for (int b = 0; b < kLookbackBatch; ++b)
+      for (int b = 0; b < kLookback; ++b)
         w[b] = (j - b >= 0) ? ld_relaxed_u32(&lb[(size_t)(j - b) * kRadix + d]) : kLbPrefix;
 #pragma unroll
-      for (int b = 0; b < kLookbackBatch; ++b) {
+      for (int b = 0; b < kLookback; ++b) {
         uint32_t x = w[b];
         if (!found && (x >> 30) == 0) {
           int spins = 0;
@@ -318,7 +289,7 @@ __global__ void __launch_bounds__(kSortThreads, 3) onesweep_kernel(OnesweepParam
           found = (x >> 30) == 2;
         }
       }
-      j -= kLookbackBatch;
+      j -= kLookback;
     }
     if (gave_up) atomicOr(&p.hdr->status, kStatusLookback);
     st_relaxed_u32(&lb[(size_t)tile * kRadix + d], kLbPrefix | ((prev + count) & kLbValue));
@@ -338,80 +309,125 @@ __global__ void __launch_bounds__(kSortThreads, 3) onesweep_kernel(OnesweepParam
     }
   }
   __syncthreads();
-  // the last pass of a variable-segment sort turns segment-local keys back into global ones
-  const uint32_t key_add = (kVarSeg && p.add_key_base) ? sm.seg_key_base : 0u;
   for (uint32_t i = threadIdx.x; i < tile_items; i += kSortThreads) {
     const uint32_t k32 = sm.keys[i];
     const uint32_t digit = (k32 >> shift) & mask;
     const uint32_t out = sm.global_base[digit] + (i - sm.block_excl[digit]);
     if (out < n) {  // always true unless a look-back gave up (the status word then says so)
-      keys_out[out] = k32 + key_add;
+      keys_out[out] = k32;
       vals_out[out] = sm.vals[i];
     }
   }
 }
 
-// ---------------------------------------------------------------- duplicate -------------------
-// duplicateWithKeys (rasterizer_impl.cu:94-140) over the depth-sorted Gaussians, in two kernels:
-//  1. instance_scan_kernel: the inclusive scan of the Gaussians' tile counts in depth order (block
-//     b takes sorted positions [1024 b, 1024 b + 1024), four per thread: block scan plus a
-//     decoupled look-back over the preceding blocks), written to p.incl; every Gaussian whose
-//     instances hold the first or last instance of an emit block (kEmitBlock instances) records
-//     its position there (p.emit_first / p.emit_last);
-//  2. instance_emit_kernel: block b writes instances [2048 b, 2048 b + 2048) of the list: every
-//     block does the same amount of work however the instances are spread over the Gaussians
-//     (the nearest splats, first in depth order, cover thousands of tiles each).  It stages the
-//     offsets and tile rects of its Gaussians in shared memory; each thread writes 8 consecutive
-//     instances (one binary search for the first one's Gaussian, then a walk through the rect and
-//     on to the next Gaussians, two 16-byte stores per array) and counts the digit histograms of
-//     the tile sort that follows.
-// One kernel doing both measured ~150 us at 400k and 1M Gaussians alike: a block's warps each
-// emitted their own Gaussians' instances, so a block held its SM slots until its busiest warp was
-// done (62 % of the stall samples were barrier waits).
+// ---------------------------------------------------------------- start of a pass -------------
+// Clears the pass's counters, histograms and look-back words in one launch (four memsets and a kernel
+// took five).
+__global__ void __launch_bounds__(256) begin_binning_kernel(const __grid_constant__ BeginParams p) {
+  chain_begin();
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    GeomHeader* hdr = p.hdr;
+    const unsigned long long total = hdr->num_rendered64;
+    uint32_t status = hdr->status & ~(kStatusCapacity | kStatusInconsistent);
+    if (total > (unsigned long long)kMaxInstances) status |= kStatusOverflow;
+    hdr->status = status;
+    hdr->num_rendered = (uint32_t)(total > 0xffffffffull ? 0xffffffffull : total);
+    hdr->dup_tile_counter = 0;
+    hdr->num_pairs = 0;
+    for (int i = 0; i < kMaxSortPasses; ++i) hdr->sort_tile_counter[i] = 0;
+  }
+  const size_t first = (size_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
+#pragma unroll
+  for (int r = 0; r < BeginParams::kRegions; ++r)
+    for (size_t i = first; i < p.bytes[r] / 16; i += stride) p.region[r][i] = make_uint4(0u, 0u, 0u, 0u);
+}
 
-// Tile rect of record `rec` (view `view`) in the duplicate's terms: instance count, rect width,
-// first column, tile-id pitch and the id of the rect's first row (view-local when per view).
-struct RecordRect {
-  uint32_t count, row_origin;
-  int pitch, width, col0;
-};
+// ---------------------------------------------------------------- coarse lists ----------------
+// duplicateWithKeys (rasterizer_impl.cu:94-140) by bins of kBinW x kBinH tiles instead of tiles, over the
+// depth-sorted Gaussians, in two kernels:
+//  1. pair_scan_kernel: the inclusive scan of the Gaussians' bin counts in depth order (block b takes
+//     sorted positions [1024 b, 1024 b + 1024), four per thread: block scan plus a decoupled look-back
+//     over the preceding blocks), written to p.incl with the tile rects; every Gaussian whose pairs
+//     hold the first or last pair of an emit block (kEmitBlock pairs) records its position there
+//     (p.emit_first / p.emit_last);
+//  2. pair_emit_kernel: block b writes pairs [2048 b, 2048 b + 2048) of the list: every block does the
+//     same amount of work however the pairs are spread over the Gaussians (the nearest splats, first
+//     in depth order, cover most bins).  It stages the offsets and bin rects of its Gaussians in
+//     shared memory; each thread writes 8 consecutive pairs (one binary search for the first one's
+//     Gaussian, then a walk through the rect and on to the next Gaussians, two 16-byte stores per
+//     array) and counts the digit histograms of the bin sort that follows.
 
-template <bool kPerView>
-__device__ __forceinline__ RecordRect record_rect(const DuplicateParams& p, uint32_t rec, uint32_t view) {
-  RecordRect r;
-  r.count = 0;
-  r.row_origin = 0;
-  r.pitch = 1;
-  r.width = 1;
-  r.col0 = 0;
-  const int radius = (rec - view * (uint32_t)p.P < (uint32_t)p.P) ? p.radii[rec] : 0;
+__device__ __forceinline__ uint32_t record_view(const TileGrid& g, uint32_t i) {
+  return (g.V == 1) ? 0u : i / (uint32_t)g.P;  // the depth order keeps records in their view
+}
+
+// Tile rect of record `rec` as the kernels keep it: first column | end << 16 (the first column may be
+// negative and the end past gx when the seam wraps) and first row | end << 16; empty: 0, 0.
+__device__ __forceinline__ uint2 record_rect(const TileGrid& grid, const int* radii, const float4* splat, uint32_t rec,
+                                             uint32_t view) {
+  uint2 r = make_uint2(0u, 0u);
+  const int radius = (rec - view * (uint32_t)grid.P < (uint32_t)grid.P) ? radii[rec] : 0;
   if (radius > 0) {
-    const float4 a = p.splat[2 * rec];
-    const int gx = p.gx[view];
+    const float4 a = splat[2 * (size_t)rec];
     int2 rmin, rmax;
-    if (p.seam_wrap)
-      tile_rect_cyclic(make_float2(a.x, a.y), radius, gx, p.gy[view], rmin, rmax);
+    if (grid.seam_wrap)
+      tile_rect_cyclic(make_float2(a.x, a.y), radius, grid.gx[view], grid.gy[view], rmin, rmax);
     else
-      tile_rect(make_float2(a.x, a.y), radius, gx, p.gy[view], rmin, rmax);
-    r.width = rmax.x - rmin.x;
-    r.count = (uint32_t)r.width * (uint32_t)(rmax.y - rmin.y);
-    if (r.count == 0) r.width = 1;
-    r.pitch = gx;
-    r.col0 = rmin.x;
-    // per-view counting writes view-local tile ids (the tile sort restores the global ids)
-    r.row_origin = (kPerView ? 0u : p.tile_base[view]) + (uint32_t)rmin.y * (uint32_t)gx;
+      tile_rect(make_float2(a.x, a.y), radius, grid.gx[view], grid.gy[view], rmin, rmax);
+    if (rmax.x > rmin.x && rmax.y > rmin.y)
+      r = make_uint2(((uint32_t)rmin.x & 0xffffu) | ((uint32_t)rmax.x << 16), (uint32_t)rmin.y | ((uint32_t)rmax.y << 16));
   }
   return r;
 }
 
-__device__ __forceinline__ uint32_t record_view(const DuplicateParams& p, uint32_t i) {
-  return (p.V == 1) ? 0u : i / (uint32_t)p.P;  // the depth order keeps records in their view
+// The bins of a tile rect: first column (the columns run on modulo the view's bx when the seam wraps),
+// columns, first row, rows.
+struct BinRect {
+  uint32_t col, cols, row, rows;
+};
+__device__ __forceinline__ BinRect bin_rect(uint2 r, int gx, int bx) {
+  BinRect b{0u, 0u, 0u, 0u};
+  int x0 = (int)(int16_t)(r.x & 0xffffu), x1 = (int)(r.x >> 16);
+  const uint32_t y0 = r.y & 0xffffu, y1 = r.y >> 16;
+  if (y1 <= y0) return b;
+  if (x0 < 0) {  // columns [x0 + gx, gx) and [0, x1): the rect is at most gx wide
+    x0 += gx;
+    x1 += gx;
+  }
+  if (x0 >= gx) {
+    x0 -= gx;
+    x1 -= gx;
+  }
+  b.col = (uint32_t)x0 / kBinW;
+  if (x1 <= gx)
+    b.cols = (uint32_t)(x1 - 1) / kBinW + 1u - b.col;
+  else
+    b.cols = min((uint32_t)bx, (uint32_t)bx - b.col + (uint32_t)(x1 - gx - 1) / kBinW + 1u);
+  b.row = y0 / kBinH;
+  b.rows = (y1 - 1u) / kBinH + 1u - b.row;
+  return b;
+}
+
+// A pair's word: the bin's tiles that the rect covers (bits [0, 8) its columns, bits [8, 12) its rows), and
+// above them the bin (at most 2^20 of them: 32 views of 2^28 pixels).  It is the key that the pairs are
+// sorted by, so the fine stage reads everything it needs in order, without a gather.
+static_assert(kBinW * kBinH == 32, "a lane per tile of a bin");
+
+__device__ __forceinline__ uint32_t tile_mask(int tx0, int ty0, int gx, bool wrap, uint2 rect) {
+  const int x0 = (int)(int16_t)(rect.x & 0xffffu) - tx0, x1 = (int)(rect.x >> 16) - tx0;
+  const int y0 = (int)(rect.y & 0xffffu) - ty0, y1 = (int)(rect.y >> 16) - ty0;
+  auto span = [](int lo, int hi, int width) {  // bits [lo, hi) of `width`
+    const int l = min(max(lo, 0), width), h = min(max(hi, 0), width);
+    return h > l ? ((1u << h) - 1u) & ~((1u << l) - 1u) : 0u;
+  };
+  uint32_t cols = span(x0, x1, kBinW);
+  if (wrap) cols = (cols | span(x0 + gx, x1 + gx, kBinW) | span(x0 - gx, x1 - gx, kBinW)) & span(0, gx - tx0, kBinW);
+  return cols | (span(y0, y1, kBinH) << kBinW);
 }
 
 constexpr int kScanItems = kScanTile / kScanBlock;  // Gaussians per scan thread
 
-template <bool kPerView>
-__global__ void __launch_bounds__(kScanBlock) instance_scan_kernel(const __grid_constant__ DuplicateParams p) {
+__global__ void __launch_bounds__(kScanBlock) pair_scan_kernel(const __grid_constant__ DuplicateParams p) {
   __shared__ uint32_t s_tile;
   __shared__ uint32_t s_warp[kScanBlock / 32];
   __shared__ unsigned long long s_excl;
@@ -419,12 +435,11 @@ __global__ void __launch_bounds__(kScanBlock) instance_scan_kernel(const __grid_
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&p.hdr->status, kStatusCapacity);
     return;
   }
-  if (kPerView && blockIdx.x == 0 && threadIdx.x < p.V) p.key_base_out[threadIdx.x] = p.tile_base[threadIdx.x];
   if (threadIdx.x == 0) s_tile = atomicAdd(&p.hdr->dup_tile_counter, 1u) + p.skip_tiles;
   __syncthreads();
   const uint32_t tile = s_tile;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint32_t items = (uint32_t)p.P * (uint32_t)p.V;
+  const uint32_t items = (uint32_t)p.grid.P * (uint32_t)p.grid.V;
   const uint32_t i0 = tile * (uint32_t)kScanTile + threadIdx.x * (uint32_t)kScanItems;
   uint32_t cnt[kScanItems];
 #pragma unroll
@@ -432,10 +447,12 @@ __global__ void __launch_bounds__(kScanBlock) instance_scan_kernel(const __grid_
     const uint32_t i = i0 + u;
     cnt[u] = 0;
     if (i < items) {
-      const RecordRect r = record_rect<kPerView>(p, p.order[i], record_view(p, i));
-      cnt[u] = r.count;
-      p.rect_row[i] = r.row_origin;
-      p.rect_cw[i] = ((uint32_t)r.col0 & 0xffffu) | ((uint32_t)r.width << 16);
+      const uint32_t view = record_view(p.grid, i);
+      const uint2 r = record_rect(p.grid, p.radii, p.splat, p.order[i], view);
+      const BinRect b = bin_rect(r, p.grid.gx[view], bins_x(p.grid.gx[view]));
+      cnt[u] = b.cols * b.rows;
+      p.rect_x[i] = r.x;
+      p.rect_y[i] = r.y;
     }
   }
   uint32_t thread_total = 0;
@@ -508,8 +525,8 @@ __global__ void __launch_bounds__(kScanBlock) instance_scan_kernel(const __grid_
     }
   }
   __syncthreads();
-  const unsigned long long R = p.hdr->num_rendered64;
-  const uint32_t nblocks = (uint32_t)((R + kEmitBlock - 1) / kEmitBlock);  // emit blocks (R fits the capacity)
+  // (past the capacity only when the scan is inconsistent: at most one pair per instance)
+  const unsigned long long max_blocks = ((unsigned long long)p.capacity + kEmitBlock - 1) / kEmitBlock;
   unsigned long long incl = s_excl + thread_excl;
 #pragma unroll
   for (int u = 0; u < kScanItems; ++u) {
@@ -518,19 +535,17 @@ __global__ void __launch_bounds__(kScanBlock) instance_scan_kernel(const __grid_
     incl += cnt[u];
     if (i >= items) continue;
     p.incl[i] = (uint32_t)min(incl, 0xffffffffull);
-    if (cnt[u] == 0 || incl > R) continue;  // (past R only when the scan is inconsistent)
-    // the emit blocks whose first instance (b * kEmitBlock) lies in [start, incl)
-    for (unsigned long long b = (start + kEmitBlock - 1) / kEmitBlock; b * kEmitBlock < incl && b < nblocks; ++b)
+    if (cnt[u] == 0) continue;
+    // the emit blocks whose first pair (b * kEmitBlock) lies in [start, incl)
+    for (unsigned long long b = (start + kEmitBlock - 1) / kEmitBlock; b * kEmitBlock < incl && b < max_blocks; ++b)
       p.emit_first[b] = i;
-    // ... and whose last instance (min((b + 1) kEmitBlock, R) - 1) does
-    for (unsigned long long b = start / kEmitBlock; b < nblocks && b * kEmitBlock < incl; ++b) {
-      const unsigned long long last = min((b + 1) * (unsigned long long)kEmitBlock, R) - 1;
-      if (last >= start && last < incl) p.emit_last[b] = i;
-    }
+    // ... and those whose last pair does, the last block (whose end the emission finds) aside
+    for (unsigned long long b = start / kEmitBlock; b < max_blocks && (b + 1) * kEmitBlock <= incl; ++b)
+      p.emit_last[b] = i;
   }
   const uint32_t last_tile = (items + kScanTile - 1) / kScanTile - 1u;
-  if (tile == last_tile && threadIdx.x == kScanBlock - 1 && s_excl + block_total != R)
-    atomicOr(&p.hdr->status, kStatusInconsistent);
+  if (tile == last_tile && threadIdx.x == kScanBlock - 1)
+    p.hdr->num_pairs = (uint32_t)min(s_excl + block_total, (unsigned long long)p.capacity);
 }
 
 constexpr int kEmitPerThread = kEmitBlock / kScanBlock;
@@ -542,50 +557,57 @@ __device__ __forceinline__ float rcp_approx_f(float x) {
   return r;
 }
 
-template <bool kPerView>
-__global__ void __launch_bounds__(kScanBlock) instance_emit_kernel(const __grid_constant__ DuplicateParams p) {
-  // digit counts of the tile sort: [slot][pass][digit], slot = view - (the block's first view)
-  // when counted per view; views past kSlots (a block spanning many small views) count directly
-  // into the global histogram
-  constexpr int kHistSlot = kTilePasses * kRadix;
-  constexpr int kSlots = kPerView ? 2 : 1;
-  __shared__ uint32_t s_hist[kSlots * kHistSlot];
-  // the block's Gaussians: inclusive offset, record, first row's tile id, first column | width,
-  // tile-id pitch | view
-  __shared__ uint32_t s_incl[kEmitStage], s_rec[kEmitStage], s_row[kEmitStage], s_cw[kEmitStage], s_pv[kEmitStage];
+__global__ void __launch_bounds__(kScanBlock) pair_emit_kernel(const __grid_constant__ DuplicateParams p) {
+  __shared__ uint32_t s_hist[kTilePasses * kRadix];  // digit counts of the bin sort
+  // the block's Gaussians: inclusive offset, record, tile rect
+  __shared__ uint32_t s_incl[kEmitStage], s_rec[kEmitStage];
+  __shared__ uint2 s_rect[kEmitStage];
+  __shared__ uint32_t s_last;
   if (!instances_fit(p.hdr, p.capacity)) return;  // the scan kernel has flagged the overflow
-  const uint32_t R = p.hdr->num_rendered;
+  const uint32_t R = pair_count(p.hdr, p.capacity);
   const uint32_t o_lo = blockIdx.x * (uint32_t)kEmitBlock;
   if (o_lo >= R) return;
   const uint32_t o_hi = min(R, o_lo + (uint32_t)kEmitBlock);  // exclusive (R <= capacity)
   const int lane = threadIdx.x & 31;
-  const uint32_t items = (uint32_t)p.P * (uint32_t)p.V;
-  for (int k = threadIdx.x; k < kSlots * kHistSlot; k += kScanBlock) s_hist[k] = 0;
+  const uint32_t items = (uint32_t)p.grid.P * (uint32_t)p.grid.V;
+  for (int k = threadIdx.x; k < kTilePasses * kRadix; k += kScanBlock) s_hist[k] = 0;
   // (both clamped: after an inconsistent scan, which the status word reports, the entries may be
   // stale; the reads stay in range)
   const uint32_t g_first = min(p.emit_first[blockIdx.x], items - 1u);
-  const uint32_t g_last = min(p.emit_last[blockIdx.x], items - 1u);
+  if (threadIdx.x == 0) {
+    uint32_t last = items - 1u;
+    if (o_hi - o_lo == (uint32_t)kEmitBlock) {
+      last = min(p.emit_last[blockIdx.x], items - 1u);
+    } else {  // the list's end: the first Gaussian whose inclusive offset reaches it
+      uint32_t lo = g_first;
+      while (lo < last) {
+        const uint32_t mid = (lo + last) >> 1;
+        if (p.incl[mid] >= R)
+          last = mid;
+        else
+          lo = mid + 1u;
+      }
+    }
+    s_last = last;
+  }
+  __syncthreads();
+  const uint32_t g_last = s_last;
   const uint32_t n = g_last >= g_first ? g_last - g_first + 1u : 1u;
-  // Gaussians between g_first and g_last with no instances (culled views' records) can make the
-  // range longer than the block's instance count: then offsets and rects are read from global memory
+  // Gaussians between g_first and g_last with no pairs (culled views' records) can make the range longer
+  // than the block's pair count: then offsets and rects are read from global memory
   const bool staged = n <= (uint32_t)kEmitStage;
   if (staged)
     for (uint32_t t = threadIdx.x; t < n; t += kScanBlock) {
-      const uint32_t i = g_first + t;
-      const uint32_t view = record_view(p, i);
-      s_incl[t] = p.incl[i];
-      s_rec[t] = p.order[i];
-      s_row[t] = p.rect_row[i];
-      s_cw[t] = p.rect_cw[i];
-      s_pv[t] = (uint32_t)p.gx[view] | (view << 16);
+      s_incl[t] = p.incl[g_first + t];
+      s_rec[t] = p.order[g_first + t];
+      s_rect[t] = make_uint2(p.rect_x[g_first + t], p.rect_y[g_first + t]);
     }
   __syncthreads();
   const uint32_t* incl = staged ? s_incl : p.incl + g_first;
   const uint32_t excl0 = g_first > 0 ? p.incl[g_first - 1] : 0u;
-  const uint32_t view0 = record_view(p, g_first);
-  // Thread t writes the kEmitPerThread consecutive instances from o0: one binary search finds the
-  // Gaussian of the first, the others step through the rect (or on to the next Gaussians with
-  // instances, whose first instance they then are) without a search or a division.
+  // Thread t writes the kEmitPerThread consecutive pairs from o0: one binary search finds the Gaussian
+  // of the first, the others step through the rect (or on to the next Gaussians with pairs, whose
+  // first pair they then are) without a search or a division.
   const uint32_t o0 = o_lo + (uint32_t)threadIdx.x * (uint32_t)kEmitPerThread;
   uint32_t j = 0;  // the first of the block's Gaussians whose inclusive offset exceeds o0
   {
@@ -599,51 +621,42 @@ __global__ void __launch_bounds__(kScanBlock) instance_emit_kernel(const __grid_
     }
   }
   uint32_t end_j = incl[j];
-  uint32_t rec = 0, row_origin = 0, view = view0;
-  int col0 = 0, width = 1, pitch = 1;
+  uint32_t rec = 0, view = 0, width = 1;
+  int gx = 1, bx = 1;
+  uint2 rect = make_uint2(0u, 0u);
+  BinRect bins{0u, 1u, 0u, 1u};
   auto load_rect = [&](uint32_t jj) {
-    uint32_t cw;
-    if (staged) {
-      rec = s_rec[jj];
-      row_origin = s_row[jj];
-      cw = s_cw[jj];
-      const uint32_t pv = s_pv[jj];
-      pitch = (int)(pv & 0xffffu);
-      view = pv >> 16;
-    } else {
-      const uint32_t i = g_first + jj;
-      view = record_view(p, i);
-      rec = p.order[i];
-      row_origin = p.rect_row[i];
-      cw = p.rect_cw[i];
-      pitch = p.gx[view];
-    }
-    col0 = (int)(int16_t)(cw & 0xffffu);
-    width = (int)(cw >> 16);
+    const uint32_t i = g_first + jj;
+    view = record_view(p.grid, i);
+    rec = staged ? s_rec[jj] : p.order[i];
+    rect = staged ? s_rect[jj] : make_uint2(p.rect_x[i], p.rect_y[i]);
+    gx = p.grid.gx[view];
+    bx = bins_x(gx);
+    bins = bin_rect(rect, gx, bx);
+    width = max(bins.cols, 1u);
   };
   load_rect(j);
-  // row and column of o0 in the rect: local / width from an approximate reciprocal (local < 2^21,
-  // a rect holds at most every tile of a view, so the truncated estimate is within one of the
-  // quotient; one step fixes it)
+  // row and column of o0 in the rect: local / width from an approximate reciprocal (local < 2^21, a rect
+  // holds at most every bin of a view, so the truncated estimate is within one of the quotient; one
+  // step fixes it)
   const uint32_t local = o0 - (j > 0 ? incl[j - 1] : excl0);
   uint32_t ry = (uint32_t)((float)local * rcp_approx_f((float)width));
-  int rem = (int)(local - ry * (uint32_t)width);
+  int rem = (int)(local - ry * width);
   if (rem < 0) {
     ry -= 1u;
-    rem += width;
-  } else if (rem >= width) {
+    rem += (int)width;
+  } else if (rem >= (int)width) {
     ry += 1u;
-    rem -= width;
+    rem -= (int)width;
   }
   uint32_t keys[kEmitPerThread], vals[kEmitPerThread];
-  const uint32_t slot_limit = kPerView ? (uint32_t)kSlots : 1u;
 #pragma unroll
   for (int k = 0; k < kEmitPerThread; ++k) {
     const uint32_t o = o0 + (uint32_t)k;
     const bool ok = o < o_hi;
     if (k > 0 && ok) {
-      // past Gaussian j: on to the next one that has instances, whose first instance o is (j stays
-      // below n even after an inconsistent scan, which the status word reports)
+      // past Gaussian j: on to the next one that has pairs, whose first pair o is (j stays below n even
+      // after an inconsistent scan, which the status word reports)
       if (o >= end_j && j + 1u < n) {
         do {
           ++j;
@@ -652,36 +665,31 @@ __global__ void __launch_bounds__(kScanBlock) instance_emit_kernel(const __grid_
         load_rect(j);
         ry = 0;
         rem = 0;
-      } else if (++rem == width) {
+      } else if (++rem == (int)width) {
         rem = 0;
         ++ry;
       }
     }
-    int tx = col0 + rem;
-    if (tx < 0) tx += pitch;  // seam wrap: columns left of 0 or right of gx - 1
-    if (tx >= pitch) tx -= pitch;
-    const uint32_t key = row_origin + ry * (uint32_t)pitch + (uint32_t)tx;
+    uint32_t col = bins.col + (uint32_t)rem;
+    if (col >= (uint32_t)bx) col -= (uint32_t)bx;  // the seam wraps
+    const uint32_t row = bins.row + ry;
+    const uint32_t key = ((p.grid.bin_base[view] + row * (uint32_t)bx + col) << kPairBinShift) |
+                         tile_mask((int)col * kBinW, (int)row * kBinH, gx, p.grid.seam_wrap != 0, rect);
     keys[k] = key;
     vals[k] = rec;
-    // digit histograms of the tile sort (the pass that would otherwise re-read every key)
-    const uint32_t slot = kPerView ? view - view0 : 0u;
-    const bool counted = ok && slot < slot_limit;
-    const unsigned live = __ballot_sync(kFullMask, counted);
+    // digit histograms of the bin sort (the pass that would otherwise re-read every key)
+    const unsigned live = __ballot_sync(kFullMask, ok);
 #pragma unroll
     for (int q = 0; q < kTilePasses; ++q)
-      if (q < p.hist_passes) {
-        const uint32_t digit = (key >> p.hist_shift[q]) & p.hist_mask[q];
-        count_digit(s_hist, slot * kHistSlot + q * kRadix + digit, counted, live, lane);
-        if (kPerView && ok && !counted)
-          atomicAdd(&p.hist[(size_t)view * kHistSlot + q * kRadix + digit], 1u);
-      }
+      if (q < p.hist_passes)
+        count_digit(s_hist, q * kRadix + ((key >> p.hist_shift[q]) & p.hist_mask[q]), ok, live, lane);
   }
   // the thread's run of the list: 16-byte stores when it is whole (o0 is a multiple of 8, the
   // lists start 256-byte aligned)
   static_assert(kEmitPerThread == 8, "two 16-byte stores per array");
   if (o0 + (uint32_t)kEmitPerThread <= o_hi) {
-    uint4* kd = reinterpret_cast<uint4*>(p.tkeys + o0);
-    uint4* vd = reinterpret_cast<uint4*>(p.tvals + o0);
+    uint4* kd = reinterpret_cast<uint4*>(p.keys + o0);
+    uint4* vd = reinterpret_cast<uint4*>(p.vals + o0);
     kd[0] = make_uint4(keys[0], keys[1], keys[2], keys[3]);
     kd[1] = make_uint4(keys[4], keys[5], keys[6], keys[7]);
     vd[0] = make_uint4(vals[0], vals[1], vals[2], vals[3]);
@@ -690,56 +698,428 @@ __global__ void __launch_bounds__(kScanBlock) instance_emit_kernel(const __grid_
 #pragma unroll
     for (int k = 0; k < kEmitPerThread; ++k)
       if (o0 + (uint32_t)k < o_hi) {
-        p.tkeys[o0 + k] = keys[k];
-        p.tvals[o0 + k] = vals[k];
+        p.keys[o0 + k] = keys[k];
+        p.vals[o0 + k] = vals[k];
       }
   }
   if (p.hist_passes == 0) return;
   __syncthreads();
-  for (int k = threadIdx.x; k < kSlots * kHistSlot; k += kScanBlock) {
+  for (int k = threadIdx.x; k < kTilePasses * kRadix; k += kScanBlock) {
     const uint32_t c = s_hist[k];
-    if (c == 0) continue;
-    if (kPerView)
-      atomicAdd(&p.hist[(size_t)(view0 + (uint32_t)(k / kHistSlot)) * kHistSlot + (k % kHistSlot)], c);
-    else
-      atomicAdd(&p.hist[k], c);
+    if (c) atomicAdd(&p.hist[k], c);
   }
 }
 
-// ---------------------------------------------------------------- tile ranges -----------------
-// A thread takes kRangesPer consecutive keys (two 16-byte loads) and the key before them, so every
-// load of the pass is in flight at once (one key per thread and iteration measured latency-bound:
-// 25 us for the 33 MB of a 1M-Gaussian view).
-constexpr int kRangesPer = 8;
+// ---------------------------------------------------------------- depth order by counting -----
+// A Gaussian's place in the (depth bits, index) order is the number of Gaussians before it.  A block has
+// kRankItems of them; its threads share the view's keys, and each compares its keys with all of the
+// block's, so a key is loaded once per block and nothing is staged.  Keys at lower indices count when
+// they are <= a Gaussian's, that is when the float below them is <; keys at higher ones when they are <.
+//
+// Bound by issue: P^2 comparisons.  An integer comparison and a predicated add both go to the ALU's 16
+// lanes (22 us for 10,000 Gaussians); here a comparison is sat(2^40 own - 2^40 key) and an add, both on
+// the FMA pipes: a key >= 2^-3 (depths are beyond the near cull at 0.2) differs from another by at least
+// 2^-26, so the difference is 0 or beyond 1 and the saturated value exactly 0 or 1, whatever its
+// rounding; culled Gaussians' infinite keys become 2^70, beyond any finite distance (at most 2^64).
+constexpr int kRankThreads = 256;
+constexpr int kRankItems = 16;
+static_assert(kRankItems * kRankItems == kRankThreads, "a thread per pair of the block's own Gaussians");
+static_assert(kRankMaxP < (1 << 24), "the counts are exact in float");
 
-__global__ void __launch_bounds__(256) ranges_kernel(RangesParams p) {
-  const uint32_t L = item_count(p.hdr, 0u, p.capacity);
-  const uint32_t stride = gridDim.x * blockDim.x * (uint32_t)kRangesPer;
-  for (uint32_t i0 = (blockIdx.x * blockDim.x + threadIdx.x) * (uint32_t)kRangesPer; i0 < L; i0 += stride) {
-    uint32_t k[kRangesPer + 1];  // k[0]: the key before i0
-    k[0] = i0 > 0 ? p.keys[i0 - 1] : 0u;
-    if (i0 + kRangesPer <= L) {  // i0 is a multiple of 8 and the list starts 256-byte aligned
-      const uint4 a = *reinterpret_cast<const uint4*>(p.keys + i0);
-      const uint4 b = *reinterpret_cast<const uint4*>(p.keys + i0 + 4);
-      k[1] = a.x, k[2] = a.y, k[3] = a.z, k[4] = a.w, k[5] = b.x, k[6] = b.y, k[7] = b.z, k[8] = b.w;
-    } else {
+__device__ __forceinline__ float fma_sat(float a, float b, float c) {
+  float r;
+  asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+
+__global__ void __launch_bounds__(kRankThreads) rank_kernel(const __grid_constant__ RankParams p) {
+  chain_begin();
+  __shared__ uint32_t s_rank[kRankItems];
+  const uint32_t P = (uint32_t)p.grid.P, view = blockIdx.y;
+  const uint32_t* keys = p.keys + (size_t)view * P;
+  const uint32_t j0 = blockIdx.x * (uint32_t)kRankItems;
+  if (threadIdx.x < kRankItems) s_rank[threadIdx.x] = 0;
+  const float far = 0x1p70f, scale = 0x1p40f;
+  float own[kRankItems], rank[kRankItems];
 #pragma unroll
-      for (int j = 0; j < kRangesPer; ++j) k[j + 1] = i0 + j < L ? p.keys[i0 + j] : 0u;
-    }
+  for (int q = 0; q < kRankItems; ++q) {
+    own[q] = j0 + q < P ? fminf(__uint_as_float(keys[j0 + q]), far) : 0.f;
+    rank[q] = 0.f;
+  }
+#pragma unroll 8
+  for (uint32_t i = threadIdx.x; i < P; i += kRankThreads) {
+    const uint32_t bits = __float_as_uint(fminf(__uint_as_float(keys[i]), far));
+    float neg = -scale * __uint_as_float(bits - (i < j0 ? 1u : 0u));
+    if (i - j0 < (uint32_t)kRankItems) neg = -0x1p126f;  // (the block's own: below)
 #pragma unroll
-    for (int j = 0; j < kRangesPer; ++j) {
-      const uint32_t idx = i0 + (uint32_t)j;
-      const uint32_t cur = k[j + 1], prev = k[j];
-      if (idx >= L || cur >= p.num_tiles) continue;  // keys always hold valid tile ids; never index past the table
-      if (idx == 0)
-        p.ranges[cur].x = 0;
-      else if (cur != prev) {
-        if (prev < p.num_tiles) p.ranges[prev].y = idx;
-        p.ranges[cur].x = idx;
-      }
-      if (idx == L - 1) p.ranges[cur].y = L;
+    for (int q = 0; q < kRankItems; ++q) rank[q] += fma_sat(own[q], scale, neg);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < kRankItems; ++q) {
+    const uint32_t sum = __reduce_add_sync(kFullMask, (uint32_t)rank[q]);
+    if ((threadIdx.x & 31) == 0 && sum) atomicAdd(&s_rank[q], sum);
+  }
+  {
+    const uint32_t a = j0 + threadIdx.x / kRankItems, c = j0 + threadIdx.x % kRankItems;
+    if (a < P && c < P) {
+      const uint32_t ka = keys[a], kc = keys[c];
+      if (kc < ka || (kc == ka && c < a)) atomicAdd(&s_rank[threadIdx.x / kRankItems], 1u);
     }
   }
+  __syncthreads();
+  const uint32_t j = j0 + threadIdx.x;
+  if (threadIdx.x < kRankItems && j < P) {
+    const uint32_t rec = view * P + j, at = view * P + s_rank[threadIdx.x];
+    const uint2 r = record_rect(p.grid, p.radii, p.splat, rec, view);
+    p.order[at] = rec;
+    p.rect_x[at] = r.x;
+    p.rect_y[at] = r.y;
+  }
+}
+
+// Tile rects in depth order, where the depth order comes from the sort and no scan needs them.
+__global__ void __launch_bounds__(256) rect_kernel(const __grid_constant__ RankParams p) {
+  const uint32_t i = blockIdx.x * 256u + threadIdx.x;
+  if (i >= (uint32_t)p.grid.P * (uint32_t)p.grid.V) return;
+  const uint2 r = record_rect(p.grid, p.radii, p.splat, p.order[i], record_view(p.grid, i));
+  p.rect_x[i] = r.x;
+  p.rect_y[i] = r.y;
+}
+
+// ---------------------------------------------------------------- tile lists ------------------
+// The fine stage works a warp at a time: a warp has one part of a bin's pairs (TileGrid::parts of them,
+// in order, eight to a block), counts its tiles' instances, and later, with the places that the scan
+// and the earlier parts' counts give it, appends the part to its tiles' lists.  No warp waits for another.
+constexpr int kListThreads = 32 * kListWarps;
+
+// A warp's part: the bin's tiles, and the pairs [first, end) of the bin's run of the sorted list, or (kAll)
+// of its view's whole depth order.
+struct BinPart {
+  int tx0, ty0;     // first tile column and row
+  int gx, gy;
+  uint32_t tile0;   // the view's first tile
+  uint32_t tiles;   // the view's tiles
+  uint32_t counts0; // the view's counts: [parts][tiles]
+  uint32_t part;    // parts or more: none
+  uint32_t parts;
+  uint32_t first, end;
+};
+
+// First index of the sorted words with a bin >= bin, by a warp (32 probes a step).
+__device__ __forceinline__ uint32_t warp_lower_bound(const uint32_t* words, uint32_t n, uint32_t bin) {
+  const uint32_t lane = threadIdx.x & 31;
+  uint32_t lo = 0, len = n;  // the answer lies in [lo, lo + len]
+  while (len > 0) {
+    const uint32_t step = (len + 31u) / 32u;
+    const bool below = lane * step < len && (words[lo + lane * step] >> kPairBinShift) < bin;
+    const uint32_t c = (uint32_t)__popc(__ballot_sync(kFullMask, below));  // probes 0 .. c - 1 are below
+    if (c == 0) return lo;
+    const uint32_t end = lo + len;
+    lo += (c - 1u) * step + 1u;
+    len = min(step - 1u, end - lo);
+  }
+  return lo;
+}
+
+template <bool kAll>
+__device__ __forceinline__ BinPart bin_part(const TileListParams& p) {
+  __shared__ uint32_t s_bounds[2];
+  const TileGrid& g = p.grid;
+  uint32_t view = 0;
+#pragma unroll 1
+  for (int v = 1; v < g.V; ++v)
+    if (g.block_base[v] <= blockIdx.x) view = (uint32_t)v;
+  BinPart b;
+  b.gx = g.gx[view];
+  b.gy = g.gy[view];
+  b.tile0 = g.tile_base[view];
+  b.tiles = (uint32_t)(b.gx * b.gy);
+  b.counts0 = g.count_base[view];
+  b.parts = g.parts[view];
+  const uint32_t per_bin = (b.parts + kListWarps - 1u) / kListWarps;  // blocks
+  const uint32_t block = blockIdx.x - g.block_base[view], local = block / per_bin;
+  b.part = (block - local * per_bin) * kListWarps + (threadIdx.x >> 5);
+  const uint32_t bx = (uint32_t)bins_x(b.gx);
+  b.ty0 = (int)(local / bx) * kBinH;
+  b.tx0 = (int)(local % bx) * kBinW;
+  uint32_t first, end;
+  if (kAll) {
+    first = view * (uint32_t)g.P;
+    end = first + (uint32_t)g.P;
+  } else {
+    const uint32_t n = pair_count(p.hdr, p.capacity);
+    if (threadIdx.x < 64) {
+      const uint32_t at = warp_lower_bound(p.words, n, g.bin_base[view] + local + (threadIdx.x >> 5));
+      if ((threadIdx.x & 31) == 0) s_bounds[threadIdx.x >> 5] = at;
+    }
+    __syncthreads();
+    first = s_bounds[0];
+    end = s_bounds[1];
+  }
+  // (parts of whole groups of 32)
+  const uint32_t len = ((end - first + b.parts - 1u) / b.parts + 31u) & ~31u;
+  b.first = (uint32_t)min((unsigned long long)end, first + (unsigned long long)b.part * len);
+  b.end = min(end, b.first + len);
+  return b;
+}
+
+// The tiles of pair e in the bin (the low bits of a pair's word).
+template <bool kAll>
+__device__ __forceinline__ uint32_t pair_tiles(const TileListParams& p, const BinPart& b, uint32_t e) {
+  return kAll ? tile_mask(b.tx0, b.ty0, b.gx, p.grid.seam_wrap != 0, make_uint2(p.rect_x[e], p.rect_y[e])) : p.words[e];
+}
+
+// The bits of a nibble as the low bits of four bytes (bit k in byte k): with a tile row's eight columns in
+// two such words, a warp counts and ranks all eight tiles with additions.
+__device__ __forceinline__ uint32_t spread4(uint32_t nibble) { return (nibble * 0x00204081u) & 0x01010101u; }
+
+// Counts of a bin's tiles over a part of its pairs: every lane keeps the 32 tiles' counts as bytes in
+// eight words (at most 255 pairs a lane between sums), which the warp then adds as halfwords.  Every tile
+// of the grid is written (0 when the instances do not fit).  (A ballot and a popcount per tile and 32
+// pairs took 38 us of the 1M-Gaussian view instead of 15.)
+template <bool kAll>
+__global__ void __launch_bounds__(kListThreads) tile_count_kernel(const __grid_constant__ TileListParams p) {
+  chain_begin();
+  const int lane = threadIdx.x & 31;
+  const bool fit = instances_fit(p.hdr, p.capacity);
+  if (kAll && !fit && blockIdx.x == 0 && threadIdx.x == 0)
+    atomicOr(&p.hdr->status, kStatusCapacity);  // (the scan flags it where there is one)
+  BinPart b = bin_part<kAll>(p);
+  if (b.part >= b.parts) return;
+  if (!fit) b.end = b.first;
+  uint32_t acc[kBinH][2] = {};
+  uint32_t mine = 0;  // instances of tile (lane / 8, lane % 8)
+  // adds the warp's bytes: tile 8 r + 4 h + k is byte k of acc[r][h]
+  auto flush = [&] {
+#pragma unroll
+    for (int r = 0; r < kBinH; ++r)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const uint32_t even = __reduce_add_sync(kFullMask, acc[r][h] & 0x00ff00ffu);        // bytes 0 and 2
+        const uint32_t odd = __reduce_add_sync(kFullMask, (acc[r][h] >> 8) & 0x00ff00ffu);  // bytes 1 and 3
+        if (lane >> 2 == 2 * r + h) {
+          const uint32_t w = lane & 1 ? odd : even;
+          mine += lane & 2 ? w >> 16 : w & 0xffffu;
+        }
+        acc[r][h] = 0u;
+      }
+  };
+  int steps = 0;
+#pragma unroll 4
+  for (uint32_t e0 = b.first; e0 < b.end; e0 += 32) {
+    const uint32_t mask = e0 + lane < b.end ? pair_tiles<kAll>(p, b, e0 + lane) : 0u;
+    const uint32_t lo = spread4(mask & 15u), hi = spread4((mask >> 4) & 15u);
+#pragma unroll
+    for (int r = 0; r < kBinH; ++r) {
+      const uint32_t on = (mask >> (kBinW + r)) & 1u;
+      acc[r][0] += lo * on;
+      acc[r][1] += hi * on;
+    }
+    if (++steps == 255) {
+      flush();
+      steps = 0;
+    }
+  }
+  if (steps) flush();
+  const int tx = b.tx0 + lane % kBinW, ty = b.ty0 + lane / kBinW;
+  if (tx < b.gx && ty < b.gy) {
+    const uint32_t t = (uint32_t)(ty * b.gx + tx);
+    if (p.counts == nullptr) {
+      p.ranges[b.tile0 + t].x = mine;
+    } else {
+      p.counts[b.counts0 + (size_t)b.part * b.tiles + t] = mine;
+      if (mine) atomicAdd(&p.totals[b.tile0 + t], mine);
+    }
+  }
+}
+
+// Tile ranges from the totals, in tile order, kTileScanBlock tiles a block: a block first sums the
+// totals before its own (without them, a single block walks all tiles and replaces the counts in the
+// ranges).  An empty tile's range is (0, 0), as the reference leaves it.
+constexpr int kTileScanThreads = 1024;
+constexpr int kTileScanItems = 8;
+constexpr uint32_t kTileScanBlock = kTileScanThreads * kTileScanItems;
+
+__global__ void __launch_bounds__(kTileScanThreads) tile_scan_kernel(const __grid_constant__ TileListParams p) {
+  chain_begin();
+  __shared__ uint32_t s_warp[32];
+  __shared__ uint32_t s_before;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t n = p.grid.num_tiles;
+  const uint32_t* totals = p.counts ? p.totals : nullptr;
+  const uint32_t begin = blockIdx.x * kTileScanBlock;
+  if (threadIdx.x == 0) s_before = 0;
+  __syncthreads();
+  uint32_t before = 0;
+#pragma unroll 8
+  for (uint32_t i = threadIdx.x; i < begin; i += kTileScanThreads) before += totals[i];
+  before = __reduce_add_sync(kFullMask, before);
+  if (lane == 0 && before) atomicAdd(&s_before, before);
+  __syncthreads();
+  uint32_t carry = s_before;
+  for (uint32_t base = begin; base < n; base += kTileScanBlock) {
+    const uint32_t t0 = base + threadIdx.x * kTileScanItems;
+    uint32_t c[kTileScanItems], sum = 0;
+#pragma unroll
+    for (int u = 0; u < kTileScanItems; ++u) c[u] = t0 + u < n ? (totals ? totals[t0 + u] : p.ranges[t0 + u].x) : 0u;
+#pragma unroll
+    for (int u = 0; u < kTileScanItems; ++u) sum += c[u];
+    uint32_t x = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(kFullMask, x, o);
+      if (lane >= o) x += y;
+    }
+    if (lane == 31) s_warp[warp] = x;
+    __syncthreads();
+    if (warp == 0) {
+      uint32_t w = s_warp[lane];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFullMask, w, o);
+        if (lane >= o) w += y;
+      }
+      s_warp[lane] = w;
+    }
+    __syncthreads();
+    uint32_t at = carry + x - sum + (warp > 0 ? s_warp[warp - 1] : 0u);
+#pragma unroll
+    for (int u = 0; u < kTileScanItems; ++u)
+      if (t0 + u < n) {
+        p.ranges[t0 + u] = c[u] ? make_uint2(at, at + c[u]) : make_uint2(0u, 0u);
+        at += c[u];
+      }
+    carry += s_warp[31];
+    if (totals) break;  // (the next tiles are another block's)
+    __syncthreads();
+  }
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0 && instances_fit(p.hdr, p.capacity) && carry != p.hdr->num_rendered)
+    atomicOr(&p.hdr->status, kStatusInconsistent);
+}
+
+// Appends a part of a bin's pairs to the lists of its 32 tiles.  A warp queues its pairs by the bin's four
+// tile rows (a pair covers one or two of them on average, so a walk per row would waste most lanes) and
+// appends 32 of a row at a time to its eight lists: a pair's place is the list's next one plus the
+// queued pairs before it that cover the tile, from a warp scan of the eight columns as bytes.  Bound by
+// issue.  Measured on a B200 (1M-Gaussian view / 16-view batch): a block per tile row, walking all of the
+// bin's pairs with ballots and popcounts per tile, 88 / 1262 us; byte scans there 75 / 967; this
+// 37 / 392 us.
+struct FillQueue {
+  uint32_t cols[kBinH][64], rec[kBinH][64];  // queued pairs of a row: columns, record
+  __align__(16) uint32_t next[32];           // next free place of every tile's list
+};
+
+template <bool kAll>
+__global__ void __launch_bounds__(kListThreads) tile_fill_kernel(const __grid_constant__ TileListParams p) {
+  chain_begin();
+  __shared__ FillQueue s_queue[kListWarps];
+  if (!instances_fit(p.hdr, p.capacity)) return;
+  const BinPart b = bin_part<kAll>(p);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned lt = (1u << lane) - 1u;
+  FillQueue& q = s_queue[warp];
+  {  // the lists' next places: the range's start and the earlier parts' counts, which the warps share
+    __shared__ uint32_t s_sum[kListWarps][32], s_own[kListWarps][32];
+    const int tx = b.tx0 + lane % kBinW, ty = b.ty0 + lane / kBinW;
+    uint32_t start = 0, sum = 0, own = 0;
+    bool safe = true;
+    if (tx < b.gx && ty < b.gy) {
+      const uint32_t t = (uint32_t)(ty * b.gx + tx);
+      const uint2 range = p.ranges[b.tile0 + t];
+      start = range.x;
+      safe = range.y <= (uint64_t)p.capacity;  // (always, after a consistent scan)
+      if (b.parts > 1) {
+        const uint32_t* c = p.counts + b.counts0 + t;
+        const uint32_t block = b.part - (uint32_t)warp;  // the block's first part
+#pragma unroll 4
+        for (uint32_t i = (uint32_t)warp; i < block; i += kListWarps) sum += c[(size_t)i * b.tiles];
+        if (b.part < b.parts) own = c[(size_t)b.part * b.tiles];
+      }
+    }
+    s_sum[warp][lane] = sum;
+    s_own[warp][lane] = own;
+    __syncthreads();
+    if (b.part >= b.parts || b.first >= b.end || !__all_sync(kFullMask, safe)) return;
+#pragma unroll
+    for (int w = 0; w < kListWarps; ++w) start += s_sum[w][lane] + (w < warp ? s_own[w][lane] : 0u);
+    q.next[lane] = start;
+  }
+  uint32_t queued[kBinH] = {};  // warp-uniform
+  // appends the first min(n, 32) pairs queued for a row
+  auto append = [&](int row, uint32_t n) {
+    __syncwarp();
+    const uint32_t m = (uint32_t)lane < n ? q.cols[row][lane] : 0u, rec = q.rec[row][lane];
+    uint32_t lo = spread4(m & 15u), hi = spread4(m >> 4);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t x = __shfl_up_sync(kFullMask, lo, o), y = __shfl_up_sync(kFullMask, hi, o);
+      if (lane >= o) {
+        lo += x;
+        hi += y;
+      }
+    }
+    const uint4 n0 = *reinterpret_cast<const uint4*>(&q.next[row * kBinW]);
+    const uint4 n1 = *reinterpret_cast<const uint4*>(&q.next[row * kBinW + 4]);
+    const uint32_t next[kBinW] = {n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, n1.z, n1.w};
+    const uint32_t all_lo = __shfl_sync(kFullMask, lo, 31), all_hi = __shfl_sync(kFullMask, hi, 31);
+    __syncwarp();
+    if (lane < kBinW) q.next[row * kBinW + lane] += ((lane < 4 ? all_lo : all_hi) >> (8 * (lane & 3))) & 255u;
+#pragma unroll
+    for (int k = 0; k < kBinW; ++k)
+      if ((m >> k) & 1u) p.out_vals[next[k] + (((k < 4 ? lo : hi) >> (8 * (k & 3))) & 255u) - 1u] = rec;
+  };
+  uint32_t mask = 0, rec = 0;
+  auto load = [&](uint32_t e) {
+    mask = 0;
+    if (e < b.end) {
+      mask = pair_tiles<kAll>(p, b, e);
+      rec = kAll ? p.order[e] : p.recs[e];
+    }
+  };
+  load(b.first + lane);
+  uint32_t mask1 = mask, rec1 = rec;  // two groups ahead
+  load(b.first + 32 + lane);
+  for (uint32_t e0 = b.first; e0 < b.end; e0 += 32) {
+    const uint32_t m = mask1, r = rec1;
+    mask1 = mask, rec1 = rec;
+    load(e0 + 64 + lane);
+#pragma unroll
+    for (int row = 0; row < kBinH; ++row) {
+      const bool in = (m >> (kBinW + row)) & 1u && (m & 255u);
+      const unsigned bal = __ballot_sync(kFullMask, in);
+      if (in) {
+        const uint32_t at = queued[row] + (uint32_t)__popc(bal & lt);
+        q.cols[row][at] = m & 255u;
+        q.rec[row][at] = r;
+      }
+      queued[row] += (uint32_t)__popc(bal);
+      if (queued[row] >= 32) {
+        append(row, 32);
+        queued[row] -= 32;
+        __syncwarp();
+        const uint32_t c = q.cols[row][32 + lane], x = q.rec[row][32 + lane];  // the rest moves to the front
+        __syncwarp();
+        if ((uint32_t)lane < queued[row]) {
+          q.cols[row][lane] = c;
+          q.rec[row][lane] = x;
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int row = 0; row < kBinH; ++row)
+    if (queued[row]) append(row, queued[row]);
+}
+
+// The sorted tile ids, which only the inspection of a pass reads: a warp per tile writes its range.
+__global__ void __launch_bounds__(256) tile_keys_kernel(const __grid_constant__ TileListParams p) {
+  chain_begin();
+  const uint32_t tile = blockIdx.x * 8u + (threadIdx.x >> 5);
+  if (tile >= p.grid.num_tiles || !instances_fit(p.hdr, p.capacity)) return;
+  const uint2 r = p.ranges[tile];
+  if (r.y > (uint64_t)p.capacity) return;
+  for (uint32_t i = r.x + (threadIdx.x & 31); i < r.y; i += 32) p.out_keys[i] = tile;
 }
 
 int sm_count() {
@@ -761,47 +1141,58 @@ void launch_histogram(const HistParams& p, int64_t max_items, cudaStream_t s) {
 }
 
 void launch_onesweep(const OnesweepParams& p, int64_t max_items, cudaStream_t s) {
-  // variable segments: each segment's last tile may be partial, so up to num_segs extra tiles
-  const int64_t blocks = p.seg_counts ? sort_tiles(max_items) + (int64_t)p.num_segs
-                         : p.seg_len  ? sort_tiles(p.seg_len) * (int64_t)p.num_segs
-                                      : sort_tiles(max_items);
+  if (p.seg_len && small_sort(p.seg_len, p.num_segs)) {  // (the depth sort: its look-back words have room)
+    onesweep_kernel<kSmallSortItems, 5, 16><<<(unsigned)sort_blocks(p.seg_len, p.num_segs), kSortThreads, 0, s>>>(p);
+    return;
+  }
+  const int64_t blocks = p.seg_len ? sort_tiles(p.seg_len) * (int64_t)p.num_segs : sort_tiles(max_items);
   if (blocks <= 0) return;
-  if (p.seg_counts)
-    onesweep_kernel<true><<<(unsigned)blocks, kSortThreads, 0, s>>>(p);
-  else
-    onesweep_kernel<false><<<(unsigned)blocks, kSortThreads, 0, s>>>(p);
+  onesweep_kernel<kSortItems, 3, kLookbackBatch><<<(unsigned)blocks, kSortThreads, 0, s>>>(p);
+}
+
+void launch_rects(const RankParams& p, cudaStream_t s) {
+  const int64_t items = (int64_t)p.grid.P * p.grid.V;
+  if (items <= 0) return;
+  rect_kernel<<<(unsigned)((items + 255) / 256), 256, 0, s>>>(p);
+}
+
+void launch_begin_binning(const BeginParams& p, cudaStream_t s) {
+  size_t total = 0;
+  for (size_t b : p.bytes) total += b / 16;
+  const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((int64_t)(total + 1023) / 1024, (int64_t)sm_count() * 8));
+  launch_chained(p.chained, begin_binning_kernel, (unsigned)blocks, 256, 0, s, p);
+}
+
+void launch_rank(const RankParams& p, cudaStream_t s) {
+  if (p.grid.P <= 0) return;
+  const dim3 grid((unsigned)(p.grid.P + kRankItems - 1) / kRankItems, (unsigned)p.grid.V);
+  launch_chained(p.chained, rank_kernel, grid, kRankThreads, 0, s, p);
 }
 
 void launch_duplicate(const DuplicateParams& p, cudaStream_t s) {
-  const int64_t items = (int64_t)p.P * p.V;
+  const int64_t items = (int64_t)p.grid.P * p.grid.V;
   if (items <= 0) return;
   const int64_t tiles = (items + kScanTile - 1) / kScanTile;
   if (tiles <= (int64_t)p.skip_tiles) return;
   // scan: one block per scan tile that is taken (block k takes tile skip_tiles + k)
-  const unsigned blocks = (unsigned)(tiles - p.skip_tiles);
-  if (p.hist_per_view)
-    instance_scan_kernel<true><<<blocks, kScanBlock, 0, s>>>(p);
-  else
-    instance_scan_kernel<false><<<blocks, kScanBlock, 0, s>>>(p);
-  // emit: one block per kEmitBlock instances the binning buffer can hold (blocks past the device's
-  // instance count return at once); a probe pass stops after the scan
+  pair_scan_kernel<<<(unsigned)(tiles - p.skip_tiles), kScanBlock, 0, s>>>(p);
+  // emit: one block per kEmitBlock pairs the binning buffer can hold (blocks past the device's pair
+  // count return at once); a probe pass stops after the scan
   if (p.skip_tiles != 0) return;
   const int64_t eblocks = emit_blocks(std::min<int64_t>(p.capacity, 0xffffffffll));
   if (eblocks <= 0) return;
-  if (p.hist_per_view)
-    instance_emit_kernel<true><<<(unsigned)eblocks, kScanBlock, 0, s>>>(p);
-  else
-    instance_emit_kernel<false><<<(unsigned)eblocks, kScanBlock, 0, s>>>(p);
+  pair_emit_kernel<<<(unsigned)eblocks, kScanBlock, 0, s>>>(p);
 }
 
-void launch_ranges(const RangesParams& p, cudaStream_t s) {
-  if (p.capacity <= 0) return;
-  // enough threads for one group of keys each at the capacity (the blocks past the device count
-  // return at once), at most 16 waves of 8 blocks per SM
-  const int64_t per_block = 256 * kRangesPer;
-  const int64_t blocks = std::max<int64_t>(
-      1, std::min<int64_t>((p.capacity + per_block - 1) / per_block, (int64_t)sm_count() * 8 * 16));
-  ranges_kernel<<<(unsigned)blocks, 256, 0, s>>>(p);
+void launch_tile_lists(const TileListParams& p, cudaStream_t s) {
+  const TileGrid& g = p.grid;
+  if (g.num_blocks == 0) return;
+  const bool all = p.words == nullptr;
+  launch_chained(p.chained, all ? tile_count_kernel<true> : tile_count_kernel<false>, g.num_blocks, kListThreads, 0, s, p);
+  const unsigned scan = p.counts ? (g.num_tiles + kTileScanBlock - 1) / kTileScanBlock : 1u;
+  launch_chained(p.chained, tile_scan_kernel, scan, kTileScanThreads, 0, s, p);
+  launch_chained(p.chained, all ? tile_fill_kernel<true> : tile_fill_kernel<false>, g.num_blocks, kListThreads, 0, s, p);
+  launch_chained(p.chained, tile_keys_kernel, (g.num_tiles + 7) / 8, 256, 0, s, p);
 }
 
 }  // namespace omnigs

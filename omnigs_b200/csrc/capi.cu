@@ -1,6 +1,7 @@
 // C-ABI entry points (include/omnigs_b200.h): argument validation, buffer carving and kernel
 // sequencing for one lonlat rasterization.  Replaces the host orchestration of
 // CudaRasterizer::LonlatRasterizer (rasterizer_impl.cu:540-795) without its mid-pass host sync.
+#include <algorithm>
 #include <atomic>
 #include <cstdio>
 #include <cstring>
@@ -47,16 +48,200 @@ cudaEvent_t take_event() {
   return e;
 }
 
-__global__ void begin_render_kernel(GeomHeader* hdr) {
-  atomicAnd(&hdr->status, ~(kStatusCapacity | kStatusInconsistent));
-  const unsigned long long total = hdr->num_rendered64;
-  if (total > (unsigned long long)kMaxInstances) atomicOr(&hdr->status, kStatusOverflow);
-  hdr->num_rendered = (uint32_t)(total > 0xffffffffull ? 0xffffffffull : total);
-  hdr->dup_tile_counter = 0;
-  for (int i = 0; i < kMaxSortPasses; ++i) hdr->sort_tile_counter[i] = 0;
-}
+int run_binning(BinningPass& b, cudaStream_t s) {
+  TileGrid& g = b.grid;
+  g.num_bins = 0;
+  for (int v = 0; v < g.V; ++v) {
+    g.bin_base[v] = g.num_bins;
+    g.num_bins += (uint32_t)bins_x(g.gx[v]) * (uint32_t)bins_y(g.gy[v]);
+  }
+  const BinningLayout& L = b.layout;
+  const int64_t records = (int64_t)g.P * g.V;
+  const bool probe = b.max_spins > 0;
+  // few Gaussians: the depth order by counting (kRankMaxP); few pairs of a Gaussian and a bin: no coarse
+  // lists, every bin reads the whole order (kWholeMaxPairs)
+  const bool ranked = !probe && g.P <= kRankMaxP;
+  const bool whole = !probe && (int64_t)g.num_bins * g.P <= kWholeMaxPairs;
+  b.small = ranked && whole;
+  TileDigits digits = TileDigits::from_bits(id_bits(g.num_bins));  // of the bin in a pair's word
+  const int64_t pair_tiles = sort_tiles(L.capacity);
+  uint32_t* hist = at<uint32_t>(b.binning, L.hist);
 
-void launch_begin_render(GeomHeader* hdr, cudaStream_t s) { begin_render_kernel<<<1, 1, 0, s>>>(hdr); }
+  // The fine stage's parts, as many as their counts have room for beside the tiles' totals: in the depth
+  // sort's first key buffer and the two buffers behind it (the rects, which the coarse stage has read);
+  // without a coarse stage, in the pairs' buffer or the key buffer alone, whichever is larger.
+  uint32_t* scratch = b.dkeys[0];
+  int64_t room = 3 * records - g.num_tiles;
+  if (whole) {
+    room = std::max(records, L.capacity) - g.num_tiles;
+    if (L.capacity > records) scratch = at<uint32_t>(b.binning, b.out ? L.tkeys0 : L.tkeys1);
+  }
+  const int64_t cap = std::max<int64_t>(1, std::min<int64_t>(kMaxListParts, room / g.num_tiles));
+  uint32_t blocks = 0, count_words = 0;
+  for (int v = 0; v < g.V; ++v) {
+    const int64_t bins = (int64_t)bins_x(g.gx[v]) * bins_y(g.gy[v]);
+    const int64_t run = whole ? g.P : (3 * (int64_t)g.P / 2 + bins - 1) / bins;
+    g.parts[v] = (uint32_t)std::max<int64_t>(1, std::min<int64_t>(cap, (run + kListPart - 1) / kListPart));
+    g.block_base[v] = blocks;
+    g.count_base[v] = count_words;
+    blocks += (uint32_t)bins * ((g.parts[v] + kListWarps - 1) / kListWarps);
+    count_words += g.parts[v] * (uint32_t)(g.gx[v] * g.gy[v]);
+  }
+  g.num_blocks = blocks;
+  uint32_t* counts = room >= (int64_t)g.num_tiles ? scratch : nullptr;
+  // the totals: in the look-back words of the passes that the bin sort does not have, cleared with the
+  // others; else behind the counts, cleared on their own
+  const int64_t lookback_words = kTilePasses * pair_tiles * kRadix;
+  uint32_t* totals = at<uint32_t>(b.binning, L.tile_lookback) + digits.passes * pair_tiles * kRadix;
+  const bool totals_there = lookback_words - digits.passes * pair_tiles * kRadix >= (int64_t)g.num_tiles + 4;
+  if (!totals_there) totals = scratch + count_words;
+
+  BeginParams begin{};
+  begin.hdr = b.hdr;
+  begin.chained = b.small;
+  if (!b.small) {
+    begin.region[0] = b.zero;
+    begin.bytes[0] = b.zero_bytes;
+    begin.region[1] = at<uint4>(b.binning, L.hist);
+    begin.bytes[1] = sizeof(uint32_t) * kMaxSortPasses * kRadix;
+  }
+  if (!whole) {
+    begin.region[2] = at<uint4>(b.binning, L.tile_lookback);
+    begin.bytes[2] = sizeof(uint32_t) * digits.passes * pair_tiles * kRadix;
+  }
+  if (counts != nullptr && totals_there) {
+    begin.region[3] = reinterpret_cast<uint4*>(totals);
+    begin.bytes[3] = (sizeof(uint32_t) * g.num_tiles + 15) / 16 * 16;
+  }
+  staged(OMNIGS_STAGE_OTHER, 1, s, [&] { launch_begin_binning(begin, s); });
+
+  const uint32_t* depth_keys = reinterpret_cast<const uint32_t*>(b.depth);
+  uint32_t* keys[2] = {at<uint32_t>(b.binning, L.tkeys0), at<uint32_t>(b.binning, L.tkeys1)};
+  uint32_t* vals[2] = {at<uint32_t>(b.binning, L.tvals0), at<uint32_t>(b.binning, L.tvals1)};
+  // the depth order ends in dvals[1]; the sort's other buffers hold the pair offsets and the tile rects
+  static_assert(((kDepthPasses - 1) & 1) == 1, "the depth order is in dvals[1]");
+  uint32_t* order = b.dvals[1];
+  uint32_t *incl = b.dkeys[0], *rect_x = b.dvals[0], *rect_y = b.dkeys[1];
+  TileListParams t{};
+  RankParams r{};
+  r.grid = g;
+  r.keys = depth_keys;
+  r.radii = b.radii;
+  r.splat = b.splat;
+  r.order = order;
+  r.rect_x = rect_x;
+  r.rect_y = rect_y;
+  r.chained = b.small;
+  if (ranked) {
+    staged(OMNIGS_STAGE_SORT, 1, s, [&] { launch_rank(r, s); });
+  } else {
+    // 1. depth sort of every view's Gaussians: one segment per view, (depth bits, index) order
+    HistParams hd{};
+    hd.keys = depth_keys;
+    hd.n_host = (uint32_t)records;
+    hd.passes = kDepthPasses;
+    for (int q = 0; q < kDepthPasses; ++q) {
+      hd.shift[q] = kRadixBits * q;
+      hd.mask[q] = kRadix - 1;
+    }
+    hd.hist = b.depth_hist;
+    hd.seg_len = (uint32_t)g.P;
+    hd.num_segs = (uint32_t)g.V;
+    staged(OMNIGS_STAGE_SORT, 1, s, [&] { launch_histogram(hd, records, s); });
+    const int64_t depth_tiles = sort_blocks(g.P, g.V);
+    for (int q = 0; q < kDepthPasses; ++q) {
+      OnesweepParams op{};
+      op.keys_in = q == 0 ? depth_keys : b.dkeys[(q + 1) & 1];
+      op.vals_in = q == 0 ? nullptr : b.dvals[(q + 1) & 1];
+      op.keys_out = b.dkeys[q & 1];
+      op.vals_out = b.dvals[q & 1];
+      op.shift = kRadixBits * q;
+      op.mask = kRadix - 1;
+      op.n_host = (uint32_t)records;
+      op.hist = b.depth_hist + q * kRadix;
+      op.lookback = b.depth_lookback + (size_t)q * depth_tiles * kRadix;
+      op.tile_counter = &b.hdr->sort_tile_counter[q];
+      op.hdr = b.hdr;
+      op.seg_len = (uint32_t)g.P;
+      op.num_segs = (uint32_t)g.V;
+      op.hist_seg_stride = kDepthPasses * kRadix;
+      staged(OMNIGS_STAGE_SORT, 1, s, [&] { launch_onesweep(op, records, s); });
+    }
+
+  }
+  if (whole) {
+    if (!ranked) staged(OMNIGS_STAGE_DUPLICATE, 1, s, [&] { launch_rects(r, s); });
+  } else {
+    // 2. coarse lists: the pairs in that order, stably sorted by bin.  The sorted pairs end in the buffer
+    // that the tile lists do not go to.
+    const int sorted = b.out ^ 1, first = (sorted + digits.passes) & 1;
+    DuplicateParams d{};
+    d.grid = g;
+    d.radii = b.radii;
+    d.splat = b.splat;
+    d.order = order;
+    d.keys = keys[first];
+    d.vals = vals[first];
+    d.scan_state = b.scan_state;
+    d.incl = incl;
+    d.rect_x = rect_x;
+    d.rect_y = rect_y;
+    d.emit_first = at<uint32_t>(b.binning, L.emit_first);
+    d.emit_last = at<uint32_t>(b.binning, L.emit_last);
+    d.capacity = b.capacity;
+    d.hdr = b.hdr;
+    d.hist = hist + kDepthPasses * kRadix;
+    d.hist_passes = digits.passes;
+    for (int q = 0; q < digits.passes; ++q) {
+      digits.shift[q] += kPairBinShift;
+      d.hist_shift[q] = digits.shift[q];
+      d.hist_mask[q] = digits.mask[q];
+    }
+    if (probe) {
+      d.max_spins = b.max_spins;
+      d.skip_tiles = 1;
+    }
+    staged(OMNIGS_STAGE_DUPLICATE, 2, s, [&] { launch_duplicate(d, s); });
+    if (probe) return check_launch("duplicate (look-back probe)");
+    for (int q = 0; q < digits.passes; ++q) {
+      const int from = (first + q) & 1;
+      OnesweepParams op{};
+      op.keys_in = keys[from];
+      op.vals_in = vals[from];
+      op.keys_out = keys[from ^ 1];
+      op.vals_out = vals[from ^ 1];
+      op.shift = digits.shift[q];
+      op.mask = digits.mask[q];
+      op.count_hdr = b.hdr;
+      op.capacity = b.capacity;
+      op.hist = hist + (kDepthPasses + q) * kRadix;
+      op.lookback = at<uint32_t>(b.binning, L.tile_lookback) + (size_t)q * pair_tiles * kRadix;
+      op.tile_counter = &b.hdr->sort_tile_counter[kDepthPasses + q];
+      op.hdr = b.hdr;
+      staged(OMNIGS_STAGE_SORT, 1, s, [&] { launch_onesweep(op, b.capacity, s); });
+    }
+    t.words = keys[sorted];
+    t.recs = vals[sorted];
+  }
+
+  // 3. tile lists and ranges
+  t.grid = g;
+  t.chained = b.small;
+  t.order = order;
+  t.rect_x = rect_x;
+  t.rect_y = rect_y;
+  t.counts = counts;
+  t.totals = totals;
+  t.out_keys = keys[b.out];
+  t.out_vals = vals[b.out];
+  t.ranges = b.ranges;
+  t.capacity = b.capacity;
+  t.hdr = b.hdr;
+  if (counts != nullptr && !totals_there && cudaMemsetAsync(totals, 0, sizeof(uint32_t) * g.num_tiles, s) != cudaSuccess)
+    return check_launch("memset tile totals");
+  staged(OMNIGS_STAGE_RANGES, 4, s, [&] { launch_tile_lists(t, s); });
+  return check_launch("binning");
+}
 
 int check_aligned(const void* a, const void* b, const void* c) {
   for (const void* q : {a, b, c})
@@ -89,7 +274,7 @@ int validate_common(int P, int D, int M, int W, int H, const void* shs, const fl
 
 namespace {
 
-// Buffer (0 or 1) that holds the sorted tile ids / point list after the tile passes.
+// Buffer (0 or 1) that receives the sorted tile ids / point list.
 int tile_final(int W, int H) { return TileDigits::make(W, H).passes & 1; }
 
 int validate_forward(const OmnigsLonlatForwardArgs* a) {
@@ -270,119 +455,37 @@ int render_impl(const OmnigsLonlatForwardArgs* a, void* geom, size_t geom_bytes,
   const BinningLayout BL = BinningLayout::make(capacity);
   if (capacity > kMaxInstances) capacity = kMaxInstances;
   const int gx = tiles_x(a->W), gy = tiles_y(a->H);
-  const TileDigits td = TileDigits::make(a->W, a->H);
+  const int fin = tile_final(a->W, a->H);
   GeomHeader* hdr = at<GeomHeader>(geom, GL.header);
-  uint32_t* hist = at<uint32_t>(binning, BL.hist);
   uint2* ranges = at<uint2>(image, IL.ranges);
-  const int64_t depth_tiles = sort_tiles(a->P);
-  const int64_t inst_tiles = sort_tiles(BL.capacity);
 
-  staged(OMNIGS_STAGE_OTHER, 1, s, [&] { launch_begin_render(hdr, s); });
-  if (cudaMemsetAsync(at<unsigned char>(geom, GL.dup_scan), 0, GL.zero_end - GL.dup_scan, s) != cudaSuccess ||
-      cudaMemsetAsync(hist, 0, sizeof(uint32_t) * kMaxSortPasses * kRadix, s) != cudaSuccess ||
-      cudaMemsetAsync(at<uint32_t>(binning, BL.tile_lookback), 0,
-                      sizeof(uint32_t) * td.passes * inst_tiles * kRadix, s) != cudaSuccess ||
-      cudaMemsetAsync(ranges, 0, sizeof(uint2) * (size_t)gx * gy, s) != cudaSuccess)
-    return check_launch("memset binning state");
-
-  // 1. depth sort of the Gaussians: (depth bits, index) order
-  const uint32_t* depth_keys = at<uint32_t>(geom, GL.depth);
-  uint32_t* dkeys[2] = {at<uint32_t>(geom, GL.dkeys0), at<uint32_t>(geom, GL.dkeys1)};
-  uint32_t* dvals[2] = {at<uint32_t>(geom, GL.dvals0), at<uint32_t>(geom, GL.dvals1)};
-  HistParams hd{};
-  hd.keys = depth_keys;
-  hd.n_host = (uint32_t)a->P;
-  hd.passes = kDepthPasses;
-  for (int q = 0; q < kDepthPasses; ++q) {
-    hd.shift[q] = kRadixBits * q;
-    hd.mask[q] = kRadix - 1;
-  }
-  hd.hist = hist;
-  staged(OMNIGS_STAGE_SORT, 1, s, [&] { launch_histogram(hd, a->P, s); });
-  for (int q = 0; q < kDepthPasses; ++q) {
-    OnesweepParams op{};
-    op.keys_in = q == 0 ? depth_keys : dkeys[(q + 1) & 1];
-    op.vals_in = q == 0 ? nullptr : dvals[(q + 1) & 1];
-    op.keys_out = dkeys[q & 1];
-    op.vals_out = dvals[q & 1];
-    op.shift = kRadixBits * q;
-    op.mask = kRadix - 1;
-    op.n_host = (uint32_t)a->P;
-    op.hist = hist + q * kRadix;
-    op.lookback = at<uint32_t>(geom, GL.depth_lookback) + (size_t)q * depth_tiles * kRadix;
-    op.tile_counter = &hdr->sort_tile_counter[q];
-    op.hdr = hdr;
-    staged(OMNIGS_STAGE_SORT, 1, s, [&] { launch_onesweep(op, a->P, s); });
-  }
-  const uint32_t* order = dvals[(kDepthPasses - 1) & 1];
-
-  // 2. duplicate in that order (fused scan of the tile counts)
-  uint32_t* tkeys[2] = {at<uint32_t>(binning, BL.tkeys0), at<uint32_t>(binning, BL.tkeys1)};
-  uint32_t* tvals[2] = {at<uint32_t>(binning, BL.tvals0), at<uint32_t>(binning, BL.tvals1)};
-  DuplicateParams d{};
-  d.P = a->P;
-  d.V = 1;
-  d.gx[0] = gx;
-  d.gy[0] = gy;
-  d.tile_base[0] = 0;
-  d.radii = a->radii;
-  d.splat = at<float4>(geom, GL.splat);
-  d.order = order;
-  d.tkeys = tkeys[0];
-  d.tvals = tvals[0];
-  d.scan_state = at<unsigned long long>(geom, GL.dup_scan);
-  d.incl = dkeys[0];  // free once the last depth pass has read it (the sorted keys are in dkeys[1])
-  // the depth sort's other free buffers: its sorted keys and its first value buffer
-  static_assert(((kDepthPasses - 1) & 1) == 1, "the depth order is in dvals[1]");
-  d.rect_row = dvals[0];
-  d.rect_cw = dkeys[1];
-  d.emit_first = at<uint32_t>(binning, BL.emit_first);
-  d.emit_last = at<uint32_t>(binning, BL.emit_last);
-  d.capacity = capacity;
-  d.hdr = hdr;
-  d.hist = hist + kDepthPasses * kRadix;
-  d.hist_passes = td.passes;
-  for (int q = 0; q < td.passes; ++q) {
-    d.hist_shift[q] = td.shift[q];
-    d.hist_mask[q] = td.mask[q];
-  }
-  if (probe != nullptr) {
-    d.max_spins = probe->max_spins;
-    d.skip_tiles = 1;
-  }
-  staged(OMNIGS_STAGE_DUPLICATE, 1, s, [&] { launch_duplicate(d, s); });
-  if (probe != nullptr) return check_launch("duplicate (look-back probe)");
-
-  // 3. stable tile sort of the instances
-  // (its digit histograms were counted by the duplicate pass)
-  for (int q = 0; q < td.passes; ++q) {
-    OnesweepParams op{};
-    op.keys_in = tkeys[q & 1];
-    op.vals_in = tvals[q & 1];
-    op.keys_out = tkeys[(q + 1) & 1];
-    op.vals_out = tvals[(q + 1) & 1];
-    op.shift = td.shift[q];
-    op.mask = td.mask[q];
-    op.count_hdr = hdr;
-    op.capacity = capacity;
-    op.hist = hist + (kDepthPasses + q) * kRadix;
-    op.lookback = at<uint32_t>(binning, BL.tile_lookback) + (size_t)q * inst_tiles * kRadix;
-    op.tile_counter = &hdr->sort_tile_counter[kDepthPasses + q];
-    op.hdr = hdr;
-    staged(OMNIGS_STAGE_SORT, 1, s, [&] { launch_onesweep(op, capacity, s); });
-  }
-  const int fin = td.passes & 1;
-  if (int rc = check_launch("binning")) return rc;
-
-  // 4. tile ranges
-  RangesParams rp{};
-  rp.keys = tkeys[fin];
-  rp.ranges = ranges;
-  rp.num_tiles = (uint32_t)gx * (uint32_t)gy;
-  rp.capacity = capacity;
-  rp.hdr = hdr;
-  staged(OMNIGS_STAGE_RANGES, 1, s, [&] { launch_ranges(rp, s); });
-  if (int rc = check_launch("ranges")) return rc;
+  BinningPass b{};
+  b.grid.P = a->P;
+  b.grid.V = 1;
+  b.grid.num_tiles = (uint32_t)gx * (uint32_t)gy;
+  b.grid.gx[0] = gx;
+  b.grid.gy[0] = gy;
+  b.depth = at<float>(geom, GL.depth);
+  b.radii = a->radii;
+  b.splat = at<float4>(geom, GL.splat);
+  b.dkeys[0] = at<uint32_t>(geom, GL.dkeys0);
+  b.dkeys[1] = at<uint32_t>(geom, GL.dkeys1);
+  b.dvals[0] = at<uint32_t>(geom, GL.dvals0);
+  b.dvals[1] = at<uint32_t>(geom, GL.dvals1);
+  b.zero = at<uint4>(geom, GL.dup_scan);
+  b.zero_bytes = GL.zero_end - GL.dup_scan;
+  b.scan_state = at<unsigned long long>(geom, GL.dup_scan);
+  b.depth_lookback = at<uint32_t>(geom, GL.depth_lookback);
+  b.depth_hist = at<uint32_t>(binning, BL.hist);
+  b.binning = binning;
+  b.layout = BL;
+  b.capacity = capacity;
+  b.ranges = ranges;
+  b.hdr = hdr;
+  b.out = fin;
+  b.max_spins = probe != nullptr ? probe->max_spins : 0;
+  if (int rc = run_binning(b, s)) return rc;
+  if (probe != nullptr) return OMNIGS_OK;
 
   RenderParams r{};
   r.P = a->P;
@@ -391,7 +494,8 @@ int render_impl(const OmnigsLonlatForwardArgs* a, void* geom, size_t geom_bytes,
   r.gx = gx;
   r.gy = gy;
   r.ranges = ranges;
-  r.point_list = tvals[fin];
+  r.point_list = at<uint32_t>(binning, fin ? BL.tvals1 : BL.tvals0);
+  r.chained = b.small;
   r.capacity = capacity;
   r.splat = at<float4>(geom, GL.splat);
   r.color = at<float4>(geom, GL.color);

@@ -10,6 +10,7 @@
 
 #include <cuda_runtime.h>
 
+#include "kernels.h"
 #include "layout.h"
 
 namespace omnigs {
@@ -71,8 +72,27 @@ void staged(int stage, int kernels, cudaStream_t s, F&& launch) {
 // Blend staging batch size per direction (0 forward, 1 backward), see blend_batch_size.
 extern std::atomic<int> g_blend_batch[2];
 
-// Clears the per-pass state in the header (status capacity bits, counters) and copies the
-// instance total into num_rendered; one thread.
-void launch_begin_render(GeomHeader* hdr, cudaStream_t s);
+// The binning of V views (binning.cu) between the preprocess and the blends, for both entry points.
+struct BinningPass {
+  TileGrid grid;                 // P, V, seam_wrap, gx, gy, tile_base, num_tiles; the bins are numbered here
+  const float* depth;            // [V][P] depth keys
+  const int* radii;
+  const float4* splat;
+  uint32_t *dkeys[2], *dvals[2]; // [V][P] each
+  uint4* zero;                   // look-back words of the scan and the depth sort, cleared by the pass
+  size_t zero_bytes;
+  unsigned long long* scan_state;
+  uint32_t* depth_lookback;      // kDepthPasses x sort tiles
+  uint32_t* depth_hist;          // [V][kDepthPasses][kRadix], inside `zero` or `hist`
+  void* binning;
+  BinningLayout layout;
+  int64_t capacity;
+  uint2* ranges;
+  GeomHeader* hdr;
+  int out;                       // binning buffer (0 or 1) that receives the sorted list
+  int max_spins;                 // look-back probe: wait limit, and stop after the scan (0: a real pass)
+  bool small;                    // set by the pass: a small scene's path was taken
+};
+int run_binning(BinningPass& b, cudaStream_t s);
 
 }  // namespace omnigs

@@ -3,6 +3,7 @@
 
 #include <cstdint>
 #include <cuda_runtime.h>
+#include <utility>
 
 namespace omnigs {
 
@@ -28,6 +29,35 @@ __device__ __forceinline__ void st_relaxed_u32(uint32_t* p, uint32_t v) {
   asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
+// Programmatic dependent launch (launch_chained): a kernel of a chain first lets the next one's blocks be
+// scheduled as its own finish starting, then waits until everything before it has completed and its
+// writes are visible.  A kernel that is launched so calls this before it touches memory; launched
+// otherwise it changes nothing.
+__device__ __forceinline__ void chain_begin() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31; }
+
+// Launches a kernel that begins with chain_begin(), with `chained` so that its launch overlaps the kernel
+// before it on the stream (also inside a captured graph).  Measured on a B200: the forward of 10,000
+// Gaussians at 512x256, whose kernels are a few microseconds each, 64.5 -> 57.2 us; where kernels are
+// longer it gains nothing, and costs 2 % of a captured train step over 200,000 Gaussians and 0.5 % of
+// the 16-view batch, so only the binning of small scenes and the blend behind it are chained.
+template <class... Params, class... Args>
+inline void launch_chained(bool chained, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = chained ? 1 : 0;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
 
 }  // namespace omnigs

@@ -66,49 +66,47 @@ struct OnesweepParams {
   uint32_t seg_len;
   uint32_t num_segs;
   uint32_t hist_seg_stride;
-  // Variable segments (seg_counts non-null): num_segs consecutive segments of seg_counts[s] items
-  // (device counts, all taken as 0 when count_hdr reports an overflow) with segment-local keys;
-  // with add_key_base the pass writes key + (segment s's key base) (the last pass restores global
-  // keys).  The key bases are the u32[kMaxBatchViews] array that directly follows the
-  // u64[kMaxBatchViews] counts (BatchLayout), so this parameter block stays at 128 bytes: at 136
-  // bytes every launch of the pass measured ~2 us slower on a B200.
-  const unsigned long long* seg_counts;
-  int add_key_base;
 };
 
-// duplicateWithKeys over V views (V = 1 for a single view).  Records are view-major (rec = v P + g);
-// instance keys are global tile ids tile_base[v] + ty gx[v] + tx and values record indices.
-struct DuplicateParams {
+// Tile and bin numbering of V views: view v owns tiles [tile_base, tile_base + gx gy) and bins
+// [bin_base, bin_base + bx by) of kBinW x kBinH tiles.
+struct TileGrid {
   int P, V;
+  uint32_t num_tiles, num_bins;
+  int seam_wrap;               // tile columns wrap modulo gx (rects from tile_rect_cyclic)
+  int gx[kMaxBatchViews], gy[kMaxBatchViews];
+  uint32_t tile_base[kMaxBatchViews], bin_base[kMaxBatchViews];
+  // the fine stage: warps that share a bin's pairs, and per view its first block and its first count
+  uint32_t num_blocks;
+  uint32_t parts[kMaxBatchViews], block_base[kMaxBatchViews], count_base[kMaxBatchViews];
+};
+
+// The coarse stage of the binning over V views (V = 1 for a single view): every Gaussian's (bin, record)
+// pairs in depth order.  Records are view-major (rec = v P + g).
+struct DuplicateParams {
+  TileGrid grid;
   const int* radii;            // [V][P]
   const float4* splat;         // [V][P][2]
   const uint32_t* order;       // [V][P] record indices sorted by (view, depth bits, index)
-  uint32_t* tkeys;             // [capacity] tile ids
-  uint32_t* tvals;             // [capacity] record indices
+  uint32_t* keys;              // [capacity] pair words (binning.cu), whose upper bits are the bin
+  uint32_t* vals;              // [capacity] record indices
   unsigned long long* scan_state;
-  uint32_t* incl;              // [V][P] scratch: inclusive instance offsets in depth order
+  uint32_t* incl;              // [V][P] scratch: inclusive pair offsets in depth order
                                // (the depth sort's first key buffer, free after its last pass)
-  // [V][P] scratch in depth order, written by the scan for the emission: each Gaussian's first
-  // row's tile id and its first column | width << 16 (the depth sort's free buffers)
-  uint32_t* rect_row;
-  uint32_t* rect_cw;
+  // [V][P] tile rects in depth order, written by the scan (the depth sort's free buffers):
+  // first column | end << 16 and first row | end << 16
+  uint32_t* rect_x;
+  uint32_t* rect_y;
   uint32_t* emit_first;        // [emit_blocks(capacity) + 1]: depth-order position of the Gaussian
-  uint32_t* emit_last;         // holding each emit block's first / last instance
+  uint32_t* emit_last;         // holding each emit block's first / last pair
   int64_t capacity;
   GeomHeader* hdr;
-  int seam_wrap;               // tile columns wrap modulo gx (rects from tile_rect_cyclic)
-  int gx[kMaxBatchViews], gy[kMaxBatchViews];
-  uint32_t tile_base[kMaxBatchViews];
-  // digit histograms of the tile sort, accumulated into hist[hist_passes][kRadix] (zeroed by the
-  // caller); hist_passes 0 counts nothing.  With hist_per_view, the keys written are view-local
-  // tile ids (without tile_base[v]) and each view's digits are counted into
-  // hist + v * kTilePasses * kRadix (requires P >= kScanBlock: a block then spans at most two views).
+  // digit histograms of the bin sort, accumulated into hist[hist_passes][kRadix] (zeroed by the
+  // caller); hist_passes 0 counts nothing
   uint32_t* hist;
   int hist_passes;
   int hist_shift[kTilePasses];
   uint32_t hist_mask[kTilePasses];
-  int hist_per_view;
-  uint32_t* key_base_out;      // with hist_per_view: tile_base[0, V) copied here for the tile sort
   // Look-back wait limit (polls; 0 = kMaxSpins) and the number of leading scan tiles no block
   // takes (0 in every real pass).  omnigs_debug_lookback_timeout sets skip_tiles = 1 and a small
   // limit: tile 0 then never publishes its prefix, so tile 1's bounded wait runs out.
@@ -116,12 +114,44 @@ struct DuplicateParams {
   uint32_t skip_tiles;
 };
 
-struct RangesParams {
-  const uint32_t* keys;        // sorted tile ids
-  uint2* ranges;
-  uint32_t num_tiles;
+// The fine stage: every tile's list from its bin's.
+struct TileListParams {
+  TileGrid grid;
+  const uint32_t* words;       // the pairs sorted by bin; NULL: every bin holds its view's whole order
+  const uint32_t* recs;
+  const uint32_t* order;       // depth order and rects (as DuplicateParams), read when there are no pairs
+  const uint32_t* rect_x;
+  const uint32_t* rect_y;
+  bool chained;
+  uint32_t* counts;            // scratch: per view [parts][tiles] counts; NULL (one part per bin): the
+                               // counts go through the ranges
+  uint32_t* totals;            // scratch: [num_tiles] totals (cleared)
+  uint32_t* out_keys;          // [capacity] sorted tile ids and record indices
+  uint32_t* out_vals;
+  uint2* ranges;               // [num_tiles]
   int64_t capacity;
-  const GeomHeader* hdr;
+  GeomHeader* hdr;
+};
+
+// Depth order by counting (few Gaussians), in place of the depth sort, and the tile rects in that order.
+struct RankParams {
+  TileGrid grid;
+  const uint32_t* keys;        // [V][P] depth bits
+  const int* radii;
+  const float4* splat;
+  uint32_t* order;
+  uint32_t* rect_x;
+  uint32_t* rect_y;
+  bool chained;
+};
+
+// Regions cleared before a binning pass, with the header's per-pass state.
+struct BeginParams {
+  GeomHeader* hdr;
+  static constexpr int kRegions = 4;
+  uint4* region[kRegions];     // 16-byte aligned
+  size_t bytes[kRegions];      // multiples of 16
+  bool chained;                // as the small scenes' other kernels (launch_chained)
 };
 
 struct RenderParams {
@@ -135,6 +165,7 @@ struct RenderParams {
   float* out_color;
   float* final_T;       // NULL with transmittance checkpointing: the forward does not store it and
   uint32_t* n_contrib;  // the backward recomputes it
+  bool chained;         // the forward, behind a small scene's binning (launch_chained)
   // backward only
   const float* dL_dpix;
   float* grad_acc;  // [P][12]
@@ -248,8 +279,11 @@ void launch_batch_preprocess_backward(const BatchParams& p, const BatchGrads& g,
 void launch_preprocess(const PreprocessParams& p, cudaStream_t s);
 void launch_histogram(const HistParams& p, int64_t max_items, cudaStream_t s);
 void launch_onesweep(const OnesweepParams& p, int64_t max_items, cudaStream_t s);
+void launch_begin_binning(const BeginParams& p, cudaStream_t s);
+void launch_rank(const RankParams& p, cudaStream_t s);
+void launch_rects(const RankParams& p, cudaStream_t s);  // rects only, in the order given
 void launch_duplicate(const DuplicateParams& p, cudaStream_t s);
-void launch_ranges(const RangesParams& p, cudaStream_t s);
+void launch_tile_lists(const TileListParams& p, cudaStream_t s);
 // Splats staged per shared-memory batch in the blend kernels: a template parameter chosen at run
 // time per direction (128, 256 or 512; set by omnigs_set_blend_batch or the autotuner).  Results
 // do not depend on it: every pixel meets the same splats in the same order.  Defaults: 128 for both

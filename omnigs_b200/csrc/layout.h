@@ -61,7 +61,8 @@ struct GeomHeader {
   uint32_t pad0;
   unsigned long long num_rendered64;
   uint32_t sort_tile_counter[kMaxSortPasses];
-  uint32_t reserved[64 - 6 - kMaxSortPasses];
+  uint32_t num_pairs;  // (Gaussian, bin) pairs of the pass (binning.cu)
+  uint32_t reserved[64 - 7 - kMaxSortPasses];
 };
 static_assert(sizeof(GeomHeader) == 256, "header must be 256 bytes");
 
@@ -71,6 +72,15 @@ inline int tiles_x(int W) { return (W + 15) / 16; }
 inline int tiles_y(int H) { return (H + 15) / 16; }
 inline int64_t sort_tiles(int64_t n) { return (n + kSortTile - 1) / kSortTile; }
 
+// A sort pass over few keys runs on small tiles (binning.cu): while those are at most kSmallSortTiles.
+constexpr int kSmallSortItems = 4;
+constexpr int kSmallSortTiles = 160;
+inline int64_t small_sort_tiles(int64_t n) { return (n + kSortThreads * kSmallSortItems - 1) / (kSortThreads * kSmallSortItems); }
+inline bool small_sort(int64_t items, int64_t segs) { return small_sort_tiles(items) * segs <= kSmallSortTiles; }
+inline int64_t sort_blocks(int64_t items, int64_t segs) {
+  return (small_sort(items, segs) ? small_sort_tiles(items) : sort_tiles(items)) * segs;
+}
+
 struct GeomLayout {
   size_t header, dup_scan, depth_lookback, zero_end, splat, color, depth, tiles_touched, dkeys0,
       dkeys1, dvals0, dvals1, grad_acc, total;
@@ -79,7 +89,7 @@ struct GeomLayout {
     size_t o = 0;
     L.header = o; o = align_up(o + sizeof(GeomHeader));
     L.dup_scan = o; o = align_up(o + sizeof(uint64_t) * ((P + kScanBlock - 1) / kScanBlock));
-    L.depth_lookback = o; o = align_up(o + sizeof(uint32_t) * kDepthPasses * sort_tiles(P) * kRadix);
+    L.depth_lookback = o; o = align_up(o + sizeof(uint32_t) * kDepthPasses * sort_blocks(P, 1) * kRadix);
     L.zero_end = o;  // everything above is cleared before each preprocess
     L.splat = o; o = align_up(o + sizeof(float) * 8 * P);
     L.color = o; o = align_up(o + sizeof(float) * 4 * P);
@@ -113,9 +123,25 @@ struct ImageLayout {
   }
 };
 
-// The duplicate pass writes the instance list in blocks of kEmitBlock instances; its scan records,
-// per such block, the depth-order positions of the Gaussians holding the block's first and last
-// instance (emit_first / emit_last).
+// Bins of the coarse stage of the binning: kBinW x kBinH tiles.
+constexpr int kBinW = 8, kBinH = 4;
+constexpr int kPairBinShift = kBinW + kBinH;  // a pair's word: its tiles in the bin, above them the bin (binning.cu)
+
+// Warps that share a bin's pairs in the fine stage: one per kListPart pairs that an even spread would give
+// a bin (one and a half bins per Gaussian), at most kMaxListParts.
+constexpr int kListPart = 128;
+constexpr int kMaxListParts = 128;
+constexpr int kListWarps = 8;                 // parts per block
+OMNIGS_HD inline int bins_x(int gx) { return (gx + kBinW - 1) / kBinW; }
+OMNIGS_HD inline int bins_y(int gy) { return (gy + kBinH - 1) / kBinH; }
+
+// Up to kRankMaxP Gaussians per view the depth order comes from counting, and up to kWholeMaxPairs
+// (Gaussian, bin) combinations every bin reads its view's whole depth order (binning.cu).
+constexpr int kRankMaxP = 12288;
+constexpr int64_t kWholeMaxPairs = int64_t(1) << 20;
+
+// The duplicate pass writes its list in blocks of kEmitBlock pairs; its scan records, per such block, the
+// depth-order positions of the Gaussians holding the block's first and last pair (emit_first / emit_last).
 constexpr int kEmitBlock = 2048;
 inline int64_t emit_blocks(int64_t capacity) { return (capacity + kEmitBlock - 1) / kEmitBlock; }
 // Gaussians per block of the duplicate's scan (4 per thread)
@@ -133,8 +159,7 @@ struct BinningLayout {
     L.tvals0 = o; o = align_up(o + sizeof(uint32_t) * C);
     L.tvals1 = o; o = align_up(o + sizeof(uint32_t) * C);
     L.hist = o; o = align_up(o + sizeof(uint32_t) * kMaxSortPasses * kRadix);
-    // room for a per-view tile sort of a batch: up to kMaxBatchViews more (partial) tiles per pass
-    L.tile_lookback = o; o = align_up(o + sizeof(uint32_t) * kTilePasses * (sort_tiles(C) + kMaxBatchViews) * kRadix);
+    L.tile_lookback = o; o = align_up(o + sizeof(uint32_t) * kTilePasses * sort_tiles(C) * kRadix);
     L.emit_first = o; o = align_up(o + sizeof(uint32_t) * (emit_blocks(C) + 1));
     L.emit_last = o; o = align_up(o + sizeof(uint32_t) * (emit_blocks(C) + 1));
     L.total = o;
@@ -159,28 +184,23 @@ struct BinningLayout {
 // BinningLayout buffer as in the single-view case).  Per-(view, Gaussian) arrays are view-major;
 // per-pixel arrays hold the views' pixels back to back, ranges the views' tiles back to back.
 //
-//   header | instances per view u64[32] | view tile bases u32[32] | duplicate-scan look-back u64[VP/256] |
+//   header | instances per view u64[32] | duplicate-scan look-back u64[VP/256] |
 //   depth-sort look-back u32[4][V sort tiles(P)][256] | depth histograms u32[V][4][256] |
-//   tile-sort histograms u32[V][3][256] |
 //   radii i32[VP] | splat records float4[2VP] | colour float4[VP] | depth f32[VP] |
 //   depth-sort keys/values u32[4][VP] | gradient accumulators float4[3VP] |
 //   final transmittance f32[pixels] | last contributor u32[pixels] | tile ranges uint2[tiles]
 struct BatchLayout {
-  size_t header, view_rendered, view_key_base, dup_scan, depth_lookback, depth_hist, tile_hist, zero_end, radii, splat, color, depth,
+  size_t header, view_rendered, dup_scan, depth_lookback, depth_hist, zero_end, radii, splat, color, depth,
       dkeys0, dkeys1, dvals0, dvals1, grad_acc, final_T, n_contrib, ranges, total;
   static BatchLayout make(int64_t P, int V, int64_t pixels, int64_t tiles) {
     BatchLayout L;
     const int64_t R = P * V;
     size_t o = 0;
     L.header = o; o = align_up(o + sizeof(GeomHeader));
-    // the view tile bases directly follow the per-view counts: the tile sort finds them there
-    static_assert(sizeof(uint64_t) * kMaxBatchViews % kAlign == 0, "view_key_base must follow view_rendered");
     L.view_rendered = o; o = align_up(o + sizeof(uint64_t) * kMaxBatchViews);
-    L.view_key_base = o; o = align_up(o + sizeof(uint32_t) * kMaxBatchViews);
     L.dup_scan = o; o = align_up(o + sizeof(uint64_t) * ((R + kScanBlock - 1) / kScanBlock));
-    L.depth_lookback = o; o = align_up(o + sizeof(uint32_t) * kDepthPasses * sort_tiles(P) * V * kRadix);
+    L.depth_lookback = o; o = align_up(o + sizeof(uint32_t) * kDepthPasses * sort_blocks(P, V) * kRadix);
     L.depth_hist = o; o = align_up(o + sizeof(uint32_t) * V * kDepthPasses * kRadix);
-    L.tile_hist = o; o = align_up(o + sizeof(uint32_t) * V * kTilePasses * kRadix);
     L.zero_end = o;  // everything above is cleared before each pass
     L.radii = o; o = align_up(o + sizeof(int32_t) * R);
     L.splat = o; o = align_up(o + sizeof(float) * 8 * R);
@@ -210,7 +230,15 @@ struct TileDigits {
   uint32_t mask[kTilePasses];
   static TileDigits make(int W, int H);
   static TileDigits from_tiles(uint32_t tiles);
+  static TileDigits from_bits(int bit);
 };
+
+// Bits of the ids 0 .. n - 1.
+inline int id_bits(uint32_t n) {
+  int bits = 1;
+  while (bits < 32 && ((uint64_t)1 << bits) < n) ++bits;
+  return bits;
+}
 
 inline uint32_t higher_msb(uint32_t n) {
   uint32_t msb = sizeof(n) * 4;
@@ -230,8 +258,9 @@ inline TileDigits TileDigits::make(int W, int H) {
   return from_tiles((uint32_t)tiles_x(W) * (uint32_t)tiles_y(H));
 }
 
-inline TileDigits TileDigits::from_tiles(uint32_t tiles) {
-  const int bit = (int)higher_msb(tiles);
+inline TileDigits TileDigits::from_tiles(uint32_t tiles) { return from_bits((int)higher_msb(tiles)); }
+
+inline TileDigits TileDigits::from_bits(int bit) {
   TileDigits t{};
   t.passes = (bit + kRadixBits - 1) / kRadixBits;
   if (t.passes < 1) t.passes = 1;

@@ -54,6 +54,7 @@ template <int kBatch>
 // on a B200 (0.511 -> 0.491 ms per 1M-Gaussian 2048x1024 view); the batched kernel measured
 // marginally slower under the same bound and keeps the compiler's choice.
 __global__ void __launch_bounds__(kBlendThreads, 12) render_forward_kernel(RenderParams p) {
+  chain_begin();
   TileJob job;
   job.tile_x = blockIdx.x;
   job.tile_y = blockIdx.y;
@@ -91,9 +92,9 @@ void launch_render_forward(const RenderParams& p, cudaStream_t s) {
   if (p.gx <= 0 || p.gy <= 0) return;
   const dim3 grid(p.gx, p.gy);
   switch (blend_batch_size(false)) {
-    case 128: render_forward_kernel<128><<<grid, kBlendThreads, 0, s>>>(p); break;
-    case 512: render_forward_kernel<512><<<grid, kBlendThreads, 0, s>>>(p); break;
-    default: render_forward_kernel<256><<<grid, kBlendThreads, 0, s>>>(p); break;
+    case 128: launch_chained(p.chained, render_forward_kernel<128>, grid, kBlendThreads, 0, s, p); break;
+    case 512: launch_chained(p.chained, render_forward_kernel<512>, grid, kBlendThreads, 0, s, p); break;
+    default: launch_chained(p.chained, render_forward_kernel<256>, grid, kBlendThreads, 0, s, p); break;
   }
 }
 
