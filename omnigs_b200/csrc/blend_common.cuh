@@ -2,6 +2,8 @@
 // alpha-support test of a splat against it, and the staging of a batch of splats into shared memory.
 #pragma once
 
+#include <type_traits>
+
 #include "device_util.cuh"
 #include "kernels.h"
 
@@ -66,7 +68,11 @@ struct BlendPatch {
   }
 
   static __device__ __forceinline__ BlendPatch make(int tile_x, int tile_y, float wrap_w = 0.f) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    return of_warp(tile_x, tile_y, threadIdx.x >> 5, wrap_w);
+  }
+  // The patch of another warp of the block (its pixels those of this thread's lane).
+  static __device__ __forceinline__ BlendPatch of_warp(int tile_x, int tile_y, int warp, float wrap_w) {
+    const int lane = threadIdx.x & 31;
     const int wx0 = tile_x * 16 + (warp & 1) * 8;
     const int wy0 = tile_y * 16 + (warp >> 1) * kPatchRows;
     BlendPatch b;
@@ -110,22 +116,6 @@ struct BlendPatch {
   }
 };
 
-// Exponent of the splat's Gaussian at offset d = centre - pixel (forward.cu:416, backward.cu:763):
-//   power = -0.5 (ca dx^2 + cc dy^2) - cb dx dy.
-// The reference leaves the rounding of this expression to the compiler's FMA contraction.  It is
-// written here with explicit roundings in the one fusion that reproduces the reference's compiled
-// results bit for bit (checked on the 1M-Gaussian 2048x1024 scene: identical transmittance, last
-// contributors and image): ca dx dx fused into the sum with the rounded cc dy dy, the cb dx dy term
-// rounded on its own.  Being explicit keeps the result independent of how the surrounding kernel is
-// structured (a thread owning several pixels lets the compiler share products between them and
-// choose other fusions).  The forward and backward use the same function, so they agree on every
-// 1/255 and saturation decision.
-__device__ __forceinline__ float splat_power(const float4& a, const float4& b, float2 d) {
-  const float ca_dx = __fmul_rn(a.z, d.x), cc_dy = __fmul_rn(b.x, d.y), cb_dx = __fmul_rn(a.w, d.x);
-  const float quad = __fmaf_rn(ca_dx, d.x, __fmul_rn(cc_dy, d.y));
-  return __fsub_rn(__fmul_rn(-0.5f, quad), __fmul_rn(cb_dx, d.y));
-}
-
 // Packed f32x2 arithmetic (one instruction for both lanes, each rounded as its scalar form).
 __device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
@@ -133,119 +123,229 @@ __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __fadd2_rn(a
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 
-// splat_power for two pixels of one column (offsets (dx, dy.x) and (dx, dy.y)), lane by lane
-// bit-identical to splat_power.
-__device__ __forceinline__ float2 splat_power2(const float4& a, const float4& b, float dx, float2 dy) {
-  const float ca_dx = __fmul_rn(a.z, dx), cb_dx = __fmul_rn(a.w, dx);
-  const float2 cc_dy = mul2(f2(b.x), dy);
-  const float2 quad = fma2(f2(ca_dx), f2(dx), mul2(cc_dy, dy));
-  return sub2(mul2(f2(-0.5f), quad), mul2(f2(cb_dx), dy));
+// Whether the blends can leave the positive-exponent test and the 0.99 clamp out for this splat
+// (a = {x, y, conic a, conic b}, b = {conic c, opacity, thr, det}):
+//  * power <= 0 at every offset: with S = a dx^2 + c dy^2 the cross term is at most
+//    sqrt(1 - det / (a c)) S / 2 in size, and the float evaluation of power is off by less than
+//    6 * 2^-24 S / 2, so det > 1e-5 a c keeps it negative (a NaN or non-positive-definite conic,
+//    det = NaN, fails the test);
+//  * opacity times an exponential of a non-positive number stays below the clamp;
+//  * with the conic below 1e9 nothing overflows, so alpha is a finite number.
+__device__ __forceinline__ bool plain_splat(const float4& a, const float4& b) {
+  return b.y < 0.98999f && b.w > 1e-5f * a.z * b.x && a.z + b.x < 1e9f;
 }
 
-// Stages instances [base, base + cnt) of the tile's list (from the back when reverse: slot t holds
-// position base_hi - 1 - t, with base the exclusive upper end) into shared memory; the colour (s_c)
-// only with kColor, the record index only when s_g is not NULL.
-template <bool kColor = true>
-__device__ __forceinline__ void stage_batch(const BlendSource& src, uint32_t range_begin, int base, int cnt,
-                                            bool reverse, float4* s_a, float4* s_b, float4* s_c,
-                                            uint32_t* s_g) {
-  for (int t = threadIdx.x; t < cnt; t += kBlendThreads) {
-    const uint32_t pos = reverse ? (uint32_t)(base - 1 - t) : (uint32_t)(base + t);
-    const uint32_t g = src.point_list[range_begin + pos];
-    if (g < src.num_records) {
-      if (s_g) s_g[t] = g;
-      s_a[t] = src.splat[2 * g];
-      s_b[t] = src.splat[2 * g + 1];
-      if (kColor) s_c[t] = src.color[g];
-    } else {  // unreachable for a consistent instance list; stage a splat that never contributes:
-              // finite, unit conic, threshold -inf (no patch test hits), opacity 0 (alpha 0)
-      if (s_g) s_g[t] = 0;
-      s_a[t] = make_float4(0.f, 0.f, 1.f, 0.f);
-      s_b[t] = make_float4(1.f, 0.f, -__int_as_float(0x7f800000), 1.f);
-      if (kColor) s_c[t] = make_float4(0.f, 0.f, 0.f, 0.f);
+// A batch of staged splats, as the blends' inner loops read it.  The loops are bound by instruction
+// issue, so the staging thread does once per splat what every warp or candidate would repeat:
+//  * it tests its splat against the block's four patches (from registers; a ballot per patch), and
+//    every warp turns its masks into a list of its candidates' offsets, so the loop over them has no
+//    bit scanning or address arithmetic;
+//  * a slot (48 bytes) holds {x, y, -a/2, -b}{-c/2, o, r, g}{b, 1 + position, record, -}.
+// The exponent at offset d = centre - pixel (forward.cu:416, backward.cu:763) is
+//   power = -0.5 (a dx^2 + c dy^2) - b dx dy,
+// whose rounding the reference leaves to the compiler's FMA contraction.  Both blends write it with
+// explicit roundings in the one fusion that reproduces the reference's compiled results bit for bit
+// (checked on the 1M-Gaussian 2048x1024 scene: identical transmittance, last contributors and image):
+// a dx dx fused into the sum with the rounded c dy dy, the b dx dy term rounded on its own.  The slot's
+// factors -1/2 and signs are exact, so applying them before the roundings changes nothing.  Forward and
+// backward agree on every 1/255 and saturation decision.
+// Slot kBatch holds a splat that reaches no pixel; it pads the lists to whole groups of four.
+constexpr uint32_t kSlotBytes = 48;
+
+template <int kBatch>
+struct BlendStage {
+  static constexpr int kListSplats = kBatch < 256 ? kBatch : 256;
+  float4 d[kBatch + 1][kSlotBytes / 16];
+  uint32_t list[kBlendWarps][kListSplats + 4];  // byte offsets of a warp's candidates, padded
+  uint32_t mask[kBatch / 32][kBlendWarps];      // candidates of a group of 32 by warp
+  uint32_t special[kBatch / 32];                // the group's splats that are not plain (plain_splat)
+};
+
+// Must be followed by a block barrier.
+template <int kBatch>
+__device__ __forceinline__ void init_stage(BlendStage<kBatch>& st) {
+  if (threadIdx.x < kSlotBytes / 16) st.d[kBatch][threadIdx.x] = make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
+// Stages instances [base, base + cnt) of the tile's list (from the back when kReverse: slot t holds
+// position base - 1 - t, with base the exclusive upper end) with their patch masks; the colour only
+// with kColor.
+template <int kBatch, bool kWrap, bool kColor, bool kReverse>
+__device__ __forceinline__ void stage_splats(BlendStage<kBatch>& st, const BlendSource& src, const TileJob& job,
+                                             int base, int cnt) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll 1
+  for (int t = threadIdx.x; t < kBatch; t += kBlendThreads) {
+    bool hits[kBlendWarps] = {}, special = false;
+    if (t < cnt) {
+      const uint32_t pos = kReverse ? (uint32_t)(base - 1 - t) : (uint32_t)(base + t);
+      const uint32_t g = src.point_list[job.range.x + pos];
+      if (g < src.num_records) {  // (always, for a consistent instance list)
+        const float4 a = src.splat[2 * (size_t)g], b = src.splat[2 * (size_t)g + 1];
+        const float4 c = kColor ? src.color[g] : make_float4(0.f, 0.f, 0.f, 0.f);
+        st.d[t][0] = make_float4(a.x, a.y, -0.5f * a.z, -a.w);
+        st.d[t][1] = make_float4(-0.5f * b.x, b.y, c.x, c.y);
+        st.d[t][2] = make_float4(c.z, __uint_as_float(pos + 1u), __uint_as_float(g), 0.f);
+        special = !plain_splat(a, b);
+#pragma unroll
+        for (int w = 0; w < kBlendWarps; ++w)
+          hits[w] = BlendPatch::of_warp(job.tile_x, job.tile_y, w, job.wrap_w).template hit<kWrap>(a, b);
+      }
+    }
+    const unsigned ms = __ballot_sync(kFullMask, special);
+    if (lane == 0) st.special[t >> 5] = ms;
+#pragma unroll
+    for (int w = 0; w < kBlendWarps; ++w) {
+      const unsigned m = __ballot_sync(kFullMask, hits[w]);
+      if (lane == 0) st.mask[t >> 5][w] = m;
     }
   }
+}
+
+// The warp's candidates among slots [max(from, first), from + kListSplats) of the staged batch, in
+// slot order: writes their offsets to its list (padded to a multiple of four), returns their number
+// and whether any is special.
+template <int kBatch>
+__device__ __forceinline__ int list_candidates(BlendStage<kBatch>& st, int from, int first, bool& special) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t* list = st.list[warp];
+  const unsigned lt = (1u << lane) - 1u;
+  int n = 0;
+  unsigned sp = 0;
+  __syncwarp();  // the warp has read its previous list
+#pragma unroll
+  for (int i = 0; i < BlendStage<kBatch>::kListSplats / 32; ++i) {
+    const int k = from / 32 + i;
+    unsigned m = st.mask[k][warp];
+    if (first > k * 32) m = first - k * 32 >= 32 ? 0u : m & (kFullMask << (first - k * 32));
+    sp |= m & st.special[k];
+    if ((m >> lane) & 1u) list[n + __popc(m & lt)] = (uint32_t)(k * 32 + lane) * kSlotBytes;
+    n += __popc(m);
+  }
+  if (lane < 4) list[n + lane] = kBatch * kSlotBytes;
+  __syncwarp();
+  special = sp != 0;
+  return n;
+}
+
+// One splat at one pixel of the forward's pass: alpha is the splat's, test_T = T (1 - alpha) with T
+// the pixel's transmittance, negated once the pixel has stopped.  Where the splat reaches the pixel
+// (alpha >= 1/255, and the exponent is not positive) and test_T stays at or above 1e-4, the colour
+// c alpha T is added (rounded as the reference's compiled blend: fused add), T becomes test_T and lc
+// the splat's position; where test_T falls below (always so for a stopped pixel, whose T is negative)
+// the pixel stops, T = -|T|.  One comparison gives both outcomes (setp's two predicates), and
+// everything else is predicated: no branches, no selects.
+template <bool kPlain, bool kColor>
+__device__ __forceinline__ void forward_pixel(float alpha, float power, float test_T, float r, float g, float b,
+                                              uint32_t at, float& T, uint32_t& lc, float& C0, float& C1, float& C2) {
+// operands: %0 T, %1 lc, %2-%4 C, %5 alpha, %6 test_T, %7 position, %8 power, %9-%11 colour
+#define OMNIGS_PIXEL_TEST                                                                       \
+  "setp.geu.f32 p, %5, 0f3B808081;\n\t" /* !(alpha < 1/255) */
+#define OMNIGS_PIXEL_TEST_ANY                                                                   \
+  "setp.leu.and.f32 p, %8, 0f00000000, p;\n\t" /* !(power > 0) */                               \
+  "setp.geu.and.f32 p, %0, 0f00000000, p;\n\t" /* a NaN alpha revives no stopped pixel */
+#define OMNIGS_PIXEL_STATE                                                                      \
+  "setp.lt.and.f32 stop|act, %6, 0f38D1B717, p;\n\t" /* test_T < 1e-4, or not */
+#define OMNIGS_PIXEL_COLOR                                                                      \
+  "mul.rn.f32 c0, %9, %5;\n\tmul.rn.f32 c1, %10, %5;\n\tmul.rn.f32 c2, %11, %5;\n\t"          \
+  "@act fma.rn.f32 %2, c0, %0, %2;\n\t@act fma.rn.f32 %3, c1, %0, %3;\n\t@act fma.rn.f32 %4, c2, %0, %4;\n\t"
+#define OMNIGS_PIXEL_UPDATE                                                                     \
+  "@act mov.f32 %0, %6;\n\t@stop or.b32 %0, %0, 0x80000000;\n\t@act mov.b32 %1, %7;\n\t"
+#define OMNIGS_PIXEL(body)                                                                      \
+  asm("{\n\t.reg .pred p, act, stop;\n\t.reg .f32 c0, c1, c2;\n\t" body "}"                   \
+      : "+f"(T), "+r"(lc), "+f"(C0), "+f"(C1), "+f"(C2)                                          \
+      : "f"(alpha), "f"(test_T), "r"(at), "f"(power), "f"(r), "f"(g), "f"(b))
+  if (kPlain && kColor)
+    OMNIGS_PIXEL(OMNIGS_PIXEL_TEST OMNIGS_PIXEL_STATE OMNIGS_PIXEL_COLOR OMNIGS_PIXEL_UPDATE);
+  else if (kPlain)
+    OMNIGS_PIXEL(OMNIGS_PIXEL_TEST OMNIGS_PIXEL_STATE OMNIGS_PIXEL_UPDATE);
+  else if (kColor)
+    OMNIGS_PIXEL(OMNIGS_PIXEL_TEST OMNIGS_PIXEL_TEST_ANY OMNIGS_PIXEL_STATE OMNIGS_PIXEL_COLOR OMNIGS_PIXEL_UPDATE);
+  else
+    OMNIGS_PIXEL(OMNIGS_PIXEL_TEST OMNIGS_PIXEL_TEST_ANY OMNIGS_PIXEL_STATE OMNIGS_PIXEL_UPDATE);
+#undef OMNIGS_PIXEL_TEST
+#undef OMNIGS_PIXEL_TEST_ANY
+#undef OMNIGS_PIXEL_STATE
+#undef OMNIGS_PIXEL_COLOR
+#undef OMNIGS_PIXEL_UPDATE
+#undef OMNIGS_PIXEL
 }
 
 // The forward's front-to-back pass over a tile's instances (forward.cu:394-456) for the thread's two
-// pixels (lane x: row py0, lane y: row py0 + 4): transmittance T and last contributor lc, and with
-// kColor the blended colour C.  Every pixel evaluates the reference's per-pair arithmetic and control
-// flow (power, alpha = min(0.99, o exp(power)), the 1/255 skip, the T < 1e-4 stop), so T and lc are
-// the same whether or not colour is blended: the forward kernel runs it with colour, the backward
-// runs it without to recompute the state it did not store.  The staging arrays hold kBatch splats.
-// The block's threads must all call it (it synchronises the block).
+// pixels (rows py0 and py0 + 4): transmittance T and last contributor lc, and with kColor the blended
+// colour C.  Every pixel evaluates the reference's per-pair arithmetic and control flow (power,
+// alpha = min(0.99, o exp(power)), the 1/255 skip, the T < 1e-4 stop), so T and lc are the same whether
+// or not colour is blended: the forward kernel runs it with colour, the backward runs it without to
+// recompute the state it did not store.
+//
+// The loop over a warp's candidates has two bodies: where all of them are plain (plain_splat) the
+// exponent's sign test and the clamp are left out.  The two pixels' arithmetic is packed (f32x2, one
+// issue slot) where both factors differ by pixel, and scalar where one is the splat's: broadcasting that
+// into a register pair costs the moves that packing saves.  Bound by instruction issue.  Measured on a
+// B200 (1M-Gaussian 2048x1024 view / 16-view batch) against a warp testing every staged splat itself and
+// walking the ballots' bits: 424 -> 410 us / 5.20 -> 5.10 ms.
 template <int kBatch, bool kWrap, bool kColor>
 __device__ __forceinline__ void forward_pass(const TileJob& job, const BlendSource& src, const BlendPatch& patch,
-                                             float4* s_a, float4* s_b, float4* s_c, float2& T, uint32_t& lc0,
-                                             uint32_t& lc1, float2& C0, float2& C1, float2& C2) {
-  static_assert(kBlendPx == 2, "the blend packs a thread's two pixels into f32x2 lanes");
-  const int lane = threadIdx.x & 31;
-  const uint2 range = job.range;
-  const int n = (int)(range.y - range.x);
-  bool done0 = !patch.inside(0, job.W, job.H), done1 = !patch.inside(1, job.W, job.H);
-  T = f2(1.0f);
-  C0 = C1 = C2 = f2(0.f);
-  lc0 = lc1 = 0;
-  const float2 pyf = make_float2(patch.pyf(0), patch.pyf(1));
+                                             BlendStage<kBatch>& st, float T[2], uint32_t lc[2], float C[2][3]) {
+  static_assert(kBlendPx == 2, "a thread owns two pixels of one column");
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    T[i] = patch.inside(i, job.W, job.H) ? 1.0f : -1.0f;  // a pixel outside the image starts stopped
+    lc[i] = 0;
+    C[i][0] = C[i][1] = C[i][2] = 0.f;
+  }
+  const float pyf[2] = {patch.pyf(0), patch.pyf(1)};
+  const int n = (int)(job.range.y - job.range.x);
+  const char* slots = reinterpret_cast<const char*>(&st.d[0][0]);
+  const uint32_t* list = st.list[threadIdx.x >> 5];
+  init_stage(st);
 
+  auto blend = [&](uint32_t off, auto plain) {
+    constexpr bool kPlain = decltype(plain)::value;
+    const float4* slot = reinterpret_cast<const float4*>(slots + off);
+    const float4 v0 = slot[0], v1 = slot[1];
+    const float2 v2 = *reinterpret_cast<const float2*>(slot + 2);
+    const float dx = (kWrap ? patch.template center_x<true>(v0.x) : v0.x) - patch.pxf;
+    const float hx = __fmul_rn(v0.z, dx), bx = __fmul_rn(v0.w, dx);
+    const float2 dy = make_float2(v0.y - pyf[0], v0.y - pyf[1]);
+    const float2 q2 = mul2(make_float2(__fmul_rn(v1.x, dy.x), __fmul_rn(v1.x, dy.y)), dy);
+    const float2 power = add2(make_float2(__fmaf_rn(hx, dx, q2.x), __fmaf_rn(hx, dx, q2.y)),
+                              make_float2(__fmul_rn(bx, dy.x), __fmul_rn(bx, dy.y)));
+    float2 alpha = make_float2(__fmul_rn(v1.y, expf(power.x)), __fmul_rn(v1.y, expf(power.y)));
+    if (!kPlain) alpha = make_float2(fminf(0.99f, alpha.x), fminf(0.99f, alpha.y));
+    const float2 test_T = mul2(make_float2(T[0], T[1]), fma2(alpha, f2(-1.0f), f2(1.0f)));
+    const uint32_t at = __float_as_uint(v2.y);
+    forward_pixel<kPlain, kColor>(alpha.x, power.x, test_T.x, v1.z, v1.w, v2.x, at, T[0], lc[0], C[0][0], C[0][1], C[0][2]);
+    forward_pixel<kPlain, kColor>(alpha.y, power.y, test_T.y, v1.z, v1.w, v2.x, at, T[1], lc[1], C[1][0], C[1][1], C[1][2]);
+  };
+  auto blend_list = [&](int cnt, auto plain) {
+#pragma unroll 1
+    for (int i = 0; i < cnt; i += 4) {
+      const uint4 o = *reinterpret_cast<const uint4*>(list + i);
+      blend(o.x, plain);
+      blend(o.y, plain);
+      blend(o.z, plain);
+      blend(o.w, plain);
+      if ((i & 4) && __all_sync(kFullMask, T[0] < 0.f && T[1] < 0.f)) break;
+    }
+  };
   for (int base = 0; base < n; base += kBatch) {
-    if (__syncthreads_and(done0 && done1)) break;
-    stage_batch<kColor>(src, range.x, base, min(kBatch, n - base), /*reverse=*/false, s_a, s_b, s_c, nullptr);
+    if (__syncthreads_and(T[0] < 0.f && T[1] < 0.f)) break;
+    stage_splats<kBatch, kWrap, kColor, /*kReverse=*/false>(st, src, job, base, min(kBatch, n - base));
     __syncthreads();
-    const int cnt = min(kBatch, n - base);
-    bool warp_done = __all_sync(kFullMask, done0 && done1);
-    for (int k = 0; k * 32 < cnt && !warp_done; ++k) {
-      const int j = k * 32 + lane;
-      // evaluated by every lane (slots past cnt hold stale or unset data, which j < cnt drops):
-      // measured 2 % faster than a branch around the test
-      const bool hit = patch.template hit<kWrap>(s_a[j], s_b[j]) && j < cnt;
-      unsigned m = __ballot_sync(kFullMask, hit);
-      while (m) {
-        const int jj = k * 32 + __ffs(m) - 1;
-        m &= m - 1;
-        // No per-lane branches: a pixel that is done, or that this splat does not reach, is
-        // inactive through act0 / act1 and its state is updated by selects (alpha 0 adds exactly
-        // 0 to the colour).  The divergent branches measured on a B200 as 13 % of the forward
-        // (0.614 -> 0.545 ms per view without the one around the pair, 0.532 without both).
-        {
-          const float4 a = s_a[jj];
-          const float4 b = s_b[jj];
-          const float dx = patch.template center_x<kWrap>(a.x) - patch.pxf;
-          const float2 dy = sub2(f2(a.y), pyf);
-          const float2 power = splat_power2(a, b, dx, dy);
-          const float2 alpha = make_float2(fminf(0.99f, b.y * expf(power.x)), fminf(0.99f, b.y * expf(power.y)));
-          bool act0 = !done0 && !(power.x > 0.0f) && !(alpha.x < 1.0f / 255.0f);
-          bool act1 = !done1 && !(power.y > 0.0f) && !(alpha.y < 1.0f / 255.0f);
-          {
-            const float2 test_T = mul2(T, sub2(f2(1.0f), alpha));
-            // a pixel whose transmittance would fall below 1e-4 stops without this splat
-            if (act0 && test_T.x < 0.0001f) {
-              done0 = true;
-              act0 = false;
-            }
-            if (act1 && test_T.y < 0.0001f) {
-              done1 = true;
-              act1 = false;
-            }
-            if (kColor) {
-              const float2 ae = make_float2(act0 ? alpha.x : 0.f, act1 ? alpha.y : 0.f);
-              const float4 c = s_c[jj];
-              // C += colour * alpha * T, rounded as the reference's compiled blend (fused add);
-              // a pixel without this splat adds exactly 0
-              C0 = fma2(mul2(f2(c.x), ae), T, C0);
-              C1 = fma2(mul2(f2(c.y), ae), T, C1);
-              C2 = fma2(mul2(f2(c.z), ae), T, C2);
-            }
-            T = make_float2(act0 ? test_T.x : T.x, act1 ? test_T.y : T.y);
-            const uint32_t idx = (uint32_t)(base + jj + 1);
-            lc0 = act0 ? idx : lc0;
-            lc1 = act1 ? idx : lc1;
-          }
-        }
-      }
-      warp_done = __all_sync(kFullMask, done0 && done1);
+#pragma unroll 1
+    for (int from = 0; from < kBatch; from += BlendStage<kBatch>::kListSplats) {
+      if (__all_sync(kFullMask, T[0] < 0.f && T[1] < 0.f)) break;
+      bool special;
+      const int cnt = list_candidates(st, from, 0, special);
+      if (special)
+        blend_list(cnt, std::false_type{});
+      else
+        blend_list(cnt, std::true_type{});
     }
   }
+  T[0] = fabsf(T[0]);
+  T[1] = fabsf(T[1]);
 }
 
 // Block -> (view, tile) of a batched blend launch: blocks run over the views' tiles in the order

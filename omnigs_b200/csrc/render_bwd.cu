@@ -9,46 +9,25 @@
 // 1 - alpha serves both of the reference's divisions by it (relative error ~1e-7 per step, far
 // inside the gradients' 1e-3 tolerance).  The per-(pixel, splat) gradients (2 screen-space mean,
 // 3 conic, 1 opacity, 3 colour) are not pushed with 9 global atomics per pixel as in the
-// reference (and the mean terms are summed as w dx and w dy with w = G dL/dalpha, without the
-// opacity and the conic, the conic terms without the opacity, all without their constant factors
-// -W/2, -H/2, -1/2: the backward preprocess applies those per Gaussian): a thread first sums them
-// over its two
-// pixels and writes the 9 sums to its warp's shared buffer; every second contributing splat the
-// warp that owns the 8 x 8 patch reduces the buffer transposed (one lane per splat and value, 32
-// terms each) and adds the accumulator records with one atomic per value.  Warps skip splats
-// that cannot reach alpha >= 1/255 in their patch or that lie behind all of their pixels' last
-// contributors, and the block starts at the batch holding its largest last contributor instead of
-// at the end of the range.
+// reference: a thread sums them over its two pixels and writes six sums to its warp's shared buffer;
+// after every fifth contributing splat the warp that owns the 8 x 8 patch reduces the buffer transposed
+// and adds the accumulator records with one atomic per value (flush_reduction).  The mean terms are
+// summed as w dx and w dy with w = G dL/dalpha, without the opacity and the conic, the conic terms
+// without the opacity, all without their constant factors -W/2, -H/2, -1/2: the backward preprocess
+// applies those per Gaussian.  A warp walks only the splats that can reach alpha >= 1/255 in its patch
+// and do not lie behind all of its pixels' last contributors (blend_common.cuh), and the block starts at
+// the batch holding its largest last contributor instead of at the end of the range.
+//
+// Bound by instruction issue (79 % of the slots on a 400k-Gaussian view).  Measured on a B200
+// (300k / 1M-Gaussian 2048x1024 view / 16-view batch): 315 / 760 / 9710 us with the warps scanning ballots
+// of their own tests, every sum in a row of its own (nine, two splats a flush) and the clamp and sign
+// tests for every splat; 271 / 669 / 8530 us now.  The same sums on the tensor cores (mma.m16n8k8, TF32
+// operands split in two) took 319 / 812 / 10600: fewer instructions, but the fragments' registers and
+// shared memory leave six blocks per SM.
 #include "blend_common.cuh"
 
 namespace omnigs {
 namespace {
-
-// Per-warp buffer of the lane values of contributing splats: row 9 h + q holds value q of buffered
-// splat h for the 32 lanes.  The row stride of 36 floats puts the 16-byte reads of 8 consecutive
-// rows (one quarter-warp) on distinct banks; the lanes' writes of one row are consecutive words.
-constexpr int kRedStride = 36;
-
-// Adds the buffered splats' lane sums to their accumulator records: lane t sums row t over the
-// 32 lanes (eight 16-byte reads, packed adds) and adds the total with one atomic.
-__device__ __forceinline__ void flush_reduction(float (*red)[kRedStride], const uint32_t* gidx, int n,
-                                                float* grad_acc, int lane) {
-  __syncwarp();
-  for (int t = lane; t < n * 9; t += 32) {
-    const int h = t / 9, q = t - 9 * h;
-    const float4* row = reinterpret_cast<const float4*>(red[t]);
-    float2 s0 = make_float2(0.f, 0.f), s1 = s0;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const float4 x = row[i];
-      s0 = add2(s0, make_float2(x.x, x.y));
-      s1 = add2(s1, make_float2(x.z, x.w));
-    }
-    s0 = add2(s0, s1);
-    atomicAdd(grad_acc + 12 * (size_t)gidx[h] + q, s0.x + s0.y);
-  }
-  __syncwarp();  // the rows are rewritten next
-}
 
 __device__ __forceinline__ float rcp_approx(float x) {
   float r;
@@ -56,44 +35,88 @@ __device__ __forceinline__ float rcp_approx(float x) {
   return r;
 }
 
-// Eight resident blocks per SM (at most 64 registers per thread) measured fastest on a B200.
-constexpr int kBlendBwdMinBlocks = 8;
+// ---- the reduction of a splat's gradients over the warp's 64 pixels ----
+// A lane keeps six sums over its two pixels (w = G dL/dalpha, d = alpha T): w, w dy, w dy^2 and d times the
+// three components of dL/dpix.  The other three, w dx, w dx^2 and w dx dy, need no rows of their own: dx is
+// the same for all pixels of a column, so the lane that adds up a row's eight columns multiplies the column
+// sums by dx.  Row 6 h + q of a warp's buffer holds sum q of buffered splat h for the 32 lanes; five splats
+// make 30 rows, one lane each.  The row stride of 36 floats puts the 16-byte reads of 8 consecutive rows
+// (one quarter-warp) on distinct banks; the lanes' writes of one row are consecutive words.
+constexpr int kRedSplats = 5;
+constexpr int kRedRows = 6;
+constexpr int kRedStride = 36;
+
+template <int kBatch>
+struct BackwardSmem {
+  BlendStage<kBatch> stage;
+  __align__(16) float red[kBlendWarps][kRedSplats * kRedRows][kRedStride];
+  float2 info[kBlendWarps][kRedSplats];  // {x of the splat less the patch's first column, its record}
+  uint32_t last[kBlendWarps];
+};
+
+// Adds the first n buffered splats' sums to their accumulator records {w dx, w dy, w dx^2, w dx dy}
+// {w dy^2, w, r, g}{b, 0, 0, 0}, one atomic per value.
+template <int kBatch>
+__device__ __forceinline__ void flush_reduction(BackwardSmem<kBatch>& sm, int n, float* grad_acc) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  __syncwarp();
+  if (lane < n * kRedRows) {
+    const int h = lane / kRedRows, q = lane - kRedRows * h;
+    const float4* row = reinterpret_cast<const float4*>(sm.red[warp][lane]);
+    float2 c[4];  // sums of the columns 2 i and 2 i + 1
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float4 lo = row[2 * i], hi = row[2 * i + 1];
+      const float2 v[4] = {make_float2(lo.x, lo.y), make_float2(lo.z, lo.w), make_float2(hi.x, hi.y), make_float2(hi.z, hi.w)};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) c[j] = i ? add2(c[j], v[j]) : v[j];
+    }
+    const float2 info = sm.info[warp][h];
+    const float2 dx0 = make_float2(info.x, info.x - 1.f);
+    float2 m1 = mul2(c[0], dx0), m2 = mul2(m1, dx0);
+#pragma unroll
+    for (int j = 1; j < 4; ++j) {
+      const float2 dx = add2(dx0, f2(-2.f * j)), t = mul2(c[j], dx);
+      m1 = add2(m1, t);
+      m2 = fma2(t, dx, m2);
+    }
+    const float2 m0 = add2(add2(c[0], c[1]), add2(c[2], c[3]));
+    float* acc = grad_acc + 12 * (size_t)__float_as_uint(info.y);
+    atomicAdd(acc + ((0x876415u >> (4 * q)) & 15u), m0.x + m0.y);  // w, w dy, w dy^2, r, g, b
+    if (q < 2) atomicAdd(acc + 3 * q, m1.x + m1.y);                // w dx, w dx dy
+    if (q == 0) atomicAdd(acc + 2, m2.x + m2.y);                   // w dx^2
+  }
+  __syncwarp();  // the rows are rewritten next
+}
+
+// Seven resident blocks per SM (at most 72 registers).  Measured on a B200 (1M-Gaussian view / 16-view
+// batch): five 717 / 9190 us, six 692 / 8800, seven 669 / 8530, eight (64 registers, spilling with the
+// seam) 696 / 9010.
+constexpr int kBlendBwdMinBlocks = 7;
 
 // kRecompute (transmittance checkpointing): the forward stored no per-pixel state; each pixel's
 // final transmittance and last contributor are recomputed first by the forward's own front-to-back
 // pass without colour (forward_pass), which yields the values the forward would have stored.
 template <int kBatch, bool kWrap, bool kRecompute>
 __device__ __forceinline__ void blend_backward_tile(const TileJob& job, const BlendSource& src, float* grad_acc) {
-  static_assert(kBlendPx == 2, "the backward blend packs a thread's two pixels into f32x2 lanes");
-  __shared__ float4 s_a[kBatch];
-  __shared__ float4 s_b[kBatch];
-  __shared__ float4 s_c[kBatch];
-  __shared__ uint32_t s_g[kBatch];
-  __shared__ uint32_t s_warp_last[kBlendWarps];
-  // Two buffered splats (18 rows: one flush round) measured fastest on a B200: larger buffers cost
-  // occupancy (shared memory, registers) faster than they save reduction instructions.  Storing
-  // the values in pairs (five 8-byte stores, two lanes reducing each pair row) measured slower:
-  // 1.03 -> 1.12 ms per 1M-Gaussian view.
-  constexpr int kRedSplats = 2;
-  __shared__ __align__(16) float s_red[kBlendWarps][kRedSplats * 9][kRedStride];
-  __shared__ uint32_t s_red_g[kBlendWarps][kRedSplats];
+  static_assert(kBlendPx == 2, "a thread owns two pixels of one column");
+  __shared__ BackwardSmem<kBatch> sm;
   const BlendPatch patch = BlendPatch::make(job.tile_x, job.tile_y, job.wrap_w);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint2 range = job.range;
-  const uint32_t n = range.y - range.x;
+  const uint32_t n = job.range.y - job.range.x;
 
-  // Per-pixel state of the thread's two pixels, lane x = row py0, lane y = row py0 + 4.
+  // Per-pixel state of the thread's two pixels (rows py0 and py0 + 4).
   const int64_t HW = (int64_t)job.H * job.W;
   float Tf[2], dp[3][2];
   uint32_t lc[2];
   if (kRecompute) {
-    float2 Tr, c0, c1, c2;
-    uint32_t l0, l1;
-    forward_pass<kBatch, kWrap, false>(job, src, patch, s_a, s_b, nullptr, Tr, l0, l1, c0, c1, c2);
-    Tf[0] = patch.inside(0, job.W, job.H) ? Tr.x : 0.f;
-    Tf[1] = patch.inside(1, job.W, job.H) ? Tr.y : 0.f;
-    lc[0] = min(l0, n);
-    lc[1] = min(l1, n);
+    float C[2][3];
+    forward_pass<kBatch, kWrap, false>(job, src, patch, sm.stage, Tf, lc, C);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      if (!patch.inside(i, job.W, job.H)) Tf[i] = 0.f;
+      lc[i] = min(lc[i], n);
+    }
   }
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
@@ -106,9 +129,7 @@ __device__ __forceinline__ void blend_backward_tile(const TileJob& job, const Bl
 #pragma unroll
     for (int ch = 0; ch < 3; ++ch) dp[ch][i] = in ? job.dL_dpix[ch * HW + pix] : 0.f;
   }
-  const float2 T_final = make_float2(Tf[0], Tf[1]);
-  const float2 neg_T_final = make_float2(-Tf[0], -Tf[1]);  // (folded into neg_T_bg below)
-  float2 T = T_final;
+  float2 T = make_float2(Tf[0], Tf[1]);
   const float2 dp0 = make_float2(dp[0][0], dp[0][1]);
   const float2 dp1 = make_float2(dp[1][0], dp[1][1]);
   const float2 dp2 = make_float2(dp[2][0], dp[2][1]);
@@ -116,110 +137,107 @@ __device__ __forceinline__ void blend_backward_tile(const TileJob& job, const Bl
   bgdot = fma2(f2(job.bg[0]), dp0, bgdot);
   bgdot = fma2(f2(job.bg[1]), dp1, bgdot);
   bgdot = fma2(f2(job.bg[2]), dp2, bgdot);
-  const float2 neg_T_bg = mul2(neg_T_final, bgdot);
+  const float2 neg_T_bg = mul2(make_float2(-Tf[0], -Tf[1]), bgdot);
   // the colour of everything behind the current splat, accumulated back to front, enters the
   // gradients only through its dot product with dL/dpix: that product is accumulated instead
   float2 acc_dp = make_float2(0.f, 0.f);
-  const float2 pyf = make_float2(patch.pyf(0), patch.pyf(1));
-
-  float(*red)[kRedStride] = s_red[threadIdx.x >> 5];
-  int nred = 0;  // buffered splats (warp-uniform)
+  const float pyf[2] = {patch.pyf(0), patch.pyf(1)};
 
   const uint32_t warp_last = __reduce_max_sync(kFullMask, max(lc[0], lc[1]));
-  if (lane == 0) s_warp_last[warp] = warp_last;
+  if (lane == 0) sm.last[warp] = warp_last;
+  init_stage(sm.stage);
   __syncthreads();
   uint32_t block_last = 0;
 #pragma unroll
-  for (int w = 0; w < kBlendWarps; ++w) block_last = max(block_last, s_warp_last[w]);
+  for (int w = 0; w < kBlendWarps; ++w) block_last = max(block_last, sm.last[w]);
 
+  const char* slots = reinterpret_cast<const char*>(&sm.stage.d[0][0]);
+  const uint32_t* list = sm.stage.list[warp];
+  int nred = 0;  // buffered splats (warp-uniform)
+  auto blend = [&](uint32_t off, auto plain) {
+    // No per-lane branches: a pixel behind its last contributor, or that this splat does not reach, is
+    // inactive, and the masked G = 0 makes alpha, w and d exactly 0 and 1 / (1 - alpha) exactly 1.
+    constexpr bool kPlain = decltype(plain)::value;
+    const float4* slot = reinterpret_cast<const float4*>(slots + off);
+    const float4 v0 = slot[0], v1 = slot[1], v2 = slot[2];
+    const float x = kWrap ? patch.template center_x<true>(v0.x) : v0.x;
+    const float dx = x - patch.pxf;
+    const float hx = __fmul_rn(v0.z, dx), bx = __fmul_rn(v0.w, dx);
+    const uint32_t at = __float_as_uint(v2.y);
+    const float2 dy = make_float2(v0.y - pyf[0], v0.y - pyf[1]);
+    const float2 q2 = mul2(make_float2(__fmul_rn(v1.x, dy.x), __fmul_rn(v1.x, dy.y)), dy);
+    const float2 power = add2(make_float2(__fmaf_rn(hx, dx, q2.x), __fmaf_rn(hx, dx, q2.y)),
+                              make_float2(__fmul_rn(bx, dy.x), __fmul_rn(bx, dy.y)));
+    float2 G = make_float2(expf(power.x), expf(power.y));
+    const float2 oG = make_float2(__fmul_rn(v1.y, G.x), __fmul_rn(v1.y, G.y));
+    bool act0 = lc[0] >= at && !(oG.x < 1.0f / 255.0f), act1 = lc[1] >= at && !(oG.y < 1.0f / 255.0f);
+    if (!kPlain) {
+      act0 = act0 && !(power.x > 0.0f);
+      act1 = act1 && !(power.y > 0.0f);
+    }
+    // a warp-uniform skip of the gradient arithmetic when no pixel of the warp blends this splat
+    if (!__any_sync(kFullMask, act0 || act1)) return;
+    G = make_float2(act0 ? G.x : 0.f, act1 ? G.y : 0.f);
+    float2 alpha = make_float2(__fmul_rn(v1.y, G.x), __fmul_rn(v1.y, G.y));
+    if (!kPlain) alpha = make_float2(act0 ? fminf(0.99f, alpha.x) : 0.f, act1 ? fminf(0.99f, alpha.y) : 0.f);
+    const float2 onem = fma2(alpha, f2(-1.f), f2(1.f));
+    const float2 inv = make_float2(rcp_approx(onem.x), rcp_approx(onem.y));
+    T = mul2(T, inv);  // transmittance in front of this splat
+    const float2 d = mul2(alpha, T);
+    // (this splat's colour minus the colour behind it) . dL/dpix; the colour behind becomes
+    // alpha c + (1 - alpha) acc, so its product with dL/dpix grows by alpha times this
+    float2 dLda;
+    dLda.x = fmaf(v2.x, dp2.x, fmaf(v1.w, dp1.x, __fmul_rn(v1.z, dp0.x)));
+    dLda.y = fmaf(v2.x, dp2.y, fmaf(v1.w, dp1.y, __fmul_rn(v1.z, dp0.y)));
+    dLda = fma2(acc_dp, f2(-1.f), dLda);
+    acc_dp = fma2(alpha, dLda, acc_dp);
+    dLda = mul2(dLda, T);
+    dLda = fma2(neg_T_bg, inv, dLda);  // the background term -T_final / (1 - alpha) bg.dL/dpix
+    // With q = G dL/dG = o G dL/dalpha and the conic (a, b, c):
+    //   dL/d(delta x) = -q (a dx + b dy), dL/d(delta y) = -q (c dy + b dx),
+    //   dL/d(conic) = -q (dx^2, dx dy, dy^2) / 2.
+    // The sums keep only w, w dx, w dy, w dx^2, ... with w = q / o = G dL/dalpha: the opacity and the
+    // conic (constant over the Gaussian's pixels) and the constant factors are applied once per Gaussian
+    // by the backward preprocess.
+    const float2 w = mul2(G, dLda), wy = mul2(w, dy);
+    float(*red)[kRedStride] = sm.red[warp] + kRedRows * nred;
+    red[0][lane] = w.x + w.y;
+    red[1][lane] = wy.x + wy.y;
+    red[2][lane] = fmaf(wy.x, dy.x, wy.y * dy.y);
+    red[3][lane] = fmaf(d.x, dp0.x, d.y * dp0.y);
+    red[4][lane] = fmaf(d.x, dp1.x, d.y * dp1.y);
+    red[5][lane] = fmaf(d.x, dp2.x, d.y * dp2.y);
+    if (lane == 0) sm.info[warp][nred] = make_float2(x - patch.wx0, v2.z);
+    if (++nred == kRedSplats) {
+      flush_reduction(sm, nred, grad_acc);
+      nred = 0;
+    }
+  };
+  auto blend_list = [&](int cnt, auto plain) {
+#pragma unroll 1
+    for (int i = 0; i < cnt; i += 2) {  // (a padded list may end in a splat that reaches no pixel)
+      const uint2 o = *reinterpret_cast<const uint2*>(list + i);
+      blend(o.x, plain);
+      blend(o.y, plain);
+    }
+  };
   for (int hi = (int)block_last; hi > 0; hi -= kBatch) {
-    const int cnt = min(kBatch, hi);
     __syncthreads();
-    stage_batch(src, range.x, hi, cnt, /*reverse=*/true, s_a, s_b, s_c, s_g);
+    stage_splats<kBatch, kWrap, true, /*kReverse=*/true>(sm.stage, src, job, hi, min(kBatch, hi));
     __syncthreads();
-    for (int k = 0; k * 32 < cnt; ++k) {
-      const int j = k * 32 + lane;
-      bool hit = false;
-      // (the branch skips the test for splats behind every last contributor of the warp: evaluating
-      // it in every lane measured 3 % slower)
-      if (j < cnt && (uint32_t)(hi - 1 - j) < warp_last) hit = patch.template hit<kWrap>(s_a[j], s_b[j]);
-      unsigned m = __ballot_sync(kFullMask, hit);
-      while (m) {
-        const int jj = k * 32 + __ffs(m) - 1;
-        m &= m - 1;
-        const uint32_t pos = (uint32_t)(hi - 1 - jj);
-        // No per-lane branches: a pixel behind its last contributor, or that this splat does not
-        // reach, is inactive through act0 / act1, and the masked alpha = G = 0 makes every one of
-        // its 9 values exactly 0.  The two divergent branches measured on a B200 as 7 % of the
-        // kernel (1.027 -> 0.955 ms per view; only the inner one removed: 1.088).
-        float v[9];
-        bool act0 = pos < lc[0], act1 = pos < lc[1];
-        {
-          const float4 a = s_a[jj];
-          const float4 b = s_b[jj];
-          const float dx = patch.template center_x<kWrap>(a.x) - patch.pxf;
-          const float2 dy = sub2(f2(a.y), pyf);
-          const float2 power = splat_power2(a, b, dx, dy);
-          const float2 G = make_float2(expf(power.x), expf(power.y));
-          const float2 alpha = make_float2(fminf(0.99f, b.y * G.x), fminf(0.99f, b.y * G.y));
-          act0 = act0 && !(power.x > 0.0f) && !(alpha.x < 1.0f / 255.0f);
-          act1 = act1 && !(power.y > 0.0f) && !(alpha.y < 1.0f / 255.0f);
-          // a warp-uniform skip of the gradient arithmetic when no pixel of the warp blends this
-          // splat (measured 0.904 -> 0.898 ms per view against testing after the arithmetic)
-          if (!__any_sync(kFullMask, act0 || act1)) continue;
-          {
-            // A pixel this splat does not touch gets alpha = G = 0 and 1 / (1 - alpha) = 1, which
-            // leaves its state unchanged and contributes zero to every gradient.
-            const float2 ae = make_float2(act0 ? alpha.x : 0.f, act1 ? alpha.y : 0.f);
-            const float2 Ge = make_float2(act0 ? G.x : 0.f, act1 ? G.y : 0.f);
-            const float2 onem = sub2(f2(1.f), ae);
-            const float2 inv = make_float2(act0 ? rcp_approx(onem.x) : 1.f, act1 ? rcp_approx(onem.y) : 1.f);
-            T = mul2(T, inv);  // transmittance in front of this splat
-            const float2 dcd = mul2(ae, T);
-            const float4 cv = s_c[jj];
-            // (this splat's colour minus the colour behind it) . dL/dpix; the colour behind becomes
-            // alpha c + (1 - alpha) acc, so its product with dL/dpix grows by alpha times this
-            float2 c_dp = mul2(f2(cv.x), dp0);
-            c_dp = fma2(f2(cv.y), dp1, c_dp);
-            c_dp = fma2(f2(cv.z), dp2, c_dp);
-            float2 dLda = sub2(c_dp, acc_dp);
-            acc_dp = fma2(ae, dLda, acc_dp);
-            dLda = mul2(dLda, T);
-            dLda = fma2(neg_T_bg, inv, dLda);  // the background term -T_final / (1 - alpha) bg.dL/dpix
-            // With q = G dL/dG = o G dL/dalpha and the conic (a, b, c):
-            //   dL/d(delta x) = -q (a dx + b dy), dL/d(delta y) = -q (c dy + b dx),
-            //   dL/d(conic) = -q (dx^2, dx dy, dy^2) / 2.
-            // The per-pixel sums keep only w dx, w dy, w dx^2, ... with w = G dL/dalpha = q / o:
-            // the opacity and the conic (constant over the Gaussian's pixels) and the constant
-            // factors -W/2, -H/2 and -1/2 are applied once per Gaussian by the backward
-            // preprocess.  The thread's two pixels share dx, so the sums over them factor through
-            // sum w, sum w dy and sum w dy^2.
-            const float2 w5 = mul2(Ge, dLda);
-            const float2 q = w5;
-            const float2 qy = mul2(q, dy);
-            const float qs = q.x + q.y, qdy = qy.x + qy.y;
-            v[0] = dx * qs;
-            v[1] = qdy;
-            v[2] = dx * v[0];
-            v[3] = dx * qdy;
-            v[4] = fmaf(qy.x, dy.x, qy.y * dy.y);
-            v[5] = w5.x + w5.y;
-            v[6] = fmaf(dcd.x, dp0.x, dcd.y * dp0.y);
-            v[7] = fmaf(dcd.x, dp1.x, dcd.y * dp1.y);
-            v[8] = fmaf(dcd.x, dp2.x, dcd.y * dp2.y);
-          }
-        }
-#pragma unroll
-        for (int q = 0; q < 9; ++q) red[nred * 9 + q][lane] = v[q];
-        if (lane == 0) s_red_g[warp][nred] = s_g[jj];
-        if (++nred == kRedSplats) {
-          flush_reduction(red, s_red_g[warp], nred, grad_acc, lane);
-          nred = 0;
-        }
-      }
+    const int first = max(0, hi - (int)warp_last);  // slots before it lie behind every last contributor
+#pragma unroll 1
+    for (int from = 0; from < kBatch; from += BlendStage<kBatch>::kListSplats) {
+      if (first >= from + BlendStage<kBatch>::kListSplats) continue;
+      bool special;
+      const int cnt = list_candidates(sm.stage, from, first, special);
+      if (special)
+        blend_list(cnt, std::false_type{});
+      else
+        blend_list(cnt, std::true_type{});
     }
   }
-  if (nred) flush_reduction(red, s_red_g[warp], nred, grad_acc, lane);
+  if (nred) flush_reduction(sm, nred, grad_acc);
 }
 
 // One view: block (x, y) back-propagates tile (x, y).
