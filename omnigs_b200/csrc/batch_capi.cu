@@ -149,6 +149,7 @@ BatchRenderParams render_params(const BatchParams& p, const BatchPlan& plan, voi
   r.P = p.P;
   r.V = p.V;
   r.ranges = at<uint2>(state, L.ranges);
+  r.block_tiles = orders_tiles(p.P, p.V, plan.tiles) ? at<uint4>(state, L.depth_lookback) : nullptr;
   r.point_list = point_list;
   r.capacity = capacity;
   r.splat = p.splat;
@@ -236,6 +237,7 @@ int omnigs_batch_render(const OmnigsBatchArgs* a, void* state, size_t state_byte
   b.layout = BL;
   b.capacity = capacity;
   b.ranges = at<uint2>(state, L.ranges);
+  b.block_tiles = orders_tiles(a->P, a->V, plan.tiles) ? reinterpret_cast<uint4*>(b.depth_lookback) : nullptr;
   b.hdr = bp.hdr;
   b.out = fin;
   uint32_t* tvals[2] = {at<uint32_t>(binning, BL.tvals0), at<uint32_t>(binning, BL.tvals1)};

@@ -823,13 +823,13 @@ __device__ __forceinline__ uint32_t warp_lower_bound(const uint32_t* words, uint
 }
 
 template <bool kAll>
-__device__ __forceinline__ BinPart bin_part(const TileListParams& p) {
+__device__ __forceinline__ BinPart bin_part(const TileListParams& p, uint32_t grid_block) {
   __shared__ uint32_t s_bounds[2];
   const TileGrid& g = p.grid;
   uint32_t view = 0;
 #pragma unroll 1
   for (int v = 1; v < g.V; ++v)
-    if (g.block_base[v] <= blockIdx.x) view = (uint32_t)v;
+    if (g.block_base[v] <= grid_block) view = (uint32_t)v;
   BinPart b;
   b.gx = g.gx[view];
   b.gy = g.gy[view];
@@ -838,7 +838,7 @@ __device__ __forceinline__ BinPart bin_part(const TileListParams& p) {
   b.counts0 = g.count_base[view];
   b.parts = g.parts[view];
   const uint32_t per_bin = (b.parts + kListWarps - 1u) / kListWarps;  // blocks
-  const uint32_t block = blockIdx.x - g.block_base[view], local = block / per_bin;
+  const uint32_t block = grid_block - g.block_base[view], local = block / per_bin;
   b.part = (block - local * per_bin) * kListWarps + (threadIdx.x >> 5);
   const uint32_t bx = (uint32_t)bins_x(b.gx);
   b.ty0 = (int)(local / bx) * kBinH;
@@ -885,7 +885,7 @@ __global__ void __launch_bounds__(kListThreads) tile_count_kernel(const __grid_c
   const bool fit = instances_fit(p.hdr, p.capacity);
   if (kAll && !fit && blockIdx.x == 0 && threadIdx.x == 0)
     atomicOr(&p.hdr->status, kStatusCapacity);  // (the scan flags it where there is one)
-  BinPart b = bin_part<kAll>(p);
+  BinPart b = bin_part<kAll>(p, blockIdx.x);
   if (b.part >= b.parts) return;
   if (!fit) b.end = b.first;
   uint32_t acc[kBinH][2] = {};
@@ -998,6 +998,95 @@ __global__ void __launch_bounds__(kTileScanThreads) tile_scan_kernel(const __gri
     atomicOr(&p.hdr->status, kStatusInconsistent);
 }
 
+// The order in which the blends take the tiles (block_tiles): heaviest first within each kOrderTiles tiles,
+// in eight classes of list length relative to their mean, in tile order inside a class (neighbours share
+// splats, and lists near the mean stay together).  Poles and dense regions hold lists many times the mean,
+// and one that starts last leaves the chip idle.  A segment is one block of the fill's launch, ahead of
+// the others and hidden behind them.  Measured on a B200, blends of a batch of views of a scene at the
+// poles, in tile order / ordered: 366 + 520 / 300 + 449 us; views with even lists change by less than 1 %.
+// (Rows from both ends inwards, without lengths: the same at the poles, but 4 % slower on even lists;
+// ordered by the scan's one block: 5 us of every view.)
+constexpr int kLoadClasses = 8;
+constexpr uint32_t kOrderTiles = 8192;
+constexpr uint32_t kOrderItems = kOrderTiles / kListThreads;  // per thread
+static_assert(kOrderTiles < 65536, "a class of one segment fits in 16 bits");
+
+__device__ __forceinline__ int load_class(uint32_t count, float mean) {
+  const float x = (float)count;
+  return (x < 4.f * mean) + (x < 2.83f * mean) + (x < 2.f * mean) + (x < 1.41f * mean) + (x < mean) +
+         (x < 0.71f * mean) + (x < 0.35f * mean);
+}
+
+// Tiles per class, as 16-bit fields.
+struct ClassCounts {
+  unsigned long long lo, hi;
+  __device__ __forceinline__ void add(int c, uint32_t n) {
+    const unsigned long long x = (unsigned long long)n << (16 * (c & 3));
+    lo += c < 4 ? x : 0ull;
+    hi += c < 4 ? 0ull : x;
+  }
+  __device__ __forceinline__ uint32_t at(int c) const { return (uint32_t)((c < 4 ? lo : hi) >> (16 * (c & 3))) & 0xffffu; }
+  __device__ __forceinline__ ClassCounts operator+(const ClassCounts& o) const { return {lo + o.lo, hi + o.hi}; }
+  __device__ __forceinline__ ClassCounts operator-(const ClassCounts& o) const { return {lo - o.lo, hi - o.hi}; }
+};
+
+__device__ __forceinline__ void order_tiles(const TileListParams& p, uint32_t segment) {
+  __shared__ uint32_t s_sum[kListWarps];
+  __shared__ ClassCounts s_class[kListWarps];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t base = segment * kOrderTiles, n = min(p.grid.num_tiles - base, kOrderTiles);
+  const uint32_t t0 = base + threadIdx.x * kOrderItems, t1 = min(t0 + kOrderItems, base + n);
+  auto count = [&](uint32_t t) {
+    const uint2 r = p.ranges[t];
+    return r.y - r.x;
+  };
+  uint32_t sum = 0;
+#pragma unroll 8
+  for (uint32_t t = t0; t < t1; ++t) sum += count(t);
+  sum = __reduce_add_sync(kFullMask, sum);
+  if (lane == 0) s_sum[warp] = sum;
+  __syncthreads();
+  sum = 0;
+#pragma unroll
+  for (int w = 0; w < kListWarps; ++w) sum += s_sum[w];
+  const float mean = (float)sum / (float)n;
+  ClassCounts own{0, 0};
+#pragma unroll 8
+  for (uint32_t t = t0; t < t1; ++t) own.add(load_class(count(t), mean), 1u);
+  ClassCounts at = own;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned long long lo = __shfl_up_sync(kFullMask, at.lo, o), hi = __shfl_up_sync(kFullMask, at.hi, o);
+    if (lane >= o) at = at + ClassCounts{lo, hi};
+  }
+  if (lane == 31) s_class[warp] = at;
+  __syncthreads();
+  at = at - own;
+  ClassCounts all{0, 0};
+#pragma unroll
+  for (int w = 0; w < kListWarps; ++w) {
+    const ClassCounts c = s_class[w];
+    if (w < warp) at = at + c;
+    all = all + c;
+  }
+  uint32_t heavier = 0;  // each class begins behind the heavier ones
+#pragma unroll
+  for (int k = 0; k < kLoadClasses; ++k) {
+    at.add(k, heavier);
+    heavier += all.at(k);
+  }
+  const uint32_t w = (uint32_t)p.tile_width;
+  uint32_t y = w ? t0 / w : 0u, x = t0 - y * w;
+#pragma unroll 4
+  for (uint32_t t = t0; t < t1; ++t) {
+    const uint2 r = p.ranges[t];
+    const int k = load_class(r.y - r.x, mean);
+    p.block_tiles[base + at.at(k)] = make_uint4(r.x, r.y, y << 16 | x, 0u);
+    at.add(k, 1u);
+    if (++x == w) x = 0, ++y;
+  }
+}
+
 // Appends a part of a bin's pairs to the lists of its 32 tiles.  A warp queues its pairs by the bin's four
 // tile rows (a pair covers one or two of them on average, so a walk per row would waste most lanes) and
 // appends 32 of a row at a time to its eight lists: a pair's place is the list's next one plus the
@@ -1014,8 +1103,10 @@ template <bool kAll>
 __global__ void __launch_bounds__(kListThreads) tile_fill_kernel(const __grid_constant__ TileListParams p) {
   chain_begin();
   __shared__ FillQueue s_queue[kListWarps];
+  const uint32_t segments = p.block_tiles ? (p.grid.num_tiles + kOrderTiles - 1) / kOrderTiles : 0u;
+  if (blockIdx.x < segments) return order_tiles(p, blockIdx.x);
   if (!instances_fit(p.hdr, p.capacity)) return;
-  const BinPart b = bin_part<kAll>(p);
+  const BinPart b = bin_part<kAll>(p, blockIdx.x - segments);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned lt = (1u << lane) - 1u;
   FillQueue& q = s_queue[warp];
@@ -1191,7 +1282,8 @@ void launch_tile_lists(const TileListParams& p, cudaStream_t s) {
   launch_chained(p.chained, all ? tile_count_kernel<true> : tile_count_kernel<false>, g.num_blocks, kListThreads, 0, s, p);
   const unsigned scan = p.counts ? (g.num_tiles + kTileScanBlock - 1) / kTileScanBlock : 1u;
   launch_chained(p.chained, tile_scan_kernel, scan, kTileScanThreads, 0, s, p);
-  launch_chained(p.chained, all ? tile_fill_kernel<true> : tile_fill_kernel<false>, g.num_blocks, kListThreads, 0, s, p);
+  const unsigned order = p.block_tiles ? (g.num_tiles + kOrderTiles - 1) / kOrderTiles : 0u;
+  launch_chained(p.chained, all ? tile_fill_kernel<true> : tile_fill_kernel<false>, g.num_blocks + order, kListThreads, 0, s, p);
   launch_chained(p.chained, tile_keys_kernel, (g.num_tiles + 7) / 8, 256, 0, s, p);
 }
 

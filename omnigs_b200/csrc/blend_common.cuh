@@ -33,6 +33,17 @@ struct TileJob {
   float wrap_w;             // image width when blending across the longitude seam, else 0
 };
 
+// The range and tile (TileListParams::block_tiles) that a block blends.  A list that gives both costs a block
+// no more dependent loads than its range alone.
+__device__ __forceinline__ uint3 block_tile(const uint4* block_tiles, const uint2* ranges, uint32_t block, uint32_t own) {
+  if (block_tiles != nullptr) {
+    const uint4 w = block_tiles[block];
+    return make_uint3(w.x, w.y, w.z);
+  }
+  const uint2 r = ranges[block];
+  return make_uint3(r.x, r.y, own);
+}
+
 // The sorted instance list and the per-record splat data it points into.
 struct BlendSource {
   const uint32_t* point_list;  // record index per instance
@@ -42,9 +53,8 @@ struct BlendSource {
   int64_t capacity;            // instances the list can hold; larger range bounds are rejected
 };
 
-// Tile range read from the ranges table, emptied if inconsistent with the list's capacity.
-__device__ __forceinline__ uint2 checked_range(const uint2* ranges, uint32_t tile, int64_t capacity) {
-  uint2 range = ranges[tile];
+// A tile's range, emptied if inconsistent with the list's capacity.
+__device__ __forceinline__ uint2 checked_range(uint2 range, int64_t capacity) {
   if (range.y > (uint64_t)capacity || range.x > range.y) range = make_uint2(0, 0);
   return range;
 }
@@ -67,12 +77,17 @@ struct BlendPatch {
     return kWrap ? ax - wrap_w * rintf((ax - wcx) / wrap_w) : ax;
   }
 
-  static __device__ __forceinline__ BlendPatch make(int tile_x, int tile_y, float wrap_w = 0.f) {
-    return of_warp(tile_x, tile_y, threadIdx.x >> 5, wrap_w);
+  // The bounds of a warp's patch in the tile whose first pixel is `origin`.
+  static __device__ __forceinline__ BlendPatch bounds(float2 origin, int warp, float wrap_w) {
+    BlendPatch b{};
+    b.wx0 = origin.x + (float)((warp & 1) * 8);
+    b.wy0 = origin.y + (float)((warp >> 1) * kPatchRows);
+    b.wcx = b.wx0 + 3.5f;
+    b.wrap_w = wrap_w;
+    return b;
   }
-  // The patch of another warp of the block (its pixels those of this thread's lane).
-  static __device__ __forceinline__ BlendPatch of_warp(int tile_x, int tile_y, int warp, float wrap_w) {
-    const int lane = threadIdx.x & 31;
+  static __device__ __forceinline__ BlendPatch make(int tile_x, int tile_y, float wrap_w = 0.f) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int wx0 = tile_x * 16 + (warp & 1) * 8;
     const int wy0 = tile_y * 16 + (warp >> 1) * kPatchRows;
     BlendPatch b;
@@ -159,27 +174,36 @@ struct BlendStage {
   uint32_t list[kBlendWarps][kListSplats + 4];  // byte offsets of a warp's candidates, padded
   uint32_t mask[kBatch / 32][kBlendWarps];      // candidates of a group of 32 by warp
   uint32_t special[kBatch / 32];                // the group's splats that are not plain (plain_splat)
+  float2 origin;                                // the tile's first pixel
+  uint32_t first;                               // its range's begin
+  uint32_t tile;                                // block_tile's (the forward's; these three are here because
+                                                // registers are scarce: 1-3 % of the blends)
 };
 
 // Must be followed by a block barrier.
 template <int kBatch>
-__device__ __forceinline__ void init_stage(BlendStage<kBatch>& st) {
+__device__ __forceinline__ void init_stage(BlendStage<kBatch>& st, const TileJob& job) {
+  if (threadIdx.x == 0) {
+    st.origin = make_float2((float)(job.tile_x * 16), (float)(job.tile_y * 16));
+    st.first = job.range.x;
+  }
   if (threadIdx.x < kSlotBytes / 16) st.d[kBatch][threadIdx.x] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
-// Stages instances [base, base + cnt) of the tile's list (from the back when kReverse: slot t holds
+// Stages instances [base, base + cnt) of the tile's list, which begins at `first` (from the back when kReverse: slot t holds
 // position base - 1 - t, with base the exclusive upper end) with their patch masks; the colour only
 // with kColor.
 template <int kBatch, bool kWrap, bool kColor, bool kReverse>
 __device__ __forceinline__ void stage_splats(BlendStage<kBatch>& st, const BlendSource& src, const TileJob& job,
-                                             int base, int cnt) {
+                                             uint32_t first, int base, int cnt) {
   const int lane = threadIdx.x & 31;
+  const float2 origin = st.origin;
 #pragma unroll 1
   for (int t = threadIdx.x; t < kBatch; t += kBlendThreads) {
     bool hits[kBlendWarps] = {}, special = false;
     if (t < cnt) {
       const uint32_t pos = kReverse ? (uint32_t)(base - 1 - t) : (uint32_t)(base + t);
-      const uint32_t g = src.point_list[job.range.x + pos];
+      const uint32_t g = src.point_list[first + pos];
       if (g < src.num_records) {  // (always, for a consistent instance list)
         const float4 a = src.splat[2 * (size_t)g], b = src.splat[2 * (size_t)g + 1];
         const float4 c = kColor ? src.color[g] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -189,7 +213,7 @@ __device__ __forceinline__ void stage_splats(BlendStage<kBatch>& st, const Blend
         special = !plain_splat(a, b);
 #pragma unroll
         for (int w = 0; w < kBlendWarps; ++w)
-          hits[w] = BlendPatch::of_warp(job.tile_x, job.tile_y, w, job.wrap_w).template hit<kWrap>(a, b);
+          hits[w] = BlendPatch::bounds(origin, w, job.wrap_w).template hit<kWrap>(a, b);
       }
     }
     const unsigned ms = __ballot_sync(kFullMask, special);
@@ -283,7 +307,7 @@ __device__ __forceinline__ void forward_pixel(float alpha, float power, float te
 // issue slot) where both factors differ by pixel, and scalar where one is the splat's: broadcasting that
 // into a register pair costs the moves that packing saves.  Bound by instruction issue.  Measured on a
 // B200 (1M-Gaussian 2048x1024 view / 16-view batch) against a warp testing every staged splat itself and
-// walking the ballots' bits: 424 -> 410 us / 5.20 -> 5.10 ms.
+// walking the ballots' bits: 424 -> 406 us / 5.20 -> 5.16 ms.
 template <int kBatch, bool kWrap, bool kColor>
 __device__ __forceinline__ void forward_pass(const TileJob& job, const BlendSource& src, const BlendPatch& patch,
                                              BlendStage<kBatch>& st, float T[2], uint32_t lc[2], float C[2][3]) {
@@ -298,7 +322,8 @@ __device__ __forceinline__ void forward_pass(const TileJob& job, const BlendSour
   const int n = (int)(job.range.y - job.range.x);
   const char* slots = reinterpret_cast<const char*>(&st.d[0][0]);
   const uint32_t* list = st.list[threadIdx.x >> 5];
-  init_stage(st);
+  init_stage(st, job);
+  __syncthreads();
 
   auto blend = [&](uint32_t off, auto plain) {
     constexpr bool kPlain = decltype(plain)::value;
@@ -331,7 +356,7 @@ __device__ __forceinline__ void forward_pass(const TileJob& job, const BlendSour
   };
   for (int base = 0; base < n; base += kBatch) {
     if (__syncthreads_and(T[0] < 0.f && T[1] < 0.f)) break;
-    stage_splats<kBatch, kWrap, kColor, /*kReverse=*/false>(st, src, job, base, min(kBatch, n - base));
+    stage_splats<kBatch, kWrap, kColor, /*kReverse=*/false>(st, src, job, st.first, base, min(kBatch, n - base));
     __syncthreads();
 #pragma unroll 1
     for (int from = 0; from < kBatch; from += BlendStage<kBatch>::kListSplats) {
@@ -348,9 +373,26 @@ __device__ __forceinline__ void forward_pass(const TileJob& job, const BlendSour
   T[1] = fabsf(T[1]);
 }
 
-// Block -> (view, tile) of a batched blend launch: blocks run over the views' tiles in the order
+// Tile `tile` (y << 16 | x) of a view.
+__device__ __forceinline__ TileJob tile_job(const RenderParams& p, uint32_t tile, uint2 range) {
+  TileJob job;
+  job.tile_x = (int)(tile & 0xffffu);
+  job.tile_y = (int)(tile >> 16);
+  job.W = p.W;
+  job.H = p.H;
+  job.range = checked_range(range, p.capacity);
+  job.bg = p.bg;
+  job.out_color = p.out_color;
+  job.final_T = p.final_T;
+  job.n_contrib = p.n_contrib;
+  job.dL_dpix = p.dL_dpix;
+  job.wrap_w = 0.f;
+  return job;
+}
+
+// The view and tile of global tile `block` of a batched blend: the tiles run over the views in the order
 // of tile_base (the host lays the views out heaviest tiles first).
-__device__ __forceinline__ TileJob batch_tile_job(const BatchRenderParams& p, uint32_t block) {
+__device__ __forceinline__ TileJob tile_job(const BatchRenderParams& p, uint32_t block, uint2 range) {
   int v = p.tile_order[0];
 #pragma unroll 1
   for (int k = 1; k < p.V; ++k) {
@@ -364,7 +406,7 @@ __device__ __forceinline__ TileJob batch_tile_job(const BatchRenderParams& p, ui
   job.tile_x = (int)(local - (uint32_t)job.tile_y * (uint32_t)bv.gx);
   job.W = bv.W;
   job.H = bv.H;
-  job.range = checked_range(p.ranges, block, p.capacity);
+  job.range = checked_range(range, p.capacity);
   job.bg = p.backgrounds + 3 * v;
   job.out_color = bv.out_color;
   job.final_T = p.final_T + bv.pixel_base;

@@ -235,6 +235,8 @@ int run_binning(BinningPass& b, cudaStream_t s) {
   t.out_keys = keys[b.out];
   t.out_vals = vals[b.out];
   t.ranges = b.ranges;
+  t.block_tiles = b.block_tiles;
+  t.tile_width = b.tile_width;
   t.capacity = b.capacity;
   t.hdr = b.hdr;
   if (counts != nullptr && !totals_there && cudaMemsetAsync(totals, 0, sizeof(uint32_t) * g.num_tiles, s) != cudaSuccess)
@@ -481,6 +483,8 @@ int render_impl(const OmnigsLonlatForwardArgs* a, void* geom, size_t geom_bytes,
   b.layout = BL;
   b.capacity = capacity;
   b.ranges = ranges;
+  b.tile_width = gx;
+  b.block_tiles = orders_tiles(a->P, 1, b.grid.num_tiles) ? reinterpret_cast<uint4*>(b.depth_lookback) : nullptr;
   b.hdr = hdr;
   b.out = fin;
   b.max_spins = probe != nullptr ? probe->max_spins : 0;
@@ -494,6 +498,7 @@ int render_impl(const OmnigsLonlatForwardArgs* a, void* geom, size_t geom_bytes,
   r.gx = gx;
   r.gy = gy;
   r.ranges = ranges;
+  r.block_tiles = b.block_tiles;
   r.point_list = at<uint32_t>(binning, fin ? BL.tvals1 : BL.tvals0);
   r.chained = b.small;
   r.capacity = capacity;
@@ -626,6 +631,7 @@ int omnigs_lonlat_backward(const OmnigsLonlatBackwardArgs* a, void* geom, size_t
   r.gx = gx;
   r.gy = gy;
   r.ranges = at<uint2>(image, IL.ranges);
+  r.block_tiles = orders_tiles(a->P, 1, (int64_t)gx * gy) ? at<uint4>(geom, GL.depth_lookback) : nullptr;
   r.point_list = at<uint32_t>(binning, fin ? BL.tvals1 : BL.tvals0);
   r.capacity = capacity;
   r.splat = at<float4>(geom, GL.splat);

@@ -88,6 +88,8 @@ struct BinningPass {
   BinningLayout layout;
   int64_t capacity;
   uint2* ranges;
+  uint4* block_tiles;            // (TileListParams)
+  int tile_width;
   GeomHeader* hdr;
   int out;                       // binning buffer (0 or 1) that receives the sorted list
   int max_spins;                 // look-back probe: wait limit, and stop after the scan (0: a real pass)

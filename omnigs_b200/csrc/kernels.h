@@ -129,6 +129,8 @@ struct TileListParams {
   uint32_t* out_keys;          // [capacity] sorted tile ids and record indices
   uint32_t* out_vals;
   uint2* ranges;               // [num_tiles]
+  uint4* block_tiles;          // [num_tiles] the blends' tiles by block (orders_tiles), or NULL: {range, tile}
+  int tile_width;              // not 0: block_tiles' tiles as (y << 16 | x) of a view that many tiles wide
   int64_t capacity;
   GeomHeader* hdr;
 };
@@ -157,6 +159,7 @@ struct BeginParams {
 struct RenderParams {
   int P, W, H, gx, gy;
   const uint2* ranges;
+  const uint4* block_tiles;  // [gx gy] tiles by block (TileListParams), or NULL: in order
   const uint32_t* point_list;
   int64_t capacity;
   const float4* splat;
@@ -256,6 +259,7 @@ struct BatchGrads {
 struct BatchRenderParams {
   int P, V;
   const uint2* ranges;          // [total tiles]
+  const uint4* block_tiles;     // [total tiles] tiles by block (TileListParams), or NULL: in order
   const uint32_t* point_list;   // record indices
   int64_t capacity;
   const float4* splat;

@@ -5,7 +5,8 @@
 // library lays them out for its own kernels:
 //
 //   geometry (per Gaussian, P):  header | duplicate-scan look-back u64[P/256] |
-//                                depth-sort look-back u32[4][sort tiles][256] |
+//                                depth-sort look-back u32[4][sort tiles][256], then the blends' tile
+//                                order uint4[tiles] (orders_tiles) |
 //                                splat records float4[2P] {x, y, conic a, b}
 //                                {conic c, opacity, cull threshold, conic determinant} |
 //                                colour float4[P] {r, g, b, clamp bits} | depth f32[P] |
@@ -81,6 +82,14 @@ inline int64_t sort_blocks(int64_t items, int64_t segs) {
   return (small_sort(items, segs) ? small_sort_tiles(items) : sort_tiles(items)) * segs;
 }
 
+// Views whose tiles the blends take heaviest first (binning.cu): the order lies in the depth sort's
+// look-back memory, which the sort has read by then.  Few Gaussians have no such sort, and their blends end
+// with the launch, not with a tile.
+constexpr int kRankMaxP = 12288;
+inline bool orders_tiles(int64_t P, int64_t V, int64_t tiles) {
+  return P > kRankMaxP && kDepthPasses * sort_blocks(P, V) * kRadix >= 4 * tiles;
+}
+
 struct GeomLayout {
   size_t header, dup_scan, depth_lookback, zero_end, splat, color, depth, tiles_touched, dkeys0,
       dkeys1, dvals0, dvals1, grad_acc, total;
@@ -137,7 +146,6 @@ OMNIGS_HD inline int bins_y(int gy) { return (gy + kBinH - 1) / kBinH; }
 
 // Up to kRankMaxP Gaussians per view the depth order comes from counting, and up to kWholeMaxPairs
 // (Gaussian, bin) combinations every bin reads its view's whole depth order (binning.cu).
-constexpr int kRankMaxP = 12288;
 constexpr int64_t kWholeMaxPairs = int64_t(1) << 20;
 
 // The duplicate pass writes its list in blocks of kEmitBlock pairs; its scan records, per such block, the
@@ -185,7 +193,7 @@ struct BinningLayout {
 // per-pixel arrays hold the views' pixels back to back, ranges the views' tiles back to back.
 //
 //   header | instances per view u64[32] | duplicate-scan look-back u64[VP/256] |
-//   depth-sort look-back u32[4][V sort tiles(P)][256] | depth histograms u32[V][4][256] |
+//   depth-sort look-back u32[4][V sort tiles(P)][256], then the blends' tile order uint4[tiles] | depth histograms u32[V][4][256] |
 //   radii i32[VP] | splat records float4[2VP] | colour float4[VP] | depth f32[VP] |
 //   depth-sort keys/values u32[4][VP] | gradient accumulators float4[3VP] |
 //   final transmittance f32[pixels] | last contributor u32[pixels] | tile ranges uint2[tiles]

@@ -21,7 +21,7 @@
 // Bound by instruction issue (79 % of the slots on a 400k-Gaussian view).  Measured on a B200
 // (300k / 1M-Gaussian 2048x1024 view / 16-view batch): 315 / 760 / 9710 us with the warps scanning ballots
 // of their own tests, every sum in a row of its own (nine, two splats a flush) and the clamp and sign
-// tests for every splat; 271 / 669 / 8530 us now.  The same sums on the tensor cores (mma.m16n8k8, TF32
+// tests for every splat; 271 / 670 / 8480 us now.  The same sums on the tensor cores (mma.m16n8k8, TF32
 // operands split in two) took 319 / 812 / 10600: fewer instructions, but the fragments' registers and
 // shared memory leave six blocks per SM.
 #include "blend_common.cuh"
@@ -145,7 +145,7 @@ __device__ __forceinline__ void blend_backward_tile(const TileJob& job, const Bl
 
   const uint32_t warp_last = __reduce_max_sync(kFullMask, max(lc[0], lc[1]));
   if (lane == 0) sm.last[warp] = warp_last;
-  init_stage(sm.stage);
+  init_stage(sm.stage, job);
   __syncthreads();
   uint32_t block_last = 0;
 #pragma unroll
@@ -223,7 +223,7 @@ __device__ __forceinline__ void blend_backward_tile(const TileJob& job, const Bl
   };
   for (int hi = (int)block_last; hi > 0; hi -= kBatch) {
     __syncthreads();
-    stage_splats<kBatch, kWrap, true, /*kReverse=*/true>(sm.stage, src, job, hi, min(kBatch, hi));
+    stage_splats<kBatch, kWrap, true, /*kReverse=*/true>(sm.stage, src, job, job.range.x, hi, min(kBatch, hi));
     __syncthreads();
     const int first = max(0, hi - (int)warp_last);  // slots before it lie behind every last contributor
 #pragma unroll 1
@@ -240,29 +240,21 @@ __device__ __forceinline__ void blend_backward_tile(const TileJob& job, const Bl
   if (nred) flush_reduction(sm, nred, grad_acc);
 }
 
-// One view: block (x, y) back-propagates tile (x, y).
+// One view: a block back-propagates one tile (block_tile).
 template <int kBatch, bool kRecompute>
 __global__ void __launch_bounds__(kBlendThreads, kBlendBwdMinBlocks) render_backward_kernel(RenderParams p) {
-  TileJob job;
-  job.tile_x = blockIdx.x;
-  job.tile_y = blockIdx.y;
-  job.W = p.W;
-  job.H = p.H;
-  job.range = checked_range(p.ranges, blockIdx.y * p.gx + blockIdx.x, p.capacity);
-  job.bg = p.bg;
-  job.out_color = nullptr;
-  job.final_T = p.final_T;
-  job.n_contrib = p.n_contrib;
-  job.dL_dpix = p.dL_dpix;
-  job.wrap_w = 0.f;
+  const uint3 tile = block_tile(p.block_tiles, p.ranges, blockIdx.y * p.gx + blockIdx.x, blockIdx.y << 16 | blockIdx.x);
+  const TileJob job = tile_job(p, tile.z, make_uint2(tile.x, tile.y));
   blend_backward_tile<kBatch, false, kRecompute>(job, BlendSource{p.point_list, p.splat, p.color, (uint32_t)p.P, p.capacity},
                                                  p.grad_acc);
 }
 
-// All views of a batch in one launch: block b back-propagates global tile b.
+// All views of a batch in one launch: a block back-propagates one of the views' tiles.
 template <int kBatch, bool kWrap>
 __global__ void __launch_bounds__(kBlendThreads, kBlendBwdMinBlocks) batch_render_backward_kernel(const __grid_constant__ BatchRenderParams p) {
-  const TileJob job = batch_tile_job(p, blockIdx.x);
+  const uint3 tile = block_tile(p.block_tiles, p.ranges, blockIdx.x, blockIdx.x);
+  if (tile.z >= p.total_tiles) return;  // (never, after a binning)
+  const TileJob job = tile_job(p, tile.z, make_uint2(tile.x, tile.y));
   blend_backward_tile<kBatch, kWrap, false>(job, BlendSource{p.point_list, p.splat, p.color, (uint32_t)p.P * (uint32_t)p.V, p.capacity},
                                             p.grad_acc);
 }

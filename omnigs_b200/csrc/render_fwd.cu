@@ -22,19 +22,25 @@
 namespace omnigs {
 namespace {
 
-// Eight resident blocks per SM (at most 64 registers) measured fastest on a B200 (1M-Gaussian 2048x1024
-// view, six / eight / ten / twelve: 407 / 410 / 420 / 434 us; 16-view batch 5.12 / 5.10 / 5.03 / 5.15 ms;
-// 300k Gaussians 157 / 160 / 168 / 174 us).
-constexpr int kBlendFwdMinBlocks = 8;
+// Resident blocks per SM, one view / a batch (at most 72 / 64 registers).  Measured on a B200: 1M-Gaussian
+// 2048x1024 view, six / seven / eight / ten: 415 / 406 / 415 / 420 us, 3M Gaussians 1006 / 985 / 1001 / 1019;
+// 16-view batch 5.44 / 5.35 / 5.16 / 5.25 ms, views at the poles 325 / 314 / 302 / 318 us.
+constexpr int kBlendFwdMinBlocks = 7, kBatchFwdMinBlocks = 8;
 
-template <int kBatch, bool kWrap>
-__device__ __forceinline__ void blend_forward_tile(const TileJob& job, const BlendSource& src) {
+// Blends the tile that make_job(tile, range) describes.  The job is made again for the stores: its pointers
+// would hold a dozen of the loop's registers.
+template <int kBatch, bool kWrap, class MakeJob>
+__device__ __forceinline__ void blend_forward_tile(const MakeJob& make_job, uint3 tile, const BlendSource& src) {
   __shared__ __align__(16) BlendStage<kBatch> stage;
-  const BlendPatch patch = BlendPatch::make(job.tile_x, job.tile_y, job.wrap_w);
   float T[2], C[2][3];
   uint32_t lc[2];
-  forward_pass<kBatch, kWrap, true>(job, src, patch, stage, T, lc, C);
-
+  {
+    const TileJob job = make_job(tile.z, make_uint2(tile.x, tile.y));
+    if (threadIdx.x == 0) stage.tile = tile.z;
+    forward_pass<kBatch, kWrap, true>(job, src, BlendPatch::make(job.tile_x, job.tile_y, job.wrap_w), stage, T, lc, C);
+  }
+  const TileJob job = make_job(stage.tile, make_uint2(0u, 0u));
+  const BlendPatch patch = BlendPatch::make(job.tile_x, job.tile_y, job.wrap_w);
   const int64_t HW = (int64_t)job.H * job.W;
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
@@ -49,30 +55,22 @@ __device__ __forceinline__ void blend_forward_tile(const TileJob& job, const Ble
   }
 }
 
-// One view: block (x, y) blends tile (x, y).
+// One view: a block blends one tile (block_tile).
 template <int kBatch>
 __global__ void __launch_bounds__(kBlendThreads, kBlendFwdMinBlocks) render_forward_kernel(RenderParams p) {
   chain_begin();
-  TileJob job;
-  job.tile_x = blockIdx.x;
-  job.tile_y = blockIdx.y;
-  job.W = p.W;
-  job.H = p.H;
-  job.range = checked_range(p.ranges, blockIdx.y * p.gx + blockIdx.x, p.capacity);
-  job.bg = p.bg;
-  job.out_color = p.out_color;
-  job.final_T = p.final_T;
-  job.n_contrib = p.n_contrib;
-  job.dL_dpix = nullptr;
-  job.wrap_w = 0.f;
-  blend_forward_tile<kBatch, false>(job, BlendSource{p.point_list, p.splat, p.color, (uint32_t)p.P, p.capacity});
+  const uint3 tile = block_tile(p.block_tiles, p.ranges, blockIdx.y * p.gx + blockIdx.x, blockIdx.y << 16 | blockIdx.x);
+  auto make_job = [&](uint32_t t, uint2 range) { return tile_job(p, t, range); };
+  blend_forward_tile<kBatch, false>(make_job, tile, BlendSource{p.point_list, p.splat, p.color, (uint32_t)p.P, p.capacity});
 }
 
-// All views of a batch in one launch: block b blends global tile b.
+// All views of a batch in one launch: a block blends one of the views' tiles.
 template <int kBatch, bool kWrap>
-__global__ void __launch_bounds__(kBlendThreads, kBlendFwdMinBlocks) batch_render_forward_kernel(const __grid_constant__ BatchRenderParams p) {
-  const TileJob job = batch_tile_job(p, blockIdx.x);
-  blend_forward_tile<kBatch, kWrap>(job, BlendSource{p.point_list, p.splat, p.color, (uint32_t)p.P * (uint32_t)p.V, p.capacity});
+__global__ void __launch_bounds__(kBlendThreads, kBatchFwdMinBlocks) batch_render_forward_kernel(const __grid_constant__ BatchRenderParams p) {
+  const uint3 tile = block_tile(p.block_tiles, p.ranges, blockIdx.x, blockIdx.x);
+  if (tile.z >= p.total_tiles) return;  // (never, after a binning)
+  auto make_job = [&](uint32_t t, uint2 range) { return tile_job(p, t, range); };
+  blend_forward_tile<kBatch, kWrap>(make_job, tile, BlendSource{p.point_list, p.splat, p.color, (uint32_t)p.P * (uint32_t)p.V, p.capacity});
 }
 
 template <bool kWrap>
