@@ -282,6 +282,7 @@ struct AdamParams {
   const float* dL_drotations;
   const OmnigsAdamHyper* hyper;  // device
   bool aligned;                  // every array starts on 16 bytes
+  int sh_tile;                   // Gaussians per SH tile (adam_sh_gaussians)
   unsigned first_chunk[4];       // first block of the xyz, scaling, rotation and opacity chunks
 };
 
@@ -336,7 +337,7 @@ __device__ __forceinline__ float adam_update(float& p, float& m, float& v, float
 
 // Every block updates a contiguous piece of one part of the model, so that all loads and stores are
 // coalesced and a block has few arrays open: the first blocks take the SH coefficients (f_dc, f_rest) of
-// kAdamTile Gaussians each, the others kAdamChunk elements of xyz, scaling, opacity or rotation.  A thread
+// a tile of Gaussians each, the others kAdamChunk elements of xyz, scaling, opacity or rotation.  A thread
 // loads its elements of p, m, v (16 bytes each when the piece is whole and the arrays are aligned) before
 // it updates any.
 //
@@ -344,10 +345,13 @@ __device__ __forceinline__ float adam_update(float& p, float& m, float& v, float
 // B200: a loop over the Gaussians with a thread each (accesses of stride 3 and 4 floats) and one over the
 // f_rest elements 596 us; blocks that take all groups of 64 Gaussians, with 30 arrays open at once,
 // 405-425 us whatever the tile, occupancy or work per thread; this split 318 us, 92 % of the copy rate.
-// A tile's f_rest is 1.9 vectors a thread: 32 Gaussians and 192 threads measured fastest (256 threads
-// 334 us, 128 threads 351 us; tiles of 64 with 256 or 384 threads 349 and 332 us).
-constexpr int kAdamTile = 32;
+// A tile is at most two vectors a thread: with 16 coefficients 32 Gaussians and 192 threads measured
+// fastest (256 threads 334 us, 128 threads 351 us; tiles of 64 with 256 or 384 threads 349 and 332 us).
+// Fewer coefficients take more Gaussians (with one, tiles of 32 left 7 of 8 threads idle: 168 us per step
+// over 1.1M Gaussians, 96 with tiles of 512).
 constexpr int kAdamThreads = 192;
+constexpr int kAdamVecs = 2;  // 16-byte vectors per thread and SH tile
+inline int adam_sh_gaussians(int M) { return kAdamVecs * kAdamThreads * 4 / (3 * M) & ~3; }
 constexpr int kAdamChunk = 2 * 4 * kAdamThreads;
 constexpr int kAdamBlocksPerSm = 5;
 
@@ -504,24 +508,44 @@ __device__ __forceinline__ void adam_sh_tile(const AdamParams& p, float* s_sh, i
   const int dc_n = 3 * ng / kW, rest_n = ng * per / kW;
   AdamScalars s_dc, s_rest;
   if (kW == 4) {  // a whole tile: everything is loaded before the gradients have arrived
-    constexpr int kRest = (kAdamTile * 45 / 4 + kAdamThreads - 1) / kAdamThreads;
-    static_assert(kAdamTile * 3 / 4 <= kAdamThreads, "one f_dc vector per thread");
-    AdamVec<kW> rp[kRest], rm[kRest], rv[kRest], dp, dm, dv;
-    const int td = kAdamThreads - 1 - t;  // f_dc on the last threads, which have the fewest f_rest vectors
-#pragma unroll
-    for (int u = 0; u < kRest; ++u) {
+    AdamVec<4> pv[kAdamVecs], mv[kAdamVecs], vv[kAdamVecs];
+    auto at = [&](int u, float*& prm, float*& m, float*& v) {  // the thread's vector u: f_rest's, then f_dc's
       const int i = t + u * kAdamThreads;
-      if (i < rest_n) rp[u] = adam_load<kW>(rest_p, i), rm[u] = adam_load<kW>(rest_m, i), rv[u] = adam_load<kW>(rest_v, i);
+      const bool rest = i < rest_n;
+      prm = rest ? rest_p : dc_p, m = rest ? rest_m : dc_m, v = rest ? rest_v : dc_v;
+      return rest ? i : i < rest_n + dc_n ? i - rest_n : -1;
+    };
+#pragma unroll
+    for (int u = 0; u < kAdamVecs; ++u) {
+      float *prm, *m, *v;
+      const int j = at(u, prm, m, v);
+      if (j >= 0) pv[u] = adam_load<4>(prm, j), mv[u] = adam_load<4>(m, j), vv[u] = adam_load<4>(v, j);
     }
-    if (td < dc_n) dp = adam_load<kW>(dc_p, td), dm = adam_load<kW>(dc_m, td), dv = adam_load<kW>(dc_v, td);
     adam_scalars2(*p.hyper, 1, 2, s_dc, s_rest);
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
 #pragma unroll
-    for (int u = 0; u < kRest; ++u)
-      if (t + u * kAdamThreads < rest_n)
-        update(rest_p, rest_m, rest_v, t + u * kAdamThreads, rp[u], rm[u], rv[u], s_rest, rest_at);
-    if (td < dc_n) update(dc_p, dc_m, dc_v, td, dp, dm, dv, s_dc, dc_at);
+    for (int u = 0; u < kAdamVecs; ++u) {
+      float *prm, *m, *v;
+      const int j = at(u, prm, m, v);
+      if (j < 0) continue;
+      // element e of f_rest lies at e + 3 (e / per) + 3 of the tile's rows, of f_dc at e + (row - 3) (e / 3)
+      const bool rest = t + u * kAdamThreads < rest_n;
+      const uint32_t by = rest ? magic : 0x55555556u;
+      const int skip = rest ? 3 : row - 3, off = rest ? 3 : 0;
+      AdamScalars s = s_dc;
+      s.step_size = rest ? s_rest.step_size : s_dc.step_size;  // (all that differs by group)
+      int pos[4];
+      AdamVec<4> g;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        pos[k] = 4 * j + k + skip * (int)__umulhi((uint32_t)(4 * j + k), by) + off;
+        g.v[k] = s_sh[pos[k]];
+      }
+      adam_vec<4>(prm, m, v, j, pv[u], mv[u], vv[u], g, s);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) s_sh[pos[k]] = pv[u].v[k];
+    }
   } else {
     adam_scalars2(*p.hyper, 1, 2, s_dc, s_rest);
     __syncthreads();
@@ -556,11 +580,11 @@ __device__ __forceinline__ void adam_sh_tile(const AdamParams& p, float* s_sh, i
 }
 
 __global__ void __launch_bounds__(kAdamThreads, kAdamBlocksPerSm) adam_gaussian_kernel(const __grid_constant__ AdamParams p) {
-  extern __shared__ float4 s_sh4[];  // [kAdamTile][M][3]
+  extern __shared__ float4 s_sh4[];  // [sh_tile][M][3]
   // SH tiles first; 16-byte accesses need whole pieces (which then start on 16 bytes if the arrays do)
   if (blockIdx.x < p.first_chunk[0]) {
-    const int g0 = blockIdx.x * kAdamTile, ng = min(kAdamTile, p.prm.P - g0);
-    if (p.aligned && ng == kAdamTile)
+    const int g0 = blockIdx.x * p.sh_tile, ng = min(p.sh_tile, p.prm.P - g0);
+    if (p.aligned && ng == p.sh_tile)
       adam_sh_tile<4>(p, reinterpret_cast<float*>(s_sh4), g0, ng);
     else
       adam_sh_tile<1>(p, reinterpret_cast<float*>(s_sh4), g0, ng);
@@ -741,12 +765,13 @@ int omnigs_adam_step(const OmnigsGaussianParams* prm, const OmnigsAdamState* st,
   // blocks: SH tiles, then chunks of xyz, scaling, rotation and opacity
   const int64_t P = prm->P;
   auto chunks = [&](int64_t per) { return (unsigned)((P * per + kAdamChunk - 1) / kAdamChunk); };
-  p.first_chunk[0] = (unsigned)((P + kAdamTile - 1) / kAdamTile);
+  p.sh_tile = adam_sh_gaussians(prm->M);
+  p.first_chunk[0] = (unsigned)((P + p.sh_tile - 1) / p.sh_tile);
   p.first_chunk[1] = p.first_chunk[0] + chunks(3);
   p.first_chunk[2] = p.first_chunk[1] + chunks(3);
   p.first_chunk[3] = p.first_chunk[2] + chunks(4);
   const unsigned blocks = p.first_chunk[3] + chunks(1);
-  const size_t smem = sizeof(float) * kAdamTile * 3 * (size_t)prm->M;
+  const size_t smem = sizeof(float) * p.sh_tile * 3 * (size_t)prm->M;
   staged(OMNIGS_STAGE_OTHER, 1, s, [&] { adam_gaussian_kernel<<<blocks, kAdamThreads, smem, s>>>(p); });
   return check_launch("adam step");
 }
