@@ -39,6 +39,7 @@ torch::autograd::tensor_list GaussianRasterizerFunction::forward(
                           raster_settings.campos_, colors_precomp, means3D, scales, rotations, cov3Ds_precomp,
                           radii, sh, std::get<3>(result), std::get<4>(result), std::get<5>(result)});
   ctx->mark_non_differentiable({radii});
+  ctx->set_materialize_grads(false);  // (no zeros for radii; the backward makes the image's if it needs them)
   return {color, radii};
 }
 

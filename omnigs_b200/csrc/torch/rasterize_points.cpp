@@ -77,12 +77,17 @@ RasterizeGaussiansCUDA(const torch::Tensor& background, const torch::Tensor& mea
   const int H = image_height;
   const int W = image_width;
   auto float_opts = means3D.options().dtype(torch::kFloat32);
-  torch::Tensor out_color = torch::full({kChannels, H, W}, 0.0, float_opts);
-  torch::Tensor radii = torch::full({P}, 0, means3D.options().dtype(torch::kInt32));
+  auto int_opts = means3D.options().dtype(torch::kInt32);
   torch::TensorOptions byte_opts = torch::TensorOptions().dtype(torch::kByte).device(means3D.device());
-  torch::Tensor geomBuffer = torch::empty({0}, byte_opts);
-  torch::Tensor binningBuffer = torch::empty({0}, byte_opts);
-  torch::Tensor imgBuffer = torch::empty({0}, byte_opts);
+  // the forward writes every pixel and radius; without Gaussians it does not run and both are zero
+  torch::Tensor out_color, radii, geomBuffer, binningBuffer, imgBuffer;
+  if (P == 0) {
+    out_color = torch::zeros({kChannels, H, W}, float_opts);
+    radii = torch::zeros({P}, int_opts);
+    geomBuffer = torch::empty({0}, byte_opts);
+    binningBuffer = torch::empty({0}, byte_opts);
+    imgBuffer = torch::empty({0}, byte_opts);
+  }
 
   int rendered = 0;
   if (P != 0) {
@@ -94,6 +99,8 @@ RasterizeGaussiansCUDA(const torch::Tensor& background, const torch::Tensor& mea
     if (sh.size(0) != 0) M = sh.size(1);
     FloatIn bg(background), m3(means3D), shs(sh), col(colors), op(opacity), sc(scales),
         rot(rotations), cov(cov3D_precomp), vm(viewmatrix), cp(campos);
+    out_color = torch::empty({kChannels, H, W}, float_opts);
+    radii = torch::empty({P}, int_opts);
     OmnigsLonlatForwardArgs a{};
     a.P = P;
     a.D = degree;
@@ -115,10 +122,10 @@ RasterizeGaussiansCUDA(const torch::Tensor& background, const torch::Tensor& mea
     a.radii = radii.data_ptr<int>();
     a.flags = g_forward_flags.load();
 
-    geomBuffer.resize_({(int64_t)omnigs_lonlat_geom_bytes(P)});
-    imgBuffer.resize_({(int64_t)omnigs_lonlat_image_bytes_flags(W, H, a.flags)});
+    geomBuffer = torch::empty({(int64_t)omnigs_lonlat_geom_bytes(P)}, byte_opts);
+    imgBuffer = torch::empty({(int64_t)omnigs_lonlat_image_bytes_flags(W, H, a.flags)}, byte_opts);
     const int64_t capacity = std::max<int64_t>(g_capacity_hint.load(), 4 * (int64_t)P);
-    binningBuffer.resize_({(int64_t)omnigs_lonlat_binning_bytes(capacity)});
+    binningBuffer = torch::empty({(int64_t)omnigs_lonlat_binning_bytes(capacity)}, byte_opts);
     auto s = reinterpret_cast<omnigs_stream_t>(stream);
     // returns once the binning has run (num_rendered and the status are final); the blend is still
     // running on the stream, so the caller's next launches overlap it
