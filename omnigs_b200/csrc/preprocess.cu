@@ -18,8 +18,10 @@
 namespace omnigs {
 namespace {
 
-// 128 threads: the per-warp SH stage (6.5 KB) of four warps.  Six resident blocks per SM (at most
-// 85 registers) measured fastest on a B200 (0.102 -> 0.078 ms at 1M Gaussians with the staging).
+// 128 threads: the per-warp SH stage (6.5 KB) of four warps, six resident blocks per SM.  Bound by the
+// latency of its loads, so the SH copies run while the geometry is computed and the colour comes last.
+// Measured on a B200 at 1M / 3M Gaussians: 75 / 196 us waiting for the SH first, 65 / 165 us now (300 MB at
+// 1M: 45 us at the copy rate).
 constexpr int kPrepBlock = 128;
 
 __global__ void __launch_bounds__(kPrepBlock, 6) preprocess_kernel(PreprocessParams p) {
@@ -28,11 +30,22 @@ __global__ void __launch_bounds__(kPrepBlock, 6) preprocess_kernel(PreprocessPar
   __shared__ float4 s_sh[kPrepBlock / 32][32 * kShStageStride];
   const int idx = blockIdx.x * kPrepBlock + threadIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const bool staged = warp_stage_sh(p.shs, idx - lane, p.P, p.M, s_sh[warp], lane);
+  const bool staged = can_stage_sh(p.shs, idx - lane, p.P, p.M);
+  if (staged) stage_sh(p.shs, idx - lane, s_sh[warp], lane);
 
-  uint32_t touched = 0;
+  // the coefficients arrive while the geometry is computed
+  SplatResult r;
+  r.radius = 0;
+  r.touched = 0;
   if (idx < p.P) {
     const float3 p_orig = {p.means3D[3 * idx], p.means3D[3 * idx + 1], p.means3D[3 * idx + 2]};
+    // (prefetched, not loaded: with the values in registers here the compiler contracts the geometry
+    // differently, and the image would no longer be the reference's bit for bit)
+    if (p.cov3D_precomp == nullptr) {
+      asm volatile("prefetch.global.L1 [%0];" ::"l"(p.scales + 3 * idx));
+      asm volatile("prefetch.global.L1 [%0];" ::"l"(p.rotations + 4 * idx));
+    }
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(p.opacities + idx));
     auto cov3d = [&](float out[6]) {
       if (p.cov3D_precomp != nullptr) {
 #pragma unroll
@@ -44,20 +57,13 @@ __global__ void __launch_bounds__(kPrepBlock, 6) preprocess_kernel(PreprocessPar
         cov3d_from_scale_rot(s, p.scale_modifier, q, out);
       }
     };
-    float shv[3 * kMaxShCoeffs];
-    if (staged)
-      read_staged_sh(s_sh[warp], lane, shv);
-    else if (p.shs != nullptr)
-      load_sh<false>(p.shs, idx, p.M, shv);
-    auto sh = [&](int k) { return v3(shv[3 * k], shv[3 * k + 1], shv[3 * k + 2]); };
-    const SplatResult r = preprocess_splat</*kFp64Poles=*/false>(
-        p_orig, p.viewmatrix, p.W, p.H, p.gx, p.gy, p.D, p.campos, p.opacities[idx],
-        p.colors_precomp != nullptr ? p.colors_precomp + 3 * idx : nullptr, /*seam_wrap=*/false, cov3d, sh);
+    auto no_sh = [](int) { return v3(0.f, 0.f, 0.f); };
+    r = preprocess_splat</*kFp64Poles=*/false, /*kColor=*/false>(p_orig, p.viewmatrix, p.W, p.H, p.gx, p.gy, p.D, p.campos,
+                                                                 p.opacities[idx], nullptr, /*seam_wrap=*/false, cov3d, no_sh);
     p.radii[idx] = r.radius;
     if (r.radius > 0) {
       p.splat[2 * idx] = r.s0;
       p.splat[2 * idx + 1] = r.s1;
-      p.color[idx] = r.col;
       const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
       p.grad_acc[3 * idx] = z4;
       p.grad_acc[3 * idx + 1] = z4;
@@ -65,7 +71,18 @@ __global__ void __launch_bounds__(kPrepBlock, 6) preprocess_kernel(PreprocessPar
     }
     p.depth[idx] = r.depth_key;
     p.tiles_touched[idx] = r.touched;
-    touched = r.touched;
+  }
+  const uint32_t touched = r.touched;
+  if (staged) wait_staged_sh();
+  if (r.radius > 0) {
+    float shv[3 * kMaxShCoeffs];
+    if (staged)
+      read_staged_sh(s_sh[warp], lane, shv);
+    else if (p.shs != nullptr)
+      load_sh<false>(p.shs, idx, p.M, shv);
+    auto sh = [&](int k) { return v3(shv[3 * k], shv[3 * k + 1], shv[3 * k + 2]); };
+    const float3 p_orig = {p.means3D[3 * idx], p.means3D[3 * idx + 1], p.means3D[3 * idx + 2]};
+    p.color[idx] = splat_color(p.D, p_orig, p.campos, p.colors_precomp != nullptr ? p.colors_precomp + 3 * idx : nullptr, sh);
   }
 
   // ---- instance total: block reduction, one atomic per block ----

@@ -23,17 +23,12 @@ namespace {
 // issued at the start (512 contiguous bytes per instruction, no registers held while the
 // covariance backward runs), the SH backward reading each coefficient from the Gaussian's row, and
 // the gradients written back through the same rows and stored 512 contiguous bytes per instruction.
-// Other warps read and write each Gaussian's coefficients on their own.  Measured on a B200 at 1M
-// Gaussians: 0.161 -> 0.134 ms; copying the rows into registers before the SH backward instead
-// measured 0.289 ms.
+// Other warps read and write each Gaussian's coefficients on their own.  Bound by the latency of the
+// loads (four blocks a SM), so all inputs are loaded before the first store.  Measured on a B200 at
+// 1M / 3M Gaussians: 161 us at 1M without the staging, 134 / 378 with it and loads between the stores,
+// 103 / 296 now (650 MB at 1M: 98 us at the copy rate).  Five or six blocks a SM spill: 111 and 117 us
+// at 1M; copying the rows into registers before the SH backward 289 us.
 constexpr int kPbThreads = 128;
-
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 __global__ void __launch_bounds__(kPbThreads) preprocess_backward_kernel(PreprocessBackwardParams p) {
   __shared__ float4 s_stage[kPbThreads / 32][32 * kShStageStride];
@@ -44,23 +39,27 @@ __global__ void __launch_bounds__(kPbThreads) preprocess_backward_kernel(Preproc
   float4* stage = s_stage[warp];
   const bool staged = p.shs != nullptr && p.dL_dsh != nullptr && M == kMaxShCoeffs && first + 32 <= p.P &&
                       ((reinterpret_cast<uintptr_t>(p.shs) | reinterpret_cast<uintptr_t>(p.dL_dsh)) & 15) == 0;
-  if (staged) {
-    const float4* src = reinterpret_cast<const float4*>(p.shs) + (size_t)first * 12;
-#pragma unroll
-    for (int i = 0; i < 12; ++i) {
-      const int e = i * 32 + lane;
-      const int gg = e / 12, part = e - gg * 12;
-      cp_async16(stage + gg * kShStageStride + part, src + e);
-    }
-    cp_async_commit();
-  }
+  if (staged) stage_sh(p.shs, first, stage, lane);
   if (idx >= p.P) return;  // (never in a staged warp)
   float* dsh = (p.dL_dsh != nullptr && M > 0) ? p.dL_dsh + (size_t)idx * M * 3 : nullptr;
-  const bool culled = !(p.radii[idx] > 0);
+  // all inputs before the first store: the compiler cannot move a load past stores that it may alias
+  const int radius = p.radii[idx];
+  const float4 g0 = p.grad_acc[3 * idx], g1 = p.grad_acc[3 * idx + 1], g2 = p.grad_acc[3 * idx + 2];
+  const float4 sa = p.splat[2 * idx];      // {x, y, conic a, conic b}
+  const float4 sb = p.splat[2 * idx + 1];  // {conic c, opacity, ...}
+  const uint32_t clamp_bits = __float_as_uint(p.color[idx].w);
+  float3 mean = {p.means3D[3 * idx], p.means3D[3 * idx + 1], p.means3D[3 * idx + 2]};
+  const bool scale_rot = p.scales != nullptr && p.cov3D_precomp == nullptr;
+  float3 scale = {0.f, 0.f, 0.f};
+  float4 rot = {0.f, 0.f, 0.f, 0.f};
+  if (scale_rot) {
+    scale = {p.scales[3 * idx], p.scales[3 * idx + 1], p.scales[3 * idx + 2]};
+    rot = {p.rotations[4 * idx], p.rotations[4 * idx + 1], p.rotations[4 * idx + 2], p.rotations[4 * idx + 3]};
+  }
+  const bool culled = !(radius > 0);
 
   V3 dL_dmeans = v3(0.f, 0.f, 0.f);
   float dcov[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  float3 mean = {0.f, 0.f, 0.f};
   float dL_dcolor[3] = {0.f, 0.f, 0.f};
   if (culled) {
     for (int k = 0; k < 3; ++k) {
@@ -82,15 +81,8 @@ __global__ void __launch_bounds__(kPbThreads) preprocess_backward_kernel(Preproc
     // a culled lane of a staged warp takes part in the warp's SH steps below with zero gradients
   } else {
     // ---- consume the accumulator record of the backward blend ----
-    const float4 g0 = p.grad_acc[3 * idx];
-    const float4 g1 = p.grad_acc[3 * idx + 1];
-    const float4 g2 = p.grad_acc[3 * idx + 2];
     // the blend sums w dx and w dy (turned into the mean terms by the opacity and the conic here)
-    // and the conic terms (by the opacity), all without their constant factors (render_bwd.cu);
-    // the conic and opacity are read before the record is cleared (the compiler cannot move loads of possibly aliasing memory past those
-    // stores)
-    const float4 sa = __ldg(&p.splat[2 * idx]);  // {x, y, conic a, conic b}
-    const float4 sb = __ldg(&p.splat[2 * idx + 1]);  // {conic c, opacity, ...}
+    // and the conic terms (by the opacity), all without their constant factors (render_bwd.cu)
     const float conic_c = sb.x, opacity = sb.y;
     const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
     p.grad_acc[3 * idx] = z4;
@@ -119,15 +111,11 @@ __global__ void __launch_bounds__(kPbThreads) preprocess_backward_kernel(Preproc
 
     // ---- computeCov2DLonLatCUDA (backward.cu:297-485) ----
     const float* vm = p.viewmatrix;
-    mean = {p.means3D[3 * idx], p.means3D[3 * idx + 1], p.means3D[3 * idx + 2]};
     float cov3D[6];
     if (p.cov3D_precomp != nullptr) {
       for (int k = 0; k < 6; ++k) cov3D[k] = p.cov3D_precomp[6 * idx + k];
     } else {
-      const float3 s = {p.scales[3 * idx], p.scales[3 * idx + 1], p.scales[3 * idx + 2]};
-      const float4 q = {p.rotations[4 * idx], p.rotations[4 * idx + 1], p.rotations[4 * idx + 2],
-                        p.rotations[4 * idx + 3]};
-      cov3d_from_scale_rot(s, p.scale_modifier, q, cov3D);
+      cov3d_from_scale_rot(scale, p.scale_modifier, rot, cov3D);
     }
     LonlatJacobian jac;
     dL_dmeans = cov2d_lonlat_backward<float>(mean, cov3D, vm, p.W, p.H, dL_dconic, dcov, jac);
@@ -146,14 +134,12 @@ __global__ void __launch_bounds__(kPbThreads) preprocess_backward_kernel(Preproc
       dshv[3 * k + 1] = g.y;
       dshv[3 * k + 2] = g.z;
     };
-    const uint32_t clamp_bits = __float_as_uint(p.color[idx].w);
     dL_dmeans = dL_dmeans + sh_backward(deg, v3(mean.x, mean.y, mean.z),
                                         v3(p.campos[0], p.campos[1], p.campos[2]), sh, clamp_bits,
                                         v3(dL_dcolor[0], dL_dcolor[1], dL_dcolor[2]), put);
   };
   if (staged) {
-    cp_async_wait_all();
-    __syncwarp();  // every lane's copies have landed
+    wait_staged_sh();
     float dshv[3 * kMaxShCoeffs];
     const int ncoef = culled ? 0 : (deg + 1) * (deg + 1);
     if (!culled) sh_grad(reinterpret_cast<const float*>(stage + lane * kShStageStride), dshv);
@@ -190,12 +176,9 @@ __global__ void __launch_bounds__(kPbThreads) preprocess_backward_kernel(Preproc
   p.dL_dmeans3D[3 * idx + 2] = dL_dmeans.z;
 
   // ---- computeCov3D backward (backward.cu:489-552) ----
-  if (p.scales != nullptr && p.cov3D_precomp == nullptr) {
-    const float3 s = {p.scales[3 * idx], p.scales[3 * idx + 1], p.scales[3 * idx + 2]};
-    const float4 q = {p.rotations[4 * idx], p.rotations[4 * idx + 1], p.rotations[4 * idx + 2],
-                      p.rotations[4 * idx + 3]};
+  if (scale_rot) {
     float dscale[3], drot[4];
-    cov3d_backward(s, p.scale_modifier, q, dcov, dscale, drot);
+    cov3d_backward(scale, p.scale_modifier, rot, dcov, dscale, drot);
     for (int k = 0; k < 3; ++k) p.dL_dscales[3 * idx + k] = dscale[k];
     for (int k = 0; k < 4; ++k) p.dL_drotations[4 * idx + k] = drot[k];
   } else {

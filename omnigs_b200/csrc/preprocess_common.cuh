@@ -52,6 +52,19 @@ struct SplatResult {
 // where the lonlat Jacobian's longitude row (~ W / (2 pi rho)) has grown ~11x over the equator's.
 constexpr float kPoleSinLat = 0.99619469809174553f;  // sin(85 deg)
 
+// The splat's colour and clamp bits, from its coefficients or precomputed.
+template <class ShLoad>
+__device__ __forceinline__ float4 splat_color(int D, float3 p_orig, const float* campos, const float* color_precomp,
+                                              ShLoad sh) {
+  if (color_precomp != nullptr)
+    return make_float4(color_precomp[0], color_precomp[1], color_precomp[2], __uint_as_float(0u));
+  const V3 pos = v3(p_orig.x, p_orig.y, p_orig.z);
+  const V3 cam = v3(campos[0], campos[1], campos[2]);
+  const V3 c = sh_color_unclamped(D, pos, cam, sh);
+  const uint32_t bits = (c.x < 0 ? 1u : 0u) | (c.y < 0 ? 2u : 0u) | (c.z < 0 ? 4u : 0u);
+  return make_float4(clamp_at_zero(c.x), clamp_at_zero(c.y), clamp_at_zero(c.z), __uint_as_float(bits));
+}
+
 // cov3d(out) fills the Gaussian's 3D covariance; it is called after the near cull and before a
 // compiler barrier, as the reference stores cov3D to global memory at that point (forward.cu:650)
 // and its 2D-covariance code then reloads the view matrix and recomputes the camera-space mean
@@ -60,8 +73,9 @@ constexpr float kPoleSinLat = 0.99619469809174553f;  // sin(85 deg)
 // registers) for the reload to happen.  sh(k) returns coefficient k as a V3.
 // seam_wrap selects the cyclic tile-column range (tile_rect_cyclic) instead of the clamped one.
 // With kFp64Poles, Gaussians beyond kPoleSinLat get their 2D covariance, conic and radius from an
-// FP64 evaluation of the same formulas (not the reference's arithmetic: a precision mode).
-template <bool kFp64Poles, class Cov3DFn, class ShLoad>
+// FP64 evaluation of the same formulas (not the reference's arithmetic: a precision mode).  Without kColor
+// the colour is left to the caller (splat_color).
+template <bool kFp64Poles, bool kColor, class Cov3DFn, class ShLoad>
 __device__ __forceinline__ SplatResult preprocess_splat(float3 p_orig, const float* vm, int W, int H,
                                                         int gx, int gy, int D, const float* campos,
                                                         float opacity, const float* color_precomp,
@@ -115,15 +129,7 @@ __device__ __forceinline__ SplatResult preprocess_splat(float3 p_orig, const flo
     tile_rect(point_image, radius, gx, gy, rmin, rmax);
   const uint32_t area = (uint32_t)(rmax.x - rmin.x) * (uint32_t)(rmax.y - rmin.y);
   if (area == 0) return res;
-  if (color_precomp == nullptr) {
-    const V3 pos = v3(p_orig.x, p_orig.y, p_orig.z);
-    const V3 cam = v3(campos[0], campos[1], campos[2]);
-    const V3 c = sh_color_unclamped(D, pos, cam, sh);
-    const uint32_t bits = (c.x < 0 ? 1u : 0u) | (c.y < 0 ? 2u : 0u) | (c.z < 0 ? 4u : 0u);
-    res.col = make_float4(clamp_at_zero(c.x), clamp_at_zero(c.y), clamp_at_zero(c.z), __uint_as_float(bits));
-  } else {
-    res.col = make_float4(color_precomp[0], color_precomp[1], color_precomp[2], __uint_as_float(0u));
-  }
+  if (kColor) res.col = splat_color(D, p_orig, campos, color_precomp, sh);
   const float2 cull = cull_quadric(point_image.x, point_image.y, conic.x, conic.y, conic.z, opacity);
   res.s0 = make_float4(point_image.x, point_image.y, conic.x, conic.y);
   res.s1 = make_float4(conic.z, opacity, cull.x, cull.y);

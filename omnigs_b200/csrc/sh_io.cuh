@@ -54,26 +54,33 @@ __device__ __forceinline__ void load_sh(const void* shs, int g, int M, float out
 }
 
 // Warp-cooperative staging of FP32 SH (M == 16): the warp's 32 consecutive Gaussians own one
-// contiguous 6 KB span, which the warp loads with 12 fully coalesced 16-byte loads per lane (each
-// instruction reads 512 contiguous bytes) into `stage`, instead of each lane reading its own 192 B
-// (every warp instruction then touches 32 separate cache lines).  `stage` holds kShStageStride
-// float4 per Gaussian: the spare float4 puts the 16-byte reads of 8 lanes (one shared-memory
-// phase) of their own records on distinct banks.  warp_stage_sh is warp-uniform; it returns false,
-// loading nothing, unless the whole warp qualifies (full warp, M == 16, 16-byte aligned).
+// contiguous 6 KB span, which the warp copies with 12 fully coalesced 16-byte cp.async per lane (each
+// instruction reads 512 contiguous bytes, and no register holds them meanwhile) into `stage`, instead of
+// each lane reading its own 192 B (every warp instruction then touches 32 separate cache lines).  `stage`
+// holds kShStageStride float4 per Gaussian: the spare float4 puts the 16-byte reads of 8 lanes (one
+// shared-memory phase) of their own records on distinct banks.  can_stage_sh is warp-uniform: full warp,
+// M == 16, 16-byte aligned.  wait_staged_sh ends the copies; the whole warp calls both.
 constexpr int kShStageStride = 13;
 
-__device__ __forceinline__ bool warp_stage_sh(const float* shs, int first, int P, int M, float4* stage, int lane) {
-  if (shs == nullptr || M != kMaxShCoeffs || first + 32 > P || (reinterpret_cast<uintptr_t>(shs) & 15) != 0)
-    return false;
+__device__ __forceinline__ bool can_stage_sh(const float* shs, int first, int P, int M) {
+  return shs != nullptr && M == kMaxShCoeffs && first + 32 <= P && (reinterpret_cast<uintptr_t>(shs) & 15) == 0;
+}
+
+__device__ __forceinline__ void stage_sh(const float* shs, int first, float4* stage, int lane) {
   const float4* src = reinterpret_cast<const float4*>(shs) + (size_t)first * 12;
 #pragma unroll
   for (int i = 0; i < 12; ++i) {
     const int e = i * 32 + lane;
     const int gg = e / 12, part = e - gg * 12;
-    stage[gg * kShStageStride + part] = __ldg(src + e);
+    const unsigned dst = (unsigned)__cvta_generic_to_shared(stage + gg * kShStageStride + part);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src + e) : "memory");
   }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+__device__ __forceinline__ void wait_staged_sh() {
+  asm volatile("cp.async.wait_all;" ::: "memory");
   __syncwarp();
-  return true;
 }
 
 // This lane's 48 staged coefficients.
