@@ -104,6 +104,8 @@ __global__ void __launch_bounds__(kBatchBlock) batch_preprocess_kernel(const __g
 // Three resident blocks per SM (at most 170 registers) for the FP32 arithmetic: 1.21 -> 0.92 ms per
 // 16-view step over 1M Gaussians on a B200, against the 190 registers (two blocks) the compiler
 // takes unbounded; the FP64-pole instantiations would spill heavily under that bound and keep theirs.
+// With the records copied a view ahead (ViewRecords) 0.90 -> 0.78 ms, and two / four blocks 0.95 / 0.77
+// (1.6 GB of records: 0.25 ms at the copy rate).
 template <bool kFp64Poles>
 constexpr int batch_bwd_min_blocks() { return kFp64Poles ? 1 : 3; }
 
@@ -111,6 +113,20 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
 }
+__device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(s), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// Waits for all groups but the newest.
+__device__ __forceinline__ void cp_async_wait_previous() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+
+// What a thread reads of its Gaussian's record in one view, copied while it works on the view before:
+// the accumulator and splat records and the clamp bits.  A slot is read and rewritten by its thread alone.
+struct ViewRecords {
+  float4 part[5][kBatchBlock];  // grad_acc[3], splat[2]
+  uint32_t clamp[kBatchBlock];
+};
 
 // A warp whose 32 Gaussians all exist and carry 16 SH coefficients (16-byte aligned) copies its
 // coefficients into shared memory with cp.async (512 contiguous bytes per instruction) and the SH
@@ -122,6 +138,7 @@ __global__ void __launch_bounds__(kBatchBlock, batch_bwd_min_blocks<kFp64Poles>(
   constexpr int kRowU4 = kShBf16 ? 6 : 12;  // 16-byte pieces of a Gaussian's coefficients
   constexpr int kStrideU4 = kRowU4 + 1;     // odd: a quarter-warp's 16-byte row reads hit distinct banks
   __shared__ uint4 s_stage[kBatchBlock / 32][32 * kStrideU4];
+  __shared__ ViewRecords s_rec[2];
   const int g = blockIdx.x * kBatchBlock + threadIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int first = g - lane;
@@ -137,16 +154,27 @@ __global__ void __launch_bounds__(kBatchBlock, batch_bwd_min_blocks<kFp64Poles>(
       const int gg = e / kRowU4, part = e - gg * kRowU4;
       cp_async16(stage + gg * kStrideU4 + part, src + e);
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");
   }
+  cp_async_commit();
   if (g >= p.P) return;  // (never in a staged warp)
+  auto fetch = [&](int v) {  // (a group even past the last view, so that one group a view is in flight)
+    if (v < p.V) {
+      const size_t rec = (size_t)v * p.P + g;
+      ViewRecords& r = s_rec[v & 1];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) cp_async16(&r.part[k][threadIdx.x], p.grad_acc + 3 * rec + k);
+#pragma unroll
+      for (int k = 0; k < 2; ++k) cp_async16(&r.part[3 + k][threadIdx.x], p.splat + 2 * rec + k);
+      cp_async4(&r.clamp[threadIdx.x], &p.color[rec].w);
+    }
+    cp_async_commit();
+  };
+  fetch(0);
   const float3 mean = {p.means3D[3 * g], p.means3D[3 * g + 1], p.means3D[3 * g + 2]};
   float cov3D[6];
   gaussian_cov3d(p, g, cov3D);
-  if (staged) {
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    __syncwarp();  // every lane's copies have landed
-  }
+  cp_async_wait_previous();
+  if (staged) __syncwarp();  // every lane's copies of the coefficients have landed
   // the rest of the kernel, given the accessor of the Gaussian's coefficients
   auto finish = [&](auto sh) {
   float dsh[3 * kMaxShCoeffs];
@@ -161,21 +189,22 @@ __global__ void __launch_bounds__(kBatchBlock, batch_bwd_min_blocks<kFp64Poles>(
   V3 dmean = v3(0.f, 0.f, 0.f), dcolor = v3(0.f, 0.f, 0.f);
   float dcov[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   float dopacity = 0.f, stat_norm = 0.f, stat_views = 0.f;
-  int max_radius = 0;
+  int max_radius = 0, next_radius = p.radii[g];
 #pragma unroll 1
   for (int v = 0; v < p.V; ++v) {
-    const size_t rec = (size_t)v * p.P + g;
-    const int radius = p.radii[rec];
+    const int radius = next_radius;
+    if (v + 1 < p.V) next_radius = p.radii[(size_t)(v + 1) * p.P + g];
+    fetch(v + 1);
+    cp_async_wait_previous();
     if (!(radius > 0)) continue;
-    const float4 g0 = p.grad_acc[3 * rec];
-    const float4 g1 = p.grad_acc[3 * rec + 1];
-    const float4 g2 = p.grad_acc[3 * rec + 2];
+    const ViewRecords& rec = s_rec[v & 1];
+    const float4 g0 = rec.part[0][threadIdx.x], g1 = rec.part[1][threadIdx.x], g2 = rec.part[2][threadIdx.x];
     const float* vm = p.viewmatrices + 16 * v;
     const int W = p.views[v].W, H = p.views[v].H;
     // the blend sums w dx and w dy (turned into the mean terms by the opacity and the conic here)
     // and the conic terms (by the opacity), all without their constant factors (render_bwd.cu)
-    const float4 sa = p.splat[2 * rec];  // {x, y, conic a, conic b}
-    const float4 sb = p.splat[2 * rec + 1];  // {conic c, opacity, ...}
+    const float4 sa = rec.part[3][threadIdx.x];  // {x, y, conic a, conic b}
+    const float4 sb = rec.part[4][threadIdx.x];  // {conic c, opacity, ...}
     const float conic_c = sb.x, opacity = sb.y;
     const float mx = opacity * fmaf(sa.z, g0.x, sa.w * g0.y), my = opacity * fmaf(sa.w, g0.x, conic_c * g0.y);
     const float ho = -0.5f * opacity;
@@ -200,7 +229,7 @@ __global__ void __launch_bounds__(kBatchBlock, batch_bwd_min_blocks<kFp64Poles>(
     if (with_sh) {
       const float* cp = p.campos + 3 * v;
       dm = dm + sh_backward(p.D, v3(mean.x, mean.y, mean.z), v3(cp[0], cp[1], cp[2]), sh,
-                            __float_as_uint(p.color[rec].w), dcol, put);
+                            rec.clamp[threadIdx.x], dcol, put);
     }
     dmean = dmean + dm;
     dcolor = dcolor + dcol;
