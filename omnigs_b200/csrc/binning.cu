@@ -42,13 +42,13 @@ constexpr uint32_t kLbValue = (1u << 30) - 1;
 constexpr unsigned long long kScanAggregate = 1ull << 62;
 constexpr unsigned long long kScanPrefix = 2ull << 62;
 constexpr unsigned long long kScanValue = (1ull << 62) - 1;
-// Predecessors a look-back reads per round.  Measured on a B200 (1M Gaussians, 2048x1024): 16 or
-// 32 per round made every sort pass slower (depth passes 21 -> 24-27 us, tile passes 90 -> 95-125
-// us), so the walk is not bound by its round trips.  Nor is the pass bound by its look-back: a
+// Predecessors a look-back reads per round.  Measured on a B200, the sorts of a 1M-Gaussian view /
+// 16-view batch: 4 / 8 / 16 / 32 a round 118 / 118 / 128 / 136 and 1106 / 1123 / 1296 / 1276 us, so the walk
+// is not bound by its round trips.  Nor is the pass bound by its look-back: a
 // reduce-then-scan in its place (a kernel counting every tile's digits and scanning the counts
 // over the tiles, then the pass without waits) made the sort slower, 0.294 -> 0.366 ms per view:
 // the count kernels took 12-27 us each and the passes got only 4-10 us faster.
-constexpr int kLookbackBatch = 8;
+constexpr int kLookbackBatch = 4;
 
 __device__ __forceinline__ bool instances_fit(const GeomHeader* hdr, int64_t capacity) {
   return (hdr->status & kStatusOverflow) == 0 && hdr->num_rendered64 <= (unsigned long long)capacity;
@@ -165,6 +165,10 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* s
 // waits on blocks that are already running) and writes runs of equal digits coalesced.  In a
 // segmented sort every segment is an independent sort whose look-back chain starts at the
 // segment's first tile; a value-less first pass numbers items by their global index.
+// Bound by a tile's own work: ranking, scans, scatter.  The tile is reordered before the look-back and its
+// values are loaded after the ranking, so that registers hold 24 words of a thread's 16 items at a time, not
+// 48.  Measured on a B200, the sorts of a 1M / 3M-Gaussian view / 16-view batch: 125 / 447 / 1202 us with
+// everything held to the end, 118 / 380 / 1020 now.
 // Launches of this pass measured ~2 us slower each on a B200 with a 136-byte parameter block than
 // with a 128-byte one.
 static_assert(sizeof(OnesweepParams) <= 128, "keep the onesweep parameter block at 128 bytes or less");
@@ -199,24 +203,20 @@ __global__ void __launch_bounds__(kSortThreads, kMinBlocks) onesweep_kernel(Ones
   const uint32_t mask = p.mask;
   const int shift = p.shift;
 
-  // load the whole tile first (independent loads in flight), then rank
-  uint32_t key[kItems], val[kItems];
+  // load the tile's keys first (independent loads in flight), then rank
+  uint32_t key[kItems];
   const uint32_t tile_base = tile * kTile + warp * (kItems * 32) + lane;
 #pragma unroll
   for (int k = 0; k < kItems; ++k) {
     const uint32_t idx = tile_base + k * 32;
     key[k] = idx < n ? keys_in[idx] : 0xffffffffu;
   }
-#pragma unroll
-  for (int k = 0; k < kItems; ++k) {
-    const uint32_t idx = tile_base + k * 32;
-    val[k] = idx < n ? (vals_in ? vals_in[idx] : (uint32_t)(seg_base + idx)) : 0u;
-  }
   // where each digit starts in the whole output
   uint32_t unused;
   sm.global_base[threadIdx.x] = block_exclusive_scan(hist[threadIdx.x], sm.scan_tmp, unused);
 
-  uint32_t rank[kItems];
+  uint32_t ranks[kItems / 2] = {};  // two a register: a warp's running count stays below 2^16
+  auto rank = [&](int k) { return k & 1 ? ranks[k / 2] >> 16 : ranks[k / 2] & 0xffffu; };
 #pragma unroll
   for (int k = 0; k < kItems; ++k) {
     const bool valid = tile_base + k * 32 < n;
@@ -237,7 +237,15 @@ __global__ void __launch_bounds__(kSortThreads, kMinBlocks) onesweep_kernel(Ones
     __syncwarp();
     if (valid && lane == leader) sm.warp_hist[warp][digit] = old + __popc(peers);
     __syncwarp();
-    rank[k] = valid ? (old + __popc(peers & lt_mask)) : 0xffffffffu;
+    const uint32_t r = old + __popc(peers & lt_mask);
+    ranks[k / 2] = k & 1 ? ranks[k / 2] | r << 16 : r;
+  }
+  // the values, in flight while the counts are summed (loaded with the keys they cost registers: spills)
+  uint32_t val[kItems];
+#pragma unroll
+  for (int k = 0; k < kItems; ++k) {
+    const uint32_t idx = tile_base + k * 32;
+    val[k] = idx < n ? (vals_in ? vals_in[idx] : (uint32_t)(seg_base + idx)) : 0u;
   }
   __syncthreads();
 
@@ -255,12 +263,26 @@ __global__ void __launch_bounds__(kSortThreads, kMinBlocks) onesweep_kernel(Ones
   sm.block_excl[d] = block_exclusive_scan(count, sm.scan_tmp, tile_items);
   __syncthreads();  // every digit's block-local start is read by other threads below
 
-  // decoupled look-back for digit d (digits above the mask are empty everywhere)
+  // digit d's count for the later tiles (digits above the mask are empty everywhere)
   uint32_t* lb = p.lookback + (size_t)(ticket - tile) * kRadix;  // this segment's chain
-  if (tile == 0 || (uint32_t)d > mask) {
-    st_relaxed_u32(&lb[(size_t)tile * kRadix + d], kLbPrefix | count);
-  } else {
-    st_relaxed_u32(&lb[(size_t)tile * kRadix + d], kLbAggregate | count);
+  const bool first = tile == 0 || (uint32_t)d > mask;
+  st_relaxed_u32(&lb[(size_t)tile * kRadix + d], (first ? kLbPrefix : kLbAggregate) | count);
+
+  // reorder the tile in shared memory by digit
+#pragma unroll
+  for (int k = 0; k < kItems; ++k) {
+    if (tile_base + k * 32 < n) {
+      const uint32_t digit = (key[k] >> shift) & mask;
+      const uint32_t pos = sm.block_excl[digit] + sm.warp_hist[warp][digit] + rank(k);
+      if (pos < (uint32_t)kTile) {  // always true: ranks are consistent within the block
+        sm.keys[pos] = key[k];
+        sm.vals[pos] = val[k];
+      }
+    }
+  }
+
+  // decoupled look-back for digit d
+  if (!first) {
     uint32_t prev = 0;
     int64_t j = (int64_t)tile - 1;
     bool gave_up = false, found = false;
@@ -296,18 +318,6 @@ __global__ void __launch_bounds__(kSortThreads, kMinBlocks) onesweep_kernel(Ones
     sm.global_base[d] += prev;
   }
 
-  // reorder the tile in shared memory by digit
-#pragma unroll
-  for (int k = 0; k < kItems; ++k) {
-    if (rank[k] != 0xffffffffu) {
-      const uint32_t digit = (key[k] >> shift) & mask;
-      const uint32_t pos = sm.block_excl[digit] + sm.warp_hist[warp][digit] + rank[k];
-      if (pos < (uint32_t)kTile) {  // always true: ranks are consistent within the block
-        sm.keys[pos] = key[k];
-        sm.vals[pos] = val[k];
-      }
-    }
-  }
   __syncthreads();
   for (uint32_t i = threadIdx.x; i < tile_items; i += kSortThreads) {
     const uint32_t k32 = sm.keys[i];
@@ -1231,14 +1241,25 @@ void launch_histogram(const HistParams& p, int64_t max_items, cudaStream_t s) {
   histogram_kernel<<<dim3((unsigned)blocks, segs), 256, 0, s>>>(p);
 }
 
-void launch_onesweep(const OnesweepParams& p, int64_t max_items, cudaStream_t s) {
+void launch_onesweep(const OnesweepParams& p, int64_t max_items, int64_t expected, cudaStream_t s) {
   if (p.seg_len && small_sort(p.seg_len, p.num_segs)) {  // (the depth sort: its look-back words have room)
     onesweep_kernel<kSmallSortItems, 5, 16><<<(unsigned)sort_blocks(p.seg_len, p.num_segs), kSortThreads, 0, s>>>(p);
     return;
   }
   const int64_t blocks = p.seg_len ? sort_tiles(p.seg_len) * (int64_t)p.num_segs : sort_tiles(max_items);
   if (blocks <= 0) return;
-  onesweep_kernel<kSortItems, 3, kLookbackBatch><<<(unsigned)blocks, kSortThreads, 0, s>>>(p);
+  // The blocks an SM holds: three have all the registers that the ranking wants, five spill.  Tiles that fit one
+  // wave of more blocks are better off so; beyond that four measured fastest.  On a B200, the sorts of a
+  // 300k / 1M / 3M-Gaussian view / 16-view batch with three, four and five: 91 / 118 / 421 / 1106,
+  // 95 / 119 / 412 / 1017 and 107 / 132 / 378 / 1037 us.  The pairs' number is only known on the device: one
+  // and a half a Gaussian are expected, as for the lists.
+  const int64_t tiles = p.seg_len ? blocks : sort_tiles(expected), sms = sm_count();
+  if (tiles <= 3 * sms)
+    onesweep_kernel<kSortItems, 3, kLookbackBatch><<<(unsigned)blocks, kSortThreads, 0, s>>>(p);
+  else if (tiles > 4 * sms && tiles <= 5 * sms)
+    onesweep_kernel<kSortItems, 5, kLookbackBatch><<<(unsigned)blocks, kSortThreads, 0, s>>>(p);
+  else
+    onesweep_kernel<kSortItems, 4, kLookbackBatch><<<(unsigned)blocks, kSortThreads, 0, s>>>(p);
 }
 
 void launch_rects(const RankParams& p, cudaStream_t s) {

@@ -165,7 +165,7 @@ int run_binning(BinningPass& b, cudaStream_t s) {
       op.seg_len = (uint32_t)g.P;
       op.num_segs = (uint32_t)g.V;
       op.hist_seg_stride = kDepthPasses * kRadix;
-      staged(OMNIGS_STAGE_SORT, 1, s, [&] { launch_onesweep(op, records, s); });
+      staged(OMNIGS_STAGE_SORT, 1, s, [&] { launch_onesweep(op, records, records, s); });
     }
 
   }
@@ -218,7 +218,7 @@ int run_binning(BinningPass& b, cudaStream_t s) {
       op.lookback = at<uint32_t>(b.binning, L.tile_lookback) + (size_t)q * pair_tiles * kRadix;
       op.tile_counter = &b.hdr->sort_tile_counter[kDepthPasses + q];
       op.hdr = b.hdr;
-      staged(OMNIGS_STAGE_SORT, 1, s, [&] { launch_onesweep(op, b.capacity, s); });
+      staged(OMNIGS_STAGE_SORT, 1, s, [&] { launch_onesweep(op, b.capacity, 3 * records / 2, s); });
     }
     t.words = keys[sorted];
     t.recs = vals[sorted];

@@ -282,7 +282,7 @@ void launch_batch_preprocess_backward(const BatchParams& p, const BatchGrads& g,
 
 void launch_preprocess(const PreprocessParams& p, cudaStream_t s);
 void launch_histogram(const HistParams& p, int64_t max_items, cudaStream_t s);
-void launch_onesweep(const OnesweepParams& p, int64_t max_items, cudaStream_t s);
+void launch_onesweep(const OnesweepParams& p, int64_t max_items, int64_t expected, cudaStream_t s);
 void launch_begin_binning(const BeginParams& p, cudaStream_t s);
 void launch_rank(const RankParams& p, cudaStream_t s);
 void launch_rects(const RankParams& p, cudaStream_t s);  // rects only, in the order given
