@@ -23,7 +23,7 @@ def _scenes(P, padded):
     return [lonlat.GaussianTensors.from_numpy(x) for x in (few, g)]
 
 
-@pytest.mark.parametrize("P,padded,W,H", [(500, 13000, 16, 16), (9000, 13000, 300, 130), (12000, 120000, 2080, 1040)])
+@pytest.mark.parametrize("P,padded,W,H", [(500, 262144, 16, 16), (9000, 262144, 300, 130), (12000, 300000, 2080, 1040)])
 def test_tile_order(cuda, P, padded, W, H):
     cam = lonlat.Camera.from_view(scenes.identity_view(W, H), background=(0.1, 0.2, 0.3))
     dpix = torch.from_numpy(scenes.upstream_grad(W, H, seed=3)).cuda()
@@ -54,7 +54,7 @@ def test_tile_order_batch(cuda):
     cams = batch.BatchCameras.from_views(views)
     dl = [torch.from_numpy(scenes.upstream_grad(W, H, seed=W)).cuda() for W, H in cams.sizes]
     runs = []
-    for gt in _scenes(7000, 13000):
+    for gt in _scenes(7000, 70000):
         images, _, state = batch.render_batch(gt, cams)
         grads = batch.BatchGradients.empty(gt.P, gt.M, cuda)
         state.backward(gt, cams, dl, grads)
