@@ -81,6 +81,12 @@ inline bool small_sort(int64_t items, int64_t segs) { return small_sort_tiles(it
 inline int64_t sort_blocks(int64_t items, int64_t segs) {
   return (small_sort(items, segs) ? small_sort_tiles(items) : sort_tiles(items)) * segs;
 }
+// Blocks that a state buffer has look-back words for: at least sort_blocks, and never fewer for more items or
+// segments, so that a buffer sized for a scene holds every smaller one.
+inline int64_t sort_room(int64_t items, int64_t segs) {
+  const int64_t small = small_sort_tiles(items) * segs, large = sort_tiles(items) * segs;
+  return small <= kSmallSortTiles ? small : (large > kSmallSortTiles ? large : kSmallSortTiles);
+}
 
 // Views whose tiles the blends take heaviest first (binning.cu): the order lies in the depth sort's
 // look-back memory, which the sort has read by then.  Below kOrderMinRecords (Gaussian, view) records the tile
@@ -100,7 +106,7 @@ struct GeomLayout {
     size_t o = 0;
     L.header = o; o = align_up(o + sizeof(GeomHeader));
     L.dup_scan = o; o = align_up(o + sizeof(uint64_t) * ((P + kScanBlock - 1) / kScanBlock));
-    L.depth_lookback = o; o = align_up(o + sizeof(uint32_t) * kDepthPasses * sort_blocks(P, 1) * kRadix);
+    L.depth_lookback = o; o = align_up(o + sizeof(uint32_t) * kDepthPasses * sort_room(P, 1) * kRadix);
     L.zero_end = o;  // everything above is cleared before each preprocess
     L.splat = o; o = align_up(o + sizeof(float) * 8 * P);
     L.color = o; o = align_up(o + sizeof(float) * 4 * P);
@@ -209,7 +215,7 @@ struct BatchLayout {
     L.header = o; o = align_up(o + sizeof(GeomHeader));
     L.view_rendered = o; o = align_up(o + sizeof(uint64_t) * kMaxBatchViews);
     L.dup_scan = o; o = align_up(o + sizeof(uint64_t) * ((R + kScanBlock - 1) / kScanBlock));
-    L.depth_lookback = o; o = align_up(o + sizeof(uint32_t) * kDepthPasses * sort_blocks(P, V) * kRadix);
+    L.depth_lookback = o; o = align_up(o + sizeof(uint32_t) * kDepthPasses * sort_room(P, V) * kRadix);
     L.depth_hist = o; o = align_up(o + sizeof(uint32_t) * V * kDepthPasses * kRadix);
     L.zero_end = o;  // everything above is cleared before each pass
     L.radii = o; o = align_up(o + sizeof(int32_t) * R);
