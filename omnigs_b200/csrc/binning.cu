@@ -16,7 +16,7 @@
 //  3. tile lists: every bin counts its tiles' instances (its pairs' tiles as bit masks), a scan of the
 //     counts in tile order gives the ranges, and every row of a bin's tiles compacts the bin's list
 //     into its tiles' lists, in order (ballots of the masks' bits).
-// Few Gaussians (kRankMaxP) are ordered by counting, which costs less than the five launches of the
+// Few Gaussians (counts_order) are ordered by counting, which costs less than the five launches of the
 // depth sort: a Gaussian's position is the number of smaller depths.  Where Gaussians times bins are
 // few (kWholeMaxPairs) there are no coarse lists: every bin reads its view's whole order.
 // Counts live on the device: every kernel reads num_rendered from the geometry header and does no
@@ -726,7 +726,7 @@ __global__ void __launch_bounds__(kScanBlock) pair_emit_kernel(const __grid_cons
 // block's, so a key is loaded once per block and nothing is staged.  Keys at lower indices count when
 // they are <= a Gaussian's, that is when the float below them is <; keys at higher ones when they are <.
 //
-// Bound by issue: P^2 comparisons.  An integer comparison and a predicated add both go to the ALU's 16
+// Bound by issue: V P^2 comparisons.  An integer comparison and a predicated add both go to the ALU's 16
 // lanes (22 us for 10,000 Gaussians); here a comparison is sat(2^40 own - 2^40 key) and an add, both on
 // the FMA pipes: a key >= 2^-3 (depths are beyond the near cull at 0.2) differs from another by at least
 // 2^-26, so the difference is 0 or beyond 1 and the saturated value exactly 0 or 1, whatever its

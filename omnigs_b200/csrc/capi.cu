@@ -58,9 +58,9 @@ int run_binning(BinningPass& b, cudaStream_t s) {
   const BinningLayout& L = b.layout;
   const int64_t records = (int64_t)g.P * g.V;
   const bool probe = b.max_spins > 0;
-  // few Gaussians: the depth order by counting (kRankMaxP); few pairs of a Gaussian and a bin: no coarse
+  // few Gaussians: the depth order by counting (counts_order); few pairs of a Gaussian and a bin: no coarse
   // lists, every bin reads the whole order (kWholeMaxPairs)
-  const bool ranked = !probe && g.P <= kRankMaxP;
+  const bool ranked = !probe && counts_order(g.P, g.V);
   const bool whole = !probe && (int64_t)g.num_bins * g.P <= kWholeMaxPairs;
   b.small = ranked && whole;
   TileDigits digits = TileDigits::from_bits(id_bits(g.num_bins));  // of the bin in a pair's word

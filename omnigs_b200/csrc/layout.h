@@ -152,8 +152,14 @@ constexpr int kListWarps = 8;                 // parts per block
 OMNIGS_HD inline int bins_x(int gx) { return (gx + kBinW - 1) / kBinW; }
 OMNIGS_HD inline int bins_y(int gy) { return (gy + kBinH - 1) / kBinH; }
 
-// Up to kRankMaxP Gaussians per view the depth order comes from counting, and up to kWholeMaxPairs
-// (Gaussian, bin) combinations every bin reads its view's whole depth order (binning.cu).
+// Few Gaussians get their depth order from counting (binning.cu), whose cost is that of V P^2 comparisons,
+// where the depth sort's is nearly flat at these sizes.  Measured on a B200, counted / sorted order, forward and
+// backward of V views: V = 2, P = 12,288 (3.0e8) 134 / 136 us; 4, 8000 (2.6e8) 131 / 136; 8, 5000 (2.0e8) 138 / 147;
+// 16, 3000 (1.4e8) 170 / 180; 32, 3000 (2.9e8) 295 / 281; 16, 5000 (4.0e8) 222 / 204; 32, 8000 (2.0e9) 558 / 388.
+constexpr int64_t kRankMaxPairs = int64_t(1) << 28;
+inline bool counts_order(int64_t P, int64_t V) { return P <= kRankMaxP && V * P * P <= kRankMaxPairs; }
+
+// Up to kWholeMaxPairs (Gaussian, bin) combinations every bin reads its view's whole depth order (binning.cu).
 constexpr int64_t kWholeMaxPairs = int64_t(1) << 20;
 
 // The duplicate pass writes its list in blocks of kEmitBlock pairs; its scan records, per such block, the

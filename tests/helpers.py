@@ -67,3 +67,23 @@ def normwise_rel(a, b) -> float:
     if den == 0.0:
         return float(np.abs(a).max()) if a.size else 0.0
     return float(np.abs(a - b).max() / den)
+
+
+def check_batch_lists(state, cams, per, P, seam=False):
+    """Tile ids, record indices and ranges of every view of a rendered batch equal the oracle's bit for bit."""
+    sv, bv = state.state_view(), state.binning_view(sum(per))
+    torch.cuda.synchronize()
+    tiles, points = to_np(bv["tile_ids"]).view(np.uint32), to_np(bv["point_list"]).view(np.uint32)
+    for v, (W, H) in enumerate(cams.sizes):
+        base, count = sv["tile_base"][v], ((W + 15) // 16) * ((H + 15) // 16)
+        mine = (tiles >= base) & (tiles < base + count)
+        assert mine.sum() == per[v]
+        ranges = to_np(sv["ranges"][v]).view(np.uint32).astype(np.int64)
+        if per[v]:
+            ranges[ranges[:, 1] > 0] -= ranges[ranges[:, 1] > 0, 0].min()
+        b = oracle.binning(W, H, to_np(sv["radii"][v]), to_np(sv["splat"][v][:, :2]), to_np(sv["depth"][v]), None,
+                           f32=True, seam_wrap=seam)
+        assert b["num_rendered"] == per[v]
+        np.testing.assert_array_equal(tiles[mine] - np.uint32(base), (b["keys"] >> np.uint64(32)).astype(np.uint32))
+        np.testing.assert_array_equal(points[mine] - np.uint32(v * P), b["point_list"])
+        np.testing.assert_array_equal(ranges.astype(np.uint32), b["ranges"])
