@@ -13,9 +13,9 @@
 //     load-balanced emission of the (bin, depth-order position) pairs in that order, and a stable
 //     LSD radix sort of the pairs by bin (one onesweep pass up to 256 bins): every bin's Gaussians
 //     in depth order.  A splat covers far fewer bins than tiles;
-//  3. tile lists: every bin counts its tiles' instances (its pairs' tiles as bit masks), a scan of the
-//     counts in tile order gives the ranges, and every row of a bin's tiles compacts the bin's list
-//     into its tiles' lists, in order (ballots of the masks' bits).
+//  3. tile lists: warps count the tiles' instances of a piece of the sorted pairs each (the pairs' tiles are
+//     bit masks), a scan of the counts in tile order gives the ranges, and the warps append their pieces
+//     to the tiles' lists, in order.
 // Few Gaussians (counts_order) are ordered by counting, which costs less than the five launches of the
 // depth sort: a Gaussian's position is the number of smaller depths.  Where Gaussians times bins are
 // few (kWholeMaxPairs) there are no coarse lists: every bin reads its view's whole order.
@@ -798,23 +798,46 @@ __global__ void __launch_bounds__(256) rect_kernel(const __grid_constant__ RankP
 }
 
 // ---------------------------------------------------------------- tile lists ------------------
-// The fine stage works a warp at a time: a warp has one part of a bin's pairs (TileGrid::parts of them,
-// in order, eight to a block), counts its tiles' instances, and later, with the places that the scan
-// and the earlier parts' counts give it, appends the part to its tiles' lists.  No warp waits for another.
+// The fine stage works a warp at a time: a warp counts its pairs by tile, and later, with the places that the
+// scan and the earlier warps' counts give it, appends them to the tiles' lists.  No warp waits for another.
+//  * From coarse lists, a warp has a piece of consecutive pairs of the sorted list, whatever bins they are
+//    in: all warps do the same work however the Gaussians are spread over the image (tile_count / tile_fill).
+//    Only a bin that runs on into the next piece needs a piece's counts there, so a slot per piece holds them
+//    (those of the piece's last bin), and a sum of its slots per block shortens the walk back to a bin's begin.
+//  * Without coarse lists, every bin reads its view's whole order, split into TileGrid::parts, eight to a block
+//    (whole_count / whole_fill).
+// Measured on a B200, all of the fine stage, with every bin split into as many parts as an even spread asks for /
+// pieces: 1M Gaussians at 2048x1024 within 0.1 rad 608 / 106 us, 3M at 4096x2048 within 0.02 rad 2930 / 490; evenly
+// spread 1M 71 / 71, 3M 264 / 279, 16 views over 1M 588 / 577, 71,000 at 2132x1093 39 / 36.
 constexpr int kListThreads = 32 * kListWarps;
+constexpr uint32_t kNoBin = 0xffffffffu >> kPairBinShift;
 
-// A warp's part: the bin's tiles, and the pairs [first, end) of the bin's run of the sorted list, or (kAll)
-// of its view's whole depth order.
-struct BinPart {
-  int tx0, ty0;     // first tile column and row
+static_assert(kMaxBatchViews == 32, "a lane per view");
+
+// A bin's place: its first tile column and row in its view.
+struct BinTiles {
+  int tx0, ty0;
   int gx, gy;
-  uint32_t tile0;   // the view's first tile
-  uint32_t tiles;   // the view's tiles
-  uint32_t counts0; // the view's counts: [parts][tiles]
-  uint32_t part;    // parts or more: none
-  uint32_t parts;
-  uint32_t first, end;
+  uint32_t tile0;  // the view's first tile
 };
+__device__ __forceinline__ BinTiles bin_tiles(const TileGrid& g, uint32_t view, uint32_t local) {
+  const uint32_t bx = (uint32_t)bins_x(g.gx[view]);
+  return {(int)(local % bx) * kBinW, (int)(local / bx) * kBinH, g.gx[view], g.gy[view], g.tile_base[view]};
+}
+// The views' first bins in shared memory, for bin_tiles by a warp (a lane per view); a block barrier follows.
+__device__ __forceinline__ void load_bases(const TileGrid& g, uint32_t (&bases)[kMaxBatchViews]) {
+  if ((int)threadIdx.x < kMaxBatchViews) bases[threadIdx.x] = (int)threadIdx.x < g.V ? g.bin_base[threadIdx.x] : kNoBin;
+}
+__device__ __forceinline__ BinTiles bin_tiles(const TileGrid& g, const uint32_t (&bases)[kMaxBatchViews], uint32_t bin) {
+  const uint32_t view = (uint32_t)__popc(__ballot_sync(kFullMask, bases[threadIdx.x & 31] <= bin)) - 1u;
+  return bin_tiles(g, view, bin - bases[view]);
+}
+// Whether the lane's tile (lane / 8, lane % 8) of the bin lies in the image, and its index.
+__device__ __forceinline__ bool lane_tile(const BinTiles& b, uint32_t& tile) {
+  const int lane = threadIdx.x & 31, tx = b.tx0 + lane % kBinW, ty = b.ty0 + lane / kBinW;
+  tile = b.tile0 + (uint32_t)(ty * b.gx + tx);
+  return tx < b.gx && ty < b.gy;
+}
 
 // First index of the sorted words with a bin >= bin, by a warp (32 probes a step).
 __device__ __forceinline__ uint32_t warp_lower_bound(const uint32_t* words, uint32_t n, uint32_t bin) {
@@ -832,93 +855,15 @@ __device__ __forceinline__ uint32_t warp_lower_bound(const uint32_t* words, uint
   return lo;
 }
 
-template <bool kAll>
-__device__ __forceinline__ BinPart bin_part(const TileListParams& p, uint32_t grid_block) {
-  __shared__ uint32_t s_bounds[2];
-  const TileGrid& g = p.grid;
-  uint32_t view = 0;
-#pragma unroll 1
-  for (int v = 1; v < g.V; ++v)
-    if (g.block_base[v] <= grid_block) view = (uint32_t)v;
-  BinPart b;
-  b.gx = g.gx[view];
-  b.gy = g.gy[view];
-  b.tile0 = g.tile_base[view];
-  b.tiles = (uint32_t)(b.gx * b.gy);
-  b.counts0 = g.count_base[view];
-  b.parts = g.parts[view];
-  const uint32_t per_bin = (b.parts + kListWarps - 1u) / kListWarps;  // blocks
-  const uint32_t block = grid_block - g.block_base[view], local = block / per_bin;
-  b.part = (block - local * per_bin) * kListWarps + (threadIdx.x >> 5);
-  const uint32_t bx = (uint32_t)bins_x(b.gx);
-  b.ty0 = (int)(local / bx) * kBinH;
-  b.tx0 = (int)(local % bx) * kBinW;
-  uint32_t first, end;
-  if (kAll) {
-    first = view * (uint32_t)g.P;
-    end = first + (uint32_t)g.P;
-  } else {
-    const uint32_t n = pair_count(p.hdr, p.capacity);
-    if (threadIdx.x < 64) {
-      const uint32_t at = warp_lower_bound(p.words, n, g.bin_base[view] + local + (threadIdx.x >> 5));
-      if ((threadIdx.x & 31) == 0) s_bounds[threadIdx.x >> 5] = at;
-    }
-    __syncthreads();
-    first = s_bounds[0];
-    end = s_bounds[1];
-  }
-  // (parts of whole groups of 32)
-  const uint32_t len = ((end - first + b.parts - 1u) / b.parts + 31u) & ~31u;
-  b.first = (uint32_t)min((unsigned long long)end, first + (unsigned long long)b.part * len);
-  b.end = min(end, b.first + len);
-  return b;
-}
-
-// The tiles of pair e in the bin (the low bits of a pair's word).
-template <bool kAll>
-__device__ __forceinline__ uint32_t pair_tiles(const TileListParams& p, const BinPart& b, uint32_t e) {
-  return kAll ? tile_mask(b.tx0, b.ty0, b.gx, p.grid.seam_wrap != 0, make_uint2(p.rect_x[e], p.rect_y[e])) : p.words[e];
-}
-
 // The bits of a nibble as the low bits of four bytes (bit k in byte k): with a tile row's eight columns in
 // two such words, a warp counts and ranks all eight tiles with additions.
 __device__ __forceinline__ uint32_t spread4(uint32_t nibble) { return (nibble * 0x00204081u) & 0x01010101u; }
 
-// Counts of a bin's tiles over a part of its pairs: every lane keeps the 32 tiles' counts as bytes in
-// eight words (at most 255 pairs a lane between sums), which the warp then adds as halfwords.  Every tile
-// of the grid is written (0 when the instances do not fit).  (A ballot and a popcount per tile and 32
-// pairs took 38 us of the 1M-Gaussian view instead of 15.)
-template <bool kAll>
-__global__ void __launch_bounds__(kListThreads) tile_count_kernel(const __grid_constant__ TileListParams p) {
-  chain_begin();
-  const int lane = threadIdx.x & 31;
-  const bool fit = instances_fit(p.hdr, p.capacity);
-  if (kAll && !fit && blockIdx.x == 0 && threadIdx.x == 0)
-    atomicOr(&p.hdr->status, kStatusCapacity);  // (the scan flags it where there is one)
-  BinPart b = bin_part<kAll>(p, blockIdx.x);
-  if (b.part >= b.parts) return;
-  if (!fit) b.end = b.first;
+// Counts of a bin's tiles: every lane keeps the 32 tiles' counts as bytes in eight words, which the warp then
+// adds.  (A ballot and a popcount per tile and 32 pairs took 38 us of the 1M-Gaussian view instead of 15.)
+struct TileCounts {
   uint32_t acc[kBinH][2] = {};
-  uint32_t mine = 0;  // instances of tile (lane / 8, lane % 8)
-  // adds the warp's bytes: tile 8 r + 4 h + k is byte k of acc[r][h]
-  auto flush = [&] {
-#pragma unroll
-    for (int r = 0; r < kBinH; ++r)
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const uint32_t even = __reduce_add_sync(kFullMask, acc[r][h] & 0x00ff00ffu);        // bytes 0 and 2
-        const uint32_t odd = __reduce_add_sync(kFullMask, (acc[r][h] >> 8) & 0x00ff00ffu);  // bytes 1 and 3
-        if (lane >> 2 == 2 * r + h) {
-          const uint32_t w = lane & 1 ? odd : even;
-          mine += lane & 2 ? w >> 16 : w & 0xffffu;
-        }
-        acc[r][h] = 0u;
-      }
-  };
-  int steps = 0;
-#pragma unroll 4
-  for (uint32_t e0 = b.first; e0 < b.end; e0 += 32) {
-    const uint32_t mask = e0 + lane < b.end ? pair_tiles<kAll>(p, b, e0 + lane) : 0u;
+  __device__ __forceinline__ void add(uint32_t mask) {
     const uint32_t lo = spread4(mask & 15u), hi = spread4((mask >> 4) & 15u);
 #pragma unroll
     for (int r = 0; r < kBinH; ++r) {
@@ -926,20 +871,196 @@ __global__ void __launch_bounds__(kListThreads) tile_count_kernel(const __grid_c
       acc[r][0] += lo * on;
       acc[r][1] += hi * on;
     }
+  }
+  // The sum over the warp of the lane's tile (lane / 8, lane % 8), after at most 255 pairs a lane; starts again at zero.
+  __device__ __forceinline__ uint32_t sum() {
+    const int lane = threadIdx.x & 31;
+    uint32_t mine = 0;
+#pragma unroll
+    for (int r = 0; r < kBinH; ++r)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {  // tile 8 r + 4 h + k is byte k of acc[r][h]
+        const uint32_t even = __reduce_add_sync(kFullMask, acc[r][h] & 0x00ff00ffu);        // bytes 0 and 2
+        const uint32_t odd = __reduce_add_sync(kFullMask, (acc[r][h] >> 8) & 0x00ff00ffu);  // bytes 1 and 3
+        if (lane >> 2 == 2 * r + h) {
+          const uint32_t w = lane & 1 ? odd : even;
+          mine = lane & 2 ? w >> 16 : w & 0xffffu;
+        }
+        acc[r][h] = 0u;
+      }
+    return mine;
+  }
+};
+
+// ---- from coarse lists: pieces of the sorted pairs
+// A piece's pairs: as many as give kPieceTarget warps (about two waves of blocks), within limits.  Measured on a B200:
+// at least 32 / 64, 20,000 Gaussians at 2132x1093 36 / 42 us of the fine stage; at most 160 / 192 / 256 / 384 / 512, the
+// 16-view batch 650 / 617 / 578 / 583 / 576 us, 3M Gaussians at 4096x2048 279 / 278 / 280 / 317 / 339; targets of
+// 5920 / 8192 / 11,000, 1M Gaussians 73 / 71 / 73.
+constexpr uint32_t kMinPiece = 32, kMaxPiece = 256, kPieceTarget = 8192;
+struct Pieces {
+  uint32_t n;       // pairs
+  uint32_t len;     // of a piece, whole groups of 32
+  uint32_t count;   // pieces
+  uint32_t blocks;  // of kListWarps pieces
+  uint32_t* sums;   // [blocks][32]: counts of the pieces' last bins, by block ...
+  uint16_t* slots;  // [count][32]: ... and by piece
+  __device__ __forceinline__ Pieces(const TileListParams& p) : n(pair_count(p.hdr, p.capacity)) {
+    len = min(max((n / kPieceTarget + 31u) & ~31u, kMinPiece), kMaxPiece);
+    count = (n + len - 1u) / len;
+    blocks = (count + kListWarps - 1u) / kListWarps;
+    sums = p.counts;
+    slots = reinterpret_cast<uint16_t*>(p.counts + 32 * (size_t)blocks);
+  }
+  __device__ __forceinline__ uint32_t first(uint32_t piece) const { return min(piece * len, n); }
+};
+// The counts take 16 words a piece and 32 a block, 5/8 n + 52 at most: room of as many words as there are pairs, in
+// whole 64, holds them (with fewer than 128 pairs, of one to four pieces, too).
+static_assert(kMinPiece >= 32 && kListWarps >= 8 && kAlign >= 64 * sizeof(uint32_t), "the counts fit");
+static_assert(kMaxPiece <= 255 * 32, "a lane's counts fit in bytes");
+
+// The warp's counts of a bin, added to its tiles' totals.
+__device__ __forceinline__ void add_total(const TileListParams& p, const uint32_t (&bases)[kMaxBatchViews], uint32_t bin,
+                                          uint32_t count) {
+  uint32_t t;
+  if (lane_tile(bin_tiles(p.grid, bases, bin), t) && count) atomicAdd(p.totals ? &p.totals[t] : &p.ranges[t].x, count);
+}
+
+// Walks a piece by a warp: use(bin, in, word, begins, ends, at_end) for every run of a bin within a group of 32 of its
+// pairs: `in` the lanes of the run, whether the bin begins with it (in this piece) and whether it or the piece ends with
+// it, at_end for the piece.  next_group(e0, after) gives the group's words, and in `after` those of the group behind.
+template <class Next, class Use>
+__device__ __forceinline__ void walk_piece(uint32_t begin, uint32_t end, Next next_group, Use use) {
+  const int lane = threadIdx.x & 31;
+  uint32_t bin = kNoBin;
+#pragma unroll 1
+  for (uint32_t e0 = begin; e0 < end; e0 += 32) {
+    uint32_t after;  // the first word of the group behind
+    const uint32_t w = next_group(e0, after);
+    unsigned left = __ballot_sync(kFullMask, e0 + lane < end);
+    const uint32_t follows = e0 + 32 < end ? __shfl_sync(kFullMask, after, 0) >> kPairBinShift : kNoBin;
+    do {  // (once, unless a bin ends within the group)
+      const uint32_t b = __shfl_sync(kFullMask, w, __ffs(left) - 1) >> kPairBinShift;
+      const bool in = ((left >> lane) & 1u) && (w >> kPairBinShift) == b;
+      left &= ~__ballot_sync(kFullMask, in);
+      use(b, in, w, b != bin, left != 0 || b != follows, left == 0 && follows == kNoBin);
+      bin = b;
+    } while (left);
+  }
+}
+
+__global__ void __launch_bounds__(kListThreads) tile_count_kernel(const __grid_constant__ TileListParams p) {
+  chain_begin();
+  __shared__ uint32_t s_own[kListWarps][32], s_bin[kListWarps], s_bases[kMaxBatchViews];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const Pieces all(p);
+  load_bases(p.grid, s_bases);
+  __syncthreads();
+  for (uint32_t block = blockIdx.x; block < all.blocks; block += gridDim.x) {
+    const uint32_t piece = block * kListWarps + (uint32_t)warp, begin = all.first(piece), end = all.first(piece + 1);
+    auto load = [&](uint32_t e) { return e < end ? p.words[e] : 0u; };
+    uint32_t w0 = load(begin + lane), w1 = load(begin + 32 + lane), own = 0, last = kNoBin;
+    TileCounts c;
+    walk_piece(begin, end, [&](uint32_t e0, uint32_t& after) {
+      const uint32_t w = w0;
+      after = w0 = w1;
+      w1 = load(e0 + 64 + lane);
+      return w;
+    }, [&](uint32_t bin, bool in, uint32_t w, bool, bool ends, bool at_end) {
+      c.add(in ? w : 0u);
+      if (!ends) return;
+      own = c.sum();
+      last = bin;
+      if (!at_end) add_total(p, s_bases, bin, own);
+    });
+    s_own[warp][lane] = own;
+    if (lane == 0) s_bin[warp] = last;
+    if (piece < all.count) all.slots[32 * (size_t)piece + lane] = (uint16_t)own;
+    __syncthreads();
+    // the pieces' last bins' totals, one addition a bin, and the block's sum
+    if (last != kNoBin && (warp == kListWarps - 1 || s_bin[warp + 1] != last)) {
+      uint32_t run = 0;
+#pragma unroll
+      for (int k = 0; k < kListWarps; ++k) run += s_bin[k] == last ? s_own[k][lane] : 0u;
+      add_total(p, s_bases, last, run);
+    }
+    if (warp == 0) {
+      uint32_t sum = 0;
+#pragma unroll
+      for (int k = 0; k < kListWarps; ++k) sum += s_own[k][lane];
+      all.sums[32 * (size_t)block + lane] = sum;
+    }
+    __syncthreads();
+  }
+}
+
+// ---- without: parts of the whole order per bin
+// A warp's part: the bin's tiles, and entries [first, end) of its view's depth order.
+struct BinPart {
+  BinTiles bin;
+  uint32_t tiles;   // the view's tiles
+  uint32_t counts0; // the view's counts: [parts][tiles]
+  uint32_t part;    // parts or more: none
+  uint32_t parts;
+  uint32_t first, end;
+};
+
+__device__ __forceinline__ BinPart bin_part(const TileListParams& p, uint32_t grid_block) {
+  const TileGrid& g = p.grid;
+  uint32_t view = 0;
+#pragma unroll 1
+  for (int v = 1; v < g.V; ++v)
+    if (g.block_base[v] <= grid_block) view = (uint32_t)v;
+  BinPart b;
+  b.tiles = (uint32_t)(g.gx[view] * g.gy[view]);
+  b.counts0 = g.count_base[view];
+  b.parts = g.parts[view];
+  const uint32_t per_bin = (b.parts + kListWarps - 1u) / kListWarps;  // blocks
+  const uint32_t block = grid_block - g.block_base[view], local = block / per_bin;
+  b.part = (block - local * per_bin) * kListWarps + (threadIdx.x >> 5);
+  b.bin = bin_tiles(g, view, local);
+  const uint32_t first = view * (uint32_t)g.P, end = first + (uint32_t)g.P;
+  // (parts of whole groups of 32)
+  const uint32_t len = ((end - first + b.parts - 1u) / b.parts + 31u) & ~31u;
+  b.first = (uint32_t)min((unsigned long long)end, first + (unsigned long long)b.part * len);
+  b.end = min(end, b.first + len);
+  return b;
+}
+
+// The tiles of the bin that entry e of the order covers.
+__device__ __forceinline__ uint32_t entry_tiles(const TileListParams& p, const BinTiles& b, uint32_t e) {
+  return tile_mask(b.tx0, b.ty0, b.gx, p.grid.seam_wrap != 0, make_uint2(p.rect_x[e], p.rect_y[e]));
+}
+
+// Every tile of the grid is written (0 when the instances do not fit).
+__global__ void __launch_bounds__(kListThreads) whole_count_kernel(const __grid_constant__ TileListParams p) {
+  chain_begin();
+  const int lane = threadIdx.x & 31;
+  const bool fit = instances_fit(p.hdr, p.capacity);
+  if (!fit && blockIdx.x == 0 && threadIdx.x == 0)
+    atomicOr(&p.hdr->status, kStatusCapacity);  // (the scan flags it where there is one)
+  BinPart b = bin_part(p, blockIdx.x);
+  if (b.part >= b.parts) return;
+  if (!fit) b.end = b.first;
+  TileCounts c;
+  uint32_t mine = 0;  // instances of the lane's tile
+  int steps = 0;
+#pragma unroll 4
+  for (uint32_t e0 = b.first; e0 < b.end; e0 += 32) {
+    c.add(e0 + lane < b.end ? entry_tiles(p, b.bin, e0 + lane) : 0u);
     if (++steps == 255) {
-      flush();
+      mine += c.sum();
       steps = 0;
     }
   }
-  if (steps) flush();
-  const int tx = b.tx0 + lane % kBinW, ty = b.ty0 + lane / kBinW;
-  if (tx < b.gx && ty < b.gy) {
-    const uint32_t t = (uint32_t)(ty * b.gx + tx);
+  if (steps) mine += c.sum();
+  uint32_t t;
+  if (lane_tile(b.bin, t)) {
     if (p.counts == nullptr) {
-      p.ranges[b.tile0 + t].x = mine;
+      p.ranges[t].x = mine;
     } else {
-      p.counts[b.counts0 + (size_t)b.part * b.tiles + t] = mine;
-      if (mine) atomicAdd(&p.totals[b.tile0 + t], mine);
+      p.counts[b.counts0 + (size_t)b.part * b.tiles + (t - b.bin.tile0)] = mine;
+      if (mine) atomicAdd(&p.totals[t], mine);
     }
   }
 }
@@ -957,7 +1078,7 @@ __global__ void __launch_bounds__(kTileScanThreads) tile_scan_kernel(const __gri
   __shared__ uint32_t s_before;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t n = p.grid.num_tiles;
-  const uint32_t* totals = p.counts ? p.totals : nullptr;
+  const uint32_t* totals = p.totals;
   const uint32_t begin = blockIdx.x * kTileScanBlock;
   if (threadIdx.x == 0) s_before = 0;
   __syncthreads();
@@ -1101,7 +1222,7 @@ __device__ __forceinline__ void order_tiles(const TileListParams& p, uint32_t se
   }
 }
 
-// Appends a part of a bin's pairs to the lists of its 32 tiles.  A warp queues its pairs by the bin's four
+// Appends pairs of a bin to the lists of its 32 tiles.  A warp queues its pairs by the bin's four
 // tile rows (a pair covers one or two of them on average, so a walk per row would waste most lanes) and
 // appends 32 of a row at a time to its eight lists: a pair's place is the list's next one plus the
 // queued pairs before it that cover the tile, from a warp scan of the eight columns as bytes.  Bound by
@@ -1113,46 +1234,51 @@ struct FillQueue {
   __align__(16) uint32_t next[32];           // next free place of every tile's list
 };
 
-template <bool kAll>
-__global__ void __launch_bounds__(kListThreads) tile_fill_kernel(const __grid_constant__ TileListParams p) {
-  chain_begin();
-  __shared__ FillQueue s_queue[kListWarps];
-  const uint32_t segments = p.block_tiles ? (p.grid.num_tiles + kOrderTiles - 1) / kOrderTiles : 0u;
-  if (blockIdx.x < segments) return order_tiles(p, blockIdx.x);
-  if (!instances_fit(p.hdr, p.capacity)) return;
-  const BinPart b = bin_part<kAll>(p, blockIdx.x - segments);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const unsigned lt = (1u << lane) - 1u;
-  FillQueue& q = s_queue[warp];
-  {  // the lists' next places: the range's start and the earlier parts' counts, which the warps share
-    __shared__ uint32_t s_sum[kListWarps][32], s_own[kListWarps][32];
-    const int tx = b.tx0 + lane % kBinW, ty = b.ty0 + lane / kBinW;
-    uint32_t start = 0, sum = 0, own = 0;
-    bool safe = true;
-    if (tx < b.gx && ty < b.gy) {
-      const uint32_t t = (uint32_t)(ty * b.gx + tx);
-      const uint2 range = p.ranges[b.tile0 + t];
-      start = range.x;
-      safe = range.y <= (uint64_t)p.capacity;  // (always, after a consistent scan)
-      if (b.parts > 1) {
-        const uint32_t* c = p.counts + b.counts0 + t;
-        const uint32_t block = b.part - (uint32_t)warp;  // the block's first part
-#pragma unroll 4
-        for (uint32_t i = (uint32_t)warp; i < block; i += kListWarps) sum += c[(size_t)i * b.tiles];
-        if (b.part < b.parts) own = c[(size_t)b.part * b.tiles];
+struct ListFill {
+  FillQueue& q;
+  uint32_t* out;
+  uint32_t queued[kBinH] = {};  // pairs queued by row (warp-uniform)
+
+  __device__ __forceinline__ ListFill(FillQueue& queue, uint32_t* out_vals) : q(queue), out(out_vals) {}
+  // Begins a bin: the lane's tile's next place.
+  __device__ __forceinline__ void begin(uint32_t next) {
+    __syncwarp();
+    q.next[threadIdx.x & 31] = next;
+  }
+  // Queues 32 pairs: the tiles m that the lane's one covers (0: none), its record r.  Appends rows that have 32, or
+  // with `ends` what there is.  (One place for both: with the rest appended by code of its own, short lists took
+  // longer by the time to fetch it.)
+  __device__ __forceinline__ void add(uint32_t m, uint32_t r, bool ends) {
+    const int lane = threadIdx.x & 31;
+    const unsigned lt = (1u << lane) - 1u;
+    const uint32_t least = ends ? 1u : 32u;
+#pragma unroll
+    for (int row = 0; row < kBinH; ++row) {
+      const bool in = (m >> (kBinW + row)) & 1u && (m & 255u);
+      const unsigned bal = __ballot_sync(kFullMask, in);
+      if (in) {
+        const uint32_t at = queued[row] + (uint32_t)__popc(bal & lt);
+        q.cols[row][at] = m & 255u;
+        q.rec[row][at] = r;
+      }
+      queued[row] += (uint32_t)__popc(bal);
+#pragma unroll 1
+      while (queued[row] >= least) {
+        append(row, queued[row]);
+        queued[row] -= min(queued[row], 32u);
+        __syncwarp();
+        const uint32_t c = q.cols[row][32 + lane], x = q.rec[row][32 + lane];  // the rest moves to the front
+        __syncwarp();
+        if ((uint32_t)lane < queued[row]) {
+          q.cols[row][lane] = c;
+          q.rec[row][lane] = x;
+        }
       }
     }
-    s_sum[warp][lane] = sum;
-    s_own[warp][lane] = own;
-    __syncthreads();
-    if (b.part >= b.parts || b.first >= b.end || !__all_sync(kFullMask, safe)) return;
-#pragma unroll
-    for (int w = 0; w < kListWarps; ++w) start += s_sum[w][lane] + (w < warp ? s_own[w][lane] : 0u);
-    q.next[lane] = start;
   }
-  uint32_t queued[kBinH] = {};  // warp-uniform
-  // appends the first min(n, 32) pairs queued for a row
-  auto append = [&](int row, uint32_t n) {
+  // Appends the first min(n, 32) pairs queued for a row.
+  __device__ __forceinline__ void append(int row, uint32_t n) {
+    const int lane = threadIdx.x & 31;
     __syncwarp();
     const uint32_t m = (uint32_t)lane < n ? q.cols[row][lane] : 0u, rec = q.rec[row][lane];
     uint32_t lo = spread4(m & 15u), hi = spread4(m >> 4);
@@ -1172,14 +1298,134 @@ __global__ void __launch_bounds__(kListThreads) tile_fill_kernel(const __grid_co
     if (lane < kBinW) q.next[row * kBinW + lane] += ((lane < 4 ? all_lo : all_hi) >> (8 * (lane & 3))) & 255u;
 #pragma unroll
     for (int k = 0; k < kBinW; ++k)
-      if ((m >> k) & 1u) p.out_vals[next[k] + (((k < 4 ? lo : hi) >> (8 * (k & 3))) & 255u) - 1u] = rec;
-  };
+      if ((m >> k) & 1u) out[next[k] + (((k < 4 ? lo : hi) >> (8 * (k & 3))) & 255u) - 1u] = rec;
+  }
+};
+
+// Blocks of a fill's launch that order the tiles instead, ahead of the others.
+__device__ __forceinline__ uint32_t order_segments(const TileListParams& p) {
+  return p.block_tiles ? (p.grid.num_tiles + kOrderTiles - 1) / kOrderTiles : 0u;
+}
+
+// The piece that the bin that runs on into piece `at` begins in, by a warp: the piece behind the nearest piece
+// boundary before `at` that the bin does not lie across; a search where that is more than 32 pieces back.
+__device__ __forceinline__ uint32_t begin_piece(const TileListParams& p, const Pieces& all, uint32_t at, uint32_t bin) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t j = at - 1u - (uint32_t)lane;  // (wraps below 0: past every piece)
+  const bool across = j < at && j > 0 && p.words[all.first(j) - 1u] >> kPairBinShift == bin;
+  const unsigned not_across = ~__ballot_sync(kFullMask, across);
+  if (not_across) return at - (uint32_t)__ffs(not_across);
+  return warp_lower_bound(p.words, all.first(at), bin) / all.len;
+}
+
+// Four resident blocks an SM (64 registers).  Measured on a B200, 1M-Gaussian view / 16-view batch: three 77 / 638 us of
+// the fine stage, four 71 / 578, five (48 registers, spills) 76 / 595, six 86 / 656.
+__global__ void __launch_bounds__(kListThreads, 4) tile_fill_kernel(const __grid_constant__ TileListParams p) {
+  chain_begin();
+  __shared__ FillQueue s_queue[kListWarps];
+  __shared__ uint32_t s_sum[kListWarps][32], s_own[kListWarps][32], s_bin[kListWarps], s_bases[kMaxBatchViews];
+  const uint32_t segments = order_segments(p);
+  if (blockIdx.x < segments) return order_tiles(p, blockIdx.x);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const Pieces all(p);
+  load_bases(p.grid, s_bases);
+  for (uint32_t block = blockIdx.x - segments; block < all.blocks; block += gridDim.x - segments) {
+    const uint32_t piece = block * kListWarps + (uint32_t)warp, begin = all.first(piece), end = all.first(piece + 1);
+    auto load = [&](uint32_t e, uint32_t& w, uint32_t& r) {
+      w = r = 0;
+      if (e < end) {
+        w = p.words[e];
+        r = p.recs[e];
+      }
+    };
+    uint32_t w0, r0, w1, r1;
+    load(begin + lane, w0, r0);
+    load(begin + 32 + lane, w1, r1);
+    // A bin that runs on into the block: its counts in the pieces before, whole blocks by their sums.
+    const uint32_t at = block * kListWarps;
+    const uint32_t before = block > 0 ? p.words[all.first(at) - 1u] >> kPairBinShift : kNoBin;
+    uint32_t sum = 0;
+    if (before == p.words[all.first(at)] >> kPairBinShift) {
+      const uint32_t from = begin_piece(p, all, at, before);
+      const uint32_t whole = (from + kListWarps - 1u) / kListWarps;  // the first whole block
+      if (from + warp < whole * kListWarps) sum = all.slots[32 * (size_t)(from + warp) + lane];
+#pragma unroll 4
+      for (uint32_t i = whole + warp; i < block; i += kListWarps) sum += all.sums[32 * (size_t)i + lane];
+    }
+    s_sum[warp][lane] = sum;
+    s_own[warp][lane] = piece < all.count ? all.slots[32 * (size_t)piece + lane] : 0u;
+    if (lane == 0) s_bin[warp] = begin < end ? p.words[end - 1] >> kPairBinShift : kNoBin;
+    __syncthreads();
+    ListFill fill(s_queue[warp], p.out_vals);
+    bool first = true, safe = false;
+    uint32_t rec = 0;
+    walk_piece(begin, end, [&](uint32_t e0, uint32_t& after) {
+      const uint32_t w = w0;
+      rec = r0;
+      after = w0 = w1, r0 = r1;
+      load(e0 + 64 + lane, w1, r1);
+      return w;
+    }, [&](uint32_t bin, bool in, uint32_t w, bool begins, bool ends, bool) {
+      if (begins) {
+        uint32_t t, place = 0;
+        safe = true;
+        if (lane_tile(bin_tiles(p.grid, s_bases, bin), t)) {
+          const uint2 range = p.ranges[t];
+          place = range.x;
+          safe = range.y <= (uint64_t)p.capacity;  // (always, after a consistent scan)
+        }
+        safe = __all_sync(kFullMask, safe);
+        if (first)  // the piece's first bin may have begun in an earlier one
+#pragma unroll
+          for (int k = 0; k < kListWarps; ++k)
+            place += (bin == before ? s_sum[k][lane] : 0u) + (k < warp && s_bin[k] == bin ? s_own[k][lane] : 0u);
+        first = false;
+        fill.begin(place);
+      }
+      if (safe) fill.add(in ? w : 0u, rec, ends);
+    });
+    __syncthreads();
+  }
+}
+
+__global__ void __launch_bounds__(kListThreads) whole_fill_kernel(const __grid_constant__ TileListParams p) {
+  chain_begin();
+  __shared__ FillQueue s_queue[kListWarps];
+  __shared__ uint32_t s_sum[kListWarps][32], s_own[kListWarps][32];
+  const uint32_t segments = order_segments(p);
+  if (blockIdx.x < segments) return order_tiles(p, blockIdx.x);
+  if (!instances_fit(p.hdr, p.capacity)) return;
+  const BinPart b = bin_part(p, blockIdx.x - segments);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // the lists' next places: the range's start and the earlier parts' counts, which the warps share
+  uint32_t t, next = 0, sum = 0, own = 0;
+  bool safe = true;
+  if (lane_tile(b.bin, t)) {
+    const uint2 range = p.ranges[t];
+    next = range.x;
+    safe = range.y <= (uint64_t)p.capacity;  // (always, after a consistent scan)
+    if (b.parts > 1) {
+      const uint32_t* c = p.counts + b.counts0 + (t - b.bin.tile0);
+      const uint32_t block = b.part - (uint32_t)warp;  // the block's first part
+#pragma unroll 4
+      for (uint32_t i = (uint32_t)warp; i < block; i += kListWarps) sum += c[(size_t)i * b.tiles];
+      if (b.part < b.parts) own = c[(size_t)b.part * b.tiles];
+    }
+  }
+  s_sum[warp][lane] = sum;
+  s_own[warp][lane] = own;
+  __syncthreads();
+  if (b.part >= b.parts || b.first >= b.end || !__all_sync(kFullMask, safe)) return;
+#pragma unroll
+  for (int w = 0; w < kListWarps; ++w) next += s_sum[w][lane] + (w < warp ? s_own[w][lane] : 0u);
+  ListFill fill(s_queue[warp], p.out_vals);
+  fill.begin(next);
   uint32_t mask = 0, rec = 0;
   auto load = [&](uint32_t e) {
     mask = 0;
     if (e < b.end) {
-      mask = pair_tiles<kAll>(p, b, e);
-      rec = kAll ? p.order[e] : p.recs[e];
+      mask = entry_tiles(p, b.bin, e);
+      rec = p.order[e];
     }
   };
   load(b.first + lane);
@@ -1189,32 +1435,8 @@ __global__ void __launch_bounds__(kListThreads) tile_fill_kernel(const __grid_co
     const uint32_t m = mask1, r = rec1;
     mask1 = mask, rec1 = rec;
     load(e0 + 64 + lane);
-#pragma unroll
-    for (int row = 0; row < kBinH; ++row) {
-      const bool in = (m >> (kBinW + row)) & 1u && (m & 255u);
-      const unsigned bal = __ballot_sync(kFullMask, in);
-      if (in) {
-        const uint32_t at = queued[row] + (uint32_t)__popc(bal & lt);
-        q.cols[row][at] = m & 255u;
-        q.rec[row][at] = r;
-      }
-      queued[row] += (uint32_t)__popc(bal);
-      if (queued[row] >= 32) {
-        append(row, 32);
-        queued[row] -= 32;
-        __syncwarp();
-        const uint32_t c = q.cols[row][32 + lane], x = q.rec[row][32 + lane];  // the rest moves to the front
-        __syncwarp();
-        if ((uint32_t)lane < queued[row]) {
-          q.cols[row][lane] = c;
-          q.rec[row][lane] = x;
-        }
-      }
-    }
+    fill.add(m, r, e0 + 32 >= b.end);
   }
-#pragma unroll
-  for (int row = 0; row < kBinH; ++row)
-    if (queued[row]) append(row, queued[row]);
 }
 
 // The sorted tile ids, which only the inspection of a pass reads: a warp per tile writes its range.
@@ -1300,15 +1522,20 @@ void launch_duplicate(const DuplicateParams& p, cudaStream_t s) {
   pair_emit_kernel<<<(unsigned)eblocks, kScanBlock, 0, s>>>(p);
 }
 
-void launch_tile_lists(const TileListParams& p, cudaStream_t s) {
+void launch_tile_lists(const TileListParams& p, int64_t expected_pairs, cudaStream_t s) {
   const TileGrid& g = p.grid;
-  if (g.num_blocks == 0) return;
-  const bool all = p.words == nullptr;
-  launch_chained(p.chained, all ? tile_count_kernel<true> : tile_count_kernel<false>, g.num_blocks, kListThreads, 0, s, p);
-  const unsigned scan = p.counts ? (g.num_tiles + kTileScanBlock - 1) / kTileScanBlock : 1u;
+  if (g.num_tiles == 0) return;
+  const bool whole = p.words == nullptr;
+  // The pairs' number is only known on the device: as many blocks as the expected ones fill, which take further
+  // pieces in turn.
+  const int64_t pairs = std::min(expected_pairs, p.capacity);
+  const int64_t piece = std::min<int64_t>(std::max<int64_t>(pairs / kPieceTarget, kMinPiece), kMaxPiece);
+  const unsigned blocks = whole ? g.num_blocks : (unsigned)(pairs / (piece * kListWarps) + 1);
+  launch_chained(p.chained, whole ? whole_count_kernel : tile_count_kernel, blocks, kListThreads, 0, s, p);
+  const unsigned scan = p.totals ? (g.num_tiles + kTileScanBlock - 1) / kTileScanBlock : 1u;
   launch_chained(p.chained, tile_scan_kernel, scan, kTileScanThreads, 0, s, p);
   const unsigned order = p.block_tiles ? (g.num_tiles + kOrderTiles - 1) / kOrderTiles : 0u;
-  launch_chained(p.chained, all ? tile_fill_kernel<true> : tile_fill_kernel<false>, g.num_blocks + order, kListThreads, 0, s, p);
+  launch_chained(p.chained, whole ? whole_fill_kernel : tile_fill_kernel, blocks + order, kListThreads, 0, s, p);
   launch_chained(p.chained, tile_keys_kernel, (g.num_tiles + 7) / 8, 256, 0, s, p);
 }
 

@@ -67,34 +67,45 @@ int run_binning(BinningPass& b, cudaStream_t s) {
   const int64_t pair_tiles = sort_tiles(L.capacity);
   uint32_t* hist = at<uint32_t>(b.binning, L.hist);
 
-  // The fine stage's parts, as many as their counts have room for beside the tiles' totals: in the depth
-  // sort's first key buffer and the two buffers behind it (the rects, which the coarse stage has read);
-  // without a coarse stage, in the pairs' buffer or the key buffer alone, whichever is larger.
-  uint32_t* scratch = b.dkeys[0];
-  int64_t room = 3 * records - g.num_tiles;
+  // Where the fine stage keeps its counts and the tiles' totals.  Buffers in use by then: the order and, in a
+  // coarse stage, the sorted pairs; without one, the rects.
+  uint32_t* counts = nullptr;
+  uint32_t* totals = nullptr;
+  bool clear_totals = false;   // on their own, behind the coarse stage, whose memory they lie in
+  const int64_t lookback_words = kTilePasses * pair_tiles * kRadix, used_words = whole ? 0 : digits.passes * pair_tiles * kRadix;
+  // the look-back words of the passes that the bin sort does not have, cleared with the others
+  uint32_t* spare = at<uint32_t>(b.binning, L.tile_lookback) + used_words;
+  if (lookback_words - used_words >= (int64_t)g.num_tiles + 4) totals = spare;
   if (whole) {
-    room = std::max(records, L.capacity) - g.num_tiles;
-    if (L.capacity > records) scratch = at<uint32_t>(b.binning, b.out ? L.tkeys0 : L.tkeys1);
+    // Parts as many as their counts have room for: in the pairs' buffer, which the tile lists do not go to, or the
+    // depth sort's first key buffer, whichever is larger; the totals behind them if there are no spare words.
+    uint32_t* scratch = L.capacity > records ? at<uint32_t>(b.binning, b.out ? L.tkeys0 : L.tkeys1) : b.dkeys[0];
+    const int64_t room = std::max(records, L.capacity) - g.num_tiles;
+    const int64_t cap = std::max<int64_t>(1, std::min<int64_t>(kMaxListParts, room / g.num_tiles));
+    uint32_t blocks = 0, count_words = 0;
+    for (int v = 0; v < g.V; ++v) {
+      const int64_t bins = (int64_t)bins_x(g.gx[v]) * bins_y(g.gy[v]);
+      g.parts[v] = (uint32_t)std::max<int64_t>(1, std::min<int64_t>(cap, ((int64_t)g.P + kListPart - 1) / kListPart));
+      g.block_base[v] = blocks;
+      g.count_base[v] = count_words;
+      blocks += (uint32_t)bins * ((g.parts[v] + kListWarps - 1) / kListWarps);
+      count_words += g.parts[v] * (uint32_t)(g.gx[v] * g.gy[v]);
+    }
+    g.num_blocks = blocks;
+    if (room >= (int64_t)g.num_tiles) {
+      counts = scratch;
+      clear_totals = totals == nullptr;
+      if (clear_totals) totals = scratch + count_words;
+    } else {
+      totals = nullptr;  // one part per bin: the counts go through the ranges
+    }
+  } else {
+    // The pieces' counts in the buffer that the tiles' ids go to in the end; the totals, without spare words, in the
+    // depth sort's first key buffer and the two behind it (the rects, which the coarse stage has read) or the ranges.
+    counts = at<uint32_t>(b.binning, b.out ? L.tkeys1 : L.tkeys0);
+    clear_totals = totals == nullptr && 3 * records >= (int64_t)g.num_tiles;
+    if (clear_totals) totals = b.dkeys[0];
   }
-  const int64_t cap = std::max<int64_t>(1, std::min<int64_t>(kMaxListParts, room / g.num_tiles));
-  uint32_t blocks = 0, count_words = 0;
-  for (int v = 0; v < g.V; ++v) {
-    const int64_t bins = (int64_t)bins_x(g.gx[v]) * bins_y(g.gy[v]);
-    const int64_t run = whole ? g.P : (3 * (int64_t)g.P / 2 + bins - 1) / bins;
-    g.parts[v] = (uint32_t)std::max<int64_t>(1, std::min<int64_t>(cap, (run + kListPart - 1) / kListPart));
-    g.block_base[v] = blocks;
-    g.count_base[v] = count_words;
-    blocks += (uint32_t)bins * ((g.parts[v] + kListWarps - 1) / kListWarps);
-    count_words += g.parts[v] * (uint32_t)(g.gx[v] * g.gy[v]);
-  }
-  g.num_blocks = blocks;
-  uint32_t* counts = room >= (int64_t)g.num_tiles ? scratch : nullptr;
-  // the totals: in the look-back words of the passes that the bin sort does not have, cleared with the
-  // others; else behind the counts, cleared on their own
-  const int64_t lookback_words = kTilePasses * pair_tiles * kRadix;
-  uint32_t* totals = at<uint32_t>(b.binning, L.tile_lookback) + digits.passes * pair_tiles * kRadix;
-  const bool totals_there = lookback_words - digits.passes * pair_tiles * kRadix >= (int64_t)g.num_tiles + 4;
-  if (!totals_there) totals = scratch + count_words;
 
   BeginParams begin{};
   begin.hdr = b.hdr;
@@ -107,11 +118,14 @@ int run_binning(BinningPass& b, cudaStream_t s) {
   }
   if (!whole) {
     begin.region[2] = at<uint4>(b.binning, L.tile_lookback);
-    begin.bytes[2] = sizeof(uint32_t) * digits.passes * pair_tiles * kRadix;
+    begin.bytes[2] = sizeof(uint32_t) * used_words;
   }
-  if (counts != nullptr && totals_there) {
+  if (totals == spare) {
     begin.region[3] = reinterpret_cast<uint4*>(totals);
     begin.bytes[3] = (sizeof(uint32_t) * g.num_tiles + 15) / 16 * 16;
+  } else if (!whole && totals == nullptr) {
+    begin.region[3] = reinterpret_cast<uint4*>(b.ranges);  // (every array has room for a multiple of 256 bytes)
+    begin.bytes[3] = (sizeof(uint2) * g.num_tiles + 15) / 16 * 16;
   }
   staged(OMNIGS_STAGE_OTHER, 1, s, [&] { launch_begin_binning(begin, s); });
 
@@ -239,9 +253,9 @@ int run_binning(BinningPass& b, cudaStream_t s) {
   t.tile_width = b.tile_width;
   t.capacity = b.capacity;
   t.hdr = b.hdr;
-  if (counts != nullptr && !totals_there && cudaMemsetAsync(totals, 0, sizeof(uint32_t) * g.num_tiles, s) != cudaSuccess)
+  if (clear_totals && cudaMemsetAsync(totals, 0, sizeof(uint32_t) * g.num_tiles, s) != cudaSuccess)
     return check_launch("memset tile totals");
-  staged(OMNIGS_STAGE_RANGES, 4, s, [&] { launch_tile_lists(t, s); });
+  staged(OMNIGS_STAGE_RANGES, 4, s, [&] { launch_tile_lists(t, 3 * records / 2, s); });
   return check_launch("binning");
 }
 

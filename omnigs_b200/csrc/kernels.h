@@ -76,7 +76,8 @@ struct TileGrid {
   int seam_wrap;               // tile columns wrap modulo gx (rects from tile_rect_cyclic)
   int gx[kMaxBatchViews], gy[kMaxBatchViews];
   uint32_t tile_base[kMaxBatchViews], bin_base[kMaxBatchViews];
-  // the fine stage: warps that share a bin's pairs, and per view its first block and its first count
+  // the fine stage without coarse lists: warps that share a bin's Gaussians, and per view its first block and its
+  // first count
   uint32_t num_blocks;
   uint32_t parts[kMaxBatchViews], block_base[kMaxBatchViews], count_base[kMaxBatchViews];
 };
@@ -123,9 +124,10 @@ struct TileListParams {
   const uint32_t* rect_x;
   const uint32_t* rect_y;
   bool chained;
-  uint32_t* counts;            // scratch: per view [parts][tiles] counts; NULL (one part per bin): the
-                               // counts go through the ranges
-  uint32_t* totals;            // scratch: [num_tiles] totals (cleared)
+  // scratch: the pieces' counts of the pairs (as many words as there are pairs), or without pairs per view
+  // [parts][tiles] counts; NULL there (one part per bin): the counts go through the ranges
+  uint32_t* counts;
+  uint32_t* totals;            // scratch: [num_tiles] totals (cleared); NULL: in the ranges (with pairs: cleared)
   uint32_t* out_keys;          // [capacity] sorted tile ids and record indices
   uint32_t* out_vals;
   uint2* ranges;               // [num_tiles]
@@ -287,7 +289,7 @@ void launch_begin_binning(const BeginParams& p, cudaStream_t s);
 void launch_rank(const RankParams& p, cudaStream_t s);
 void launch_rects(const RankParams& p, cudaStream_t s);  // rects only, in the order given
 void launch_duplicate(const DuplicateParams& p, cudaStream_t s);
-void launch_tile_lists(const TileListParams& p, cudaStream_t s);
+void launch_tile_lists(const TileListParams& p, int64_t expected_pairs, cudaStream_t s);
 // Splats staged per shared-memory batch in the blend kernels: a template parameter chosen at run
 // time per direction (128, 256 or 512; set by omnigs_set_blend_batch or the autotuner).  Results
 // do not depend on it: every pixel meets the same splats in the same order.  Defaults: 128 for both

@@ -144,10 +144,10 @@ struct ImageLayout {
 constexpr int kBinW = 8, kBinH = 4;
 constexpr int kPairBinShift = kBinW + kBinH;  // a pair's word: its tiles in the bin, above them the bin (binning.cu)
 
-// Warps that share a bin's pairs in the fine stage: one per kListPart pairs that an even spread would give
-// a bin (one and a half bins per Gaussian), at most kMaxListParts.
+// Without coarse lists, warps that share a bin's Gaussians in the fine stage: one per kListPart, at most
+// kMaxListParts (bins are so few where that counts that 2048 warps each fill the chip).
 constexpr int kListPart = 128;
-constexpr int kMaxListParts = 128;
+constexpr int kMaxListParts = 2048;
 constexpr int kListWarps = 8;                 // parts per block
 OMNIGS_HD inline int bins_x(int gx) { return (gx + kBinW - 1) / kBinW; }
 OMNIGS_HD inline int bins_y(int gy) { return (gy + kBinH - 1) / kBinH; }
