@@ -164,30 +164,29 @@ __device__ __forceinline__ bool plain_splat(const float4& a, const float4& b) {
 // a dx dx fused into the sum with the rounded c dy dy, the b dx dy term rounded on its own.  The slot's
 // factors -1/2 and signs are exact, so applying them before the roundings changes nothing.  Forward and
 // backward agree on every 1/255 and saturation decision.
-// Slot kBatch holds a splat that reaches no pixel; it pads the lists to whole groups of four.
 constexpr uint32_t kSlotBytes = 48;
 
 template <int kBatch>
 struct BlendStage {
   static constexpr int kListSplats = kBatch < 256 ? kBatch : 256;
-  float4 d[kBatch + 1][kSlotBytes / 16];
-  uint32_t list[kBlendWarps][kListSplats + 4];  // byte offsets of a warp's candidates, padded
+  float4 d[kBatch][kSlotBytes / 16];
+  uint32_t list[kBlendWarps][kListSplats];      // byte offsets of a warp's candidates
   uint32_t mask[kBatch / 32][kBlendWarps];      // candidates of a group of 32 by warp
   uint32_t special[kBatch / 32];                // the group's splats that are not plain (plain_splat)
   float2 origin;                                // the tile's first pixel
   uint32_t first;                               // its range's begin
-  uint32_t tile;                                // block_tile's (the forward's; these three are here because
-                                                // registers are scarce: 1-3 % of the blends)
+  uint32_t tile, view;                          // block_tile's and its view (the forward's; these four are here
+                                                // because registers are scarce: 1-3 % of the blends)
 };
 
-// Must be followed by a block barrier.
+// Every warp writes what it reads (the same values), so no barrier is needed.
 template <int kBatch>
 __device__ __forceinline__ void init_stage(BlendStage<kBatch>& st, const TileJob& job) {
-  if (threadIdx.x == 0) {
+  if ((threadIdx.x & 31) == 0) {
     st.origin = make_float2((float)(job.tile_x * 16), (float)(job.tile_y * 16));
     st.first = job.range.x;
   }
-  if (threadIdx.x < kSlotBytes / 16) st.d[kBatch][threadIdx.x] = make_float4(0.f, 0.f, 0.f, 0.f);
+  __syncwarp();
 }
 
 // Stages instances [base, base + cnt) of the tile's list, which begins at `first` (from the back when kReverse: slot t holds
@@ -199,7 +198,7 @@ __device__ __forceinline__ void stage_splats(BlendStage<kBatch>& st, const Blend
   const int lane = threadIdx.x & 31;
   const float2 origin = st.origin;
 #pragma unroll 1
-  for (int t = threadIdx.x; t < kBatch; t += kBlendThreads) {
+  for (int t = threadIdx.x; t - lane < cnt; t += kBlendThreads) {  // (whole groups of 32)
     bool hits[kBlendWarps] = {}, special = false;
     if (t < cnt) {
       const uint32_t pos = kReverse ? (uint32_t)(base - 1 - t) : (uint32_t)(base + t);
@@ -226,27 +225,32 @@ __device__ __forceinline__ void stage_splats(BlendStage<kBatch>& st, const Blend
   }
 }
 
-// The warp's candidates among slots [max(from, first), from + kListSplats) of the staged batch, in
-// slot order: writes their offsets to its list (padded to a multiple of four), returns their number
-// and whether any is special.
+// The warp's candidates among slots [max(from, first), min(from + kListSplats, cnt)) of the staged batch of cnt, in slot
+// order: writes their offsets to its list, returns their number and whether any is special.  (Short lists are a large
+// part of the blends' time in sparse views, so groups past cnt are not looked at, and nothing is padded.)
 template <int kBatch>
-__device__ __forceinline__ int list_candidates(BlendStage<kBatch>& st, int from, int first, bool& special) {
+__device__ __forceinline__ int list_candidates(BlendStage<kBatch>& st, int from, int first, int cnt, bool& special) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t* list = st.list[warp];
   const unsigned lt = (1u << lane) - 1u;
   int n = 0;
   unsigned sp = 0;
   __syncwarp();  // the warp has read its previous list
-#pragma unroll
-  for (int i = 0; i < BlendStage<kBatch>::kListSplats / 32; ++i) {
-    const int k = from / 32 + i;
+  auto group = [&](int k) {
     unsigned m = st.mask[k][warp];
     if (first > k * 32) m = first - k * 32 >= 32 ? 0u : m & (kFullMask << (first - k * 32));
     sp |= m & st.special[k];
     if ((m >> lane) & 1u) list[n + __popc(m & lt)] = (uint32_t)(k * 32 + lane) * kSlotBytes;
     n += __popc(m);
+  };
+  constexpr int kGroups = BlendStage<kBatch>::kListSplats / 32;
+  if (cnt > from + (kGroups - 1) * 32) {
+#pragma unroll
+    for (int i = 0; i < kGroups; ++i) group(from / 32 + i);
+  } else {
+#pragma unroll 1
+    for (int k = from / 32; k * 32 < cnt; ++k) group(k);
   }
-  if (lane < 4) list[n + lane] = kBatch * kSlotBytes;
   __syncwarp();
   special = sp != 0;
   return n;
@@ -307,7 +311,7 @@ __device__ __forceinline__ void forward_pixel(float alpha, float power, float te
 // issue slot) where both factors differ by pixel, and scalar where one is the splat's: broadcasting that
 // into a register pair costs the moves that packing saves.  Bound by instruction issue.  Measured on a
 // B200 (1M-Gaussian 2048x1024 view / 16-view batch) against a warp testing every staged splat itself and
-// walking the ballots' bits: 424 -> 406 us / 5.20 -> 5.16 ms.
+// walking the ballots' bits: 424 -> 397 us / 5.20 -> 5.02 ms (short lists aside: blend_forward_short).
 template <int kBatch, bool kWrap, bool kColor>
 __device__ __forceinline__ void forward_pass(const TileJob& job, const BlendSource& src, const BlendPatch& patch,
                                              BlendStage<kBatch>& st, float T[2], uint32_t lc[2], float C[2][3]) {
@@ -323,7 +327,6 @@ __device__ __forceinline__ void forward_pass(const TileJob& job, const BlendSour
   const char* slots = reinterpret_cast<const char*>(&st.d[0][0]);
   const uint32_t* list = st.list[threadIdx.x >> 5];
   init_stage(st, job);
-  __syncthreads();
 
   auto blend = [&](uint32_t off, auto plain) {
     constexpr bool kPlain = decltype(plain)::value;
@@ -344,25 +347,29 @@ __device__ __forceinline__ void forward_pass(const TileJob& job, const BlendSour
     forward_pixel<kPlain, kColor>(alpha.y, power.y, test_T.y, v1.z, v1.w, v2.x, at, T[1], lc[1], C[1][0], C[1][1], C[1][2]);
   };
   auto blend_list = [&](int cnt, auto plain) {
+    int i = 0;
 #pragma unroll 1
-    for (int i = 0; i < cnt; i += 4) {
+    for (; i + 4 <= cnt; i += 4) {
       const uint4 o = *reinterpret_cast<const uint4*>(list + i);
       blend(o.x, plain);
       blend(o.y, plain);
       blend(o.z, plain);
       blend(o.w, plain);
-      if ((i & 4) && __all_sync(kFullMask, T[0] < 0.f && T[1] < 0.f)) break;
+      if ((i & 4) && __all_sync(kFullMask, T[0] < 0.f && T[1] < 0.f)) return;
     }
+#pragma unroll 1
+    for (; i < cnt; ++i) blend(list[i], plain);
   };
   for (int base = 0; base < n; base += kBatch) {
-    if (__syncthreads_and(T[0] < 0.f && T[1] < 0.f)) break;
-    stage_splats<kBatch, kWrap, kColor, /*kReverse=*/false>(st, src, job, st.first, base, min(kBatch, n - base));
+    if (base > 0 && __syncthreads_and(T[0] < 0.f && T[1] < 0.f)) break;
+    const int staged = min(kBatch, n - base);
+    stage_splats<kBatch, kWrap, kColor, /*kReverse=*/false>(st, src, job, st.first, base, staged);
     __syncthreads();
 #pragma unroll 1
-    for (int from = 0; from < kBatch; from += BlendStage<kBatch>::kListSplats) {
+    for (int from = 0; from < staged; from += BlendStage<kBatch>::kListSplats) {
       if (__all_sync(kFullMask, T[0] < 0.f && T[1] < 0.f)) break;
       bool special;
-      const int cnt = list_candidates(st, from, 0, special);
+      const int cnt = list_candidates(st, from, 0, staged, special);
       if (special)
         blend_list(cnt, std::false_type{});
       else
@@ -373,8 +380,9 @@ __device__ __forceinline__ void forward_pass(const TileJob& job, const BlendSour
   T[1] = fabsf(T[1]);
 }
 
-// Tile `tile` (y << 16 | x) of a view.
-__device__ __forceinline__ TileJob tile_job(const RenderParams& p, uint32_t tile, uint2 range) {
+// The view of a block's tile, and that tile: of one view, whose tiles are y << 16 | x.
+__device__ __forceinline__ uint32_t tile_view(const RenderParams&, uint32_t) { return 0u; }
+__device__ __forceinline__ TileJob tile_job(const RenderParams& p, uint32_t, uint32_t tile, uint2 range) {
   TileJob job;
   job.tile_x = (int)(tile & 0xffffu);
   job.tile_y = (int)(tile >> 16);
@@ -390,15 +398,18 @@ __device__ __forceinline__ TileJob tile_job(const RenderParams& p, uint32_t tile
   return job;
 }
 
-// The view and tile of global tile `block` of a batched blend: the tiles run over the views in the order
-// of tile_base (the host lays the views out heaviest tiles first).
-__device__ __forceinline__ TileJob tile_job(const BatchRenderParams& p, uint32_t block, uint2 range) {
-  int v = p.tile_order[0];
-#pragma unroll 1
-  for (int k = 1; k < p.V; ++k) {
-    const int w = p.tile_order[k];
-    if (p.views[w].tile_base <= block) v = w;
-  }
+// Of a batch, whose tiles are numbered over the views in the order of tile_base (the host lays the views out
+// heaviest tiles first).
+__device__ __forceinline__ uint32_t tile_view(const BatchRenderParams& p, uint32_t block) {
+  // the largest first tile not beyond the block, a lane per view (one by one, 32 views took a tenth of the
+  // forward blend of few Gaussians)
+  static_assert(kMaxBatchViews == 32, "a lane per view");
+  const int lane = threadIdx.x & 31;
+  uint32_t base = lane < p.V ? p.views[lane].tile_base : 0xffffffffu;
+  base = base <= block ? base + 1u : 0u;
+  return (uint32_t)__ffs(__ballot_sync(kFullMask, base == __reduce_max_sync(kFullMask, base))) - 1u;
+}
+__device__ __forceinline__ TileJob tile_job(const BatchRenderParams& p, uint32_t v, uint32_t block, uint2 range) {
   const BatchView& bv = p.views[v];
   const uint32_t local = block - bv.tile_base;
   TileJob job;

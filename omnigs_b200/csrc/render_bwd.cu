@@ -104,6 +104,7 @@ __device__ __forceinline__ void blend_backward_tile(const TileJob& job, const Bl
   const BlendPatch patch = BlendPatch::make(job.tile_x, job.tile_y, job.wrap_w);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t n = job.range.y - job.range.x;
+  if (n == 0) return;
 
   // Per-pixel state of the thread's two pixels (rows py0 and py0 + 4).
   const int64_t HW = (int64_t)job.H * job.W;
@@ -214,23 +215,26 @@ __device__ __forceinline__ void blend_backward_tile(const TileJob& job, const Bl
     }
   };
   auto blend_list = [&](int cnt, auto plain) {
+    int i = 0;
 #pragma unroll 1
-    for (int i = 0; i < cnt; i += 2) {  // (a padded list may end in a splat that reaches no pixel)
+    for (; i + 2 <= cnt; i += 2) {
       const uint2 o = *reinterpret_cast<const uint2*>(list + i);
       blend(o.x, plain);
       blend(o.y, plain);
     }
+    if (i < cnt) blend(list[i], plain);
   };
   for (int hi = (int)block_last; hi > 0; hi -= kBatch) {
     __syncthreads();
-    stage_splats<kBatch, kWrap, true, /*kReverse=*/true>(sm.stage, src, job, job.range.x, hi, min(kBatch, hi));
+    const int staged = min(kBatch, hi);
+    stage_splats<kBatch, kWrap, true, /*kReverse=*/true>(sm.stage, src, job, job.range.x, hi, staged);
     __syncthreads();
     const int first = max(0, hi - (int)warp_last);  // slots before it lie behind every last contributor
 #pragma unroll 1
-    for (int from = 0; from < kBatch; from += BlendStage<kBatch>::kListSplats) {
+    for (int from = 0; from < staged; from += BlendStage<kBatch>::kListSplats) {
       if (first >= from + BlendStage<kBatch>::kListSplats) continue;
       bool special;
-      const int cnt = list_candidates(sm.stage, from, first, special);
+      const int cnt = list_candidates(sm.stage, from, first, staged, special);
       if (special)
         blend_list(cnt, std::false_type{});
       else
@@ -244,7 +248,7 @@ __device__ __forceinline__ void blend_backward_tile(const TileJob& job, const Bl
 template <int kBatch, bool kRecompute>
 __global__ void __launch_bounds__(kBlendThreads, kBlendBwdMinBlocks) render_backward_kernel(RenderParams p) {
   const uint3 tile = block_tile(p.block_tiles, p.ranges, blockIdx.y * p.gx + blockIdx.x, blockIdx.y << 16 | blockIdx.x);
-  const TileJob job = tile_job(p, tile.z, make_uint2(tile.x, tile.y));
+  const TileJob job = tile_job(p, tile_view(p, tile.z), tile.z, make_uint2(tile.x, tile.y));
   blend_backward_tile<kBatch, false, kRecompute>(job, BlendSource{p.point_list, p.splat, p.color, (uint32_t)p.P, p.capacity},
                                                  p.grad_acc);
 }
@@ -254,7 +258,7 @@ template <int kBatch, bool kWrap>
 __global__ void __launch_bounds__(kBlendThreads, kBlendBwdMinBlocks) batch_render_backward_kernel(const __grid_constant__ BatchRenderParams p) {
   const uint3 tile = block_tile(p.block_tiles, p.ranges, blockIdx.x, blockIdx.x);
   if (tile.z >= p.total_tiles) return;  // (never, after a binning)
-  const TileJob job = tile_job(p, tile.z, make_uint2(tile.x, tile.y));
+  const TileJob job = tile_job(p, tile_view(p, tile.z), tile.z, make_uint2(tile.x, tile.y));
   blend_backward_tile<kBatch, kWrap, false>(job, BlendSource{p.point_list, p.splat, p.color, (uint32_t)p.P * (uint32_t)p.V, p.capacity},
                                             p.grad_acc);
 }
