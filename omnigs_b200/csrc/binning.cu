@@ -81,6 +81,7 @@ __device__ __forceinline__ void count_digit(uint32_t* hist, uint32_t digit, bool
 constexpr int kHistUnroll = 4;  // keys per thread loaded before any of them is counted
 
 __global__ void __launch_bounds__(256) histogram_kernel(const __grid_constant__ HistParams p) {
+  chain_begin();
   __shared__ uint32_t s_hist[kDepthPasses][kRadix];
   for (int i = threadIdx.x; i < kDepthPasses * kRadix; i += blockDim.x) (&s_hist[0][0])[i] = 0;
   __syncthreads();
@@ -180,6 +181,7 @@ static_assert(sizeof(OnesweepParams) <= 128, "keep the onesweep parameter block 
 // those: 282 -> 276 us for the whole forward of 150,000 Gaussians (147 tiles), nothing at 300,000 (293).
 template <int kItems, int kMinBlocks, int kLookback>
 __global__ void __launch_bounds__(kSortThreads, kMinBlocks) onesweep_kernel(OnesweepParams p) {
+  chain_begin();
   constexpr int kTile = kSortThreads * kItems;
   __shared__ SortSmem<kTile> sm;
   const uint32_t n = p.seg_len ? p.seg_len : item_count(p.count_hdr, p.n_host, p.capacity);
@@ -438,6 +440,7 @@ __device__ __forceinline__ uint32_t tile_mask(int tx0, int ty0, int gx, bool wra
 constexpr int kScanItems = kScanTile / kScanBlock;  // Gaussians per scan thread
 
 __global__ void __launch_bounds__(kScanBlock) pair_scan_kernel(const __grid_constant__ DuplicateParams p) {
+  chain_begin();
   __shared__ uint32_t s_tile;
   __shared__ uint32_t s_warp[kScanBlock / 32];
   __shared__ unsigned long long s_excl;
@@ -568,6 +571,7 @@ __device__ __forceinline__ float rcp_approx_f(float x) {
 }
 
 __global__ void __launch_bounds__(kScanBlock) pair_emit_kernel(const __grid_constant__ DuplicateParams p) {
+  chain_begin();
   __shared__ uint32_t s_hist[kTilePasses * kRadix];  // digit counts of the bin sort
   // the block's Gaussians: inclusive offset, record, tile rect
   __shared__ uint32_t s_incl[kEmitStage], s_rec[kEmitStage];
@@ -790,6 +794,7 @@ __global__ void __launch_bounds__(kRankThreads) rank_kernel(const __grid_constan
 
 // Tile rects in depth order, where the depth order comes from the sort and no scan needs them.
 __global__ void __launch_bounds__(256) rect_kernel(const __grid_constant__ RankParams p) {
+  chain_begin();
   const uint32_t i = blockIdx.x * 256u + threadIdx.x;
   if (i >= (uint32_t)p.grid.P * (uint32_t)p.grid.V) return;
   const uint2 r = record_rect(p.grid, p.radii, p.splat, p.order[i], record_view(p.grid, i));
@@ -1458,18 +1463,18 @@ int sm_count() {
 
 }  // namespace
 
-void launch_histogram(const HistParams& p, int64_t max_items, cudaStream_t s) {
+void launch_histogram(const HistParams& p, int64_t max_items, bool chained, cudaStream_t s) {
   const unsigned segs = p.seg_len ? std::max(1u, p.num_segs) : 1u;
   const int64_t per_seg = p.seg_len ? (int64_t)p.seg_len : max_items;
   const int64_t blocks = std::max<int64_t>(
       1, std::min<int64_t>((per_seg + 256 * kHistUnroll - 1) / (256 * kHistUnroll),
                            std::max<int64_t>(1, sm_count() * 4 / segs)));
-  histogram_kernel<<<dim3((unsigned)blocks, segs), 256, 0, s>>>(p);
+  launch_chained(chained, histogram_kernel, dim3((unsigned)blocks, segs), 256, 0, s, p);
 }
 
-void launch_onesweep(const OnesweepParams& p, int64_t max_items, int64_t expected, cudaStream_t s) {
+void launch_onesweep(const OnesweepParams& p, int64_t max_items, int64_t expected, bool chained, cudaStream_t s) {
   if (p.seg_len && small_sort(p.seg_len, p.num_segs)) {  // (the depth sort: its look-back words have room)
-    onesweep_kernel<kSmallSortItems, 5, 16><<<(unsigned)sort_blocks(p.seg_len, p.num_segs), kSortThreads, 0, s>>>(p);
+    launch_chained(chained, onesweep_kernel<kSmallSortItems, 5, 16>, (unsigned)sort_blocks(p.seg_len, p.num_segs), kSortThreads, 0, s, p);
     return;
   }
   const int64_t blocks = p.seg_len ? sort_tiles(p.seg_len) * (int64_t)p.num_segs : sort_tiles(max_items);
@@ -1481,17 +1486,17 @@ void launch_onesweep(const OnesweepParams& p, int64_t max_items, int64_t expecte
   // and a half a Gaussian are expected, as for the lists.
   const int64_t tiles = p.seg_len ? blocks : sort_tiles(expected), sms = sm_count();
   if (tiles <= 3 * sms)
-    onesweep_kernel<kSortItems, 3, kLookbackBatch><<<(unsigned)blocks, kSortThreads, 0, s>>>(p);
+    launch_chained(chained, onesweep_kernel<kSortItems, 3, kLookbackBatch>, (unsigned)blocks, kSortThreads, 0, s, p);
   else if (tiles > 4 * sms && tiles <= 5 * sms)
-    onesweep_kernel<kSortItems, 5, kLookbackBatch><<<(unsigned)blocks, kSortThreads, 0, s>>>(p);
+    launch_chained(chained, onesweep_kernel<kSortItems, 5, kLookbackBatch>, (unsigned)blocks, kSortThreads, 0, s, p);
   else
-    onesweep_kernel<kSortItems, 4, kLookbackBatch><<<(unsigned)blocks, kSortThreads, 0, s>>>(p);
+    launch_chained(chained, onesweep_kernel<kSortItems, 4, kLookbackBatch>, (unsigned)blocks, kSortThreads, 0, s, p);
 }
 
 void launch_rects(const RankParams& p, cudaStream_t s) {
   const int64_t items = (int64_t)p.grid.P * p.grid.V;
   if (items <= 0) return;
-  rect_kernel<<<(unsigned)((items + 255) / 256), 256, 0, s>>>(p);
+  launch_chained(p.chained, rect_kernel, (unsigned)((items + 255) / 256), 256, 0, s, p);
 }
 
 void launch_begin_binning(const BeginParams& p, cudaStream_t s) {
@@ -1507,19 +1512,19 @@ void launch_rank(const RankParams& p, cudaStream_t s) {
   launch_chained(p.chained, rank_kernel, grid, kRankThreads, 0, s, p);
 }
 
-void launch_duplicate(const DuplicateParams& p, cudaStream_t s) {
+void launch_duplicate(const DuplicateParams& p, bool chained, cudaStream_t s) {
   const int64_t items = (int64_t)p.grid.P * p.grid.V;
   if (items <= 0) return;
   const int64_t tiles = (items + kScanTile - 1) / kScanTile;
   if (tiles <= (int64_t)p.skip_tiles) return;
   // scan: one block per scan tile that is taken (block k takes tile skip_tiles + k)
-  pair_scan_kernel<<<(unsigned)(tiles - p.skip_tiles), kScanBlock, 0, s>>>(p);
+  launch_chained(chained, pair_scan_kernel, (unsigned)(tiles - p.skip_tiles), kScanBlock, 0, s, p);
   // emit: one block per kEmitBlock pairs the binning buffer can hold (blocks past the device's pair
   // count return at once); a probe pass stops after the scan
   if (p.skip_tiles != 0) return;
   const int64_t eblocks = emit_blocks(std::min<int64_t>(p.capacity, 0xffffffffll));
   if (eblocks <= 0) return;
-  pair_emit_kernel<<<(unsigned)eblocks, kScanBlock, 0, s>>>(p);
+  launch_chained(chained, pair_emit_kernel, (unsigned)eblocks, kScanBlock, 0, s, p);
 }
 
 void launch_tile_lists(const TileListParams& p, int64_t expected_pairs, cudaStream_t s) {

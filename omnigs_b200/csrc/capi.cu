@@ -48,6 +48,12 @@ cudaEvent_t take_event() {
   return e;
 }
 
+// Whether the stream is being captured into a graph.
+static bool capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(s, &status) == cudaSuccess && status == cudaStreamCaptureStatusActive;
+}
+
 int run_binning(BinningPass& b, cudaStream_t s) {
   TileGrid& g = b.grid;
   g.num_bins = 0;
@@ -62,7 +68,8 @@ int run_binning(BinningPass& b, cudaStream_t s) {
   // lists, every bin reads the whole order (kWholeMaxPairs)
   const bool ranked = !probe && counts_order(g.P, g.V);
   const bool whole = !probe && (int64_t)g.num_bins * g.P <= kWholeMaxPairs;
-  b.small = ranked && whole;
+  const bool small = ranked && whole;
+  b.chained = small || (!probe && records <= kChainRecords && !capturing(s));
   TileDigits digits = TileDigits::from_bits(id_bits(g.num_bins));  // of the bin in a pair's word
   const int64_t pair_tiles = sort_tiles(L.capacity);
   uint32_t* hist = at<uint32_t>(b.binning, L.hist);
@@ -109,8 +116,8 @@ int run_binning(BinningPass& b, cudaStream_t s) {
 
   BeginParams begin{};
   begin.hdr = b.hdr;
-  begin.chained = b.small;
-  if (!b.small) {
+  begin.chained = b.chained;
+  if (!small) {
     begin.region[0] = b.zero;
     begin.bytes[0] = b.zero_bytes;
     begin.region[1] = at<uint4>(b.binning, L.hist);
@@ -145,7 +152,7 @@ int run_binning(BinningPass& b, cudaStream_t s) {
   r.order = order;
   r.rect_x = rect_x;
   r.rect_y = rect_y;
-  r.chained = b.small;
+  r.chained = b.chained;
   if (ranked) {
     staged(OMNIGS_STAGE_SORT, 1, s, [&] { launch_rank(r, s); });
   } else {
@@ -161,7 +168,7 @@ int run_binning(BinningPass& b, cudaStream_t s) {
     hd.hist = b.depth_hist;
     hd.seg_len = (uint32_t)g.P;
     hd.num_segs = (uint32_t)g.V;
-    staged(OMNIGS_STAGE_SORT, 1, s, [&] { launch_histogram(hd, records, s); });
+    staged(OMNIGS_STAGE_SORT, 1, s, [&] { launch_histogram(hd, records, b.chained, s); });
     const int64_t depth_tiles = sort_blocks(g.P, g.V);
     for (int q = 0; q < kDepthPasses; ++q) {
       OnesweepParams op{};
@@ -179,7 +186,7 @@ int run_binning(BinningPass& b, cudaStream_t s) {
       op.seg_len = (uint32_t)g.P;
       op.num_segs = (uint32_t)g.V;
       op.hist_seg_stride = kDepthPasses * kRadix;
-      staged(OMNIGS_STAGE_SORT, 1, s, [&] { launch_onesweep(op, records, records, s); });
+      staged(OMNIGS_STAGE_SORT, 1, s, [&] { launch_onesweep(op, records, records, b.chained, s); });
     }
 
   }
@@ -215,7 +222,7 @@ int run_binning(BinningPass& b, cudaStream_t s) {
       d.max_spins = b.max_spins;
       d.skip_tiles = 1;
     }
-    staged(OMNIGS_STAGE_DUPLICATE, 2, s, [&] { launch_duplicate(d, s); });
+    staged(OMNIGS_STAGE_DUPLICATE, 2, s, [&] { launch_duplicate(d, b.chained, s); });
     if (probe) return check_launch("duplicate (look-back probe)");
     for (int q = 0; q < digits.passes; ++q) {
       const int from = (first + q) & 1;
@@ -232,7 +239,7 @@ int run_binning(BinningPass& b, cudaStream_t s) {
       op.lookback = at<uint32_t>(b.binning, L.tile_lookback) + (size_t)q * pair_tiles * kRadix;
       op.tile_counter = &b.hdr->sort_tile_counter[kDepthPasses + q];
       op.hdr = b.hdr;
-      staged(OMNIGS_STAGE_SORT, 1, s, [&] { launch_onesweep(op, b.capacity, 3 * records / 2, s); });
+      staged(OMNIGS_STAGE_SORT, 1, s, [&] { launch_onesweep(op, b.capacity, 3 * records / 2, b.chained, s); });
     }
     t.words = keys[sorted];
     t.recs = vals[sorted];
@@ -240,7 +247,7 @@ int run_binning(BinningPass& b, cudaStream_t s) {
 
   // 3. tile lists and ranges
   t.grid = g;
-  t.chained = b.small;
+  t.chained = b.chained;
   t.order = order;
   t.rect_x = rect_x;
   t.rect_y = rect_y;
@@ -514,7 +521,7 @@ int render_impl(const OmnigsLonlatForwardArgs* a, void* geom, size_t geom_bytes,
   r.ranges = ranges;
   r.block_tiles = b.block_tiles;
   r.point_list = at<uint32_t>(binning, fin ? BL.tvals1 : BL.tvals0);
-  r.chained = b.small;
+  r.chained = b.chained;
   r.capacity = capacity;
   r.splat = at<float4>(geom, GL.splat);
   r.color = at<float4>(geom, GL.color);

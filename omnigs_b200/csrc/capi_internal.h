@@ -93,7 +93,7 @@ struct BinningPass {
   GeomHeader* hdr;
   int out;                       // binning buffer (0 or 1) that receives the sorted list
   int max_spins;                 // look-back probe: wait limit, and stop after the scan (0: a real pass)
-  bool small;                    // set by the pass: a small scene's path was taken
+  bool chained;                  // set by the pass: its kernels are chained (launch_chained)
 };
 int run_binning(BinningPass& b, cudaStream_t s);
 

@@ -41,10 +41,9 @@ __device__ __forceinline__ void chain_begin() {
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31; }
 
 // Launches a kernel that begins with chain_begin(), with `chained` so that its launch overlaps the kernel
-// before it on the stream (also inside a captured graph).  Measured on a B200: the forward of 10,000
-// Gaussians at 512x256, whose kernels are a few microseconds each, 64.5 -> 57.2 us; where kernels are
-// longer it gains nothing, and costs 2 % of a captured train step over 200,000 Gaussians and 0.5 % of
-// the 16-view batch, so only the binning of small scenes and the blend behind it are chained.
+// before it on the stream (also inside a captured graph).  Where kernels are a few microseconds long that is
+// much of their time (64.5 -> 57.2 us for the forward of 10,000 Gaussians at 512x256); where they are longer it
+// costs more than it gains (kChainRecords).
 template <class... Params, class... Args>
 inline void launch_chained(bool chained, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
   cudaLaunchConfig_t cfg{};

@@ -155,7 +155,7 @@ struct BeginParams {
   static constexpr int kRegions = 4;
   uint4* region[kRegions];     // 16-byte aligned
   size_t bytes[kRegions];      // multiples of 16
-  bool chained;                // as the small scenes' other kernels (launch_chained)
+  bool chained;
 };
 
 struct RenderParams {
@@ -170,7 +170,7 @@ struct RenderParams {
   float* out_color;
   float* final_T;       // NULL with transmittance checkpointing: the forward does not store it and
   uint32_t* n_contrib;  // the backward recomputes it
-  bool chained;         // the forward, behind a small scene's binning (launch_chained)
+  bool chained;         // the forward, behind a chained binning (launch_chained)
   // backward only
   const float* dL_dpix;
   float* grad_acc;  // [P][12]
@@ -283,12 +283,13 @@ void launch_batch_preprocess_backward(const BatchParams& p, const BatchGrads& g,
                                       cudaStream_t s);
 
 void launch_preprocess(const PreprocessParams& p, cudaStream_t s);
-void launch_histogram(const HistParams& p, int64_t max_items, cudaStream_t s);
-void launch_onesweep(const OnesweepParams& p, int64_t max_items, int64_t expected, cudaStream_t s);
+// `chained`: as launch_chained's, also in the other parameter blocks
+void launch_histogram(const HistParams& p, int64_t max_items, bool chained, cudaStream_t s);
+void launch_onesweep(const OnesweepParams& p, int64_t max_items, int64_t expected, bool chained, cudaStream_t s);
 void launch_begin_binning(const BeginParams& p, cudaStream_t s);
 void launch_rank(const RankParams& p, cudaStream_t s);
 void launch_rects(const RankParams& p, cudaStream_t s);  // rects only, in the order given
-void launch_duplicate(const DuplicateParams& p, cudaStream_t s);
+void launch_duplicate(const DuplicateParams& p, bool chained, cudaStream_t s);
 void launch_tile_lists(const TileListParams& p, int64_t expected_pairs, cudaStream_t s);
 // Splats staged per shared-memory batch in the blend kernels: a template parameter chosen at run
 // time per direction (128, 256 or 512; set by omnigs_set_blend_batch or the autotuner).  Results

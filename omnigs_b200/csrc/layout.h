@@ -162,6 +162,13 @@ inline bool counts_order(int64_t P, int64_t V) { return P <= kRankMaxP && V * P 
 // Up to kWholeMaxPairs (Gaussian, bin) combinations every bin reads its view's whole depth order (binning.cu).
 constexpr int64_t kWholeMaxPairs = int64_t(1) << 20;
 
+// Up to kChainRecords (Gaussian, view) records the binning's kernels are chained (launch_chained): it is a row of a dozen
+// launches there.  Measured on a B200, forward without / with: 20,000 Gaussians at 2132x1093 163 / 141 us, 70,000 at
+// 2048x1024 184 / 165, 300,000 402 / 387; 1M 677 / 674; forward and backward 3M at 4096x2048 3924 / 3999, six views of
+// 20,000 at 1024x512 299 / 288.  A captured graph has no such gaps, and chained it measured slower (a train step over four
+// views of 200,000 Gaussians 1282 / 1303 us), except where everything is short (every bin reads the whole counted order).
+constexpr int64_t kChainRecords = int64_t(1) << 19;
+
 // The duplicate pass writes its list in blocks of kEmitBlock pairs; its scan records, per such block, the
 // depth-order positions of the Gaussians holding the block's first and last pair (emit_first / emit_last).
 constexpr int kEmitBlock = 2048;

@@ -25,7 +25,7 @@ namespace {
 constexpr int kPrepBlock = 128;
 
 __global__ void __launch_bounds__(kPrepBlock, 6) preprocess_kernel(PreprocessParams p) {
-  chain_begin();  // (the binning of a small scene is launched behind it)
+  chain_begin();  // (a chained binning is launched behind it)
   __shared__ uint32_t s_warp[kPrepBlock / 32];
   __shared__ float4 s_sh[kPrepBlock / 32][32 * kShStageStride];
   const int idx = blockIdx.x * kPrepBlock + threadIdx.x;
