@@ -577,150 +577,151 @@ __global__ void __launch_bounds__(kScanBlock) pair_emit_kernel(const __grid_cons
   __shared__ uint32_t s_incl[kEmitStage], s_rec[kEmitStage];
   __shared__ uint2 s_rect[kEmitStage];
   __shared__ uint32_t s_last;
-  if (!instances_fit(p.hdr, p.capacity)) return;  // the scan kernel has flagged the overflow
-  const uint32_t R = pair_count(p.hdr, p.capacity);
-  const uint32_t o_lo = blockIdx.x * (uint32_t)kEmitBlock;
-  if (o_lo >= R) return;
-  const uint32_t o_hi = min(R, o_lo + (uint32_t)kEmitBlock);  // exclusive (R <= capacity)
-  const int lane = threadIdx.x & 31;
-  const uint32_t items = (uint32_t)p.grid.P * (uint32_t)p.grid.V;
-  for (int k = threadIdx.x; k < kTilePasses * kRadix; k += kScanBlock) s_hist[k] = 0;
-  // (both clamped: after an inconsistent scan, which the status word reports, the entries may be
-  // stale; the reads stay in range)
-  const uint32_t g_first = min(p.emit_first[blockIdx.x], items - 1u);
-  if (threadIdx.x == 0) {
-    uint32_t last = items - 1u;
-    if (o_hi - o_lo == (uint32_t)kEmitBlock) {
-      last = min(p.emit_last[blockIdx.x], items - 1u);
-    } else {  // the list's end: the first Gaussian whose inclusive offset reaches it
-      uint32_t lo = g_first;
-      while (lo < last) {
-        const uint32_t mid = (lo + last) >> 1;
-        if (p.incl[mid] >= R)
-          last = mid;
+  const uint32_t R = pair_count(p.hdr, p.capacity);  // (0 when the scan kernel has flagged an overflow)
+#pragma unroll 1
+  for (uint32_t block = blockIdx.x; block < (R + kEmitBlock - 1u) / kEmitBlock; block += gridDim.x) {
+    const uint32_t o_lo = block * (uint32_t)kEmitBlock;
+    const uint32_t o_hi = min(R, o_lo + (uint32_t)kEmitBlock);  // exclusive (R <= capacity)
+    const int lane = threadIdx.x & 31;
+    const uint32_t items = (uint32_t)p.grid.P * (uint32_t)p.grid.V;
+    for (int k = threadIdx.x; k < kTilePasses * kRadix; k += kScanBlock) s_hist[k] = 0;
+    // (both clamped: after an inconsistent scan, which the status word reports, the entries may be
+    // stale; the reads stay in range)
+    const uint32_t g_first = min(p.emit_first[block], items - 1u);
+    if (threadIdx.x == 0) {
+      uint32_t last = items - 1u;
+      if (o_hi - o_lo == (uint32_t)kEmitBlock) {
+        last = min(p.emit_last[block], items - 1u);
+      } else {  // the list's end: the first Gaussian whose inclusive offset reaches it
+        uint32_t lo = g_first;
+        while (lo < last) {
+          const uint32_t mid = (lo + last) >> 1;
+          if (p.incl[mid] >= R)
+            last = mid;
+          else
+            lo = mid + 1u;
+        }
+      }
+      s_last = last;
+    }
+    __syncthreads();
+    const uint32_t g_last = s_last;
+    const uint32_t n = g_last >= g_first ? g_last - g_first + 1u : 1u;
+    // Gaussians between g_first and g_last with no pairs (culled views' records) can make the range longer
+    // than the block's pair count: then offsets and rects are read from global memory
+    const bool staged = n <= (uint32_t)kEmitStage;
+    if (staged)
+      for (uint32_t t = threadIdx.x; t < n; t += kScanBlock) {
+        s_incl[t] = p.incl[g_first + t];
+        s_rec[t] = p.order[g_first + t];
+        s_rect[t] = make_uint2(p.rect_x[g_first + t], p.rect_y[g_first + t]);
+      }
+    __syncthreads();
+    const uint32_t* incl = staged ? s_incl : p.incl + g_first;
+    const uint32_t excl0 = g_first > 0 ? p.incl[g_first - 1] : 0u;
+    // Thread t writes the kEmitPerThread consecutive pairs from o0: one binary search finds the Gaussian
+    // of the first, the others step through the rect (or on to the next Gaussians with pairs, whose
+    // first pair they then are) without a search or a division.
+    const uint32_t o0 = o_lo + (uint32_t)threadIdx.x * (uint32_t)kEmitPerThread;
+    uint32_t j = 0;  // the first of the block's Gaussians whose inclusive offset exceeds o0
+    {
+      uint32_t hi = n - 1u;
+      while (j < hi) {
+        const uint32_t mid = (j + hi) >> 1;
+        if (incl[mid] > o0)
+          hi = mid;
         else
-          lo = mid + 1u;
+          j = mid + 1u;
       }
     }
-    s_last = last;
-  }
-  __syncthreads();
-  const uint32_t g_last = s_last;
-  const uint32_t n = g_last >= g_first ? g_last - g_first + 1u : 1u;
-  // Gaussians between g_first and g_last with no pairs (culled views' records) can make the range longer
-  // than the block's pair count: then offsets and rects are read from global memory
-  const bool staged = n <= (uint32_t)kEmitStage;
-  if (staged)
-    for (uint32_t t = threadIdx.x; t < n; t += kScanBlock) {
-      s_incl[t] = p.incl[g_first + t];
-      s_rec[t] = p.order[g_first + t];
-      s_rect[t] = make_uint2(p.rect_x[g_first + t], p.rect_y[g_first + t]);
+    uint32_t end_j = incl[j];
+    uint32_t rec = 0, view = 0, width = 1;
+    int gx = 1, bx = 1;
+    uint2 rect = make_uint2(0u, 0u);
+    BinRect bins{0u, 1u, 0u, 1u};
+    auto load_rect = [&](uint32_t jj) {
+      const uint32_t i = g_first + jj;
+      view = record_view(p.grid, i);
+      rec = staged ? s_rec[jj] : p.order[i];
+      rect = staged ? s_rect[jj] : make_uint2(p.rect_x[i], p.rect_y[i]);
+      gx = p.grid.gx[view];
+      bx = bins_x(gx);
+      bins = bin_rect(rect, gx, bx);
+      width = max(bins.cols, 1u);
+    };
+    load_rect(j);
+    // row and column of o0 in the rect: local / width from an approximate reciprocal (local < 2^21, a rect
+    // holds at most every bin of a view, so the truncated estimate is within one of the quotient; one
+    // step fixes it)
+    const uint32_t local = o0 - (j > 0 ? incl[j - 1] : excl0);
+    uint32_t ry = (uint32_t)((float)local * rcp_approx_f((float)width));
+    int rem = (int)(local - ry * width);
+    if (rem < 0) {
+      ry -= 1u;
+      rem += (int)width;
+    } else if (rem >= (int)width) {
+      ry += 1u;
+      rem -= (int)width;
     }
-  __syncthreads();
-  const uint32_t* incl = staged ? s_incl : p.incl + g_first;
-  const uint32_t excl0 = g_first > 0 ? p.incl[g_first - 1] : 0u;
-  // Thread t writes the kEmitPerThread consecutive pairs from o0: one binary search finds the Gaussian
-  // of the first, the others step through the rect (or on to the next Gaussians with pairs, whose
-  // first pair they then are) without a search or a division.
-  const uint32_t o0 = o_lo + (uint32_t)threadIdx.x * (uint32_t)kEmitPerThread;
-  uint32_t j = 0;  // the first of the block's Gaussians whose inclusive offset exceeds o0
-  {
-    uint32_t hi = n - 1u;
-    while (j < hi) {
-      const uint32_t mid = (j + hi) >> 1;
-      if (incl[mid] > o0)
-        hi = mid;
-      else
-        j = mid + 1u;
-    }
-  }
-  uint32_t end_j = incl[j];
-  uint32_t rec = 0, view = 0, width = 1;
-  int gx = 1, bx = 1;
-  uint2 rect = make_uint2(0u, 0u);
-  BinRect bins{0u, 1u, 0u, 1u};
-  auto load_rect = [&](uint32_t jj) {
-    const uint32_t i = g_first + jj;
-    view = record_view(p.grid, i);
-    rec = staged ? s_rec[jj] : p.order[i];
-    rect = staged ? s_rect[jj] : make_uint2(p.rect_x[i], p.rect_y[i]);
-    gx = p.grid.gx[view];
-    bx = bins_x(gx);
-    bins = bin_rect(rect, gx, bx);
-    width = max(bins.cols, 1u);
-  };
-  load_rect(j);
-  // row and column of o0 in the rect: local / width from an approximate reciprocal (local < 2^21, a rect
-  // holds at most every bin of a view, so the truncated estimate is within one of the quotient; one
-  // step fixes it)
-  const uint32_t local = o0 - (j > 0 ? incl[j - 1] : excl0);
-  uint32_t ry = (uint32_t)((float)local * rcp_approx_f((float)width));
-  int rem = (int)(local - ry * width);
-  if (rem < 0) {
-    ry -= 1u;
-    rem += (int)width;
-  } else if (rem >= (int)width) {
-    ry += 1u;
-    rem -= (int)width;
-  }
-  uint32_t keys[kEmitPerThread], vals[kEmitPerThread];
-#pragma unroll
-  for (int k = 0; k < kEmitPerThread; ++k) {
-    const uint32_t o = o0 + (uint32_t)k;
-    const bool ok = o < o_hi;
-    if (k > 0 && ok) {
-      // past Gaussian j: on to the next one that has pairs, whose first pair o is (j stays below n even
-      // after an inconsistent scan, which the status word reports)
-      if (o >= end_j && j + 1u < n) {
-        do {
-          ++j;
-          end_j = incl[j];
-        } while (end_j <= o && j + 1u < n);
-        load_rect(j);
-        ry = 0;
-        rem = 0;
-      } else if (++rem == (int)width) {
-        rem = 0;
-        ++ry;
+    uint32_t keys[kEmitPerThread], vals[kEmitPerThread];
+  #pragma unroll
+    for (int k = 0; k < kEmitPerThread; ++k) {
+      const uint32_t o = o0 + (uint32_t)k;
+      const bool ok = o < o_hi;
+      if (k > 0 && ok) {
+        // past Gaussian j: on to the next one that has pairs, whose first pair o is (j stays below n even
+        // after an inconsistent scan, which the status word reports)
+        if (o >= end_j && j + 1u < n) {
+          do {
+            ++j;
+            end_j = incl[j];
+          } while (end_j <= o && j + 1u < n);
+          load_rect(j);
+          ry = 0;
+          rem = 0;
+        } else if (++rem == (int)width) {
+          rem = 0;
+          ++ry;
+        }
       }
+      uint32_t col = bins.col + (uint32_t)rem;
+      if (col >= (uint32_t)bx) col -= (uint32_t)bx;  // the seam wraps
+      const uint32_t row = bins.row + ry;
+      const uint32_t key = ((p.grid.bin_base[view] + row * (uint32_t)bx + col) << kPairBinShift) |
+                           tile_mask((int)col * kBinW, (int)row * kBinH, gx, p.grid.seam_wrap != 0, rect);
+      keys[k] = key;
+      vals[k] = rec;
+      // digit histograms of the bin sort (the pass that would otherwise re-read every key)
+      const unsigned live = __ballot_sync(kFullMask, ok);
+  #pragma unroll
+      for (int q = 0; q < kTilePasses; ++q)
+        if (q < p.hist_passes)
+          count_digit(s_hist, q * kRadix + ((key >> p.hist_shift[q]) & p.hist_mask[q]), ok, live, lane);
     }
-    uint32_t col = bins.col + (uint32_t)rem;
-    if (col >= (uint32_t)bx) col -= (uint32_t)bx;  // the seam wraps
-    const uint32_t row = bins.row + ry;
-    const uint32_t key = ((p.grid.bin_base[view] + row * (uint32_t)bx + col) << kPairBinShift) |
-                         tile_mask((int)col * kBinW, (int)row * kBinH, gx, p.grid.seam_wrap != 0, rect);
-    keys[k] = key;
-    vals[k] = rec;
-    // digit histograms of the bin sort (the pass that would otherwise re-read every key)
-    const unsigned live = __ballot_sync(kFullMask, ok);
-#pragma unroll
-    for (int q = 0; q < kTilePasses; ++q)
-      if (q < p.hist_passes)
-        count_digit(s_hist, q * kRadix + ((key >> p.hist_shift[q]) & p.hist_mask[q]), ok, live, lane);
-  }
-  // the thread's run of the list: 16-byte stores when it is whole (o0 is a multiple of 8, the
-  // lists start 256-byte aligned)
-  static_assert(kEmitPerThread == 8, "two 16-byte stores per array");
-  if (o0 + (uint32_t)kEmitPerThread <= o_hi) {
-    uint4* kd = reinterpret_cast<uint4*>(p.keys + o0);
-    uint4* vd = reinterpret_cast<uint4*>(p.vals + o0);
-    kd[0] = make_uint4(keys[0], keys[1], keys[2], keys[3]);
-    kd[1] = make_uint4(keys[4], keys[5], keys[6], keys[7]);
-    vd[0] = make_uint4(vals[0], vals[1], vals[2], vals[3]);
-    vd[1] = make_uint4(vals[4], vals[5], vals[6], vals[7]);
-  } else {
-#pragma unroll
-    for (int k = 0; k < kEmitPerThread; ++k)
-      if (o0 + (uint32_t)k < o_hi) {
-        p.keys[o0 + k] = keys[k];
-        p.vals[o0 + k] = vals[k];
-      }
-  }
-  if (p.hist_passes == 0) return;
-  __syncthreads();
-  for (int k = threadIdx.x; k < kTilePasses * kRadix; k += kScanBlock) {
-    const uint32_t c = s_hist[k];
-    if (c) atomicAdd(&p.hist[k], c);
+    // the thread's run of the list: 16-byte stores when it is whole (o0 is a multiple of 8, the
+    // lists start 256-byte aligned)
+    static_assert(kEmitPerThread == 8, "two 16-byte stores per array");
+    if (o0 + (uint32_t)kEmitPerThread <= o_hi) {
+      uint4* kd = reinterpret_cast<uint4*>(p.keys + o0);
+      uint4* vd = reinterpret_cast<uint4*>(p.vals + o0);
+      kd[0] = make_uint4(keys[0], keys[1], keys[2], keys[3]);
+      kd[1] = make_uint4(keys[4], keys[5], keys[6], keys[7]);
+      vd[0] = make_uint4(vals[0], vals[1], vals[2], vals[3]);
+      vd[1] = make_uint4(vals[4], vals[5], vals[6], vals[7]);
+    } else {
+  #pragma unroll
+      for (int k = 0; k < kEmitPerThread; ++k)
+        if (o0 + (uint32_t)k < o_hi) {
+          p.keys[o0 + k] = keys[k];
+          p.vals[o0 + k] = vals[k];
+        }
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < kTilePasses * kRadix; k += kScanBlock) {
+      const uint32_t c = s_hist[k];
+      if (c) atomicAdd(&p.hist[k], c);
+    }
+    __syncthreads();  // (the next pairs' stage and histograms)
   }
 }
 
@@ -1037,6 +1038,9 @@ __device__ __forceinline__ uint32_t entry_tiles(const TileListParams& p, const B
   return tile_mask(b.tx0, b.ty0, b.gx, p.grid.seam_wrap != 0, make_uint2(p.rect_x[e], p.rect_y[e]));
 }
 
+// Whether a word's tiles are any of the bin's: a row and a column.
+__device__ __forceinline__ bool covers(uint32_t mask) { return (mask & 255u) != 0 && ((mask >> kBinW) & 15u) != 0; }
+
 // Every tile of the grid is written (0 when the instances do not fit).
 __global__ void __launch_bounds__(kListThreads) whole_count_kernel(const __grid_constant__ TileListParams p) {
   chain_begin();
@@ -1050,10 +1054,15 @@ __global__ void __launch_bounds__(kListThreads) whole_count_kernel(const __grid_
   TileCounts c;
   uint32_t mine = 0;  // instances of the lane's tile
   int steps = 0;
-#pragma unroll 4
-  for (uint32_t e0 = b.first; e0 < b.end; e0 += 32) {
-    c.add(e0 + lane < b.end ? entry_tiles(p, b.bin, e0 + lane) : 0u);
-    if (++steps == 255) {
+  for (uint32_t e0 = b.first; e0 < b.end; e0 += 128) {
+    uint32_t mask[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) mask[u] = e0 + 32 * u + lane < b.end ? entry_tiles(p, b.bin, e0 + 32 * u + lane) : 0u;
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (__any_sync(kFullMask, covers(mask[u]))) c.add(mask[u]);  // (few groups, where the bins are many)
+    steps += 4;
+    if (steps > 255 - 4) {
       mine += c.sum();
       steps = 0;
     }
@@ -1440,7 +1449,8 @@ __global__ void __launch_bounds__(kListThreads) whole_fill_kernel(const __grid_c
     const uint32_t m = mask1, r = rec1;
     mask1 = mask, rec1 = rec;
     load(e0 + 64 + lane);
-    fill.add(m, r, e0 + 32 >= b.end);
+    const bool last = e0 + 32 >= b.end;
+    if (last || __any_sync(kFullMask, covers(m))) fill.add(m, r, last);
   }
 }
 
@@ -1512,18 +1522,18 @@ void launch_rank(const RankParams& p, cudaStream_t s) {
   launch_chained(p.chained, rank_kernel, grid, kRankThreads, 0, s, p);
 }
 
-void launch_duplicate(const DuplicateParams& p, bool chained, cudaStream_t s) {
+void launch_duplicate(const DuplicateParams& p, int64_t expected_pairs, bool chained, cudaStream_t s) {
   const int64_t items = (int64_t)p.grid.P * p.grid.V;
   if (items <= 0) return;
   const int64_t tiles = (items + kScanTile - 1) / kScanTile;
   if (tiles <= (int64_t)p.skip_tiles) return;
   // scan: one block per scan tile that is taken (block k takes tile skip_tiles + k)
   launch_chained(chained, pair_scan_kernel, (unsigned)(tiles - p.skip_tiles), kScanBlock, 0, s, p);
-  // emit: one block per kEmitBlock pairs the binning buffer can hold (blocks past the device's pair
-  // count return at once); a probe pass stops after the scan
-  if (p.skip_tiles != 0) return;
-  const int64_t eblocks = emit_blocks(std::min<int64_t>(p.capacity, 0xffffffffll));
-  if (eblocks <= 0) return;
+  // emit: a block per kEmitBlock pairs of which there may be three a Gaussian, further ones in turn (with a block per
+  // kEmitBlock pairs that the binning buffer can hold, 3M Gaussians' duplicate stage took 187 us instead of 157; with
+  // blocks for half as many pairs, 150,000 Gaussians' 40 instead of 31); a probe pass stops after the scan
+  if (p.skip_tiles != 0 || p.capacity <= 0) return;
+  const int64_t eblocks = emit_blocks(std::min<int64_t>(p.capacity, expected_pairs)) + 1;
   launch_chained(chained, pair_emit_kernel, (unsigned)eblocks, kScanBlock, 0, s, p);
 }
 
@@ -1531,8 +1541,8 @@ void launch_tile_lists(const TileListParams& p, int64_t expected_pairs, cudaStre
   const TileGrid& g = p.grid;
   if (g.num_tiles == 0) return;
   const bool whole = p.words == nullptr;
-  // The pairs' number is only known on the device: as many blocks as the expected ones fill, which take further
-  // pieces in turn.
+  // The pairs' number is only known on the device: as many blocks as the expected ones fill (three a Gaussian, rather too
+  // many: those without a piece end at once), which take further pieces in turn.
   const int64_t pairs = std::min(expected_pairs, p.capacity);
   const int64_t piece = std::min<int64_t>(std::max<int64_t>(pairs / kPieceTarget, kMinPiece), kMaxPiece);
   const unsigned blocks = whole ? g.num_blocks : (unsigned)(pairs / (piece * kListWarps) + 1);

@@ -108,10 +108,16 @@ int run_binning(BinningPass& b, cudaStream_t s) {
     }
   } else {
     // The pieces' counts in the buffer that the tiles' ids go to in the end; the totals, without spare words, in the
-    // depth sort's first key buffer and the two behind it (the rects, which the coarse stage has read) or the ranges.
+    // depth sort's first key buffer and the two behind it (the rects, which the coarse stage has read), where the lists
+    // go after the scan, or in the ranges.
     counts = at<uint32_t>(b.binning, b.out ? L.tkeys1 : L.tkeys0);
-    clear_totals = totals == nullptr && 3 * records >= (int64_t)g.num_tiles;
-    if (clear_totals) totals = b.dkeys[0];
+    if (totals == nullptr) {
+      if (3 * records >= (int64_t)g.num_tiles)
+        totals = b.dkeys[0];
+      else if (L.capacity >= (int64_t)g.num_tiles)
+        totals = at<uint32_t>(b.binning, b.out ? L.tvals1 : L.tvals0);
+      clear_totals = totals != nullptr;
+    }
   }
 
   BeginParams begin{};
@@ -222,7 +228,7 @@ int run_binning(BinningPass& b, cudaStream_t s) {
       d.max_spins = b.max_spins;
       d.skip_tiles = 1;
     }
-    staged(OMNIGS_STAGE_DUPLICATE, 2, s, [&] { launch_duplicate(d, b.chained, s); });
+    staged(OMNIGS_STAGE_DUPLICATE, 2, s, [&] { launch_duplicate(d, 3 * records, b.chained, s); });
     if (probe) return check_launch("duplicate (look-back probe)");
     for (int q = 0; q < digits.passes; ++q) {
       const int from = (first + q) & 1;
@@ -262,7 +268,7 @@ int run_binning(BinningPass& b, cudaStream_t s) {
   t.hdr = b.hdr;
   if (clear_totals && cudaMemsetAsync(totals, 0, sizeof(uint32_t) * g.num_tiles, s) != cudaSuccess)
     return check_launch("memset tile totals");
-  staged(OMNIGS_STAGE_RANGES, 4, s, [&] { launch_tile_lists(t, 3 * records / 2, s); });
+  staged(OMNIGS_STAGE_RANGES, 4, s, [&] { launch_tile_lists(t, 3 * records, s); });
   return check_launch("binning");
 }
 

@@ -289,7 +289,7 @@ void launch_onesweep(const OnesweepParams& p, int64_t max_items, int64_t expecte
 void launch_begin_binning(const BeginParams& p, cudaStream_t s);
 void launch_rank(const RankParams& p, cudaStream_t s);
 void launch_rects(const RankParams& p, cudaStream_t s);  // rects only, in the order given
-void launch_duplicate(const DuplicateParams& p, bool chained, cudaStream_t s);
+void launch_duplicate(const DuplicateParams& p, int64_t expected_pairs, bool chained, cudaStream_t s);
 void launch_tile_lists(const TileListParams& p, int64_t expected_pairs, cudaStream_t s);
 // Splats staged per shared-memory batch in the blend kernels: a template parameter chosen at run
 // time per direction (128, 256 or 512; set by omnigs_set_blend_batch or the autotuner).  Results
