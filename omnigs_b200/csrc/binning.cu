@@ -562,7 +562,10 @@ __global__ void __launch_bounds__(kScanBlock) pair_scan_kernel(const __grid_cons
 }
 
 constexpr int kEmitPerThread = kEmitBlock / kScanBlock;
-constexpr int kEmitStage = 1025;  // Gaussians of a block staged in shared memory (more: read from global memory)
+// Gaussians of a block staged in shared memory: as many as it can have pairs, and one.  Measured on a B200, stages of 1025 /
+// 2049: the 16-view batch 540 / 528 us, 3M Gaussians 159 / 156 (at some 1.4 pairs a Gaussian most blocks have more than 1025;
+// none staged: 545 and 161, but 150,000 Gaussians 31 / 27).
+constexpr int kEmitStage = kEmitBlock + 1;
 
 __device__ __forceinline__ float rcp_approx_f(float x) {
   float r;
@@ -608,7 +611,7 @@ __global__ void __launch_bounds__(kScanBlock) pair_emit_kernel(const __grid_cons
     const uint32_t g_last = s_last;
     const uint32_t n = g_last >= g_first ? g_last - g_first + 1u : 1u;
     // Gaussians between g_first and g_last with no pairs (culled views' records) can make the range longer
-    // than the block's pair count: then offsets and rects are read from global memory
+    // than the block's pairs: then offsets and rects are read from global memory
     const bool staged = n <= (uint32_t)kEmitStage;
     if (staged)
       for (uint32_t t = threadIdx.x; t < n; t += kScanBlock) {
