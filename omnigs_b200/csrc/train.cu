@@ -50,7 +50,7 @@ struct LossParams {
 constexpr int kLossThreads = 128;
 constexpr int kLossCols = kLossThreads - 2 * kHalf;
 constexpr int kLossInCols = kLossThreads + 2 * kHalf;
-constexpr int kLossMinChunk = 16;
+constexpr int kLossMinChunk = 4;
 constexpr int kLossBlocksPerSm = 3;  // (168 registers; four measured 171 us against 137)
 
 // Block sums of (a, b) into partials[2 * block] (no contended atomics; loss_finalize adds them).
@@ -109,8 +109,7 @@ __device__ __forceinline__ float2 window_step(float2 (&acc)[kWin - 1], const flo
 // there on a B200, against two kernels through a 75 MB workspace, each with its horizontal and
 // vertical pass in shared memory: 213 -> 137 us (157 us with the pairs in scalar arithmetic, 140 us
 // with the two horizontal passes on either side of the barrier).  Strips recompute ten columns a side
-// and chunks ten rows at each end, so a chunk is as high as a grid of one wave allows
-// (omnigs_l1_dssim).
+// and chunks ten rows at each end (loss_chunk).
 __global__ void __launch_bounds__(kLossThreads, kLossBlocksPerSm) ssim_loss_kernel(const __grid_constant__ LossParams p) {
   __shared__ float2 s_in[2][kLossInCols];          // (img, gt) of the current and next input row
   __shared__ float2 s_ab[2][kLossInCols];          // (A, B) of a statistics row, from column xs - 5 of thread 0
@@ -651,12 +650,22 @@ int validate_params(const OmnigsGaussianParams* prm, const OmnigsActivated* act)
   return OMNIGS_OK;
 }
 
-// Workspace part of the loss kernel's block sums: two doubles per block, whose strips are wider than 32
-// columns and whose chunks are at least kLossMinChunk rows.  (The rest of the workspace holds the
-// gradient when that goes over one of the images.)
+// Workspace part of the loss kernel's block sums, the first; the last holds the gradient when that goes over one of the
+// images.  Two doubles a block, whose strips are wider than 32 columns; blocks of less than 16 rows also use what lies
+// between, two floats a pixel.
 size_t loss_sums_bytes(int C, int H, int W) {
-  const size_t blocks = (size_t)C * ((W + 31) / 32) * ((H + kLossMinChunk - 1) / kLossMinChunk);
+  const size_t blocks = (size_t)C * ((W + 31) / 32) * ((H + 15) / 16);
   return align_up(sizeof(double) * 2 * blocks);
+}
+
+// Rows of a block: as many as one wave of blocks takes (a chunk recomputes 20 rows), but at least 16 where such chunks give
+// every SM a block, and at least kLossMinChunk where they do not.  Measured on a B200, three channels, 16 rows / fewer: 16x16
+// 25 / 19 us, 128x256 28 / 22, 512x100 28 / 23; where they do, 256x512 32 / 33-38.
+int loss_chunk(int C, int rows, int W, int sms) {
+  const int64_t columns = (int64_t)((W + kLossCols - 1) / kLossCols) * C;
+  const bool small = columns * ((rows + 15) / 16) < sms;
+  const int chunks = (int)std::max<int64_t>(1, (int64_t)sms * (small ? 1 : kLossBlocksPerSm) / columns);
+  return std::max(small ? kLossMinChunk : 16, (rows + chunks - 1) / chunks);
 }
 
 }  // namespace
@@ -695,7 +704,7 @@ int omnigs_l1_dssim(const float* image, const float* gt, int C, int H, int W, in
     return x < y + bytes && y < x + bytes;
   };
   const bool in_place = overlaps(image) || overlaps(gt);
-  p.dimg = in_place ? reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + loss_sums_bytes(C, H, W)) : dL_dimage;
+  p.dimg = in_place ? reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + loss_sums_bytes(C, H, W) + 2 * bytes) : dL_dimage;
   p.C = C;
   p.H = H;
   p.W = W;
@@ -709,14 +718,11 @@ int omnigs_l1_dssim(const float* image, const float* gt, int C, int H, int W, in
     sum += p.w[k];
   }
   for (int k = 0; k < kWin; ++k) p.w[k] /= sum;
-  // One wave of blocks, each as many rows as that takes (a chunk recomputes 20 rows of statistics and
-  // input filtering), but at least kLossMinChunk.
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int strips = (W + kLossCols - 1) / kLossCols;
-  const int chunks = std::max(1, (int)((int64_t)sms * kLossBlocksPerSm / ((int64_t)strips * C)));
-  p.chunk = std::max(kLossMinChunk, (rows + chunks - 1) / chunks);
+  p.chunk = loss_chunk(C, rows, W, sms);
   const dim3 grid(strips, (rows + p.chunk - 1) / p.chunk, C);
   const int blocks = (int)(grid.x * grid.y * grid.z);
   staged(OMNIGS_STAGE_OTHER, 2, s, [&] {
