@@ -157,7 +157,9 @@ __device__ __forceinline__ void blend_backward_tile(const TileJob& job, const Bl
   int nred = 0;  // buffered splats (warp-uniform)
   auto blend = [&](uint32_t off, auto plain) {
     // No per-lane branches: a pixel behind its last contributor, or that this splat does not reach, is
-    // inactive, and the masked G = 0 makes alpha, w and d exactly 0 and 1 / (1 - alpha) exactly 1.
+    // inactive, and the masked G = 0 makes alpha, w and d exactly 0 and 1 / (1 - alpha) exactly 1: sm_100's
+    // approximate reciprocal of 1 is 1, which its documented error bound does not say (a test holds the gradients
+    // of a pixel under 700 such splats to the bit; selecting 1 instead takes two more issue slots a splat).
     constexpr bool kPlain = decltype(plain)::value;
     const float4* slot = reinterpret_cast<const float4*>(slots + off);
     const float4 v0 = slot[0], v1 = slot[1], v2 = slot[2];
