@@ -229,11 +229,13 @@ def traffic_from_profiles() -> dict:
 
 
 def stage_bytes(P, V, R, N, Tl):
-    """Algorithmic (compulsory) HBM bytes of each stage for one view."""
+    """Algorithmic (compulsory) HBM bytes of each stage for one view.  Of the binning (duplicate, sort, ranges): the splats'
+    records and depth keys in, the depth order, the sorted tile ids and records and the tile ranges out; the pairs of a splat
+    and a bin that it makes in between are its own."""
     return {
         "preprocess": 44 * P + 192 * V + 8 * P + 40 * V + 8 * P,  # + the fused scan of tiles_touched
-        "duplicate": 20 * V + 12 * R,
-        "sort": 24 * R,
+        "duplicate": 20 * V,
+        "sort": 8 * P,
         "ranges": 8 * R + 8 * Tl,
         "render_forward": 40 * R + 8 * Tl + 12 * N + 8 * N,
         "render_backward": 40 * R + 8 * Tl + 12 * N + 8 * N + 44 * V,

@@ -109,18 +109,6 @@ __global__ void __launch_bounds__(kBatchBlock) batch_preprocess_kernel(const __g
 template <bool kFp64Poles>
 constexpr int batch_bwd_min_blocks() { return kFp64Poles ? 1 : 3; }
 
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-// Waits for all groups but the newest.
-__device__ __forceinline__ void cp_async_wait_previous() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
-
 // What a thread reads of its Gaussian's record in one view, copied while it works on the view before:
 // the accumulator and splat records and the clamp bits.  A slot is read and rewritten by its thread alone.
 struct ViewRecords {

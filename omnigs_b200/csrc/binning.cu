@@ -59,10 +59,6 @@ __device__ __forceinline__ bool instances_fit(const GeomHeader* hdr, int64_t cap
 __device__ __forceinline__ uint32_t pair_count(const GeomHeader* hdr, int64_t capacity) {
   return instances_fit(hdr, capacity) ? (uint32_t)min((long long)hdr->num_pairs, (long long)capacity) : 0u;
 }
-// Element count of a sort/histogram: a host value, or the device's pair count.
-__device__ __forceinline__ uint32_t item_count(const GeomHeader* count_hdr, uint32_t n_host, int64_t capacity) {
-  return count_hdr == nullptr ? n_host : pair_count(count_hdr, capacity);
-}
 
 // ---------------------------------------------------------------- digit histograms ------------
 // Adds the warp's digits (lanes in `live`, a prefix of the warp) to a shared histogram.  Keys of a
@@ -85,7 +81,7 @@ __global__ void __launch_bounds__(256) histogram_kernel(const __grid_constant__ 
   __shared__ uint32_t s_hist[kDepthPasses][kRadix];
   for (int i = threadIdx.x; i < kDepthPasses * kRadix; i += blockDim.x) (&s_hist[0][0])[i] = 0;
   __syncthreads();
-  const uint32_t n = p.seg_len ? p.seg_len : item_count(p.count_hdr, p.n_host, p.capacity);
+  const uint32_t n = p.seg_len;
   const size_t seg_base = (size_t)blockIdx.y * n;  // gridDim.y segments
   const int lane = threadIdx.x & 31;
   const uint32_t stride = gridDim.x * blockDim.x;
@@ -184,7 +180,7 @@ __global__ void __launch_bounds__(kSortThreads, kMinBlocks) onesweep_kernel(Ones
   chain_begin();
   constexpr int kTile = kSortThreads * kItems;
   __shared__ SortSmem<kTile> sm;
-  const uint32_t n = p.seg_len ? p.seg_len : item_count(p.count_hdr, p.n_host, p.capacity);
+  const uint32_t n = p.seg_len ? p.seg_len : pair_count(p.hdr, p.capacity);
   const uint32_t tiles_per_seg = (n + kTile - 1) / kTile;
   const uint32_t ntiles = tiles_per_seg * (p.seg_len ? p.num_segs : 1u);
   if (threadIdx.x == 0) sm.tile = atomicAdd(p.tile_counter, 1u);
@@ -1476,11 +1472,10 @@ int sm_count() {
 
 }  // namespace
 
-void launch_histogram(const HistParams& p, int64_t max_items, bool chained, cudaStream_t s) {
-  const unsigned segs = p.seg_len ? std::max(1u, p.num_segs) : 1u;
-  const int64_t per_seg = p.seg_len ? (int64_t)p.seg_len : max_items;
+void launch_histogram(const HistParams& p, bool chained, cudaStream_t s) {
+  const unsigned segs = std::max(1u, p.num_segs);
   const int64_t blocks = std::max<int64_t>(
-      1, std::min<int64_t>((per_seg + 256 * kHistUnroll - 1) / (256 * kHistUnroll),
+      1, std::min<int64_t>(((int64_t)p.seg_len + 256 * kHistUnroll - 1) / (256 * kHistUnroll),
                            std::max<int64_t>(1, sm_count() * 4 / segs)));
   launch_chained(chained, histogram_kernel, dim3((unsigned)blocks, segs), 256, 0, s, p);
 }

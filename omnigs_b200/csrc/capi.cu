@@ -165,7 +165,6 @@ int run_binning(BinningPass& b, cudaStream_t s) {
     // 1. depth sort of every view's Gaussians: one segment per view, (depth bits, index) order
     HistParams hd{};
     hd.keys = depth_keys;
-    hd.n_host = (uint32_t)records;
     hd.passes = kDepthPasses;
     for (int q = 0; q < kDepthPasses; ++q) {
       hd.shift[q] = kRadixBits * q;
@@ -174,7 +173,7 @@ int run_binning(BinningPass& b, cudaStream_t s) {
     hd.hist = b.depth_hist;
     hd.seg_len = (uint32_t)g.P;
     hd.num_segs = (uint32_t)g.V;
-    staged(OMNIGS_STAGE_SORT, 1, s, [&] { launch_histogram(hd, records, b.chained, s); });
+    staged(OMNIGS_STAGE_SORT, 1, s, [&] { launch_histogram(hd, b.chained, s); });
     const int64_t depth_tiles = sort_blocks(g.P, g.V);
     for (int q = 0; q < kDepthPasses; ++q) {
       OnesweepParams op{};
@@ -184,7 +183,6 @@ int run_binning(BinningPass& b, cudaStream_t s) {
       op.vals_out = b.dvals[q & 1];
       op.shift = kRadixBits * q;
       op.mask = kRadix - 1;
-      op.n_host = (uint32_t)records;
       op.hist = b.depth_hist + q * kRadix;
       op.lookback = b.depth_lookback + (size_t)q * depth_tiles * kRadix;
       op.tile_counter = &b.hdr->sort_tile_counter[q];
@@ -239,7 +237,6 @@ int run_binning(BinningPass& b, cudaStream_t s) {
       op.vals_out = vals[from ^ 1];
       op.shift = digits.shift[q];
       op.mask = digits.mask[q];
-      op.count_hdr = b.hdr;
       op.capacity = b.capacity;
       op.hist = hist + (kDepthPasses + q) * kRadix;
       op.lookback = at<uint32_t>(b.binning, L.tile_lookback) + (size_t)q * pair_tiles * kRadix;

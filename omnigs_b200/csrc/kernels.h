@@ -30,19 +30,15 @@ struct PreprocessParams {
   GeomHeader* hdr;           // num_rendered64 is accumulated here
 };
 
-// Digit histograms of up to kDepthPasses digits of u32 keys.
-// With seg_len > 0 the keys are num_segs independent segments of seg_len items each (the views of
-// a batch) and every segment gets its own histograms, at hist + seg * passes * kRadix.
+// Digit histograms of up to kDepthPasses digits of u32 keys: num_segs independent segments of seg_len items
+// each (the views), every segment with its own histograms, at hist + seg * passes * kRadix.
 struct HistParams {
   const uint32_t* keys;
-  uint32_t n_host;             // item count when count_hdr is null
-  const GeomHeader* count_hdr; // else the device num_rendered (0 if over capacity)
-  int64_t capacity;
   int passes;
   int shift[kDepthPasses];
   uint32_t mask[kDepthPasses];
   uint32_t* hist;              // [segments][passes][kRadix], zeroed by the caller
-  uint32_t seg_len;            // 0: one segment of all items
+  uint32_t seg_len;
   uint32_t num_segs;
 };
 
@@ -54,15 +50,13 @@ struct OnesweepParams {
   uint32_t* vals_out;
   int shift;
   uint32_t mask;
-  uint32_t n_host;
-  const GeomHeader* count_hdr;
-  int64_t capacity;
+  int64_t capacity;            // (seg_len == 0)
   const uint32_t* hist;        // this pass's [kRadix] histogram (of segment 0)
   uint32_t* lookback;          // [sort tiles][kRadix], zeroed by the caller
   uint32_t* tile_counter;      // zeroed by the caller
-  GeomHeader* hdr;             // status bits
+  GeomHeader* hdr;             // status bits; the pairs' number
   // Segmented sort (each segment sorted on its own, in place): seg_len items per segment, the
-  // histogram of segment s at hist + s * hist_seg_stride.  seg_len == 0: one segment.
+  // histogram of segment s at hist + s * hist_seg_stride.  seg_len == 0: one segment, the pass's pairs.
   uint32_t seg_len;
   uint32_t num_segs;
   uint32_t hist_seg_stride;
@@ -284,7 +278,7 @@ void launch_batch_preprocess_backward(const BatchParams& p, const BatchGrads& g,
 
 void launch_preprocess(const PreprocessParams& p, cudaStream_t s);
 // `chained`: as launch_chained's, also in the other parameter blocks
-void launch_histogram(const HistParams& p, int64_t max_items, bool chained, cudaStream_t s);
+void launch_histogram(const HistParams& p, bool chained, cudaStream_t s);
 void launch_onesweep(const OnesweepParams& p, int64_t max_items, int64_t expected, bool chained, cudaStream_t s);
 void launch_begin_binning(const BeginParams& p, cudaStream_t s);
 void launch_rank(const RankParams& p, cudaStream_t s);

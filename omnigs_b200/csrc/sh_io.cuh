@@ -8,6 +8,8 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include "device_util.cuh"
+
 namespace omnigs {
 
 constexpr int kMaxShCoeffs = 16;
@@ -72,14 +74,13 @@ __device__ __forceinline__ void stage_sh(const float* shs, int first, float4* st
   for (int i = 0; i < 12; ++i) {
     const int e = i * 32 + lane;
     const int gg = e / 12, part = e - gg * 12;
-    const unsigned dst = (unsigned)__cvta_generic_to_shared(stage + gg * kShStageStride + part);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src + e) : "memory");
+    cp_async16(stage + gg * kShStageStride + part, src + e);
   }
-  asm volatile("cp.async.commit_group;" ::: "memory");
+  cp_async_commit();
 }
 
 __device__ __forceinline__ void wait_staged_sh() {
-  asm volatile("cp.async.wait_all;" ::: "memory");
+  cp_async_wait_all();
   __syncwarp();
 }
 

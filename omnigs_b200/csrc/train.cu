@@ -495,8 +495,7 @@ __device__ __forceinline__ void adam_sh_tile(const AdamParams& p, float* s_sh, i
 #pragma unroll 4
   for (int i = t; i < ng * row / kW; i += kAdamThreads) {
     if (kW == 4) {
-      const unsigned dst = (unsigned)__cvta_generic_to_shared(s_sh + 4 * i);
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(dsh + 4 * i) : "memory");
+      cp_async16(s_sh + 4 * i, dsh + 4 * i);
     } else {
       s_sh[i] = dsh[i];
     }
@@ -529,7 +528,7 @@ __device__ __forceinline__ void adam_sh_tile(const AdamParams& p, float* s_sh, i
       if (j >= 0) pv[u] = adam_load<4>(prm, j), mv[u] = adam_load<4>(m, j), vv[u] = adam_load<4>(v, j);
     }
     adam_scalars2(*p.hyper, 1, 2, s_dc, s_rest);
-    asm volatile("cp.async.wait_all;" ::: "memory");
+    cp_async_wait_all();
     __syncthreads();
 #pragma unroll
     for (int u = 0; u < kAdamVecs; ++u) {
