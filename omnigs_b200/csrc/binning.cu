@@ -23,8 +23,8 @@
 // work if it exceeds the binning capacity.  Waits on other blocks are bounded.
 //
 // Measured on a B200 against emitting every instance and sorting the list by tile id in two or three
-// passes, all stages of the binning: 1M Gaussians at 2048x1024 (8.6M instances) 353 -> 239 us, 3M at
-// 4096x2048 (72M) 1895 -> 905 us, 16 views over 1M Gaussians (112M) 3.49 -> 2.35 ms, 10,000 at 512x256
+// passes, all stages of the binning: 1M Gaussians at 2048x1024 (8.6M instances) 353 -> 238 us, 3M at
+// 4096x2048 (72M) 1895 -> 813 us, 16 views over 1M Gaussians (112M) 3.49 -> 2.14 ms, 10,000 at 512x256
 // 115 -> 49 us.  The sort passes over the instances were what it cost (80 us each over 8.2M), and the
 // pairs are a fifth of them.
 #include <algorithm>
@@ -165,7 +165,7 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* s
 // Bound by a tile's own work: ranking, scans, scatter.  The tile is reordered before the look-back and its
 // values are loaded after the ranking, so that registers hold 24 words of a thread's 16 items at a time, not
 // 48.  Measured on a B200, the sorts of a 1M / 3M-Gaussian view / 16-view batch: 125 / 447 / 1202 us with
-// everything held to the end, 118 / 380 / 1020 now.
+// everything held to the end, 117 / 382 / 1020 now.
 // Launches of this pass measured ~2 us slower each on a B200 with a 136-byte parameter block than
 // with a 128-byte one.
 static_assert(sizeof(OnesweepParams) <= 128, "keep the onesweep parameter block at 128 bytes or less");
@@ -1239,7 +1239,7 @@ __device__ __forceinline__ void order_tiles(const TileListParams& p, uint32_t se
 // tile rows (a pair covers one or two of them on average, so a walk per row would waste most lanes) and
 // appends 32 of a row at a time to its eight lists: a pair's place is the list's next one plus the
 // queued pairs before it that cover the tile, from a warp scan of the eight columns as bytes.  Bound by
-// issue.  Measured on a B200 (1M-Gaussian view / 16-view batch): a block per tile row, walking all of the
+// issue (56 % of the slots) and shared memory (41 %).  Measured on a B200 (1M-Gaussian view / 16-view batch): a block per tile row, walking all of the
 // bin's pairs with ballots and popcounts per tile, 88 / 1262 us; byte scans there 75 / 967; this
 // 37 / 392 us.
 struct FillQueue {
@@ -1489,9 +1489,10 @@ void launch_onesweep(const OnesweepParams& p, int64_t max_items, int64_t expecte
   if (blocks <= 0) return;
   // The blocks an SM holds: three have all the registers that the ranking wants, five spill.  Tiles that fit one
   // wave of more blocks are better off so; beyond that four measured fastest.  On a B200, the sorts of a
-  // 300k / 1M / 3M-Gaussian view / 16-view batch with three, four and five: 91 / 118 / 421 / 1106,
-  // 95 / 119 / 412 / 1017 and 107 / 132 / 378 / 1037 us.  The pairs' number is only known on the device: one
-  // and a half a Gaussian are expected, as for the lists.
+  // 300k / 1M / 3M-Gaussian view / 16-view batch with three, four and five: 89 / 117 / 417 / 1088,
+  // 92 / 118 / 408 / 1026 and 104 / 129 / 372 / 1035 us; by this rule 90 / 117 / 382 / 1025.  Five against four within
+  // their window: 2.45M Gaussians 212 / 205, 2.7M 358 / 372, 3M at 1024x512 212 / 238, eight views of 350,000 199 / 210.
+  // The pairs' number is only known on the device: one and a half a Gaussian are expected.
   const int64_t tiles = p.seg_len ? blocks : sort_tiles(expected), sms = sm_count();
   if (tiles <= 3 * sms)
     launch_chained(chained, onesweep_kernel<kSortItems, 3, kLookbackBatch>, (unsigned)blocks, kSortThreads, 0, s, p);

@@ -51,7 +51,11 @@ cudaEvent_t take_event() {
 // Whether the stream is being captured into a graph.
 static bool capturing(cudaStream_t s) {
   cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-  return cudaStreamIsCapturing(s, &status) == cudaSuccess && status == cudaStreamCaptureStatusActive;
+  if (cudaStreamIsCapturing(s, &status) != cudaSuccess) {
+    cudaGetLastError();  // (the legacy stream beside a capture: the launches will say so)
+    return true;
+  }
+  return status == cudaStreamCaptureStatusActive;
 }
 
 int run_binning(BinningPass& b, cudaStream_t s) {

@@ -288,8 +288,8 @@ void launch_tile_lists(const TileListParams& p, int64_t expected_pairs, cudaStre
 // Splats staged per shared-memory batch in the blend kernels: a template parameter chosen at run
 // time per direction (128, 256 or 512; set by omnigs_set_blend_batch or the autotuner).  Results
 // do not depend on it: every pixel meets the same splats in the same order.  Defaults: 128 for both
-// directions (the faster of the three for each on the 1M-Gaussian 2048x1024 view on a B200:
-// forward 0.512 vs 0.522 ms at 256, backward 1.149 vs 1.163 ms at 256).
+// directions.  Measured on a B200 (1M-Gaussian 2048x1024 view, 128 / 256 / 512): forward 0.463 / 0.449 / 0.485 ms,
+// backward 0.785 / 0.847 / 0.941.  (The forward's kernel for short lists has a size of its own.)
 constexpr int kDefaultBatch = 128;
 constexpr int kDefaultBwdBatch = 128;
 int blend_batch_size(bool backward);

@@ -163,8 +163,8 @@ inline bool counts_order(int64_t P, int64_t V) { return P <= kRankMaxP && V * P 
 constexpr int64_t kWholeMaxPairs = int64_t(1) << 20;
 
 // Up to kChainRecords (Gaussian, view) records the binning's kernels are chained (launch_chained): it is a row of a dozen
-// launches there.  Measured on a B200, forward without / with: 20,000 Gaussians at 2132x1093 163 / 141 us, 70,000 at
-// 2048x1024 184 / 165, 300,000 402 / 387; 1M 677 / 674; forward and backward 3M at 4096x2048 3924 / 3999, six views of
+// launches there.  Measured on a B200, forward without / with: 20,000 Gaussians at 2132x1093 148 / 125 us, 71,000
+// there 198 / 176, 300,000 402 / 387; 1M 677 / 674; forward and backward 3M at 4096x2048 3924 / 3999, six views of
 // 20,000 at 1024x512 299 / 288.  A captured graph has no such gaps, and chained it measured slower (a train step over four
 // views of 200,000 Gaussians 1282 / 1303 us), except where everything is short (every bin reads the whole counted order).
 constexpr int64_t kChainRecords = int64_t(1) << 19;

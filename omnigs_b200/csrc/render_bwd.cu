@@ -18,10 +18,10 @@
 // and do not lie behind all of its pixels' last contributors (blend_common.cuh), and the block starts at
 // the batch holding its largest last contributor instead of at the end of the range.
 //
-// Bound by instruction issue (79 % of the slots on a 400k-Gaussian view).  Measured on a B200
+// Bound by instruction issue (78 % of the slots on a 400k-Gaussian view).  Measured on a B200
 // (300k / 1M-Gaussian 2048x1024 view / 16-view batch): 315 / 760 / 9710 us with the warps scanning ballots
 // of their own tests, every sum in a row of its own (nine, two splats a flush) and the clamp and sign
-// tests for every splat; 271 / 670 / 8480 us now.  The same sums on the tensor cores (mma.m16n8k8, TF32
+// tests for every splat; 272 / 673 / 8430 us now.  The same sums on the tensor cores (mma.m16n8k8, TF32
 // operands split in two) took 319 / 812 / 10600: fewer instructions, but the fragments' registers and
 // shared memory leave six blocks per SM.
 #include "blend_common.cuh"
@@ -90,8 +90,7 @@ __device__ __forceinline__ void flush_reduction(BackwardSmem<kBatch>& sm, int n,
 }
 
 // Seven resident blocks per SM (at most 72 registers).  Measured on a B200 (1M-Gaussian view / 16-view
-// batch): five 717 / 9190 us, six 692 / 8800, seven 669 / 8530, eight (64 registers, spilling with the
-// seam) 696 / 9010.
+// batch): six 678 / 8610 us, seven 673 / 8430, eight (64 registers, spilling with the seam) 696 / 8840.
 constexpr int kBlendBwdMinBlocks = 7;
 
 // kRecompute (transmittance checkpointing): the forward stored no per-pixel state; each pixel's

@@ -4,8 +4,8 @@
 // Loss (include/loss_utils.h:30-131, as used at src/gaussian_mapper.cpp:384-409):
 //   L = (1 - lambda) mean|img - gt| + lambda (1 - mean SSIM(img, gt)),
 // SSIM with the 11x11 Gaussian window (sigma 1.5, zero padding 5, per channel), C1 = 0.01^2,
-// C2 = 0.03^2.  The window is separable, so every 2D convolution runs as a horizontal then a
-// vertical 11-tap pass in shared memory.  The gradient follows from
+// C2 = 0.03^2.  The window is separable, so every 2D convolution runs as a horizontal 11-tap pass over a
+// shared row and a vertical one as running sums in registers.  The gradient follows from
 //   dSSIM/dimg(p) = 1/N [ (w * A)(p) + 2 img(p) (w * B)(p) + gt(p) (w * Cm)(p) ]
 // with per-pixel A = dS/dmu1, B = dS/d(w * img^2), Cm = dS/d(w * img gt) (the window is
 // symmetric, so the adjoint convolution is the same convolution).  One kernel walks the image down
@@ -343,9 +343,10 @@ __device__ __forceinline__ float adam_update(float& p, float& m, float& v, float
 // The pass is bound by HBM: 1.88 GB per step over 1M Gaussians (16 SH coefficients).  Measured there on a
 // B200: a loop over the Gaussians with a thread each (accesses of stride 3 and 4 floats) and one over the
 // f_rest elements 596 us; blocks that take all groups of 64 Gaussians, with 30 arrays open at once,
-// 405-425 us whatever the tile, occupancy or work per thread; this split 318 us, 92 % of the copy rate.
+// 405-425 us whatever the tile, occupancy or work per thread; this split 326 us, 89 % of the copy rate.
 // A tile is at most two vectors a thread: with 16 coefficients 32 Gaussians and 192 threads measured
-// fastest (256 threads 334 us, 128 threads 351 us; tiles of 64 with 256 or 384 threads 349 and 332 us).
+// fastest (318 us over one model's buffers; 256 threads 334 us, 128 threads 351 us; tiles of 64 with 256 or 384
+// threads 349 and 332 us).
 // Fewer coefficients take more Gaussians (with one, tiles of 32 left 7 of 8 threads idle: 168 us per step
 // over 1.1M Gaussians, 96 with tiles of 512).
 constexpr int kAdamThreads = 192;
