@@ -1380,18 +1380,17 @@ __global__ void __launch_bounds__(kListThreads, 4) tile_fill_kernel(const __grid
       return w;
     }, [&](uint32_t bin, bool in, uint32_t w, bool begins, bool ends, bool) {
       if (begins) {
-        uint32_t t, place = 0;
-        safe = true;
+        uint32_t t, place = 0, last = 0;
         if (lane_tile(bin_tiles(p.grid, s_bases, bin), t)) {
           const uint2 range = p.ranges[t];
-          place = range.x;
-          safe = range.y <= (uint64_t)p.capacity;  // (always, after a consistent scan)
+          place = range.x, last = range.y;
         }
-        safe = __all_sync(kFullMask, safe);
         if (first)  // the piece's first bin may have begun in an earlier one
 #pragma unroll
           for (int k = 0; k < kListWarps; ++k)
             place += (bin == before ? s_sum[k][lane] : 0u) + (k < warp && s_bin[k] == bin ? s_own[k][lane] : 0u);
+        // (always, after a sort whose waits ended; a piece's writes then end in the list, or in the arrays behind it)
+        safe = __all_sync(kFullMask, place <= last && last <= (uint64_t)p.capacity);
         first = false;
         fill.begin(place);
       }
