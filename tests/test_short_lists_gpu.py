@@ -127,4 +127,4 @@ def test_short_lists_cost_less_with_their_kernel(cuda):
             capi.timing_enable(False)
         return t
 
-    assert best(n) < 0.97 * best(_loose(W, H))
+    assert best(n) < 0.99 * best(_loose(W, H))
